@@ -278,3 +278,27 @@ def test_gpu_trained_network_beats_the_plain_init(u3dg):
         psnr.append(t.evaluatePsnr())
         t.close()
     assert psnr[1] > psnr[0] + 0.1, psnr
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 15, 64, 65, 1025, 4161, 9344, 9345])
+def test_gpu_mlp_gradient_at_tile_and_chunk_edges(u3dg, n):
+    # One row, partial k tiles and row chunks (64 rows and more per chunk), and both sides of the row
+    # count at which the layers take the larger tile. Gradients are compared by the 2-norm per array:
+    # float32 products and sums of up to n terms in chunks, so well within 1e-5 of the 64-bit values
+    # (2^-24 times the square root of the longest chain, times a cancellation of about 100).
+    p = _params(41, scale=0.7).astype(np.float32)
+    x, t = _batch(n, seed=n)
+    x, t = x.astype(np.float32), t.astype(np.float32)
+    net = u3dg.WarmStartNet(p)
+    loss, g = net.loss_grad(x, t)
+    rl, rg = wo.mlp_loss_grad(p.astype(np.float64), x.astype(np.float64), t.astype(np.float64))
+    assert abs(loss - rl) <= 1e-5 * rl
+    o = 0
+    for i, k in wo.LAYERS:
+        for a, b in ((o, o + i * k), (o + i * k, o + i * k + k)):
+            assert np.linalg.norm(g[a:b] - rg[a:b]) <= 1e-5 * np.linalg.norm(rg[a:b]), (n, i, k, a)
+        o += i * k + k
+    y = net.forward(x)
+    ref, _ = wo.mlp_forward(p.astype(np.float64), x.astype(np.float64))
+    assert np.max(np.abs(y - ref)) <= 1e-4 * max(1.0, np.max(np.abs(ref)))

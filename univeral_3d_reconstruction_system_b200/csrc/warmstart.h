@@ -27,10 +27,20 @@ size_t warmViewRefBytes();
 void fillWarmViewRef(void *dst, const u3dg_camera &cam, const uint8_t *rgbDev);
 void launchWarmFeatures(const float *xyz, const float *rgb, int n, const int *nbr, const float *nd2,
                         const float *baseScale, const void *views, int nViews, float *feat, cudaStream_t s);
-void launchGemm(const float *A, int sAm, int sAk, const float *B, int sBk, int sBn, float *C, int ldc, int M, int N,
-                int K, const float *bias, bool relu, cudaStream_t s);
-void launchReluBackward(float *d, const float *y, size_t count, cudaStream_t s);
-void launchColumnSum(const float *d, int n, int out, float *db, cudaStream_t s);
+// y (n x out) = x (n x in) W^T + b, then ReLU (relu).
+void launchLayer(const float *x, int in, const float *W, const float *b, float *y, int out, int n, bool relu,
+                 cudaStream_t s);
+// dIn (n x in) = dOut (n x out) W, zero where the layer's input activation act is not positive.
+void launchLayerInputGrad(const float *dOut, int out, const float *W, int in, const float *act, float *dIn, int n,
+                          cudaStream_t s);
+// One partial gradient per row chunk of a layer's weights and biases, at offsets w and b of
+// parameter-sized arrays (partial: gradPartialEntries(n) floats); launchReduceGrad adds the chunks of
+// every parameter in chunk order once all layers are done.
+constexpr int kGradChunks = 64;
+void launchLayerParamGrad(const float *dOut, int out, const float *act, int in, int n, float *partial, size_t w,
+                          size_t b, cudaStream_t s);
+void launchReduceGrad(const float *partial, int n, float *grad, cudaStream_t s);
+size_t gradPartialEntries(int n);
 int mseBlocks();
 void launchMse(const float *y, const float *t, const float *w, int n, float *dy, double *partial, float *lossOut,
                cudaStream_t s);

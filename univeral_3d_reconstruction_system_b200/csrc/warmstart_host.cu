@@ -57,6 +57,7 @@ struct u3dg_mlp {
     int step = 0;
     size_t cap = 0; // rows the activation scratch holds
     DevBuf<float> x, h1, h2, h3, y, t, dy, dh, dh2, w11, lossDev;
+    DevBuf<float> gradPartial; // weight-gradient partials of the row chunks
     DevBuf<double> partial;
 
     u3dg_mlp()
@@ -108,28 +109,27 @@ struct u3dg_mlp {
         for (int l = 0; l < kWarmLayers; ++l) {
             const int in = kWarmIn[l], out = kWarmOut[l];
             float *dst = (l == kWarmLayers - 1) ? y.p : act(l + 1);
-            launchGemm(act(l), in, 1, W(l), 1, in, dst, out, n, out, in, B(l), l < kWarmLayers - 1, stream);
+            launchLayer(act(l), in, W(l), B(l), dst, out, n, l < kWarmLayers - 1, stream);
         }
     }
     // Gradient of the weighted MSE against t (rows in x / t): loss into lossDev, gradients into grad.
     void lossGrad(int n)
     {
+        gradPartial.reserve(gradPartialEntries(n));
         forward(n);
         launchMse(y.p, t.p, w11.p, n, dy.p, partial.p, lossDev.p, stream);
         float *dOut = dy.p;
         for (int l = kWarmLayers - 1; l >= 0; --l) {
             const int in = kWarmIn[l], out = kWarmOut[l];
             const LayerOffsets &o = offsets();
-            // dW = dOut^T In (out x in), db = column sums of dOut.
-            launchGemm(dOut, 1, out, act(l), in, 1, grad.p + o.w[l], in, out, in, n, nullptr, false, stream);
-            launchColumnSum(dOut, n, out, grad.p + o.b[l], stream);
+            launchLayerParamGrad(dOut, out, act(l), in, n, gradPartial.p, o.w[l], o.b[l], stream);
             if (l > 0) {
                 float *dIn = (dOut == dh.p) ? dh2.p : dh.p;
-                launchGemm(dOut, out, 1, W(l), in, 1, dIn, in, n, in, out, nullptr, false, stream);
-                launchReluBackward(dIn, act(l), size_t(n) * in, stream);
+                launchLayerInputGrad(dOut, out, W(l), in, act(l), dIn, n, stream);
                 dOut = dIn;
             }
         }
+        launchReduceGrad(gradPartial.p, n, grad.p, stream);
     }
     void adam(float lr)
     {
