@@ -302,3 +302,19 @@ def test_gpu_mlp_gradient_at_tile_and_chunk_edges(u3dg, n):
     y = net.forward(x)
     ref, _ = wo.mlp_forward(p.astype(np.float64), x.astype(np.float64))
     assert np.max(np.abs(y - ref)) <= 1e-4 * max(1.0, np.max(np.abs(ref)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nq, np_", [(1, 2049), (33, 1024), (131, 1025), (5, 31), (0, 7), (4, 0)])
+def test_gpu_knn_at_group_and_stage_edges(u3dg, nq, np_):
+    # Queries beyond a warp's group of four and a CTA's 32, candidates at the edges of a warp's 32 and of
+    # the 1024 staged at once, on a lattice full of equal distances: exact (integers and small squares).
+    rng = np.random.default_rng(nq + np_)
+    q = (rng.integers(-3, 4, size=(nq, 3)) * 0.5).astype(np.float32)
+    p = (rng.integers(-3, 4, size=(np_, 3)) * 0.5).astype(np.float32)
+    for k in (1, 3, 16):
+        for exclude in (False, True):
+            idx, d2 = u3dg.knn(q, p, k, exclude_self=exclude)
+            ri, rd = wo.knn(q, p, k, exclude_self=exclude)
+            np.testing.assert_array_equal(idx, ri)
+            np.testing.assert_array_equal(d2, rd)
