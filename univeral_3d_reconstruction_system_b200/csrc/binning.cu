@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(kThreads) radixRowScanKernel(int *hist, int G,
 // earlier items) + its rank in its warp. After the round the last item of each (warp, digit) advances
 // the digit's base and clears that count, so only the touched counts are reset.
 // kTiles (the single pass of a tile sort, digit = tile): instead of the sorted keys and values, the
-// scatter writes each entry's (Gaussian id, emission index) pair (fin.entries[pos]), and block 0
+// scatter writes each entry's Gaussian id (fin.entries[pos]) and its position (fin.listPos), and block 0
 // writes the tile offsets, which are the digit bases it starts from.
 // Where a pass of the depth sort keeps its items: (key, value) pairs in and out, so each item is one
 // load and one scattered 8-byte store; the last pass writes the values only (the keys are done).
@@ -219,7 +219,8 @@ __global__ void __launch_bounds__(kThreads) radixScatterKernel(const uint32_t *k
                     cross += warpCounts[w][d];
                 const int pos = base[d] + cross + local[r];
                 if (kTiles) {
-                    fin.entries[pos] = make_int2(fin.emitGid[val[r]], int(val[r]));
+                    fin.entries[pos] = fin.emitGid[val[r]];
+                    fin.listPos[val[r]] = make_int2(pos, d);
                 } else if (io.out) {
                     io.out[pos] = make_uint2(key[r], val[r]);
                 } else if (io.valsOnly) {
@@ -307,7 +308,7 @@ __global__ void __launch_bounds__(kThreads) scanPartialKernel(int *partial, int 
 }
 
 // cap.counts (may be null): block 0 also runs the bin pass's capacity check on the total.
-__global__ void __launch_bounds__(kThreads) scanDownsweepKernel(const int *in, const uint32_t *perm, int *out, int n,
+__global__ void __launch_bounds__(kThreads) scanDownsweepKernel(const int *in, const uint32_t *perm, int *out, int *outById, int n,
                                                                 const int *partial, int B, ScanCapacity cap)
 {
     pdlEntry();
@@ -323,8 +324,11 @@ __global__ void __launch_bounds__(kThreads) scanDownsweepKernel(const int *in, c
     int run = blockExclusiveScan(s, total) + partial[blockIdx.x];
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
-        if (base + r < n)
+        if (base + r < n) {
             out[base + r] = run;
+            if (outById)
+                outById[perm[base + r]] = run;
+        }
         run += v[r];
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -436,13 +440,15 @@ __global__ void __launch_bounds__(256) emitKernel(const uint32_t *sortedIds, con
     }
 }
 
-__global__ void finalizeKernel(const uint32_t *sortedEmit, const int *emitGid, const BinCounts *c, int2 *entries)
+__global__ void finalizeKernel(const uint32_t *sortedKeys, const uint32_t *sortedEmit, const int *emitGid,
+                               const BinCounts *c, int *entries, int2 *listPos)
 {
     pdlEntry();
     const int total = c->effTotal;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < total; s += gridDim.x * blockDim.x) {
         const uint32_t e = sortedEmit[s];
-        entries[s] = make_int2(emitGid[e], int(e));
+        entries[s] = emitGid[e];
+        listPos[e] = make_int2(s, int(sortedKeys[s]));
     }
 }
 
@@ -530,13 +536,13 @@ void radixSortDepth(const uint32_t *keys, uint2 *pairsA, uint2 *pairsB, uint32_t
 
 size_t scanPartialEntries(int n) { return size_t((n + kScanTile - 1) / kScanTile) + 1; }
 
-static void scanLaunches(const int *in, const uint32_t *perm, int *out, int n, int *partial, const ScanCapacity &cap,
-                         cudaStream_t s)
+static void scanLaunches(const int *in, const uint32_t *perm, int *out, int *outById, int n, int *partial,
+                         const ScanCapacity &cap, cudaStream_t s)
 {
     const int B = (n + kScanTile - 1) / kScanTile;
     { launchPdl(scanReduceKernel, B, kThreads, 0, s, in, perm, n, partial); countLaunch(); }
     { launchPdl(scanPartialKernel, 1, kThreads, 0, s, partial, B); countLaunch(); }
-    { launchPdl(scanDownsweepKernel, B, kThreads, 0, s, in, perm, out, n, partial, B, cap); countLaunch(); }
+    { launchPdl(scanDownsweepKernel, B, kThreads, 0, s, in, perm, out, outById, n, partial, B, cap); countLaunch(); }
 }
 
 void exclusiveScan(const int *in, int *out, int n, int *partial, cudaStream_t s)
@@ -545,18 +551,18 @@ void exclusiveScan(const int *in, int *out, int n, int *partial, cudaStream_t s)
         cudaMemsetAsync(out, 0, sizeof(int), s);
         return;
     }
-    scanLaunches(in, nullptr, out, n, partial, ScanCapacity{0, nullptr, 0, nullptr}, s);
+    scanLaunches(in, nullptr, out, nullptr, n, partial, ScanCapacity{0, nullptr, 0, nullptr}, s);
 }
 
-void exclusiveScanChecked(const int *in, const uint32_t *perm, int *out, int n, int *partial, const ScanCapacity &cap,
-                          cudaStream_t s)
+void exclusiveScanChecked(const int *in, const uint32_t *perm, int *out, int *outById, int n, int *partial,
+                          const ScanCapacity &cap, cudaStream_t s)
 {
     if (n <= 0) {
         cudaMemsetAsync(out, 0, sizeof(int), s);
         launchCapacityCheck(out, cap.capacity, cap.counts, cap.iteration, s, cap.desc);
         return;
     }
-    scanLaunches(in, perm, out, n, partial, cap, s);
+    scanLaunches(in, perm, out, outById, n, partial, cap, s);
 }
 
 size_t cullRowEntries(size_t n) { return n * kCullRows; }
@@ -577,10 +583,10 @@ void launchEmit(const uint32_t *sortedIds, const int *offs, const int4 *rect, in
 }
 
 void launchFinalizeBins(const uint32_t *sortedKeys, const uint32_t *sortedEmit, const int *emitGid, const BinCounts *c,
-                        int capacity, int tiles, int2 *entries, int *tileOffsets, cudaStream_t s)
+                        int capacity, int tiles, int *entries, int2 *listPos, int *tileOffsets, cudaStream_t s)
 {
     if (capacity > 0)
-        { launchPdl(finalizeKernel, std::min(grid(capacity, 256), 148 * 16), 256, 0, s, sortedEmit, emitGid, c, entries); countLaunch(); }
+        { launchPdl(finalizeKernel, std::min(grid(capacity, 256), 148 * 16), 256, 0, s, sortedKeys, sortedEmit, emitGid, c, entries, listPos); countLaunch(); }
     { launchPdl(tileOffsetsKernel, grid(tiles + 1, 256), 256, 0, s, sortedKeys, c, tiles, tileOffsets); countLaunch(); }
 }
 

@@ -641,9 +641,7 @@ int u3dg_rasterizer_tiles(u3dg_rasterizer *r, int *tiles_x, int *tiles_y, int *o
             U3DG_CUDA(cudaMemcpyAsync(offsets, R.ws.tileOffsets.p, (tiles + 1) * sizeof(int), cudaMemcpyDeviceToHost, s));
         const size_t L = std::min(list_capacity, size_t(R.ws.total()));
         if (list && L)
-            // The Gaussian ids: the first int of each (id, emission index) entry.
-            U3DG_CUDA(cudaMemcpy2DAsync(list, sizeof(int), R.ws.entries.p, sizeof(int2), sizeof(int), L,
-                                        cudaMemcpyDeviceToHost, s));
+            U3DG_CUDA(cudaMemcpyAsync(list, R.ws.entries.p, L * sizeof(int), cudaMemcpyDeviceToHost, s));
         R.stream.sync();
     });
 }
@@ -705,6 +703,7 @@ int u3dg_bin_tiles(const float *depth, const int *radius, const int *rect, size_
         ws.radius.reserve(nn);
         ws.cnt.reserve(nn);
         ws.offs.reserve(nn + 1);
+        ws.offsById.reserve(nn);
         ws.scanPartial.reserve(scanPartialEntries(int(nn)) + 1);
         std::vector<uint32_t> keys(n);
         std::vector<int4> rc(n);
@@ -743,8 +742,7 @@ int u3dg_bin_tiles(const float *depth, const int *radius, const int *rect, size_
         U3DG_CUDA(cudaMemcpyAsync(offsets, ws.tileOffsets.p, (tiles + 1) * sizeof(int), cudaMemcpyDeviceToHost, st.s));
         const size_t L = std::min(list_capacity, size_t(ws.total()));
         if (list && L)
-            U3DG_CUDA(cudaMemcpy2DAsync(list, sizeof(int), ws.entries.p, sizeof(int2), sizeof(int), L,
-                                        cudaMemcpyDeviceToHost, st.s));
+            U3DG_CUDA(cudaMemcpyAsync(list, ws.entries.p, L * sizeof(int), cudaMemcpyDeviceToHost, st.s));
         if (list_length)
             *list_length = size_t(ws.total());
         st.sync();

@@ -135,7 +135,8 @@ void RasterWorkspace::eachIntersectionBuffer(size_t capacity, F &&f)
     f(iVals1, capacity);
     f(emitGid, capacity);
     f(entries, capacity);
-    f(partial, capacity * kG2d * size_t(partialSlots));
+    f(listPos, capacity);
+    f(partial, capacity * kPartial * size_t(partialSlots));
 }
 
 void RasterWorkspace::reserveIntersections(size_t capacity)
@@ -171,7 +172,7 @@ void RasterWorkspace::project(const Params &P, int count, const u3dg_camera &c, 
     const int per = st.tile_size > 16 ? st.tile_size / 16 : 1;
     if (per * per > partialSlots) { // a tile size spanning more backward CTAs than before
         partialSlots = per * per;
-        partial.reserve(size_t(icap) * kG2d * size_t(partialSlots), true);
+        partial.reserve(size_t(icap) * kPartial * size_t(partialSlots), true);
     }
     ProjOut out{rec.p, depthKey.p, depth.p, rect.p, radius.p, flags.p, cov2d.p, cnt.p, rowTab.p, culled() ? 1 : 0};
     launchProject(P, n, cam, st, tilesX, tilesY, shRest, shDegree, out, stream, desc);
@@ -191,10 +192,10 @@ void RasterWorkspace::eachGaussianBuffer(size_t nn, F &&f)
     f(rowTab, cullRowEntries(nn));
     f(cnt, nn);
     f(offs, nn + 1);
+    f(offsById, nn);
     f(scanPartial, scanPartialEntries(int(nn)) + 1);
     f(flags, nn);
     f(cov2d, nn);
-    f(g2d, nn * kG2d);
     f(hist, std::max(radixHistEntries(std::max(int(nn), icap)), size_t(256)));
 }
 
@@ -219,6 +220,7 @@ void RasterWorkspace::planPixels(DeviceSlab &slab, size_t pixels, int tx, int ty
     const int pb = tileSize <= 8 ? 8 : 16;
     const int per = tileSize > pb ? tileSize / pb : 1;
     slab.add(blockOrder, size_t(std::max(1, tx * per * ty * per)));
+    slab.add(blockStop, size_t(std::max(1, tx * per * ty * per)));
 }
 
 void RasterWorkspace::bin(cudaStream_t stream, int iteration, const StepDesc *desc)
@@ -233,7 +235,7 @@ void RasterWorkspace::bin(cudaStream_t stream, int iteration, const StepDesc *de
     // The projection counted each Gaussian's tiles (and, culling, its row table); the scan takes the
     // counts in depth-rank order.
     const SplatRec *cullRec = culled() ? rec.p : nullptr;
-    exclusiveScanChecked(cnt.p, sortedIds, offs.p, n, scanPartial.p, ScanCapacity{icap, counts.p, iteration, desc},
+    exclusiveScanChecked(cnt.p, sortedIds, offs.p, offsById.p, n, scanPartial.p, ScanCapacity{icap, counts.p, iteration, desc},
                          stream);
     launchEmit(sortedIds, offs.p, rect.p, n, counts.p, icap, tilesX, cullRec, st.tile_size, rowTab.p, iKeys0.p,
                emitGid.p, stream);
@@ -242,11 +244,11 @@ void RasterWorkspace::bin(cudaStream_t stream, int iteration, const StepDesc *de
         ++bits;
     bits = std::max(bits, 1);
     // Up to 2048 tiles: one pass whose scatter also writes the lists' entries and the tile offsets.
-    const TileFinish fin{emitGid.p, entries.p, tileOffsets.p, tiles};
+    const TileFinish fin{emitGid.p, entries.p, listPos.p, tileOffsets.p, tiles};
     const int tilePasses = radixSortPairs(iKeys0.p, iKeys1.p, iVals0.p, iVals1.p, &counts.p->effTotal, icap, bits,
                                           hist.p, rowTotals.p, &keysOut, &valsOut, stream, &fin);
     if (tilePasses != 1)
-        launchFinalizeBins(keysOut, valsOut, emitGid.p, counts.p, icap, tiles, entries.p, tileOffsets.p, stream);
+        launchFinalizeBins(keysOut, valsOut, emitGid.p, counts.p, icap, tiles, entries.p, listPos.p, tileOffsets.p, stream);
 }
 
 void RasterWorkspace::forwardChecked(const Params &P, int count, const u3dg_camera &c, const u3dg_raster_settings &s,
@@ -285,7 +287,7 @@ RasterArgs RasterWorkspace::rasterArgs() const
     a.blocksX = tilesX * per;
     a.blocksY = tilesY * per;
     a.subSlots = per * per;
-    a.subStride = size_t(icap) * kG2d;
+    a.subStride = size_t(icap) * kPartial;
     a.blockOrder = blockOrder.p;
     a.counters = blockCounters.p;
     a.forwardBlock = forwardBlock;
@@ -303,6 +305,7 @@ void RasterWorkspace::composite(cudaStream_t stream)
     const int pb = st.tile_size <= 8 ? 8 : 16;
     const int per = st.tile_size > pb ? st.tile_size / pb : 1;
     blockOrder.reserve(size_t(std::max(1, tilesX * per * tilesY * per)));
+    blockStop.reserve(size_t(std::max(1, tilesX * per * tilesY * per)));
     const RasterArgs a = rasterArgs();
     launchBlockOrder(a, blockOrder.p, stream);
     launchCompositeForward(a, rgb.p, finalT.p, nContrib.p, stream);
@@ -310,7 +313,7 @@ void RasterWorkspace::composite(cudaStream_t stream)
 
 void RasterWorkspace::backwardComposite(const float *dLdRgb, cudaStream_t stream)
 {
-    launchCompositeBackward(rasterArgs(), dLdRgb, finalT.p, nContrib.p, partial.p, stream);
+    launchCompositeBackward(rasterArgs(), dLdRgb, finalT.p, nContrib.p, partial.p, blockStop.p, stream);
 }
 
 ChainArgs RasterWorkspace::chainArgs(const Params &P) const
@@ -323,13 +326,16 @@ ChainArgs RasterWorkspace::chainArgs(const Params &P) const
     a.radius = radius.p;
     a.rec = rec.p;
     a.flags = flags.p;
-    a.offs = offs.p;
-    a.sortedIds = sortedIds;
+    a.offs = offsById.p;
+    a.tileCount = cnt.p;
+    a.listPos = listPos.p;
+    a.stop = blockStop.p;
     a.partial = partial.p;
     const int per = st.tile_size > 16 ? st.tile_size / 16 : 1;
     a.subSlots = per * per;
-    a.subStride = size_t(icap) * kG2d;
-    a.g2d = g2d.p;
+    a.subStride = size_t(icap) * kPartial;
+    a.tilesX = tilesX;
+    a.blocksX = tilesX * per;
     a.counts = counts.p;
     return a;
 }

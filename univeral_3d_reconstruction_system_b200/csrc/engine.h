@@ -198,20 +198,21 @@ struct RasterWorkspace {
     DevBuf<uint2> depthPairs[2];           // the depth sort's (key, id) pairs between passes
     DevBuf<float> depth;
     DevBuf<int4> rect;
-    DevBuf<int> radius, cnt, offs, scanPartial, hist, rowTotals; // cnt: tiles per Gaussian (projection)
+    DevBuf<int> radius, cnt, offs, offsById, scanPartial, hist, rowTotals; // cnt: tiles per Gaussian (projection)
     DevBuf<uint32_t> rowTab; // tile culling: per Gaussian, the first rows' spans (emission lookup)
     DevBuf<uint8_t> flags;
     DevBuf<float4> cov2d;
-    DevBuf<float> g2d; // per Gaussian: summed 2D gradients (chain-rule input)
     // per intersection (capacity icap)
     DevBuf<uint32_t> iKeys0, iKeys1, iVals0, iVals1;
     DevBuf<int> emitGid;
-    DevBuf<int2> entries; // per tile-sorted entry: Gaussian id, emission index
-    DevBuf<float> partial;             // partialSlots arrays of icap * 9 floats
+    DevBuf<int> entries;   // per tile-sorted entry: Gaussian id
+    DevBuf<int2> listPos;  // per emission: list position, tile
+    DevBuf<float> partial; // partialSlots arrays of icap * kPartial floats
     int icap = 0;
     int partialSlots = 1;              // slot arrays the backward needs: (tile size / 16)^2 above 16
     // per tile / pixel
     DevBuf<int> tileOffsets, nContrib;
+    DevBuf<int> blockStop; // per backward block: list position behind its last contributor
     DevBuf<int> blockOrder, blockCounters; // compositing schedule: pixel blocks by list length, counters
     DevBuf<float> rgb, finalT;
     // device-side sizes of the last pass and their pinned host copy

@@ -187,87 +187,77 @@ __device__ __forceinline__ void adamOne(float &p, float &m, float &v, float g, f
     p -= stepSize * m / (sqrtf(v) * invSqrtBc2 + 1e-15f);
 }
 
-// The 9 summed 2D gradients of every Gaussian from the per-(tile, Gaussian) partials of the
-// compositing backward. Emission order is depth-rank order, so a rank's partials are contiguous: one
-// warp per 32 consecutive ranks walks their partials 32 entries at a time (coalesced), lane j holding
-// entry j of the chunk; a segmented inclusive scan over the lanes (segments = ranks) adds the entries
-// of each rank in lane order, and each rank's lane adds the scan value at its last entry in the chunk.
-// The order of the additions is fixed, so the sums are deterministic. Written per Gaussian id.
-__global__ void __launch_bounds__(256) partialSumKernel(const float *partial, int subSlots, size_t subStride,
-                                                        const int *offs, const uint32_t *sortedIds, int n,
-                                                        const BinCounts *counts, float *g2d)
+// The 9 summed 2D gradients of Gaussian i: its partials of the compositing backward, in emission order.
+// Every intersection names its list position and tile (listPos); those behind the last contributor of
+// their block's pixels (stop) have no partial and are passed over, so a Gaussian deep behind others
+// costs its 8-byte positions only. A lane adds up its own Gaussian, four intersections' loads in flight
+// at a time; Gaussians in more tiles than kGatherLane are added by the whole warp (lanes strided, then a
+// butterfly), so that a few image-sized ones do not hold up a kernel. Both orders are fixed, so the sums
+// are deterministic. All lanes of a warp call it (cnt = 0 without a Gaussian).
+constexpr int kGatherLane = 32;
+
+__device__ __forceinline__ void addPartial(const ChainArgs &a, const int2 &lp, float (&g)[kG2d])
 {
-    pdlEntry();
-    if (counts != nullptr && counts->abortIter >= 0)
-        return;
-    const int lane = threadIdx.x & 31;
-    const int warps = int((gridDim.x * blockDim.x) >> 5);
-    for (int w = int((blockIdx.x * blockDim.x + threadIdx.x) >> 5); w * 32 < n; w += warps) {
-        const int r = w * 32 + lane;
-        const bool valid = r < n;
-        const int o = valid ? offs[r] : INT_MAX;
-        const int oEnd = valid ? offs[r + 1] : INT_MAX;
-        const int first = offs[w * 32], last = offs[min(w * 32 + 32, n)];
-        float acc[kG2d];
-#pragma unroll
-        for (int k = 0; k < kG2d; ++k)
-            acc[k] = 0.0f;
-        for (int c0 = first; c0 < last; c0 += 32) {
-            const int e = c0 + lane;
-            const bool in = e < last;
-            // Owner of entry e: the last lane whose start offset is not above e.
-            int owner = 0;
-#pragma unroll
-            for (int step = 16; step > 0; step >>= 1) {
-                const int oc = __shfl_sync(0xffffffffu, o, owner + step);
-                if (oc <= e)
-                    owner += step;
-            }
-            float v[kG2d];
-#pragma unroll
-            for (int k = 0; k < kG2d; ++k)
-                v[k] = in ? partial[size_t(e) * kG2d + k] : 0.0f;
-            // Tiles covered by several CTAs: their slots, added in slot order.
-            for (int sl = 1; sl < subSlots; ++sl) {
-                const float *p = partial + size_t(sl) * subStride;
-#pragma unroll
-                for (int k = 0; k < kG2d; ++k)
-                    v[k] = __fadd_rn(v[k], in ? p[size_t(e) * kG2d + k] : 0.0f);
-            }
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int ownerUp = __shfl_up_sync(0xffffffffu, owner, d);
-                const bool same = lane >= d && ownerUp == owner;
-#pragma unroll
-                for (int k = 0; k < kG2d; ++k) {
-                    const float up = __shfl_up_sync(0xffffffffu, v[k], d);
-                    if (same)
-                        v[k] = __fadd_rn(v[k], up);
-                }
-            }
-            // This lane's rank: its last entry inside the chunk, if any.
-            const int lastE = min(min(oEnd, last), c0 + 32) - 1;
-            const bool has = valid && o < c0 + 32 && oEnd > c0 && lastE >= max(o, c0);
-            const int src = has ? lastE - c0 : lane;
-#pragma unroll
-            for (int k = 0; k < kG2d; ++k) {
-                const float got = __shfl_sync(0xffffffffu, v[k], src);
-                if (has)
-                    acc[k] = __fadd_rn(acc[k], got);
-            }
+    for (int sl = 0; sl < a.subSlots; ++sl) {
+        int block = lp.y;
+        if (a.subSlots > 1) { // tiles covered by several blocks: slot sl is its block's position, row-major
+            const int per = a.blocksX / a.tilesX;
+            block = (lp.y / a.tilesX * per + sl / per) * a.blocksX + lp.y % a.tilesX * per + sl % per;
         }
-        if (valid) {
-            float *dst = g2d + size_t(sortedIds[r]) * kG2d;
+        if (lp.x >= a.stop[block])
+            continue;
+        const float4 *p = reinterpret_cast<const float4 *>(a.partial + sl * a.subStride) + size_t(lp.x) * (kPartial / 4);
+        const float4 u = p[0], v = p[1];
+        const float w = p[2].x;
+        g[0] += u.x;
+        g[1] += u.y;
+        g[2] += u.z;
+        g[3] += u.w;
+        g[4] += v.x;
+        g[5] += v.y;
+        g[6] += v.z;
+        g[7] += v.w;
+        g[8] += w;
+    }
+}
+
+__device__ __forceinline__ void gatherPartials(const ChainArgs &a, int start, int cnt, float (&g)[kG2d])
+{
+    const int lane = threadIdx.x & 31;
 #pragma unroll
-            for (int k = 0; k < kG2d; ++k)
-                dst[k] = acc[k];
+    for (int k = 0; k < kG2d; ++k)
+        g[k] = 0.0f;
+    const int own = cnt <= kGatherLane ? cnt : 0;
+    for (int k = 0; k < own; k += 4) {
+        int2 lp[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+            lp[r] = k + r < own ? a.listPos[start + k + r] : make_int2(INT_MAX, 0);
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+            addPartial(a, lp[r], g);
+    }
+    for (uint32_t many = __ballot_sync(0xffffffffu, cnt > kGatherLane); many; many &= many - 1) {
+        const int owner = __ffs(many) - 1;
+        const int s0 = __shfl_sync(0xffffffffu, start, owner), c0 = __shfl_sync(0xffffffffu, cnt, owner);
+        float h[kG2d] = {};
+        for (int k = lane; k < c0; k += 32)
+            addPartial(a, a.listPos[s0 + k], h);
+#pragma unroll
+        for (int k = 0; k < kG2d; ++k) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                h[k] += __shfl_xor_sync(0xffffffffu, h[k], o);
+            if (lane == owner)
+                g[k] = h[k];
         }
     }
 }
 
 // Rasterizer::backward pass 2 (Rasterizer.cpp:432-544) for one Gaussian per thread, fused either with
 // Adam::step (kAdam: the trainer; gradients never leave registers) or with adding the gradients into
-// caller arrays (the unit entry point). The per-Gaussian 2D gradient comes from partialSumKernel.
+// caller arrays (the unit entry point). It starts from the Gaussian's summed partials (gatherPartials),
+// which never go through memory.
 // Resident CTAs per SM the compiler must allow for: caps registers per thread at 65536 / (256 * n)
 // (64 at 4; the kernel is latency-bound, and 4 CTAs per SM beat fewer with more registers).
 #ifndef U3DG_CHAIN_MIN_BLOCKS
@@ -279,15 +269,18 @@ __global__ void __launch_bounds__(256, U3DG_CHAIN_MIN_BLOCKS) chainKernel(ChainA
 {
     pdlEntry();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n || (a.counts != nullptr && a.counts->abortIter >= 0))
+    if (a.counts != nullptr && a.counts->abortIter >= 0)
+        return;
+    float g[kG2d];
+    {
+        const bool seen = i < a.n && a.radius[i] > 0;
+        gatherPartials(a, seen ? a.offs[i] : 0, seen ? a.tileCount[i] : 0, g);
+    }
+    if (i >= a.n)
         return;
     const Params &P = a.params;
     float gMeans[3] = {0, 0, 0}, gScales[3] = {0, 0, 0}, gQuats[4] = {0, 0, 0, 0}, gOpac = 0, gColors[3] = {0, 0, 0};
     if (a.radius[i] > 0) {
-        float g[kG2d];
-#pragma unroll
-        for (int k = 0; k < kG2d; ++k)
-            g[k] = a.g2d[size_t(i) * kG2d + k];
         const u3dg_camera &cam = a.desc ? a.desc->cam : a.cam;
         const float dmx = g[0], dmy = g[1], dA = g[2], dB = g[3], dC = g[4];
         if (a.gradAccum != nullptr) {
@@ -613,8 +606,6 @@ void launchChain(const ChainArgs &a, bool adam, cudaStream_t s)
 {
     if (a.n <= 0)
         return;
-    { launchPdl(partialSumKernel, std::min(blocks((long long)(a.n + 31) / 32 * 32, 256), 148 * 16), 256, 0, s, 
-          a.partial, std::max(a.subSlots, 1), a.subStride, a.offs, a.sortedIds, a.n, a.counts, a.g2d); countLaunch(); }
     if (adam)
         { launchPdl(chainKernel<true>, blocks(a.n, 256), 256, 0, s, a); countLaunch(); }
     else

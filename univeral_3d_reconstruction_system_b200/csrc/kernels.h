@@ -85,12 +85,15 @@ struct ChainArgs {
     const int *radius;
     const SplatRec *rec;
     const uint8_t *flags;
-    const int *offs;      // per rank: first intersection in emission order (n + 1 entries)
-    const uint32_t *sortedIds; // Gaussian id per depth rank
-    const float *partial; // per intersection, in emission order: 9 summed 2D gradients (subSlots arrays)
+    const int *offs;      // per Gaussian: first intersection in emission order
+    const int *tileCount; // per Gaussian: its intersections
+    const int2 *listPos;  // per intersection, in emission order: position in the tile lists, tile
+    const int *stop;      // per backward block: the list position behind its pixels' last contributor
+    const float *partial; // per list position below its block's stop: 9 summed 2D gradients (kPartial
+                          // floats; subSlots arrays)
     int subSlots;         // slot arrays of partial (RasterArgs::subSlots), subStride floats apart
     size_t subStride;
-    float *g2d;           // per Gaussian: the 9 partials summed (written by launchChain's first kernel)
+    int tilesX, blocksX;  // tiles per row; backward blocks per row
     const BinCounts *counts; // the kernel does nothing when counts->abortIter >= 0
     float *gradAccum;     // |dL/dmean2d| NDC statistic (may be null)
     int *gradCount;       // visibility count (may be null)
@@ -127,13 +130,14 @@ void launchOpacityReset(float *opac, float *mOpac, float *vOpac, int n, float ca
 int radixBlocks(int nMax);
 size_t radixHistEntries(int nMax);
 // Outputs of a tile sort done in one pass (keys of at most 11 bits, digit = tile): instead of the
-// sorted keys and values, the scatter writes every sorted entry as one 8-byte pair (entries[pos] =
-// (Gaussian id = emitGid[emission index], emission index)), and the tile offsets (tiles + 1 entries;
-// the last is the item count). One scattered 8-byte store per entry instead of two 4-byte ones: the
-// scatter's cost is its scattered stores.
+// sorted keys and values, the scatter writes every sorted entry's Gaussian id (entries[pos] =
+// emitGid[emission index]), where each emission went (listPos[emission index] = (pos, tile), in
+// emission order and so coalesced) and the tile offsets (tiles + 1 entries; the last is the item
+// count). The one scattered store per entry is 4 bytes: the scatter's cost is its scattered stores.
 struct TileFinish {
     const int *emitGid;
-    int2 *entries;
+    int *entries;
+    int2 *listPos;
     int *tileOffsets;
     int tiles;
 };
@@ -162,8 +166,9 @@ struct ScanCapacity {
     int iteration;
     const StepDesc *desc;
 };
-void exclusiveScanChecked(const int *in, const uint32_t *perm, int *out, int n, int *partial, const ScanCapacity &cap,
-                          cudaStream_t s);
+// outById[perm[i]] gets out[i].
+void exclusiveScanChecked(const int *in, const uint32_t *perm, int *out, int *outById, int n, int *partial,
+                          const ScanCapacity &cap, cudaStream_t s);
 // Entries of the per-Gaussian row table of tile culling (ProjOut::rowTab) for n Gaussians.
 size_t cullRowEntries(size_t n);
 // Checks *total against the intersection capacity (see BinCounts); exclusiveScanChecked does the same
@@ -175,16 +180,16 @@ void launchCapacityCheck(const int *total, int capacity, BinCounts *c, int itera
 void launchEmit(const uint32_t *sortedIds, const int *offs, const int4 *rect, int n, const BinCounts *c, int capacity,
                 int tilesX, const SplatRec *cullRec, int tileSize, const uint32_t *rowTab, uint32_t *keys, int *emitGid,
                 cudaStream_t s);
-// After a tile sort of several passes (more than 2048 tiles): the (Gaussian id, emission index) pair of
-// every sorted entry and the tile offsets (a binary search in the sorted keys). A one-pass tile sort
+// After a tile sort of several passes (more than 2048 tiles): the Gaussian id of every sorted entry, the
+// list position and tile of every emission and the tile offsets (a binary search in the sorted keys). A one-pass tile sort
 // writes both itself (TileFinish).
 void launchFinalizeBins(const uint32_t *sortedKeys, const uint32_t *sortedEmit, const int *emitGid, const BinCounts *c,
-                        int capacity, int tiles, int2 *entries, int *tileOffsets, cudaStream_t s);
+                        int capacity, int tiles, int *entries, int2 *listPos, int *tileOffsets, cudaStream_t s);
 
 // raster.cu
 struct RasterArgs {
     const int *tileOffsets;
-    const int2 *entries; // per tile-sorted entry: Gaussian id, emission index (where backward stores partials)
+    const int *entries; // per tile-sorted entry: Gaussian id
     const SplatRec *rec;
     int width, height, tileSize, tilesX;
     float bg[3];
@@ -206,10 +211,11 @@ struct RasterArgs {
 // order[blocksX * blocksY].
 void launchBlockOrder(const RasterArgs &a, int *order, cudaStream_t s);
 void launchCompositeForward(const RasterArgs &a, float *rgb, float *finalT, int *nContrib, cudaStream_t s);
-// partial: 9 floats per intersection in emission order, in a.subSlots slot arrays (every slot of every
-// entry is written: no zeroing needed).
+// partial: kPartial floats per list position, in a.subSlots slot arrays; stop: per pixel block, the list
+// position behind its pixels' last contributor. Partials from there on are not written: they are zero,
+// and ChainArgs' reader skips them.
 void launchCompositeBackward(const RasterArgs &a, const float *dLdRgb, const float *finalT, const int *nContrib,
-                             float *partial, cudaStream_t s);
+                             float *partial, int *stop, cudaStream_t s);
 
 // loss.cu
 struct LossScratch {

@@ -6,9 +6,10 @@
 // contributions before the warp sum, so one warp reduction covers 64 pixels. The 9 sums per list entry
 // (dmean2d xy, dconic ABC, drgb, dalpha) go through a reduce-scatter (14 shuffles), land in a
 // per-warp shared-memory slot, and are added over the warps in warp order after the batch: the result
-// does not depend on scheduling. Each (tile, Gaussian) partial is stored once at the entry's emission
-// index, zero for entries behind every pixel's last contributor; the chain-rule kernel sums a
-// Gaussian's partials in tile order. Tiles of 32 or 64 pixels span 4 or 16 CTAs (16x16 blocks): each
+// does not depend on scheduling. Each (tile, Gaussian) partial is stored once, at the entry's list
+// position (a tile's partials are contiguous); entries behind every pixel's last contributor, where
+// lists are long more than half, are neither written nor read (stop); the chain-rule kernel sums a
+// Gaussian's partials in emission order. Tiles of 32 or 64 pixels span 4 or 16 CTAs (16x16 blocks): each
 // stores into its own slot array and the chain-rule kernel adds the slots in a fixed order, so every
 // tile size gives deterministic gradients (no atomics).
 //
@@ -116,14 +117,14 @@ template <int PB, int BD, bool kBg>
 __device__ __forceinline__ void backwardBlock(const RasterArgs &a, int bx, int by, const float *dLdRgb,
                                               const float *finalTIn, const int *nContribIn, float *partial,
                                               float4 *sP, float4 *sQ, float4 *sR,
-                                              uint32_t (*mask)[RasterShape<PB, BD>::NG], int &sMax, float *sWarp)
+                                              uint32_t (*mask)[RasterShape<PB, BD>::NG], int &sMax, float *sWarp, int &stop)
 {
     using S = RasterShape<PB, BD>;
     constexpr int NT = S::NT, NW = S::NW, NB = S::NB, NG = S::NG;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const WarpBlock<PB> wb(warp, lane, bx, by);
     const int tile = tileOf<PB>(a, bx, by);
-    const int start = a.tileOffsets[tile], end = a.tileOffsets[tile + 1];
+    const int start = a.tileOffsets[tile];
     const bool in0 = wb.px < a.width && wb.py0 < a.height, in1 = wb.px < a.width && wb.py1 < a.height;
     if (a.subSlots > 1) { // this block's slot array: its position in the tile, row-major
         const int per = a.tileSize / PB;
@@ -148,14 +149,9 @@ __device__ __forceinline__ void backwardBlock(const RasterArgs &a, int bx, int b
     __syncthreads();
     const int jmax = sMax;
     // Entries behind every pixel's last contributor get no gradient (the reference's per-tile
-    // accumulators start at zero); their partials are still written, as the chain-rule kernel sums
-    // every intersection of a Gaussian.
-    for (int j = jmax + tid; j < end - start; j += NT) {
-            float *dst = partial + size_t(a.entries[start + j].y) * kG2d;
-#pragma unroll
-            for (int k = 0; k < kG2d; ++k)
-                dst[k] = 0.0f;
-        }
+    // accumulators start at zero): the chain-rule kernel skips them by this position.
+    if (tid == 0)
+        stop = start + jmax;
     float *myWarp = sWarp + size_t(warp) * NB * kG2d;
     for (int bEnd = jmax; bEnd > 0; bEnd -= NB) {
         const int bStart = max(0, bEnd - NB), cnt = bEnd - bStart;
@@ -280,10 +276,10 @@ __device__ __forceinline__ void backwardBlock(const RasterArgs &a, int bx, int b
                 for (int q = 0; q < kG2d; ++q)
                     sum[q] += sWarp[(size_t(w) * NB + e) * kG2d + q];
             finishEntry(sQ[e], sum);
-            float *dst = partial + size_t(a.entries[start + bStart + e].y) * kG2d;
-#pragma unroll
-            for (int q = 0; q < kG2d; ++q)
-                dst[q] = sum[q];
+            float4 *dst = reinterpret_cast<float4 *>(partial) + size_t(start + bStart + e) * (kPartial / 4);
+            dst[0] = make_float4(sum[0], sum[1], sum[2], sum[3]);
+            dst[1] = make_float4(sum[4], sum[5], sum[6], sum[7]);
+            dst[2] = make_float4(sum[8], 0.0f, 0.0f, 0.0f);
         }
     }
 }
@@ -302,7 +298,7 @@ __device__ __forceinline__ void backwardBlock(const RasterArgs &a, int bx, int b
 template <int PB, int BD, bool kBg>
 __global__ void __launch_bounds__(RasterShape<PB>::NT, U3DG_BWD_MIN_BLOCKS) compositeBackwardKernel(RasterArgs a, const float *dLdRgb,
                                                                               const float *finalTIn,
-                                                                              const int *nContribIn, float *partial)
+                                                                              const int *nContribIn, float *partial, int *stop)
 {
     pdlEntry();
     using S = RasterShape<PB, BD>;
@@ -317,7 +313,7 @@ __global__ void __launch_bounds__(RasterShape<PB>::NT, U3DG_BWD_MIN_BLOCKS) comp
     int *counter = a.counters + 2; // backward: counters[2..3]
     for (int b = nextBlock(a, counter, &sNext); b < units; b = nextBlock(a, counter, &sNext))
         backwardBlock<PB, BD, kBg>(a, b % a.blocksX, b / a.blocksX, dLdRgb, finalTIn, nContribIn, partial, sP, sQ, sR,
-                              mask, sMax, sWarp);
+                              mask, sMax, sWarp, stop[b]);
 }
 
 template <class K>
@@ -336,7 +332,7 @@ int residentCtas(K kernel, int threads, size_t smem)
 
 template <int PB, int BD, bool kBg>
 static void launchBackward(const RasterArgs &a, const float *dLdRgb, const float *finalT, const int *nContrib,
-                           float *partial, cudaStream_t s)
+                           float *partial, int *stop, cudaStream_t s)
 {
     using S = RasterShape<PB, BD>;
     const size_t smem = size_t(S::NW) * S::NB * kG2d * sizeof(float); // 18 KB (BD 1) or 36 KB (BD 2) at PB 16
@@ -345,11 +341,11 @@ static void launchBackward(const RasterArgs &a, const float *dLdRgb, const float
         return residentCtas(compositeBackwardKernel<PB, BD, kBg>, S::NT, smem);
     }();
     const int units = a.blocksX * a.blocksY;
-    { launchPdl(compositeBackwardKernel<PB, BD, kBg>, std::min(units, ctas), S::NT, smem, s, a, dLdRgb, finalT, nContrib, partial); countLaunch(); }
+    { launchPdl(compositeBackwardKernel<PB, BD, kBg>, std::min(units, ctas), S::NT, smem, s, a, dLdRgb, finalT, nContrib, partial, stop); countLaunch(); }
 }
 
 void launchCompositeBackward(const RasterArgs &a, const float *dLdRgb, const float *finalT, const int *nContrib,
-                             float *partial, cudaStream_t s)
+                             float *partial, int *stop, cudaStream_t s)
 {
     if (a.blocksX * a.blocksY <= 0)
         return;
@@ -358,11 +354,11 @@ void launchCompositeBackward(const RasterArgs &a, const float *dLdRgb, const flo
     auto run = [&](auto kBg) {
         constexpr bool B = decltype(kBg)::value;
         if (a.tileSize <= 8)
-            deep ? launchBackward<8, 2, B>(a, dLdRgb, finalT, nContrib, partial, s)
-                 : launchBackward<8, 1, B>(a, dLdRgb, finalT, nContrib, partial, s);
+            deep ? launchBackward<8, 2, B>(a, dLdRgb, finalT, nContrib, partial, stop, s)
+                 : launchBackward<8, 1, B>(a, dLdRgb, finalT, nContrib, partial, stop, s);
         else
-            deep ? launchBackward<16, 2, B>(a, dLdRgb, finalT, nContrib, partial, s)
-                 : launchBackward<16, 1, B>(a, dLdRgb, finalT, nContrib, partial, s);
+            deep ? launchBackward<16, 2, B>(a, dLdRgb, finalT, nContrib, partial, stop, s)
+                 : launchBackward<16, 1, B>(a, dLdRgb, finalT, nContrib, partial, stop, s);
     };
     if (bg)
         run(std::true_type{});
