@@ -37,3 +37,82 @@ def test_gaussians_in_few_and_many_tiles(u3dg, oracle, width, height, tile):
     cam = make_camera(width, height, 0.8 * width)
     w = rng.uniform(-1, 1, (height, width, 3)).astype(np.float32)
     _close(u3dg, oracle, small, cam, RasterSettings(tile_size=tile, background=(0.1, 0.2, 0.3)), w, 2e-4)
+
+
+def _stack(n, rng, opacity):
+    """n Gaussians one behind the other, each over the whole of a small image."""
+    m = random_model(n, rng, 0.05, 3.0, 0.5, 1.0)
+    m.means[:, 2] = np.linspace(2.0, 4.0, n)
+    m.opacities[:] = np.log(opacity / (1 - opacity))
+    return m
+
+
+@pytest.mark.parametrize("tile", [8, 16, 32])
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 128, 129, 257, 700])
+def test_backward_at_segment_edges(u3dg, oracle, n, tile):
+    # Lists that end at, before and behind a segment's 64 (256 at tile 32) entries, blended to the end (no
+    # pixel terminates: at most 700 alphas of 0.008) and over a background; some pixels terminate in a
+    # second, opaque stack. Sums over 1,200 pixels: within 1e-4.
+    rng = np.random.default_rng(n)
+    w = rng.uniform(-1, 1, (37, 33, 3)).astype(np.float32)
+    cam = make_camera(33, 37, 30.0)
+    _close(u3dg, oracle, _stack(n, rng, 0.008), cam, RasterSettings(tile_size=tile, background=(0.3, 0.1, 0.2)), w, 1e-4)
+    mixed = _stack(n, rng, 0.008)
+    mixed.opacities[n // 2:] = 1.0
+    mixed.scales[n // 2:] -= 3.0
+    _close(u3dg, oracle, mixed, cam, RasterSettings(tile_size=tile), w, 1e-4)
+
+
+def test_a_non_finite_pixel_gradient_reaches_only_what_blends_there(u3dg):
+    rng = np.random.default_rng(3)
+    m = random_model(200, rng, 1.0, 3.0, 0.02, 0.1)
+    cam, st = make_camera(64, 48, 50.0), RasterSettings()
+    w = rng.uniform(-1, 1, (48, 64, 3)).astype(np.float32)
+    r = u3dg.Rasterizer()
+    r.forward(m, cam, st)
+    clean = r.backward(m, w)
+    w[20, 30, 1] = np.inf
+    r.forward(m, cam, st)
+    bad = r.backward(m, w)
+    hit = ~np.isfinite(bad.opacities)
+    # The Gaussians that blend at that pixel, found by the image's change when each is removed.
+    base = r.forward(m, cam, st)[20, 30]
+    blends = np.zeros(m.size(), bool)
+    for i in range(m.size()):
+        one = m.copy()
+        one.opacities[i] = -30.0
+        blends[i] = np.any(r.forward(one, cam, st)[20, 30] != base)
+    assert 0 < blends.sum() < m.size() // 2
+    assert np.all(hit <= blends)
+    for k in ("means", "scales", "quats", "opacities", "colors"):
+        a, b = getattr(bad, k)[~blends], getattr(clean, k)[~blends]
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("background", [(0.0, 0.0, 0.0), (0.2, 0.4, 0.1)])
+def test_a_non_finite_colour_reaches_only_the_pixels_it_covers(u3dg, background):
+    rng = np.random.default_rng(4)
+    m = random_model(120, rng, 1.0, 3.0, 0.02, 0.08)
+    m.means[7] = [0.0, 0.0, 2.5]
+    cam, st = make_camera(64, 48, 50.0), RasterSettings(background=background)
+    w = rng.uniform(-1, 1, (48, 64, 3)).astype(np.float32)
+    r = u3dg.Rasterizer()
+    clean_image = r.forward(m, cam, st)
+    clean = r.backward(m, w)
+    m.colors[7, 0] = np.inf
+    image = r.forward(m, cam, st)
+    bad = r.backward(m, w)
+    covered = np.any(image != clean_image, axis=-1)
+    assert 0 < covered.sum() < covered.size // 4
+    # Gaussians none of whose pixels the coloured one covers keep their gradients.
+    far = np.array([np.isfinite(bad.opacities[i]) for i in range(m.size())])
+    assert far.sum() > 20
+    same = [i for i in range(m.size()) if np.array_equal(bad.means[i], clean.means[i])]
+    w0 = np.where(covered[..., None], 0.0, w).astype(np.float32)
+    m.colors[7, 0] = 0.0
+    r.forward(m, cam, st)
+    masked = r.backward(m, w0)
+    r.forward(m, cam, st)
+    whole = r.backward(m, w)
+    untouched = [i for i in range(m.size()) if np.array_equal(masked.opacities[i], whole.opacities[i])]
+    assert untouched and set(untouched) - {7} <= set(same)

@@ -503,7 +503,7 @@ static u3dg_rasterizer &rz(u3dg_rasterizer *r)
 }
 
 static void rasterForward(u3dg_rasterizer &r, const u3dg_model *model, const float *shRest, int degree,
-                          const u3dg_camera *camera, const u3dg_raster_settings *settings, float *rgb)
+                          const u3dg_camera *camera, const u3dg_raster_settings *settings, float *rgb, bool keep)
 {
     requireModel(model, "model");
     if (!camera || !settings || !rgb)
@@ -522,7 +522,7 @@ static void rasterForward(u3dg_rasterizer &r, const u3dg_model *model, const flo
         U3DG_CUDA(cudaMemcpyAsync(sh.p, shRest, model->count * K * 3 * sizeof(float), cudaMemcpyHostToDevice, s));
         shDev = sh.p;
     }
-    r.ws.forwardChecked(r.model.params(), int(model->count), *camera, *settings, shDev, degree, s);
+    r.ws.forwardChecked(r.model.params(), int(model->count), *camera, *settings, shDev, degree, s, keep);
     U3DG_CUDA(cudaGetLastError());
     U3DG_CUDA(cudaMemcpyAsync(rgb, r.ws.rgb.p, size_t(camera->width) * camera->height * 3 * sizeof(float),
                               cudaMemcpyDeviceToHost, s));
@@ -533,7 +533,7 @@ static void rasterForward(u3dg_rasterizer &r, const u3dg_model *model, const flo
 int u3dg_rasterizer_forward(u3dg_rasterizer *r, const u3dg_model *model, const u3dg_camera *camera,
                             const u3dg_raster_settings *settings, float *rgb)
 {
-    return guarded([&] { rasterForward(rz(r), model, nullptr, 0, camera, settings, rgb); });
+    return guarded([&] { rasterForward(rz(r), model, nullptr, 0, camera, settings, rgb, true); });
 }
 
 int u3dg_rasterizer_backward(u3dg_rasterizer *r, const u3dg_model *model, const float *dl_drgb, u3dg_model *grads,
@@ -1212,7 +1212,7 @@ int u3dg_render_sh(const u3dg_model *model, const float *sh_rest, int degree, co
         requireDevice();
         u3dg_rasterizer r;
         U3DG_CUDA(cudaGetDevice(&r.device));
-        rasterForward(r, model, sh_rest, degree, camera, settings, rgb);
+        rasterForward(r, model, sh_rest, degree, camera, settings, rgb, false);
     });
 }
 

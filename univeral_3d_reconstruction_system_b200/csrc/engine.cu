@@ -19,6 +19,9 @@
 
 #include "engine.h"
 
+#ifndef U3DG_SEG16
+#define U3DG_SEG16 64
+#endif
 #include <algorithm>
 #include <atomic>
 #include <climits>
@@ -221,6 +224,11 @@ void RasterWorkspace::planPixels(DeviceSlab &slab, size_t pixels, int tx, int ty
     const int per = tileSize > pb ? tileSize / pb : 1;
     slab.add(blockOrder, size_t(std::max(1, tx * per * ty * per)));
     slab.add(blockStop, size_t(std::max(1, tx * per * ty * per)));
+    const size_t slots = icap / segmentOf(tileSize) + size_t(tx) * ty + 1;
+    slab.add(segments, slots * tileSize * tileSize);
+    slab.add(units, slots * per * per);
+    slab.add(blockMax, size_t(tx) * ty * (tileSize / 8) * (tileSize / 8));
+    slab.add(unitCount, 1);
 }
 
 void RasterWorkspace::bin(cudaStream_t stream, int iteration, const StepDesc *desc)
@@ -252,11 +260,11 @@ void RasterWorkspace::bin(cudaStream_t stream, int iteration, const StepDesc *de
 }
 
 void RasterWorkspace::forwardChecked(const Params &P, int count, const u3dg_camera &c, const u3dg_raster_settings &s,
-                                     const float *shRest, int shDegree, cudaStream_t stream)
+                                     const float *shRest, int shDegree, cudaStream_t stream, bool keep)
 {
     for (int attempt = 0; attempt < 8; ++attempt) {
         clearCounts(stream);
-        forward(P, count, c, s, shRest, shDegree, stream, 0);
+        forward(P, count, c, s, shRest, shDegree, stream, 0, keep);
         U3DG_CUDA(cudaMemcpyAsync(hostCounts.p, counts.p, sizeof(BinCounts), cudaMemcpyDeviceToHost, stream));
         U3DG_CUDA(cudaStreamSynchronize(stream));
         if (hostCounts.p->abortIter < 0)
@@ -290,13 +298,36 @@ RasterArgs RasterWorkspace::rasterArgs() const
     a.subStride = size_t(icap) * kPartial;
     a.blockOrder = blockOrder.p;
     a.counters = blockCounters.p;
+    a.segment = segmentOf(st.tile_size);
+    a.ck = segments.p;
+    a.blockMax = blockMax.p;
     a.forwardBlock = forwardBlock;
     a.forwardDepth = forwardDepth;
     a.backwardDepth = backwardDepth;
     return a;
 }
 
-void RasterWorkspace::composite(cudaStream_t stream)
+// Entries per segment: 64 for tiles of up to 16 pixels, and as many more for larger tiles as keep what a
+// segment holds (16 bytes per pixel of the tile) at 64 bytes per entry of intersection capacity, beside
+// the 48 of its partial. Backward us at 64 / 128 / 256 entries (tile 16; before segments): 4k Gaussians
+// at 96x72 51 / 78 / 115 (128), 80k at 320x240 62 / 91 / 146 (180), 150k at 480x360 99 / 103 / 147 (196),
+// 300k at 640x480 145 / 153 / 162 (243); the forward pays 2 to 12 us for keeping them.
+int RasterWorkspace::segmentOf(int tileSize)
+{
+    return tileSize <= 16 ? U3DG_SEG16 : tileSize * tileSize / 4;
+}
+
+void RasterWorkspace::reserveSegments()
+{
+    const int ts = st.tile_size, pb = ts <= 8 ? 8 : 16, per = ts > pb ? ts / pb : 1;
+    const size_t tiles = size_t(tilesX) * tilesY, slots = segmentSlots(tiles);
+    segments.reserve(slots * ts * ts);
+    units.reserve(slots * per * per);
+    blockMax.reserve(tiles * (ts / 8) * (ts / 8));
+    unitCount.reserve(1);
+}
+
+void RasterWorkspace::composite(cudaStream_t stream, bool keep)
 {
     const size_t P = size_t(cam.width) * cam.height;
     rgb.reserve(P * 3);
@@ -306,14 +337,19 @@ void RasterWorkspace::composite(cudaStream_t stream)
     const int per = st.tile_size > pb ? st.tile_size / pb : 1;
     blockOrder.reserve(size_t(std::max(1, tilesX * per * tilesY * per)));
     blockStop.reserve(size_t(std::max(1, tilesX * per * tilesY * per)));
-    const RasterArgs a = rasterArgs();
-    launchBlockOrder(a, blockOrder.p, stream);
+    if (keep)
+        reserveSegments();
+    RasterArgs a = rasterArgs();
+    if (!keep)
+        a.segment = 0;
     launchCompositeForward(a, rgb.p, finalT.p, nContrib.p, stream);
 }
 
 void RasterWorkspace::backwardComposite(const float *dLdRgb, cudaStream_t stream)
 {
-    launchCompositeBackward(rasterArgs(), dLdRgb, finalT.p, nContrib.p, partial.p, blockStop.p, stream);
+    const RasterArgs a = rasterArgs();
+    launchBackwardUnits(a, blockStop.p, units.p, unitCount.p, stream);
+    launchCompositeBackward(a, dLdRgb, finalT.p, nContrib.p, partial.p, blockStop.p, units.p, unitCount.p, stream);
 }
 
 ChainArgs RasterWorkspace::chainArgs(const Params &P) const
@@ -736,7 +772,7 @@ void TrainerImpl::launchStep(const StepValues &sv, const StepDesc *desc, BinCoun
     ws.bin(stream, sv.d.iteration, desc);
     if (tm)
         tm->mark(2, stream);
-    ws.composite(stream);
+    ws.composite(stream, true);
     if (tm)
         tm->mark(3, stream);
     // Loss (Trainer.cpp:67-71) and the step's stats (Trainer.cpp:88-92).

@@ -213,6 +213,9 @@ struct RasterWorkspace {
     // per tile / pixel
     DevBuf<int> tileOffsets, nContrib;
     DevBuf<int> blockStop; // per backward block: list position behind its last contributor
+    DevBuf<float4> segments;                      // RasterArgs::ck
+    DevBuf<int> blockMax, unitCount;
+    DevBuf<int2> units;                           // the backward's (block, segment) units
     DevBuf<int> blockOrder, blockCounters; // compositing schedule: pixel blocks by list length, counters
     DevBuf<float> rgb, finalT;
     // device-side sizes of the last pass and their pinned host copy
@@ -251,18 +254,24 @@ struct RasterWorkspace {
     // Depth sort + tile binning from depthKey / rect / radius. Never waits for the device: an overflow of
     // the intersection buffers is recorded in `counts` (tagged with `iteration`) and bins nothing.
     void bin(cudaStream_t stream, int iteration, const StepDesc *desc = nullptr);
-    void composite(cudaStream_t stream);
+    // keep: also what a backward needs (RasterArgs::segment).
+    void composite(cudaStream_t stream, bool keep);
+    // Entries per segment of a tile list, and the segment slots and units that the intersection capacity
+    // and tile count need.
+    static int segmentOf(int tileSize);
+    size_t segmentSlots(size_t tiles) const { return size_t(icap) / size_t(segmentOf(st.tile_size)) + tiles + 1; }
+    void reserveSegments();
     void forward(const Params &P, int count, const u3dg_camera &c, const u3dg_raster_settings &s, const float *shRest,
-                 int shDegree, cudaStream_t stream, int iteration)
+                 int shDegree, cudaStream_t stream, int iteration, bool keep)
     {
         project(P, count, c, s, shRest, shDegree, stream);
         bin(stream, iteration);
-        composite(stream);
+        composite(stream, keep);
     }
     // A forward that is complete when it returns: waits, and on an overflow grows the intersection
     // buffers and runs again. For the unit entry points and evaluation, not the training loop.
     void forwardChecked(const Params &P, int count, const u3dg_camera &c, const u3dg_raster_settings &s,
-                        const float *shRest, int shDegree, cudaStream_t stream);
+                        const float *shRest, int shDegree, cudaStream_t stream, bool keep = false);
     // Intersections binned by the last completed pass (valid after a wait).
     int total() const { return hostCounts.p->effTotal; }
     // Compositing backward into `partial`.

@@ -194,10 +194,19 @@ struct RasterArgs {
     int width, height, tileSize, tilesX;
     float bg[3];
     float minAlpha, minTransmittance;
-    // Persistent scheduling over the pixel blocks (PB x PB, PB = 8 for tile size 8, else 16).
+    // Pixel blocks of the compositing kernels (PB x PB, PB = 8 for tile size 8, else 16).
     int blocksX, blocksY;
-    const int *blockOrder; // pixel blocks, heaviest tile list first (launchBlockOrder)
-    int *counters;         // 4 ints, zero between launches: forward [0..1], backward [2..3]
+    int *blockOrder; // persistent forward: pixel blocks, heaviest tile list first
+    int *counters;   // 4 ints, zero between launches: forward [0..1], backward [2..3]
+    // What a forward keeps for the backward (segment > 0; 0: images only). A tile's list is cut every
+    // `segment` entries; for each segment but the first that a pixel reaches, ck holds the colour the
+    // pixel blends in it and its transmittance before it, so that the backward can replay every segment
+    // by itself. Slot tileOffsets[tile] / segment + tile + s holds segment s of a tile, a float4 per
+    // pixel (8x8 blocks row-major, pixels row-major within). blockMax: per 8x8 block, its pixels'
+    // largest contributor count.
+    int segment;
+    float4 *ck;
+    int *blockMax;
     int forwardBlock;      // pixel block edge of the forward kernel: 8 or 16 (tiles > 8 only; same results)
     int forwardDepth;      // list entries staged per thread per batch, forward: 1 or 2 (same results)
     int backwardDepth;     // the same for the backward kernel
@@ -207,15 +216,16 @@ struct RasterArgs {
     int subSlots;
     size_t subStride;
 };
-// Orders the pixel blocks by the list length of their tile, longest first (log-scale buckets), into
-// order[blocksX * blocksY].
-void launchBlockOrder(const RasterArgs &a, int *order, cudaStream_t s);
+// Work of the backward: (pixel block, segment) of every segment with a contributor into units,
+// their number into unitCount, and per pixel block the list position behind its last contributor into
+// stop.
+void launchBackwardUnits(const RasterArgs &a, int *stop, int2 *units, int *unitCount, cudaStream_t s);
 void launchCompositeForward(const RasterArgs &a, float *rgb, float *finalT, int *nContrib, cudaStream_t s);
-// partial: kPartial floats per list position, in a.subSlots slot arrays; stop: per pixel block, the list
-// position behind its pixels' last contributor. Partials from there on are not written: they are zero,
-// and ChainArgs' reader skips them.
+// partial: kPartial floats per list position, in a.subSlots slot arrays. Partials from a block's stop on
+// are not written: they are zero, and ChainArgs' reader skips them.
 void launchCompositeBackward(const RasterArgs &a, const float *dLdRgb, const float *finalT, const int *nContrib,
-                             float *partial, int *stop, cudaStream_t s);
+                             float *partial, const int *stop, const int2 *units, const int *unitCount,
+                             cudaStream_t s);
 
 // loss.cu
 struct LossScratch {

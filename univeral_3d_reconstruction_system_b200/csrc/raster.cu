@@ -24,7 +24,7 @@ namespace u3dg {
 
 namespace {
 
-template <int PB, int BD>
+template <int PB, int BD, bool kKeep>
 __device__ __forceinline__ void forwardBlock(const RasterArgs &a, int bx, int by, float *rgb, float *finalT,
                                              int *nContrib, float4 *sP, float4 *sQ, float4 *sR,
                                              uint32_t (*mask)[RasterShape<PB, BD>::NG])
@@ -43,13 +43,34 @@ __device__ __forceinline__ void forwardBlock(const RasterArgs &a, int bx, int by
     const float2 one = make_float2(1.0f, 1.0f);
     const float minA = a.minAlpha, minT = a.minTransmittance;
     const float4 *rec = reinterpret_cast<const float4 *>(a.rec);
-    for (int b0 = start; b0 < end; b0 += NB) {
+    // kKeep: the colour blended since the current segment began and the transmittance it began with,
+    // written when it ends (RasterArgs::ck).
+    float2 lr = cr, lg = cr, lb = cr, begin = one;
+    int segment = 0, segEnd = kKeep ? start + a.segment : end;
+    auto keepSegment = [&] {
+        if (segment == 0)
+            return;
+        float4 *slot = a.ck + (size_t(start / a.segment + tile + segment) * a.tileSize) * a.tileSize;
+        if (in0)
+            slot[slotPixel(a.tileSize, wb.px, wb.py0)] = make_float4(lr.x, lg.x, lb.x, begin.x);
+        if (in1)
+            slot[slotPixel(a.tileSize, wb.px, wb.py1)] = make_float4(lr.y, lg.y, lb.y, begin.y);
+    };
+    for (int b0 = start, bEnd; b0 < end; b0 = bEnd) {
         if (__syncthreads_count(done0 && done1) == NT)
             break;
+        if (kKeep && b0 == segEnd) {
+            keepSegment();
+            ++segment;
+            segEnd += a.segment;
+            lr = lg = lb = make_float2(0.0f, 0.0f);
+            begin = T;
+        }
+        bEnd = min(min(b0 + NB, segEnd), end);
 #pragma unroll
         for (int r = 0; r < BD; ++r) {
             const int slot = r * NT + tid;
-            stage<PB, BD>(rec, a.entries, b0 + slot, b0 + slot < end, slot, sP, sQ, sR, mask, bx, by);
+            stage<PB, NG>(rec, a.entries, b0 + slot, b0 + slot < bEnd, slot, sP, sQ, sR, mask, bx, by);
         }
         __syncthreads();
         for (int k = 0; k < NG && !(done0 && done1); ++k) {
@@ -95,6 +116,11 @@ __device__ __forceinline__ void forwardBlock(const RasterArgs &a, int bx, int by
                     cr = fma2rn(make_float2(R.x, R.x), w, cr);
                     cg = fma2rn(make_float2(R.y, R.y), w, cg);
                     cb = fma2rn(make_float2(R.z, R.z), w, cb);
+                    if (kKeep) {
+                        lr = fma2rn(make_float2(R.x, R.x), w, lr);
+                        lg = fma2rn(make_float2(R.y, R.y), w, lg);
+                        lb = fma2rn(make_float2(R.z, R.z), w, lb);
+                    }
                     const int idx = b0 - start + j + 1;
                     if (v0) {
                         T.x = nT.x;
@@ -109,6 +135,12 @@ __device__ __forceinline__ void forwardBlock(const RasterArgs &a, int bx, int by
                     break;
             }
         }
+    }
+    if (kKeep) {
+        keepSegment();
+        const int most = __reduce_max_sync(0xffffffffu, max(last0, last1));
+        if (lane == 0)
+            a.blockMax[(wb.py0 >> 3) * (a.tilesX * (a.tileSize >> 3)) + (wb.px >> 3)] = most;
     }
     const float T0 = T.x, T1 = T.y, r0 = cr.x, r1 = cr.y, g0 = cg.x, g1 = cg.y, b0c = cb.x, b1c = cb.y;
     if (in0) {
@@ -135,7 +167,7 @@ __device__ __forceinline__ void forwardBlock(const RasterArgs &a, int bx, int by
 #define U3DG_FWD_MIN_BLOCKS 10
 #endif
 
-template <int PB, int BD>
+template <int PB, int BD, bool kKeep>
 __global__ void __launch_bounds__(RasterShape<PB>::NT, U3DG_FWD_MIN_BLOCKS) compositeForwardKernel(RasterArgs a, float *rgb, float *finalT,
                                                                               int *nContrib)
 {
@@ -149,12 +181,15 @@ __global__ void __launch_bounds__(RasterShape<PB>::NT, U3DG_FWD_MIN_BLOCKS) comp
     __shared__ int sNext;
     const int units = a.blocksX * a.blocksY;
     if (a.counters == nullptr) { // one CTA per pixel block (every block resident in one wave)
-        forwardBlock<PB, BD>(a, int(blockIdx.x) % a.blocksX, int(blockIdx.x) / a.blocksX, rgb, finalT, nContrib, sP,
+        forwardBlock<PB, BD, kKeep>(a, int(blockIdx.x) % a.blocksX, int(blockIdx.x) / a.blocksX, rgb, finalT, nContrib, sP,
                              sQ, sR, mask);
         return;
     }
-    for (int b = nextBlock(a, a.counters, &sNext); b < units; b = nextBlock(a, a.counters, &sNext))
-        forwardBlock<PB, BD>(a, b % a.blocksX, b / a.blocksX, rgb, finalT, nContrib, sP, sQ, sR, mask);
+    // Heaviest tile lists first (a.blockOrder), so that the long lists start early.
+    for (int u = nextUnit(units, a.counters, &sNext); u < units; u = nextUnit(units, a.counters, &sNext)) {
+        const int b = a.blockOrder[u];
+        forwardBlock<PB, BD, kKeep>(a, b % a.blocksX, b / a.blocksX, rgb, finalT, nContrib, sP, sQ, sR, mask);
+    }
 }
 
 // One CTA: the pixel blocks bucketed by the list length of their tile on a log scale (four buckets
@@ -228,51 +263,63 @@ int residentCtas(K kernel, int threads, size_t smem)
 
 } // namespace
 
-void launchBlockOrder(const RasterArgs &a, int *order, cudaStream_t s)
+// Orders the pixel blocks by the list length of their tile, longest first, into a.blockOrder.
+static void launchBlockOrder(const RasterArgs &a, cudaStream_t s)
 {
-    const int units = a.blocksX * a.blocksY;
-    if (units <= 0)
-        return;
     const int pb = a.tileSize <= 8 ? 8 : 16;
-    { launchPdl(blockOrderKernel, 1, 1024, 0, s, a.tileOffsets, a.blocksX, a.blocksY, pb, a.tileSize, a.tilesX, order); countLaunch(); }
+    { launchPdl(blockOrderKernel, 1, 1024, 0, s, a.tileOffsets, a.blocksX, a.blocksY, pb, a.tileSize, a.tilesX, a.blockOrder); countLaunch(); }
 }
 
-template <int PB, int BD>
+template <int PB, int BD, bool kKeep>
 static void launchForward(const RasterArgs &a, float *rgb, float *finalT, int *nContrib, cudaStream_t s)
 {
     // When every pixel block fits on the GPU at once, one CTA per block in natural order (no work
     // counter); otherwise the persistent schedule on counters[0..1].
     const int units = a.blocksX * a.blocksY;
-    static const int ctas = residentCtas(compositeForwardKernel<PB, BD>, RasterShape<PB>::NT, 0);
+    static const int ctas = residentCtas(compositeForwardKernel<PB, BD, kKeep>, RasterShape<PB>::NT, 0);
     RasterArgs f = a;
     if (units <= ctas)
         f.counters = nullptr;
-    { launchPdl(compositeForwardKernel<PB, BD>, std::min(units, ctas), RasterShape<PB>::NT, 0, s, f, rgb, finalT, nContrib); countLaunch(); }
+    else
+        launchBlockOrder(a, s);
+    { launchPdl(compositeForwardKernel<PB, BD, kKeep>, std::min(units, ctas), RasterShape<PB>::NT, 0, s, f, rgb, finalT, nContrib); countLaunch(); }
 }
 
 // 8x8 CTAs over the lists of larger tiles: one CTA per pixel block in natural order, as many waves as
-// it takes (the blocks are short; the persistent order is computed for the backward's blocks).
-template <int BD>
+// it takes (the blocks are short).
+template <int BD, bool kKeep>
 static void launchForwardSplit(const RasterArgs &a, float *rgb, float *finalT, int *nContrib, cudaStream_t s)
 {
     RasterArgs f = a;
     f.blocksX = (a.width + 7) / 8;
     f.blocksY = (a.height + 7) / 8;
     f.counters = nullptr;
-    { launchPdl(compositeForwardKernel<8, BD>, f.blocksX * f.blocksY, RasterShape<8>::NT, 0, s, f, rgb, finalT, nContrib); countLaunch(); }
+    { launchPdl(compositeForwardKernel<8, BD, kKeep>, f.blocksX * f.blocksY, RasterShape<8>::NT, 0, s, f, rgb, finalT, nContrib); countLaunch(); }
+}
+
+template <bool kKeep>
+static void launchForwardAny(const RasterArgs &a, float *rgb, float *finalT, int *nContrib, cudaStream_t s)
+{
+    const bool deep = a.forwardDepth >= 2;
+    if (a.tileSize > 8 && a.forwardBlock == 8)
+        deep ? launchForwardSplit<2, kKeep>(a, rgb, finalT, nContrib, s)
+             : launchForwardSplit<1, kKeep>(a, rgb, finalT, nContrib, s);
+    else if (a.tileSize <= 8)
+        deep ? launchForward<8, 2, kKeep>(a, rgb, finalT, nContrib, s)
+             : launchForward<8, 1, kKeep>(a, rgb, finalT, nContrib, s);
+    else
+        deep ? launchForward<16, 2, kKeep>(a, rgb, finalT, nContrib, s)
+             : launchForward<16, 1, kKeep>(a, rgb, finalT, nContrib, s);
 }
 
 void launchCompositeForward(const RasterArgs &a, float *rgb, float *finalT, int *nContrib, cudaStream_t s)
 {
     if (a.blocksX * a.blocksY <= 0)
         return;
-    const bool deep = a.forwardDepth >= 2;
-    if (a.tileSize > 8 && a.forwardBlock == 8)
-        deep ? launchForwardSplit<2>(a, rgb, finalT, nContrib, s) : launchForwardSplit<1>(a, rgb, finalT, nContrib, s);
-    else if (a.tileSize <= 8)
-        deep ? launchForward<8, 2>(a, rgb, finalT, nContrib, s) : launchForward<8, 1>(a, rgb, finalT, nContrib, s);
+    if (a.segment > 0)
+        launchForwardAny<true>(a, rgb, finalT, nContrib, s);
     else
-        deep ? launchForward<16, 2>(a, rgb, finalT, nContrib, s) : launchForward<16, 1>(a, rgb, finalT, nContrib, s);
+        launchForwardAny<false>(a, rgb, finalT, nContrib, s);
 }
 
 } // namespace u3dg

@@ -82,15 +82,12 @@ __device__ __forceinline__ int tileOf(const RasterArgs &a, int bx, int by)
     return (by * PB / a.tileSize) * a.tilesX + bx * PB / a.tileSize;
 }
 
-// Persistent scheduling: every CTA takes pixel blocks from a device counter until none are left,
-// heaviest tile lists first (a.blockOrder), so the long lists start early and no CTA waits for a
-// second wave. Returns the next block index for the whole CTA (>= a.blocksX * a.blocksY: done); the
-// last CTA to run out resets the counter for the next launch. counter[0] hands out blocks, counter[1]
-// counts finished CTAs.
-__device__ __forceinline__ int nextBlock(const RasterArgs &a, int *counter, int *sNext)
+// Persistent scheduling: every CTA takes work units from a device counter until none are left. Returns
+// the next unit's index for the whole CTA (>= units: done); the last CTA to run out resets the counter
+// for the next launch. counter[0] hands out units, counter[1] counts finished CTAs.
+__device__ __forceinline__ int nextUnit(int units, int *counter, int *sNext)
 {
-    const int units = a.blocksX * a.blocksY;
-    __syncthreads(); // every thread is done with the previous block's shared memory
+    __syncthreads(); // every thread is done with the previous unit's shared memory
     if (threadIdx.x == 0) {
         int u = atomicAdd(counter, 1);
         if (u >= units) {
@@ -103,17 +100,23 @@ __device__ __forceinline__ int nextBlock(const RasterArgs &a, int *counter, int 
         *sNext = u;
     }
     __syncthreads();
-    const int u = *sNext;
-    return u < units ? a.blockOrder[u] : units;
+    return *sNext;
 }
 
-// Stages batch entry `slot` (if valid) and the masks: mask[w][g] bit b <=> entry 32g + b meets warp w.
-template <int PB, int BD>
-__device__ __forceinline__ void stage(const float4 *rec, const int *entries, int idx, bool valid, int slot, float4 *sP,
-                                      float4 *sQ, float4 *sR, uint32_t (*mask)[RasterShape<PB, BD>::NG], int bx,
-                                      int by)
+// Index of a pixel in its tile's segment slot (RasterArgs::ck).
+__device__ __forceinline__ int slotPixel(int tileSize, int px, int py)
 {
-    constexpr int NW = RasterShape<PB, BD>::NW, WX = RasterShape<PB, BD>::WX;
+    const int x = px % tileSize, y = py % tileSize;
+    return ((y >> 3) * (tileSize >> 3) + (x >> 3)) * 64 + (y & 7) * 8 + (x & 7);
+}
+
+// Stages batch entry `slot` (if valid) and the masks of NG words: mask[w][g] bit b <=> entry 32g + b meets
+// 8x8 block w (slots are a warp's lanes in order).
+template <int PB, int NG>
+__device__ __forceinline__ void stage(const float4 *rec, const int *entries, int idx, bool valid, int slot, float4 *sP,
+                                      float4 *sQ, float4 *sR, uint32_t (*mask)[NG], int bx, int by)
+{
+    constexpr int NW = RasterShape<PB>::NW, WX = RasterShape<PB>::WX;
     float4 p = make_float4(0.0f, 0.0f, -1.0f, -1.0f), q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float powMin = 0.0f, iA = 0.0f, iC = 0.0f;
     if (valid) {
