@@ -227,17 +227,17 @@ int u3dg_trainer_time_steps(u3dg_trainer *trainer, int count, float *ms);
  * graph launches ran so far. */
 int u3dg_trainer_set_graphs(u3dg_trainer *trainer, int enable);
 int u3dg_trainer_graph_launches(u3dg_trainer *trainer, long long *launches);
-/* No reference counterpart. Compositing schedule: forward_block is the pixel block edge of the
- * forward kernel for tiles of 16 and 32 pixels, 8 (default: several 8x8 CTAs walk each tile list) or
- * 16; forward_depth and backward_depth are the list entries each thread of the forward and of the
+/* No reference counterpart. Compositing schedule: backward_depth is the list entries each thread of the
  * backward kernel stages per shared-memory batch, 1 (default) or 2 (deeper batches halve the block
- * barriers per Gaussian at the cost of shared memory). The rendered images, gradients and trained
- * models are bit-identical for every setting. */
+ * barriers per Gaussian at the cost of shared memory; no effect at tile size 16). forward_block (8 or
+ * 16) and forward_depth (1 or 2) have no effect: the forward kernel picks its own from the image size.
+ * The rendered images, gradients and trained models are bit-identical for every setting. */
 int u3dg_trainer_set_raster_schedule(u3dg_trainer *trainer, int forward_block, int forward_depth,
                                      int backward_depth);
 /* No reference counterpart. Tile culling (on by default): a Gaussian is listed only in the tiles of
  * its rectangle that its contributing ellipse (alpha >= min_alpha) can reach, with a conservative
- * margin; the trained models are bit-identical with it on (1) or off (0). */
+ * margin; images and per-entry gradients are the same with it on (1) or off (0), and the trained models
+ * agree to rounding (the segments in which a list is replayed begin at other entries). */
 int u3dg_trainer_set_tile_culling(u3dg_trainer *trainer, int enable);
 void u3dg_trainer_destroy(u3dg_trainer *trainer);
 

@@ -116,3 +116,31 @@ def test_a_non_finite_colour_reaches_only_the_pixels_it_covers(u3dg, background)
     whole = r.backward(m, w)
     untouched = [i for i in range(m.size()) if np.array_equal(masked.opacities[i], whole.opacities[i])]
     assert untouched and set(untouched) - {7} <= set(same)
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 63, 64, 65, 129, 700])
+@pytest.mark.parametrize("opacity", [0.008, 0.6])
+def test_forward_kernels_agree_and_match_the_oracle(u3dg, oracle, n, opacity):
+    # The left 256 columns of a 512x272 image (2,176 blocks of 8x8: one warp per block) and the same columns
+    # as an image of their own (1,088 blocks: a team per block), with everything left of the optical axis
+    # so that both project alike: the same bits, at lists around the batch sizes, ended by the cut-off or
+    # not; and within 1e-5 of the oracle.
+    rng = np.random.default_rng(n)
+    m = _stack(n, rng, opacity)
+    m.means[:, 0] = rng.uniform(-1.1, -0.35, n) * m.means[:, 2] * 0.5
+    m.means[:, 1] = rng.uniform(-0.3, 0.3, n)
+    m.scales -= 2.0
+    wide = make_camera(512, 272, 480.0)
+    left = make_camera(512, 272, 480.0)
+    left.width = 256
+    out = []
+    for cam in (wide, left):
+        r = u3dg.Rasterizer()
+        image = r.forward(m, cam, RasterSettings(background=(0.1, 0.2, 0.3)))
+        ft, nc = r.pixel_state()
+        out.append([x.reshape(272, cam.width, -1)[:, :256] for x in (image, ft, nc)])
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+    assert out[0][2].max() > 0
+    ref = oracle.render(m, left, RasterSettings(background=(0.1, 0.2, 0.3)))
+    assert np.max(np.abs(out[1][0] - ref)) <= 1e-5

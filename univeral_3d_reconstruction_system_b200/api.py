@@ -159,13 +159,13 @@ class Trainer:
         return int(v.value)
 
     def set_raster_schedule(self, forward_block: int = 8, forward_depth: int = 1, backward_depth: int = 1) -> None:
-        """Compositing schedule (identical results for every setting): the forward kernel's pixel block
-        edge for tiles of 16 and 32 pixels (8 or 16) and the list entries each forward / backward
-        thread stages per shared-memory batch (1 or 2)."""
+        """Compositing schedule (identical results for every setting): the list entries each backward
+        thread stages per shared-memory batch (1 or 2). The forward's settings (8 or 16, 1 or 2) have
+        no effect: its kernel is picked from the image size."""
         check(load().u3dg_trainer_set_raster_schedule(self._h, forward_block, forward_depth, backward_depth))
 
     def set_tile_culling(self, enable: bool) -> None:
-        """List Gaussians only in tiles their contributing ellipse reaches (default on; same models)."""
+        """List Gaussians only in tiles their contributing ellipse reaches (default on; models agree to rounding)."""
         check(load().u3dg_trainer_set_tile_culling(self._h, 1 if enable else 0))
 
     def set_profiling(self, enable: bool) -> None:

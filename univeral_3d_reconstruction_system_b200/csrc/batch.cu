@@ -72,8 +72,6 @@ int u3dg_batch_create(const u3dg_model *initial, const u3dg_image *const *images
             o.raster.tile_size = rs.tileSize;
             auto t = std::make_unique<u3dg_trainer>();
             t->impl = std::make_unique<TrainerImpl>(initial[s], images[s], image_counts[s], extents[s], o);
-            t->impl->ws.forwardBlock = rs.forwardBlock;
-            t->impl->ws.forwardDepth = rs.forwardDepth;
             t->impl->ws.backwardDepth = rs.backwardDepth;
             t->ownedByBatch = true;
             b->schedules.push_back(rs);

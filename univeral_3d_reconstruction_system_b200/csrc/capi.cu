@@ -416,8 +416,6 @@ int u3dg_trainer_set_raster_schedule(u3dg_trainer *trainer, int forward_block, i
             if (d != 1 && d != 2)
                 throw StatusError(U3DG_ERR_INVALID_ARG, "batch depth must be 1 or 2");
         t.finish();
-        t.ws.forwardBlock = forward_block;
-        t.ws.forwardDepth = forward_depth;
         t.ws.backwardDepth = backward_depth;
         t.resetGraphs(); // its kernels were recorded for the other depth
     });

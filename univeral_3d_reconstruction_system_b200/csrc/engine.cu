@@ -19,9 +19,6 @@
 
 #include "engine.h"
 
-#ifndef U3DG_SEG16
-#define U3DG_SEG16 64
-#endif
 #include <algorithm>
 #include <atomic>
 #include <climits>
@@ -103,9 +100,9 @@ RasterWorkspace::RasterWorkspace()
     c.abortIter = -1;
     *hostCounts.p = c;
     U3DG_CUDA(cudaMemcpy(counts.p, &c, sizeof(c), cudaMemcpyHostToDevice));
-    // The compositing kernels' block counters start at zero and are reset by each launch's last CTA.
-    blockCounters.reserve(4, true);
-    U3DG_CUDA(cudaMemset(blockCounters.p, 0, 4 * sizeof(int)));
+    // The backward's unit counters start at zero and are reset by each launch's last CTA.
+    unitCounters.reserve(2, true);
+    U3DG_CUDA(cudaMemset(unitCounters.p, 0, 2 * sizeof(int)));
 }
 
 void RasterWorkspace::clearCounts(cudaStream_t stream)
@@ -222,7 +219,6 @@ void RasterWorkspace::planPixels(DeviceSlab &slab, size_t pixels, int tx, int ty
     slab.add(rowTotals, size_t(radixDigits()));
     const int pb = tileSize <= 8 ? 8 : 16;
     const int per = tileSize > pb ? tileSize / pb : 1;
-    slab.add(blockOrder, size_t(std::max(1, tx * per * ty * per)));
     slab.add(blockStop, size_t(std::max(1, tx * per * ty * per)));
     const size_t slots = icap / segmentOf(tileSize) + size_t(tx) * ty + 1;
     slab.add(segments, slots * tileSize * tileSize);
@@ -296,13 +292,10 @@ RasterArgs RasterWorkspace::rasterArgs() const
     a.blocksY = tilesY * per;
     a.subSlots = per * per;
     a.subStride = size_t(icap) * kPartial;
-    a.blockOrder = blockOrder.p;
-    a.counters = blockCounters.p;
+    a.counters = unitCounters.p;
     a.segment = segmentOf(st.tile_size);
     a.ck = segments.p;
     a.blockMax = blockMax.p;
-    a.forwardBlock = forwardBlock;
-    a.forwardDepth = forwardDepth;
     a.backwardDepth = backwardDepth;
     return a;
 }
@@ -314,7 +307,7 @@ RasterArgs RasterWorkspace::rasterArgs() const
 // 300k at 640x480 145 / 153 / 162 (243); the forward pays 2 to 12 us for keeping them.
 int RasterWorkspace::segmentOf(int tileSize)
 {
-    return tileSize <= 16 ? U3DG_SEG16 : tileSize * tileSize / 4;
+    return tileSize <= 16 ? 64 : tileSize * tileSize / 4;
 }
 
 void RasterWorkspace::reserveSegments()
@@ -335,7 +328,6 @@ void RasterWorkspace::composite(cudaStream_t stream, bool keep)
     nContrib.reserve(P);
     const int pb = st.tile_size <= 8 ? 8 : 16;
     const int per = st.tile_size > pb ? st.tile_size / pb : 1;
-    blockOrder.reserve(size_t(std::max(1, tilesX * per * tilesY * per)));
     blockStop.reserve(size_t(std::max(1, tilesX * per * tilesY * per)));
     if (keep)
         reserveSegments();
@@ -1229,19 +1221,16 @@ RasterSchedule autotuneSchedule(const u3dg_model &initial, const u3dg_image *img
     static const int kTiles[3] = {16, 8, 32};
     RasterSchedule best{opt.raster.tile_size, 8, 1, 1, 0.0f};
     for (int tile : kTiles) {
-        // Two runs per tile: forward 16x16 blocks at depth 1 with the backward at depth 1, and forward
-        // 8x8 blocks at depth 2 with the backward at depth 2 (tile 8: both forwards use 8x8 blocks, at
-        // depth 1 and 2). Each times graph runs of whole steps, then profiled steps for the compositing
-        // kernels' own times; the forward and backward settings are picked independently (the kernels
-        // do not interact) and the tile's step time is the first run's corrected by their gains.
-        float stepMs[2] = {}, fwdMs[2] = {}, bwdMs[2] = {};
+        // Two runs per tile, the backward at depth 1 and 2. Each times graph runs of whole steps, then
+        // profiled steps for the backward's own time; the tile's step time is the first run's corrected by
+        // the gain.
+        float stepMs[2] = {}, bwdMs[2] = {};
         for (int d = 0; d < 2; ++d) {
             u3dg_train_options o = opt;
             o.raster.tile_size = tile;
             o.iterations = std::max(o.iterations, 64);
             TrainerImpl t(initial, imgs, count, extent, o);
-            t.ws.forwardBlock = d == 0 ? 16 : 8;
-            t.ws.forwardDepth = t.ws.backwardDepth = d + 1;
+            t.ws.backwardDepth = d + 1;
             t.stepTo(3 + TrainerImpl::kGraphSteps); // warm-up, including the first graph capture
             t.finish();
             cudaEvent_t e0, e1;
@@ -1261,13 +1250,12 @@ RasterSchedule autotuneSchedule(const u3dg_model &initial, const u3dg_image *img
             t.stepTo(t.iteration + TrainerImpl::kGraphSteps);
             t.sync();
             const u3dg_phase_times &acc = t.timer->acc;
-            fwdMs[d] = acc.steps ? acc.forward_ms / float(acc.steps) : 0.0f;
             bwdMs[d] = acc.steps ? acc.backward_ms / float(acc.steps) : 0.0f;
         }
-        const int f = fwdMs[1] < fwdMs[0] ? 1 : 0, b = bwdMs[1] < bwdMs[0] ? 1 : 0;
-        const float ms = stepMs[0] - (fwdMs[0] - fwdMs[f]) - (bwdMs[0] - bwdMs[b]);
+        const int b = bwdMs[1] < bwdMs[0] ? 1 : 0;
+        const float ms = stepMs[0] - (bwdMs[0] - bwdMs[b]);
         if (best.msPerStep == 0.0f || ms < best.msPerStep)
-            best = RasterSchedule{tile, f == 0 && tile > 8 ? 16 : 8, f + 1, b + 1, ms};
+            best = RasterSchedule{tile, 8, 1, b + 1, ms};
     }
     return best;
 }

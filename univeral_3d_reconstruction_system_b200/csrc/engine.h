@@ -216,17 +216,16 @@ struct RasterWorkspace {
     DevBuf<float4> segments;                      // RasterArgs::ck
     DevBuf<int> blockMax, unitCount;
     DevBuf<int2> units;                           // the backward's (block, segment) units
-    DevBuf<int> blockOrder, blockCounters; // compositing schedule: pixel blocks by list length, counters
+    DevBuf<int> unitCounters; // RasterArgs::counters
     DevBuf<float> rgb, finalT;
     // device-side sizes of the last pass and their pinned host copy
     DevBuf<BinCounts> counts;
     HostPinned<BinCounts> hostCounts;
 
     int n = 0, tilesX = 0, tilesY = 0;
-    // Compositing schedule (none changes a result): the forward kernel's pixel block edge (8 or 16,
-    // for tiles of 16 and 32 pixels) and the list entries each compositing thread stages per
-    // shared-memory batch (1 or 2).
-    int forwardBlock = 8, forwardDepth = 1, backwardDepth = 1;
+    // List entries each thread of the compositing backward stages per shared-memory batch (1 or 2; no
+    // effect on a result).
+    int backwardDepth = 1;
     // Tile culling: list a Gaussian only in the tiles of its rectangle that its contributing ellipse
     // can reach (trainers; the rasterizer unit boundary keeps the reference's lists).
     bool cullTiles = false;
@@ -565,10 +564,9 @@ struct BatchGraph {
 // graph holding all of their chunks (bg, may be null: no combined graph).
 void stepBatch(const std::vector<TrainerImpl *> &trainers, int count, BatchGraph *bg = nullptr);
 
-// Tile size (8 or 16: the sizes whose results are deterministic), forward pixel block (8 or 16) and
-// compositing batch depths (1 or 2 staged list entries per thread per batch, for the forward and the
-// backward kernel) with the shortest step time for a scene, timed on throwaway trainers started from
-// the same model.
+// Tile size (8, 16 or 32) and batch depth of the compositing backward (1 or 2) with the shortest step time
+// for a scene, timed on throwaway trainers started from the same model; the forward's block and depth
+// are always 8 and 1.
 struct RasterSchedule {
     int tileSize, forwardBlock, forwardDepth, backwardDepth;
     float msPerStep;

@@ -194,10 +194,9 @@ struct RasterArgs {
     int width, height, tileSize, tilesX;
     float bg[3];
     float minAlpha, minTransmittance;
-    // Pixel blocks of the compositing kernels (PB x PB, PB = 8 for tile size 8, else 16).
+    // Pixel blocks of the backward (PB x PB, PB = 8 for tile size 8, else 16).
     int blocksX, blocksY;
-    int *blockOrder; // persistent forward: pixel blocks, heaviest tile list first
-    int *counters;   // 4 ints, zero between launches: forward [0..1], backward [2..3]
+    int *counters; // 2 ints, zero between launches: the backward's units handed out, CTAs done
     // What a forward keeps for the backward (segment > 0; 0: images only). A tile's list is cut every
     // `segment` entries; for each segment but the first that a pixel reaches, ck holds the colour the
     // pixel blends in it and its transmittance before it, so that the backward can replay every segment
@@ -207,9 +206,7 @@ struct RasterArgs {
     int segment;
     float4 *ck;
     int *blockMax;
-    int forwardBlock;      // pixel block edge of the forward kernel: 8 or 16 (tiles > 8 only; same results)
-    int forwardDepth;      // list entries staged per thread per batch, forward: 1 or 2 (same results)
-    int backwardDepth;     // the same for the backward kernel
+    int backwardDepth;     // list entries staged per thread per batch, backward: 1 or 2 (same results)
     // Tiles larger than the backward's 16x16 pixel block are covered by several CTAs: each writes its
     // sums into its own slot array (slot = the block's position in its tile, row-major), subSlots
     // arrays of subStride floats apart, and the chain rule adds a Gaussian's slots in slot order.

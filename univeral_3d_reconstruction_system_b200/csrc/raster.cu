@@ -1,325 +1,427 @@
 // raster.cu - tile compositing forward (Rasterizer::forward, Rasterizer.cpp:281-329).
 //
-// Layout and staging in raster_common.cuh: a CTA per 16x16 or 8x8 pixel block, two pixels per thread,
-// 8x8 pixels per warp, batches of one or two list entries per thread staged in shared memory with
-// per-warp masks of the entries whose contributing box meets the warp's block. A tile of 16 or 32
-// pixels may be covered by several 8x8 CTAs that each walk the whole tile list (RasterArgs::
-// forwardBlock): more, shorter CTAs keep the SMs busy while the heaviest tiles finish. Each warp walks its set bits in list
-// order and blends both of its pixels' columns, front to back, with the reference's cut-offs
-// (alpha <= 0.99, skip alpha < minAlpha, stop when T (1 - alpha) < minTransmittance). A CTA stops when
-// every pixel has terminated (__syncthreads_count). Skipped entries are exactly those the reference
-// skips for these pixels, so the output is unchanged.
+// The unit of work is an 8x8 pixel block, two pixels per lane of a warp, walking the depth-sorted list of
+// the tile it lies in (all blocks of a larger tile walk the same list). Entries are staged in shared memory
+// in batches with a mask of those whose contributing box and ellipse meet the block (raster_common.cuh),
+// so only the set bits are walked, front to back, with the reference's cut-offs (alpha <= 0.99, skip
+// alpha < minAlpha, stop when T (1 - alpha) < minTransmittance). Skipped entries are exactly those the
+// reference skips for these pixels, so the output is unchanged.
+//
+// What an entry adds to a pixel needs its alpha, which is the same whatever lies before it, and the
+// transmittance, which is one product after the other. Evaluated one entry at a time, an entry cost a
+// warp's lane 320 cycles from loads over the exponential to the cut-off, and a launch lasted as long as its
+// longest list took one warp (a block's last pixel terminates after about 150 entries on average, in an
+// image's longest after 1,000 to 1,500; part-trained 300k model at 640x480: SMs idle 64 % of the time).
+// Here the alphas of several entries are evaluated together and the path from entry to entry is the one
+// product (Blend::entry). Two kernels with the same arithmetic and so the same bits:
+//   compositeForwardKernel      one warp per block, four entries at a time: 190 cycles per entry
+//   compositeForwardTeamKernel  four warps per block evaluate for one that blends: 70 cycles per entry, but
+//                               up to a batch of entries evaluated in vain at the end of every block
+// The second where blocks are too few to fill the GPU: us per launch one warp / team / before at 96x72
+// pixels 46 / 27 / 71, 320x240 (1,200 blocks) 65 / 57 / 96, 480x360 (2,700) 76 / 84 / 102, 640x480 106 / 130 /
+// 134.
 //
 // Compiled with -fmad=false: the contribution decisions (power, alpha, the transmittance cut-off) and
 // the transmittance round exactly like the reference's, so the same entries contribute. The colour
 // sums alone use explicit fused multiply-adds (within 1e-7 of the unfused sums; images are compared
-// within 1e-5). A thread's two pixels are blended together in sm_100's paired FP32 instructions
+// within 1e-5). A lane's two pixels are blended together in sm_100's paired FP32 instructions
 // (add2rn / mul2rn / fma2rn, raster_common.cuh), which round each lane like the scalar operation.
 
 #include "raster_common.cuh"
 
-#include <algorithm>
+#include <cstdint>
 
 namespace u3dg {
 
 namespace {
 
-template <int PB, int BD, bool kKeep>
-__device__ __forceinline__ void forwardBlock(const RasterArgs &a, int bx, int by, float *rgb, float *finalT,
-                                             int *nContrib, float4 *sP, float4 *sQ, float4 *sR,
-                                             uint32_t (*mask)[RasterShape<PB, BD>::NG])
+// The alphas of one entry at a lane's two pixels (column fx, rows -nfy): the falloff exponent in powerAt's
+// order (products paired, sums scalar; -0.5 q is exact, so one fused step rounds like the two). Reaches a
+// pixel if the exponent is in range; its exponential is only needed then.
+struct EntryPower {
+    float2 pw;
+    float alpha;
+    bool v0, v1;
+};
+
+__device__ __forceinline__ EntryPower entryPower(const float4 &P, const float4 &Q, float fx, float2 nfy, bool on0, bool on1)
 {
-    using S = RasterShape<PB, BD>;
-    constexpr int NT = S::NT, NB = S::NB, NG = S::NG;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const WarpBlock<PB> wb(warp, lane, bx, by);
-    const int tile = tileOf<PB>(a, bx, by);
-    const int start = a.tileOffsets[tile], end = a.tileOffsets[tile + 1];
-    const bool in0 = wb.px < a.width && wb.py0 < a.height, in1 = wb.px < a.width && wb.py1 < a.height;
-    bool done0 = !in0, done1 = !in1;
-    float2 T = make_float2(1.0f, 1.0f), cr = make_float2(0.0f, 0.0f), cg = cr, cb = cr;
-    int last0 = 0, last1 = 0;
-    const float fx = float(wb.px), fy0 = float(wb.py0), fy1 = float(wb.py1);
-    const float2 one = make_float2(1.0f, 1.0f);
-    const float minA = a.minAlpha, minT = a.minTransmittance;
-    const float4 *rec = reinterpret_cast<const float4 *>(a.rec);
+    const ColumnTerms ct = columnTerms(Q, __fsub_rn(P.x, fx));
+    const float2 dy = add2rn(both(P.y), nfy);
+    const float2 cdd = mul2rn(mul2rn(both(Q.z), dy), dy);
+    const float2 q = make_float2(__fadd_rn(ct.axx, cdd.x), __fadd_rn(ct.axx, cdd.y));
+    EntryPower e;
+    e.pw = fma2rn(both(-0.5f), q, mul2rn(both(-ct.bx), dy));
+    e.alpha = Q.w;
+    e.v0 = on0 && !(e.pw.x > 0.0f || e.pw.x < P.z);
+    e.v1 = on1 && !(e.pw.y > 0.0f || e.pw.y < P.z);
+    return e;
+}
+
+// Negative zero where the entry is not blended.
+__device__ __forceinline__ float2 entryAlpha(const EntryPower &e, float minA)
+{
+    const float2 raw = mul2rn(both(e.alpha), make_float2(rasterExp(e.pw.x), rasterExp(e.pw.y)));
+    const float a0 = (raw.x < kMaxAlpha) ? raw.x : kMaxAlpha;
+    const float a1 = (raw.y < kMaxAlpha) ? raw.y : kMaxAlpha;
+    return make_float2(e.v0 && !(a0 < minA) ? a0 : -0.0f, e.v1 && !(a1 < minA) ? a1 : -0.0f);
+}
+
+// A lane's two pixels while their list is blended, front to back (Rasterizer.cpp:305-318), in paired FP32
+// instructions where each lane rounds like the scalar operation. T is the running product of 1 - alpha,
+// not stopped at the cut-off: it never grows, so a pixel is live exactly while T is at least the minimum,
+// and the path from entry to entry is one multiplication. Tf is T before the entry that fell below it.
+template <bool kKeep>
+struct Blend {
+    float2 T, Tf, cr, cg, cb;
     // kKeep: the colour blended since the current segment began and the transmittance it began with,
     // written when it ends (RasterArgs::ck).
-    float2 lr = cr, lg = cr, lb = cr, begin = one;
-    int segment = 0, segEnd = kKeep ? start + a.segment : end;
-    auto keepSegment = [&] {
+    float2 lr, lg, lb, begin;
+    int last0, last1, segment, left;
+
+    __device__ __forceinline__ Blend(bool in0, bool in1, int segmentSize)
+    {
+        T = make_float2(in0 ? 1.0f : -1.0f, in1 ? 1.0f : -1.0f); // outside the image: never live
+        Tf = begin = both(1.0f);
+        cr = cg = cb = lr = lg = lb = both(0.0f);
+        last0 = last1 = segment = 0;
+        left = segmentSize;
+    }
+    // al: the entry's alphas (negative zero: not blended), idx its list position + 1. kStrict: R may hold a
+    // non-finite colour, which must reach only the pixels it blends into (0 * inf is not 0): the colour is
+    // taken as 0 where a pixel's weight is.
+    template <bool kStrict>
+    __device__ __forceinline__ void entry(const float2 &al, const float4 &R, int idx, float minT)
+    {
+        const float2 nT = mul2rn(T, fma2rn(al, both(-1.0f), both(1.0f)));
+        const bool on0 = nT.x >= minT, on1 = nT.y >= minT;
+        float2 w = mul2rn(al, T);
+        w.x = on0 ? w.x : 0.0f;
+        w.y = on1 ? w.y : 0.0f;
+        T = nT;
+        Tf.x = on0 ? nT.x : Tf.x;
+        Tf.y = on1 ? nT.y : Tf.y;
+        float2 r = both(R.x), g = both(R.y), b = both(R.z);
+        if (kStrict) {
+            const bool s0 = w.x != 0.0f, s1 = w.y != 0.0f;
+            r = make_float2(s0 ? r.x : 0.0f, s1 ? r.y : 0.0f);
+            g = make_float2(s0 ? g.x : 0.0f, s1 ? g.y : 0.0f);
+            b = make_float2(s0 ? b.x : 0.0f, s1 ? b.y : 0.0f);
+        }
+        cr = fma2rn(r, w, cr);
+        cg = fma2rn(g, w, cg);
+        cb = fma2rn(b, w, cb);
+        if (kKeep) {
+            lr = fma2rn(r, w, lr);
+            lg = fma2rn(g, w, lg);
+            lb = fma2rn(b, w, lb);
+        }
+        last0 = on0 && __float_as_int(al.x) >= 0 ? idx : last0;
+        last1 = on1 && __float_as_int(al.y) >= 0 ? idx : last1;
+    }
+    __device__ __forceinline__ void keepSegment(const RasterArgs &a, int slot0, int px, int py0, bool in0, bool in1) const
+    {
         if (segment == 0)
             return;
-        float4 *slot = a.ck + (size_t(start / a.segment + tile + segment) * a.tileSize) * a.tileSize;
+        float4 *slot = a.ck + (size_t(slot0 + segment) * a.tileSize) * a.tileSize;
         if (in0)
-            slot[slotPixel(a.tileSize, wb.px, wb.py0)] = make_float4(lr.x, lg.x, lb.x, begin.x);
+            slot[slotPixel(a.tileSize, px, py0)] = make_float4(lr.x, lg.x, lb.x, begin.x);
         if (in1)
-            slot[slotPixel(a.tileSize, wb.px, wb.py1)] = make_float4(lr.y, lg.y, lb.y, begin.y);
-    };
-    for (int b0 = start, bEnd; b0 < end; b0 = bEnd) {
-        if (__syncthreads_count(done0 && done1) == NT)
-            break;
-        if (kKeep && b0 == segEnd) {
-            keepSegment();
+            slot[slotPixel(a.tileSize, px, py0 + 4)] = make_float4(lr.y, lg.y, lb.y, begin.y);
+    }
+    // Before a batch of `batch` entries (batches do not cross segments).
+    __device__ __forceinline__ void beginBatch(const RasterArgs &a, int batch, int slot0, int px, int py0, bool in0, bool in1)
+    {
+        if (kKeep && left == 0) {
+            keepSegment(a, slot0, px, py0, in0, in1);
             ++segment;
-            segEnd += a.segment;
-            lr = lg = lb = make_float2(0.0f, 0.0f);
-            begin = T;
+            left = a.segment;
+            lr = lg = lb = both(0.0f);
+            begin = Tf;
         }
-        bEnd = min(min(b0 + NB, segEnd), end);
+        left -= batch;
+    }
+    __device__ __forceinline__ void store(const RasterArgs &a, int slot0, int px, int py0, bool in0, bool in1, float *rgb,
+                                          float *finalT, int *nContrib) const
+    {
+        if (kKeep) {
+            keepSegment(a, slot0, px, py0, in0, in1);
+            const int most = __reduce_max_sync(0xffffffffu, max(last0, last1));
+            if ((threadIdx.x & 31) == 0)
+                a.blockMax[(py0 >> 3) * (a.tilesX * (a.tileSize >> 3)) + (px >> 3)] = most;
+        }
+        auto put = [&](int py, float T1, float r, float g, float b, int last) {
+            const size_t pix = size_t(py) * a.width + px;
+            rgb[pix * 3] = r + T1 * a.bg[0];
+            rgb[pix * 3 + 1] = g + T1 * a.bg[1];
+            rgb[pix * 3 + 2] = b + T1 * a.bg[2];
+            finalT[pix] = T1;
+            nContrib[pix] = last;
+        };
+        if (in0)
+            put(py0, Tf.x, cr.x, cg.x, cb.x, last0);
+        if (in1)
+            put(py0 + 4, Tf.y, cr.y, cg.y, cb.y, last1);
+    }
+};
+
+// One warp per 8x8 pixel block: kGroup entries at a time, first the alphas of all of them, then the
+// blending. At most 96 registers, so that 20 blocks share an SM (640x480 us at groups of 1 / 2 / 4: 129 /
+// 112 / 106).
+constexpr int kSoloBatch = 32, kGroup = 4;
+
+struct SoloShared {
+    float4 P[kSoloBatch], Q[kSoloBatch], R[kSoloBatch];
+    uint32_t mask[1][1];
+};
+
+template <bool kKeep, bool kStrict>
+__device__ __forceinline__ void soloBatch(const SoloShared &sh, Blend<kKeep> &px, int first, float fx, float2 nfy, float minA,
+                                          float minT)
+{
+    uint32_t bits = sh.mask[0][0];
+    while (bits) {
+        const bool on0 = px.T.x >= minT, on1 = px.T.y >= minT;
+        if (!__any_sync(0xffffffffu, on0 || on1))
+            break;
+        float2 al[kGroup];
+        int j[kGroup];
 #pragma unroll
-        for (int r = 0; r < BD; ++r) {
-            const int slot = r * NT + tid;
-            stage<PB, NG>(rec, a.entries, b0 + slot, b0 + slot < bEnd, slot, sP, sQ, sR, mask, bx, by);
+        for (int u = 0; u < kGroup; ++u) {
+            const bool has = bits != 0;
+            j[u] = has ? __ffs(bits) - 1 : j[0];
+            bits &= bits - 1;
+            al[u] = entryAlpha(entryPower(sh.P[j[u]], sh.Q[j[u]], fx, nfy, has && on0, has && on1), minA);
         }
-        __syncthreads();
-        for (int k = 0; k < NG && !(done0 && done1); ++k) {
-            uint32_t bits = mask[warp][k];
-            while (bits) {
-                const int j = 32 * k + __ffs(bits) - 1;
-                bits &= bits - 1;
-                // One front-to-back blending step of Rasterizer.cpp:305-318 for both of the thread's
-                // pixels at once, in paired FP32 instructions where each lane rounds like the scalar
-                // operation: the falloff exponent in powerAt's order (products paired, sums scalar),
-                // alpha, 1 - alpha, T (1 - alpha) and alpha T, and the colour sums as paired fused
-                // multiply-adds; the cut-offs per pixel.
-                const float4 P = sP[j], Q = sQ[j];
-                const ColumnTerms ct = columnTerms(Q, P.x - fx);
-                const float2 dy = make_float2(P.y - fy0, P.y - fy1);
-                const float2 cdd = mul2rn(mul2rn(make_float2(Q.z, Q.z), dy), dy);
-                const float2 bdy = mul2rn(make_float2(ct.bx, ct.bx), dy);
-                const float2 hq = mul2rn(make_float2(-0.5f, -0.5f), make_float2(__fadd_rn(ct.axx, cdd.x), __fadd_rn(ct.axx, cdd.y)));
-                const float2 pw = make_float2(__fsub_rn(hq.x, bdy.x), __fsub_rn(hq.y, bdy.y));
-                bool v0 = !done0 && !(pw.x > 0.0f || pw.x < P.z);
-                bool v1 = !done1 && !(pw.y > 0.0f || pw.y < P.z);
-                if (v0 || v1) {
-                    // A pixel that is out gets exp(0), whose alpha it never uses.
-                    const float2 G = make_float2(rasterExp(v0 ? pw.x : 0.0f), rasterExp(v1 ? pw.y : 0.0f));
-                    const float2 raw = mul2rn(make_float2(Q.w, Q.w), G);
-                    const float al0 = (raw.x < kMaxAlpha) ? raw.x : kMaxAlpha;
-                    const float al1 = (raw.y < kMaxAlpha) ? raw.y : kMaxAlpha;
-                    v0 = v0 && !(al0 < minA);
-                    v1 = v1 && !(al1 < minA);
-                    const float2 nT = mul2rn(T, add2rn(one, make_float2(-al0, -al1)));
-                    if (v0 && nT.x < minT) {
-                        done0 = true;
-                        v0 = false;
-                    }
-                    if (v1 && nT.y < minT) {
-                        done1 = true;
-                        v1 = false;
-                    }
-                    float2 w = mul2rn(make_float2(al0, al1), T);
-                    w.x = v0 ? w.x : 0.0f; // a pixel that does not blend adds R * 0 = 0 to its sums
-                    w.y = v1 ? w.y : 0.0f;
-                    const float4 R = sR[j];
-                    cr = fma2rn(make_float2(R.x, R.x), w, cr);
-                    cg = fma2rn(make_float2(R.y, R.y), w, cg);
-                    cb = fma2rn(make_float2(R.z, R.z), w, cb);
-                    if (kKeep) {
-                        lr = fma2rn(make_float2(R.x, R.x), w, lr);
-                        lg = fma2rn(make_float2(R.y, R.y), w, lg);
-                        lb = fma2rn(make_float2(R.z, R.z), w, lb);
-                    }
-                    const int idx = b0 - start + j + 1;
-                    if (v0) {
-                        T.x = nT.x;
-                        last0 = idx;
-                    }
-                    if (v1) {
-                        T.y = nT.y;
-                        last1 = idx;
-                    }
-                }
-                if (done0 && done1)
-                    break;
-            }
-        }
-    }
-    if (kKeep) {
-        keepSegment();
-        const int most = __reduce_max_sync(0xffffffffu, max(last0, last1));
-        if (lane == 0)
-            a.blockMax[(wb.py0 >> 3) * (a.tilesX * (a.tileSize >> 3)) + (wb.px >> 3)] = most;
-    }
-    const float T0 = T.x, T1 = T.y, r0 = cr.x, r1 = cr.y, g0 = cg.x, g1 = cg.y, b0c = cb.x, b1c = cb.y;
-    if (in0) {
-        const size_t pix = size_t(wb.py0) * a.width + wb.px;
-        rgb[pix * 3] = r0 + T0 * a.bg[0];
-        rgb[pix * 3 + 1] = g0 + T0 * a.bg[1];
-        rgb[pix * 3 + 2] = b0c + T0 * a.bg[2];
-        finalT[pix] = T0;
-        nContrib[pix] = last0;
-    }
-    if (in1) {
-        const size_t pix = size_t(wb.py1) * a.width + wb.px;
-        rgb[pix * 3] = r1 + T1 * a.bg[0];
-        rgb[pix * 3 + 1] = g1 + T1 * a.bg[1];
-        rgb[pix * 3 + 2] = b1c + T1 * a.bg[2];
-        finalT[pix] = T1;
-        nContrib[pix] = last1;
-    }
-}
-
-// Resident CTAs per SM the compiler must allow for: caps registers per thread at 65536 / (NT * n)
-// (48 at 10 for NT = 128).
-#ifndef U3DG_FWD_MIN_BLOCKS
-#define U3DG_FWD_MIN_BLOCKS 10
-#endif
-
-template <int PB, int BD, bool kKeep>
-__global__ void __launch_bounds__(RasterShape<PB>::NT, U3DG_FWD_MIN_BLOCKS) compositeForwardKernel(RasterArgs a, float *rgb, float *finalT,
-                                                                              int *nContrib)
-{
-    pdlEntry();
-    using S = RasterShape<PB, BD>;
-    constexpr int NB = S::NB, NW = S::NW, NG = S::NG;
-    __shared__ float4 sP[NB]; // mx, my, powMin, ey
-    __shared__ float4 sQ[NB]; // A, B, C, alpha
-    __shared__ float4 sR[NB]; // r, g, b, powMin
-    __shared__ uint32_t mask[NW][NG];
-    __shared__ int sNext;
-    const int units = a.blocksX * a.blocksY;
-    if (a.counters == nullptr) { // one CTA per pixel block (every block resident in one wave)
-        forwardBlock<PB, BD, kKeep>(a, int(blockIdx.x) % a.blocksX, int(blockIdx.x) / a.blocksX, rgb, finalT, nContrib, sP,
-                             sQ, sR, mask);
-        return;
-    }
-    // Heaviest tile lists first (a.blockOrder), so that the long lists start early.
-    for (int u = nextUnit(units, a.counters, &sNext); u < units; u = nextUnit(units, a.counters, &sNext)) {
-        const int b = a.blockOrder[u];
-        forwardBlock<PB, BD, kKeep>(a, b % a.blocksX, b / a.blocksX, rgb, finalT, nContrib, sP, sQ, sR, mask);
-    }
-}
-
-// One CTA: the pixel blocks bucketed by the list length of their tile on a log scale (four buckets
-// per power of two), longest first. The order only schedules work (every block's result is the same
-// whichever CTA computes it when), so blocks within a bucket may come in any order.
-constexpr int kOrderBuckets = 132;
-
-__device__ __forceinline__ int lengthBucket(unsigned len)
-{
-    if (len == 0)
-        return kOrderBuckets - 1;
-    const int msb = 31 - __clz(len);
-    const int sub = msb >= 2 ? int((len >> (msb - 2)) & 3u) : int((len << (2 - msb)) & 3u);
-    return kOrderBuckets - 2 - (msb * 4 + sub); // longer lists: smaller bucket index
-}
-
-__global__ void __launch_bounds__(1024) blockOrderKernel(const int *tileOffsets, int blocksX, int blocksY, int pb,
-                                                         int tileSize, int tilesX, int *order)
-{
-    pdlEntry();
-    __shared__ int count[kOrderBuckets];
-    __shared__ int cursor[kOrderBuckets];
-    const int units = blocksX * blocksY;
-    for (int b = threadIdx.x; b < kOrderBuckets; b += blockDim.x)
-        count[b] = 0;
-    __syncthreads();
-    for (int u = threadIdx.x; u < units; u += blockDim.x) {
-        const int bx = u % blocksX, by = u / blocksX;
-        const int t = (by * pb / tileSize) * tilesX + bx * pb / tileSize;
-        atomicAdd(&count[lengthBucket(unsigned(tileOffsets[t + 1] - tileOffsets[t]))], 1);
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) { // exclusive scan of the bucket counts: each lane owns kPer consecutive buckets
-        constexpr int kPer = (kOrderBuckets + 31) / 32;
-        const int lane = threadIdx.x, b0 = lane * kPer;
-        int own = 0;
-        for (int b = b0; b < b0 + kPer && b < kOrderBuckets; ++b)
-            own += count[b];
-        int incl = own;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o)
-                incl += y;
-        }
-        int run = incl - own;
-        for (int b = b0; b < b0 + kPer && b < kOrderBuckets; ++b) {
-            cursor[b] = run;
-            run += count[b];
-        }
+        for (int u = 0; u < kGroup; ++u)
+            px.template entry<kStrict>(al[u], sh.R[j[u]], first + j[u], minT);
     }
-    __syncthreads();
-    for (int u = threadIdx.x; u < units; u += blockDim.x) {
-        const int bx = u % blocksX, by = u / blocksX;
-        const int t = (by * pb / tileSize) * tilesX + bx * pb / tileSize;
-        const int pos = atomicAdd(&cursor[lengthBucket(unsigned(tileOffsets[t + 1] - tileOffsets[t]))], 1);
-        order[pos] = u;
-    }
-}
-
-// CTAs that can be resident at once for a kernel (cached per kernel and dynamic shared memory size).
-template <class K>
-int residentCtas(K kernel, int threads, size_t smem)
-{
-    int dev = 0, sms = 0, perSm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, threads, smem);
-    return std::max(1, sms * std::max(1, perSm));
-}
-
-} // namespace
-
-// Orders the pixel blocks by the list length of their tile, longest first, into a.blockOrder.
-static void launchBlockOrder(const RasterArgs &a, cudaStream_t s)
-{
-    const int pb = a.tileSize <= 8 ? 8 : 16;
-    { launchPdl(blockOrderKernel, 1, 1024, 0, s, a.tileOffsets, a.blocksX, a.blocksY, pb, a.tileSize, a.tilesX, a.blockOrder); countLaunch(); }
-}
-
-template <int PB, int BD, bool kKeep>
-static void launchForward(const RasterArgs &a, float *rgb, float *finalT, int *nContrib, cudaStream_t s)
-{
-    // When every pixel block fits on the GPU at once, one CTA per block in natural order (no work
-    // counter); otherwise the persistent schedule on counters[0..1].
-    const int units = a.blocksX * a.blocksY;
-    static const int ctas = residentCtas(compositeForwardKernel<PB, BD, kKeep>, RasterShape<PB>::NT, 0);
-    RasterArgs f = a;
-    if (units <= ctas)
-        f.counters = nullptr;
-    else
-        launchBlockOrder(a, s);
-    { launchPdl(compositeForwardKernel<PB, BD, kKeep>, std::min(units, ctas), RasterShape<PB>::NT, 0, s, f, rgb, finalT, nContrib); countLaunch(); }
-}
-
-// 8x8 CTAs over the lists of larger tiles: one CTA per pixel block in natural order, as many waves as
-// it takes (the blocks are short).
-template <int BD, bool kKeep>
-static void launchForwardSplit(const RasterArgs &a, float *rgb, float *finalT, int *nContrib, cudaStream_t s)
-{
-    RasterArgs f = a;
-    f.blocksX = (a.width + 7) / 8;
-    f.blocksY = (a.height + 7) / 8;
-    f.counters = nullptr;
-    { launchPdl(compositeForwardKernel<8, BD, kKeep>, f.blocksX * f.blocksY, RasterShape<8>::NT, 0, s, f, rgb, finalT, nContrib); countLaunch(); }
 }
 
 template <bool kKeep>
-static void launchForwardAny(const RasterArgs &a, float *rgb, float *finalT, int *nContrib, cudaStream_t s)
+__global__ void __launch_bounds__(32, 20) compositeForwardKernel(RasterArgs a, float *rgb, float *finalT, int *nContrib)
 {
-    const bool deep = a.forwardDepth >= 2;
-    if (a.tileSize > 8 && a.forwardBlock == 8)
-        deep ? launchForwardSplit<2, kKeep>(a, rgb, finalT, nContrib, s)
-             : launchForwardSplit<1, kKeep>(a, rgb, finalT, nContrib, s);
-    else if (a.tileSize <= 8)
-        deep ? launchForward<8, 2, kKeep>(a, rgb, finalT, nContrib, s)
-             : launchForward<8, 1, kKeep>(a, rgb, finalT, nContrib, s);
+    pdlEntry();
+    __shared__ SoloShared sh;
+    const int bx = int(blockIdx.x) % a.blocksX, by = int(blockIdx.x) / a.blocksX; // 8x8 blocks
+    const int lane = threadIdx.x;
+    const WarpBlock wb(lane, bx, by);
+    const int tile = tileOf<8>(a, bx, by);
+    const int start = a.tileOffsets[tile], end = a.tileOffsets[tile + 1];
+    const float fx = float(wb.px);
+    const float2 nfy = make_float2(-float(wb.py0), -float(wb.py1));
+    const float4 *rec = reinterpret_cast<const float4 *>(a.rec);
+    const bool in0 = wb.px < a.width && wb.py0 < a.height, in1 = wb.px < a.width && wb.py1 < a.height;
+    const int slot0 = kKeep ? start / a.segment + tile : 0;
+    Blend<kKeep> px(in0, in1, a.segment);
+    // The records of the next batch and the ids of the one after it are on their way meanwhile.
+    auto idOf = [&](int b0) { return b0 + lane < end ? a.entries[b0 + lane] : -1; };
+    StagedRecord next = loadRecord(rec, idOf(start));
+    int gid = idOf(start + kSoloBatch);
+    for (int b0 = start; b0 < end; b0 += kSoloBatch) {
+        if (!__any_sync(0xffffffffu, px.T.x >= a.minTransmittance || px.T.y >= a.minTransmittance))
+            break;
+        px.beginBatch(a, kSoloBatch, slot0, wb.px, wb.py0, in0, in1);
+        stage<1, 1>(next, b0 + lane < end, lane, sh.P, sh.Q, sh.R, sh.mask, bx, by);
+        const bool odd = !finite(next.c.x) || !finite(next.c.y) || !finite(next.c.z);
+        const bool strict = __any_sync(0xffffffffu, odd);
+        __syncwarp();
+        next = loadRecord(rec, gid);
+        gid = idOf(b0 + 2 * kSoloBatch);
+        if (strict)
+            soloBatch<kKeep, true>(sh, px, b0 - start + 1, fx, nfy, a.minAlpha, a.minTransmittance);
+        else
+            soloBatch<kKeep, false>(sh, px, b0 - start + 1, fx, nfy, a.minAlpha, a.minTransmittance);
+        __syncwarp();
+    }
+    px.store(a, slot0, wb.px, wb.py0, in0, in1, rgb, finalT, nContrib);
+}
+
+// One 8x8 pixel block by a team of warps. What an entry adds to a pixel needs its alpha, which is the same
+// whatever lies before it, and the transmittance, which is one product after the other. The evaluating
+// warps stage a batch of kBatch list entries and compute the alphas of those that meet the block (every
+// kEval-th each, two at a time) into shared memory while the blending warp, one batch behind, takes them
+// in list order through the transmittance, the cut-off and the colour sums.
+constexpr int kEval = 4, kBatch = 64, kBlendGroup = 4, kEvalGroup = 2;
+constexpr int kTeamThreads = 32 * (kEval + 1);
+static_assert(kEval * 32 >= kBatch, "every entry of a batch has an evaluating thread");
+
+struct TeamShared {
+    float2 alpha[2][kBatch][32]; // per entry and lane: the lane's two pixels (negative zero: not blended)
+    float4 P[kBatch], Q[kBatch], R[2][kBatch];
+    uint32_t mask[2][1][kBatch / 32];
+    int odd[2][kBatch / 32]; // a non-finite colour among a staging warp's entries
+    uint2 live[2];           // the lanes whose first / second pixel is live
+};
+
+// Barriers by name, as the two roles meet at different places of the code.
+__device__ __forceinline__ void evaluatorsMeet() { asm volatile("bar.sync 1, %0;" ::"n"(kEval * 32) : "memory"); }
+__device__ __forceinline__ void teamMeets() { asm volatile("bar.sync 2, %0;" ::"n"(kTeamThreads) : "memory"); }
+
+// Alphas of the batch's entries that meet the block, evaluating warp `w` of kEval. An entry that reaches no
+// live pixel (on0, on1: the lane's pixels as of two batches ago) leaves the mask before its exponentials:
+// towards the end of a block few pixels are live.
+__device__ __forceinline__ void evaluateBatch(TeamShared &sh, int buf, int w, int lane, float fx, float2 nfy, float minA,
+                                              bool on0, bool on1)
+{
+    static_assert(kEval == 4, "every fourth entry");
+#pragma unroll
+    for (int half = 0; half < kBatch / 32; ++half) {
+        uint32_t mine = sh.mask[buf][0][half] & (0x11111111u << w), none = 0;
+        while (mine) {
+            int j[kEvalGroup];
+            EntryPower e[kEvalGroup];
+            bool any = false;
+#pragma unroll
+            for (int u = 0; u < kEvalGroup; ++u) {
+                const bool has = mine != 0;
+                j[u] = has ? __ffs(mine) - 1 : j[0];
+                mine &= mine - 1;
+                e[u] = entryPower(sh.P[32 * half + j[u]], sh.Q[32 * half + j[u]], fx, nfy, on0, on1);
+                any = any || e[u].v0 || e[u].v1;
+            }
+            if (!__any_sync(0xffffffffu, any)) {
+#pragma unroll
+                for (int u = 0; u < kEvalGroup; ++u)
+                    none |= 1u << j[u];
+                continue;
+            }
+#pragma unroll
+            for (int u = 0; u < kEvalGroup; ++u)
+                sh.alpha[buf][32 * half + j[u]][lane] = entryAlpha(e[u], minA);
+        }
+        if (none && lane == 0)
+            atomicAnd(&sh.mask[buf][0][half], ~none);
+    }
+}
+
+template <bool kKeep, bool kStrict>
+__device__ __forceinline__ void blendBatch(const TeamShared &sh, int buf, int lane, Blend<kKeep> &px, int first, float minT)
+{
+#pragma unroll
+    for (int half = 0; half < kBatch / 32; ++half) {
+        uint32_t bits = sh.mask[buf][0][half];
+        while (bits) {
+            int j[kBlendGroup];
+            float2 al[kBlendGroup];
+#pragma unroll
+            for (int u = 0; u < kBlendGroup; ++u) {
+                const bool has = bits != 0;
+                j[u] = 32 * half + (has ? __ffs(bits) - 1 : 0);
+                bits &= bits - 1;
+                al[u] = sh.alpha[buf][j[u]][lane];
+                if (!has)
+                    al[u] = both(-0.0f);
+            }
+#pragma unroll
+            for (int u = 0; u < kBlendGroup; ++u)
+                px.template entry<kStrict>(al[u], sh.R[buf][j[u]], first + j[u], minT);
+        }
+    }
+}
+
+template <bool kKeep>
+__global__ void __launch_bounds__(kTeamThreads, 6) compositeForwardTeamKernel(RasterArgs a, float *rgb,
+                                                                                           float *finalT, int *nContrib)
+{
+    pdlEntry();
+    __shared__ TeamShared sh;
+    const int bx = int(blockIdx.x) % a.blocksX, by = int(blockIdx.x) / a.blocksX; // 8x8 blocks
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const WarpBlock wb(lane, bx, by);
+    const int tile = tileOf<8>(a, bx, by);
+    const int start = a.tileOffsets[tile], end = a.tileOffsets[tile + 1];
+    const int batches = (end - start + kBatch - 1) / kBatch;
+    const bool in0 = wb.px < a.width && wb.py0 < a.height, in1 = wb.px < a.width && wb.py1 < a.height;
+    const float minT = a.minTransmittance;
+    if (warp > 0) {
+        const int e = threadIdx.x - 32;
+        const float fx = float(wb.px);
+        const float2 nfy = make_float2(-float(wb.py0), -float(wb.py1));
+        const float4 *rec = reinterpret_cast<const float4 *>(a.rec);
+        auto idOf = [&](int t) {
+            const int i = start + t * kBatch + e;
+            return e < kBatch && i < end ? a.entries[i] : -1;
+        };
+        // The records of the next batch and the ids of the one after it are on their way meanwhile.
+        bool on0 = in0, on1 = in1;
+        StagedRecord next = loadRecord(rec, idOf(0));
+        int gid = idOf(1);
+        for (int t = 0; t < batches; ++t) {
+            const int buf = t & 1;
+            if (e < kBatch) {
+                const bool valid = start + t * kBatch + e < end;
+                stage<1, kBatch / 32>(next, valid, e, sh.P, sh.Q, sh.R[buf], sh.mask[buf], bx, by);
+                const bool odd = !finite(next.c.x) || !finite(next.c.y) || !finite(next.c.z);
+                const bool any = __any_sync(0xffffffffu, odd);
+                if (lane == 0)
+                    sh.odd[buf][e >> 5] = any;
+            }
+            evaluatorsMeet();
+            next = loadRecord(rec, gid);
+            gid = idOf(t + 2);
+            evaluateBatch(sh, buf, warp - 1, lane, fx, nfy, a.minAlpha, on0, on1);
+            teamMeets(); // batch t is evaluated, batch t - 1 blended
+            if (t > 0) {
+                const uint2 live = sh.live[buf ^ 1];
+                if (!(live.x | live.y))
+                    return; // and so does the blending warp
+                on0 = live.x >> lane & 1u;
+                on1 = live.y >> lane & 1u;
+            }
+        }
+        return;
+    }
+    const int slot0 = kKeep ? start / a.segment + tile : 0;
+    Blend<kKeep> px(in0, in1, a.segment);
+    if (batches > 0)
+        teamMeets(); // batch 0 is evaluated
+    for (int t = 0; t < batches; ++t) {
+        const int buf = t & 1;
+        px.beginBatch(a, kBatch, slot0, wb.px, wb.py0, in0, in1);
+        if (sh.odd[buf][0] | sh.odd[buf][1])
+            blendBatch<kKeep, true>(sh, buf, lane, px, t * kBatch + 1, minT);
+        else
+            blendBatch<kKeep, false>(sh, buf, lane, px, t * kBatch + 1, minT);
+        if (t + 1 == batches)
+            break;
+        const uint2 live = make_uint2(__ballot_sync(0xffffffffu, px.T.x >= minT), __ballot_sync(0xffffffffu, px.T.y >= minT));
+        if (lane == 0)
+            sh.live[buf] = live;
+        teamMeets(); // batch t + 1 is evaluated, this one's buffers are free
+        if (!(live.x | live.y))
+            break;
+    }
+    px.store(a, slot0, wb.px, wb.py0, in0, in1, rgb, finalT, nContrib);
+}
+
+// Blocks up to which the team is faster (between 1,200 and 2,700, see above): about 14 per SM.
+constexpr int kTeamLimit = 2048;
+
+} // namespace
+
+template <bool kKeep>
+static void launchForward(const RasterArgs &a, float *rgb, float *finalT, int *nContrib, cudaStream_t s)
+{
+    const int blocks = a.blocksX * a.blocksY;
+    if (blocks <= kTeamLimit)
+        { launchPdl(compositeForwardTeamKernel<kKeep>, blocks, kTeamThreads, 0, s, a, rgb, finalT, nContrib); countLaunch(); }
     else
-        deep ? launchForward<16, 2, kKeep>(a, rgb, finalT, nContrib, s)
-             : launchForward<16, 1, kKeep>(a, rgb, finalT, nContrib, s);
+        { launchPdl(compositeForwardKernel<kKeep>, blocks, 32, 0, s, a, rgb, finalT, nContrib); countLaunch(); }
 }
 
 void launchCompositeForward(const RasterArgs &a, float *rgb, float *finalT, int *nContrib, cudaStream_t s)
 {
-    if (a.blocksX * a.blocksY <= 0)
+    RasterArgs f = a;
+    f.blocksX = (a.width + 7) / 8;
+    f.blocksY = (a.height + 7) / 8;
+    if (f.blocksX * f.blocksY <= 0)
         return;
     if (a.segment > 0)
-        launchForwardAny<true>(a, rgb, finalT, nContrib, s);
+        launchForward<true>(f, rgb, finalT, nContrib, s);
     else
-        launchForwardAny<false>(a, rgb, finalT, nContrib, s);
+        launchForward<false>(f, rgb, finalT, nContrib, s);
 }
 
 } // namespace u3dg

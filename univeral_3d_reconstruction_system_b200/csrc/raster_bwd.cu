@@ -110,10 +110,6 @@ __device__ __forceinline__ float rcpApprox(float x)
     return y;
 }
 
-__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
-
-__device__ __forceinline__ bool finite(float v) { return fabsf(v) < __int_as_float(0x7f800000); }
-
 template <int PB, int BD, bool kBg>
 __device__ __forceinline__ void backwardUnit(const RasterArgs &a, int block, int segment, const float *dLdRgb,
                                              const float *finalTIn, const int *nContribIn, float *partial,
@@ -203,7 +199,8 @@ __device__ __forceinline__ void backwardUnit(const RasterArgs &a, int block, int
         for (int r = 0; r < BD; ++r) {
             const int slot = r * NT + tid;
             const bool valid = slot < cnt;
-            stage<PB, NG>(rec, a.entries, start + bStart + slot, valid, slot, sP, sQ, sR, mask, bx, by);
+            stage<S::WX, NG>(loadRecord(rec, valid ? a.entries[start + bStart + slot] : -1), valid, slot, sP, sQ, sR, mask, bx,
+                          by);
             if (valid && !(finite(sR[slot].x) && finite(sR[slot].y) && finite(sR[slot].z)))
                 sOdd = 1;
         }
@@ -365,8 +362,7 @@ __global__ void __launch_bounds__(BackwardShape<PB>::NT, U3DG_BWD_MIN_BLOCKS * 6
     __shared__ int sOdd, sNext;
     extern __shared__ __align__(16) float sBlock[]; // per 8x8 block: NB entries x 9 sums
     const int count = *unitCount;
-    int *counter = a.counters + 2; // backward: counters[2..3]
-    for (int u = nextUnit(count, counter, &sNext); u < count; u = nextUnit(count, counter, &sNext)) {
+    for (int u = nextUnit(count, a.counters, &sNext); u < count; u = nextUnit(count, a.counters, &sNext)) {
         const int2 unit = units[u];
         backwardUnit<PB, BD, kBg>(a, unit.x, unit.y, dLdRgb, finalTIn, nContribIn, partial, stop, sP, sQ, sR, mask,
                                   sOdd, sBlock);
@@ -462,7 +458,7 @@ void launchCompositeBackward(const RasterArgs &a, const float *dLdRgb, const flo
 {
     if (a.blocksX * a.blocksY <= 0)
         return;
-    const bool deep = a.backwardDepth >= 2;
+    const bool deep = a.backwardDepth >= 2 && a.tileSize != 16; // segments of 64 entries are one batch at tile 16
     const bool bg = a.bg[0] != 0.0f || a.bg[1] != 0.0f || a.bg[2] != 0.0f;
     auto run = [&](auto kBg) {
         constexpr bool B = decltype(kBg)::value;

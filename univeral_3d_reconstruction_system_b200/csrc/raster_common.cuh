@@ -1,11 +1,9 @@
 // raster_common.cuh - pixel layout and batch staging shared by the compositing kernels.
 //
-// A CTA covers a PB x PB pixel block (PB = 16, or 8 for tile size 8) with PB*PB/2 threads; a warp
-// owns an 8 x 8 pixel block and each thread two pixels of the same column, rows r and r + 4. A tile's
-// depth-sorted list is walked in batches of BD records per thread (the batch depth, 1 or 2); while
-// staging a batch, each warp votes which of its 32 entries meet each warp's pixel block (the Gaussian's
-// conservative contributing box, SplatRec::ex / ey, against the block), so each warp later walks only
-// the set bits of its mask. The batch depth changes how many entries are staged per barrier, not any
+// Work is divided by 8x8 pixel blocks. A tile's depth-sorted list is walked in batches staged in shared
+// memory; while staging, each warp votes which of its 32 entries meet a block (the Gaussian's conservative
+// contributing box, SplatRec::ex / ey, and ellipse against the block), so that a block's warp walks only
+// the set bits of its mask. The batch size changes how many entries are staged per barrier, not any
 // result: every entry is evaluated the same way in the same order.
 #pragma once
 
@@ -13,41 +11,11 @@
 
 namespace u3dg {
 
-template <int PB, int BD = 1>
-struct RasterShape {
-    static constexpr int NT = PB * PB / 2; // threads
-    static constexpr int NW = NT / 32;     // warps
-    static constexpr int WX = PB / 8;      // warp blocks per row
-    static constexpr int NB = NT * BD;     // batch entries
-    static constexpr int NG = NB / 32;     // 32-entry groups of a batch (mask words per warp)
-};
-
-// This thread's two pixels and its warp's 8x8 block, in pixel block (bx, by).
-template <int PB>
+// The two pixels of a warp's lane in 8x8 block (bx, by): one column, rows 4 apart.
 struct WarpBlock {
     int px, py0, py1;
-    float x0, x1, y0, y1; // warp block, inclusive
-    __device__ WarpBlock(int warp, int lane, int bx, int by)
-    {
-        constexpr int WX = RasterShape<PB>::WX;
-        const int wx0 = bx * PB + (warp % WX) * 8, wy0 = by * PB + (warp / WX) * 8;
-        px = wx0 + (lane & 7);
-        py0 = wy0 + (lane >> 3);
-        py1 = py0 + 4;
-        x0 = float(wx0);
-        x1 = float(wx0 + 7);
-        y0 = float(wy0);
-        y1 = float(wy0 + 7);
-    }
+    __device__ WarpBlock(int lane, int bx, int by) : px(bx * 8 + (lane & 7)), py0(by * 8 + (lane >> 3)), py1(py0 + 4) {}
 };
-
-template <int PB>
-__device__ __forceinline__ bool meets(const float4 &p, int w, int bx, int by)
-{
-    constexpr int WX = RasterShape<PB>::WX;
-    const float x0 = float(bx * PB + (w % WX) * 8), y0 = float(by * PB + (w / WX) * 8);
-    return !(p.x + p.z < x0 || p.x - p.z > x0 + 7.0f || p.y + p.w < y0 || p.y - p.w > y0 + 7.0f);
-}
 
 // Whether the contributing ellipse of a staged entry, {d : A dx^2 + 2 B dx dy + C dy^2 <= -2 powMin}
 // (power >= powMin), can reach a pixel centre of the 8x8 block [x0, x0 + 7] x [y0, y0 + 7]: the
@@ -110,39 +78,54 @@ __device__ __forceinline__ int slotPixel(int tileSize, int px, int py)
     return ((y >> 3) * (tileSize >> 3) + (x >> 3)) * 64 + (y & 7) * 8 + (x & 7);
 }
 
-// Stages batch entry `slot` (if valid) and the masks of NG words: mask[w][g] bit b <=> entry 32g + b meets
-// 8x8 block w (slots are a warp's lanes in order).
-template <int PB, int NG>
-__device__ __forceinline__ void stage(const float4 *rec, const int *entries, int idx, bool valid, int slot, float4 *sP,
-                                      float4 *sQ, float4 *sR, uint32_t (*mask)[NG], int bx, int by)
+// A list entry's raster record on its way to shared memory (p.z < 0: none).
+struct StagedRecord {
+    float4 p, q, c;
+};
+
+__device__ __forceinline__ StagedRecord loadRecord(const float4 *rec, int gid)
 {
-    constexpr int NW = RasterShape<PB>::NW, WX = RasterShape<PB>::WX;
-    float4 p = make_float4(0.0f, 0.0f, -1.0f, -1.0f), q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float powMin = 0.0f, iA = 0.0f, iC = 0.0f;
-    if (valid) {
-        const float4 *r = rec + size_t(entries[idx]) * 3;
-        p = r[0];
-        q = r[1];
-        const float4 c = r[2];
-        // The blending loops read the mean from sP and the exponent floor (SplatRec::powMin) from its
-        // third slot; the contributing box is only needed for the masks below.
-        sP[slot] = make_float4(p.x, p.y, c.w, p.w);
-        sQ[slot] = q;
-        sR[slot] = c;
-        powMin = c.w;
-        iA = __frcp_rn(q.x);
-        iC = __frcp_rn(q.z);
+    StagedRecord s;
+    s.p = make_float4(0.0f, 0.0f, -1.0f, -1.0f);
+    s.q = s.c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (gid >= 0) {
+        const float4 *r = rec + size_t(gid) * 3;
+        s.p = r[0];
+        s.q = r[1];
+        s.c = r[2];
     }
-    // The ellipse test refines the box test where the box extents are finite (well-conditioned
-    // covariances and a positive minimum alpha).
-    const bool fine = p.z < __int_as_float(0x7f800000);
+    return s;
+}
+
+// Whether a record can contribute to a pixel of the 8x8 block at (x0, y0): its box against the block,
+// refined by the ellipse test where the box extents are finite (well-conditioned covariances and a
+// positive minimum alpha).
+__device__ __forceinline__ bool entryMeets(const StagedRecord &s, float x0, float y0)
+{
+    const float4 &p = s.p;
+    if (p.x + p.z < x0 || p.x - p.z > x0 + 7.0f || p.y + p.w < y0 || p.y - p.w > y0 + 7.0f)
+        return false;
+    return !(p.z < __int_as_float(0x7f800000)) || ellipseMeets(p.x, p.y, s.q, s.c.w, __frcp_rn(s.q.x), __frcp_rn(s.q.z), x0, y0);
+}
+
+// Stages batch entry `slot` (if valid) and the masks of NG words: mask[w][g] bit b <=> entry 32g + b meets
+// 8x8 block w (of WX per row) of pixel block (bx, by). Slots are a warp's lanes in order.
+template <int WX, int NG>
+__device__ __forceinline__ void stage(const StagedRecord &s, bool valid, int slot, float4 *sP, float4 *sQ, float4 *sR,
+                                      uint32_t (*mask)[NG], int bx, int by)
+{
+    constexpr int PB = 8 * WX;
+    if (valid) {
+        // The blending loop reads the mean from sP and the exponent floor (SplatRec::powMin) from its third
+        // slot; the contributing box is only needed for the masks below.
+        sP[slot] = make_float4(s.p.x, s.p.y, s.c.w, s.p.w);
+        sQ[slot] = s.q;
+        sR[slot] = s.c;
+    }
     const int group = slot >> 5, lane = slot & 31;
 #pragma unroll
-    for (int w = 0; w < NW; ++w) {
-        bool hit = valid && meets<PB>(p, w, bx, by);
-        if (hit && fine)
-            hit = ellipseMeets(p.x, p.y, q, powMin, iA, iC, float(bx * PB + (w % WX) * 8), float(by * PB + (w / WX) * 8));
-        const uint32_t bits = __ballot_sync(0xffffffffu, hit);
+    for (int w = 0; w < WX * WX; ++w) {
+        const uint32_t bits = __ballot_sync(0xffffffffu, valid && entryMeets(s, float(bx * PB + (w % WX) * 8), float(by * PB + (w / WX) * 8)));
         if (lane == 0)
             mask[w][group] = bits;
     }
@@ -213,5 +196,9 @@ __device__ __forceinline__ float2 fma2rn(float2 a, float2 b, float2 c)
         : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
     return d;
 }
+
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+
+__device__ __forceinline__ bool finite(float v) { return fabsf(v) < __int_as_float(0x7f800000); }
 
 } // namespace u3dg
