@@ -118,3 +118,30 @@ def test_invalid_arguments_are_rejected():
     assert b"NULL" in lib.u3dg_last_error()
     assert lib.u3dg_init_gaussians_from_points(None, None, 5, None) == _abi.ERR_INVALID_ARG
     assert lib.u3dg_read_splat_ply(b"/nonexistent/x.ply", None, 0, C.byref(C.c_size_t()), None) == _abi.ERR_IO
+
+
+def test_a_batch_s_trainer_never_destroys_the_batch_s_handle(monkeypatch):
+    # The batch owns its trainers' handles, which are freed with it; a Trainer of it that lives longer must
+    # not hand the freed handle to the library.
+    from univeral_3d_reconstruction_system_b200 import api
+
+    class Library:
+        destroyed = []
+
+        def u3dg_trainer_destroy(self, h):
+            self.destroyed.append(h)
+
+        def u3dg_batch_destroy(self, h):
+            pass
+
+    library = Library()
+    monkeypatch.setattr(api, "load", lambda: library)
+    batch = api.Batch.__new__(api.Batch)
+    batch._h = 1
+    borrowed, own = api.Trainer.__new__(api.Trainer), api.Trainer.__new__(api.Trainer)
+    borrowed._h, borrowed._owner, own._h = 2, batch, 3
+    batch.close()
+    borrowed.close()
+    own.close()
+    assert library.destroyed == [3]
+    assert borrowed._h is None and own._h is None

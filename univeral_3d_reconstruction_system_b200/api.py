@@ -68,9 +68,10 @@ class Trainer:
 
     def __del__(self):
         h = getattr(self, "_h", None)
-        if h:
+        # A batch's trainer belongs to the batch, and is gone with it: the handle is not touched then.
+        if h and getattr(self, "_owner", None) is None:
             load().u3dg_trainer_destroy(h)
-            self._h = None
+        self._h = None
 
     def close(self):
         self.__del__()
