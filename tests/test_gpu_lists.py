@@ -144,3 +144,28 @@ def test_forward_kernels_agree_and_match_the_oracle(u3dg, oracle, n, opacity):
     assert out[0][2].max() > 0
     ref = oracle.render(m, left, RasterSettings(background=(0.1, 0.2, 0.3)))
     assert np.max(np.abs(out[1][0] - ref)) <= 1e-5
+
+
+@pytest.mark.parametrize("n, tiles_x, tiles_y, wide", [(1, 1, 1, 1), (511, 3, 2, 2), (512, 5, 7, 3), (513, 64, 32, 5), (2049, 45, 45, 4),
+                                                       (20_011, 64, 32, 3), (1500, 46, 45, 3), (700, 20, 15, 20)])
+def test_tile_lists_at_chunk_and_path_edges(u3dg, oracle, n, tiles_x, tiles_y, wide):
+    # Chunks of 512 ranks, their last rank and the next; exactly 2048 tiles (one tile per digit) and just
+    # more (sorted by tile id); chunks with more intersections than they list (700 Gaussians in up to 300
+    # tiles); equal depths; invisible Gaussians. Exact.
+    rng = np.random.default_rng(n + tiles_x)
+    depth = rng.choice(rng.uniform(0.5, 80.0, max(1, n // 3)).astype(np.float32), n)
+    radius = (rng.random(n) < 0.9).astype(np.int32) * 7
+    x0, y0 = rng.integers(0, tiles_x, n), rng.integers(0, tiles_y, n)
+    x1 = np.minimum(tiles_x, x0 + 1 + rng.integers(0, wide, n))
+    y1 = np.minimum(tiles_y, y0 + 1 + rng.integers(0, wide, n))
+    rect = np.stack([x0, y0, x1, y1], 1).astype(np.int32)
+    offsets, ids = u3dg.binTiles(depth, radius, rect, tiles_x, tiles_y)
+    # Rasterizer.cpp:206-261: visible Gaussians by depth, ties by index, appended to each tile of their rect.
+    lists = [[] for _ in range(tiles_x * tiles_y)]
+    for i in np.argsort(depth, kind="stable"):
+        if radius[i] > 0:
+            for ty in range(y0[i], y1[i]):
+                for tx in range(x0[i], x1[i]):
+                    lists[ty * tiles_x + tx].append(i)
+    np.testing.assert_array_equal(offsets, np.concatenate([[0], np.cumsum([len(x) for x in lists])]))
+    np.testing.assert_array_equal(ids, np.concatenate([np.array(x, np.int32) for x in lists]) if len(ids) else ids)

@@ -2,30 +2,31 @@
 //
 // The reference sorts the visible Gaussians by the float bits of their depth with a stable LSD
 // radix sort (ties keep index order), then buckets them per tile in that order, so every tile list
-// is depth-sorted. Here the same order comes from two stable radix sorts:
+// is depth-sorted. Here the same order comes from two stable sorts:
 //   1. (depth bits, Gaussian id) over all Gaussians -> depth rank; invisible ones get key
-//      0xFFFFFFFF and sort last;
-//   2. intersections are emitted in depth-rank order (an exclusive scan of per-rank tile counts
-//      gives each Gaussian its slots), keyed by tile id, and sorted stably by the tile id only.
-// Within a tile the emission order, i.e. (depth bits, id), survives, which is exactly the
-// reference's list.
+//      0xFFFFFFFF and sort last: four passes of 8 bits, a histogram and a scatter kernel each
+//      (radixSortDepth);
+//   2. the ranks' intersections, in rank order, by tile. Up to 2048 tiles (binByTile) they are never
+//      written out: a chunk of ranks counts its intersections per tile, the counts are scanned over the
+//      chunks, and the chunk then goes through its intersections again and writes each one's Gaussian id
+//      straight to its place in the tile lists. With more tiles they are emitted in rank order (an
+//      exclusive scan of per-rank tile counts gives each Gaussian its slots), keyed by tile id, and
+//      sorted by radix passes on the tile id.
+// Within a tile the rank order, i.e. (depth bits, id), survives, which is exactly the reference's list.
+// Emission order, in which the chain rule adds up a Gaussian's partials, is rank order too.
 //
-// The intersection count is only known on the device, so nothing here waits for the host: the tile
-// sort reads its item count from device memory (the depth sort takes the host-known Gaussian count),
-// grids are sized for the capacity, and a capacity check (in the scan of the per-rank tile counts)
-// turns an overflow into an empty bin list plus a flag the host reads later (it then grows the
-// buffers and replays the step).
+// The intersection count is only known on the device, so nothing here waits for the host: a capacity
+// check on the count turns an overflow into empty lists plus a flag the host reads later (it then grows
+// the buffers and replays the step). Grids of the first path follow the host-known Gaussian count; those
+// of the second are sized for the capacity.
 //
-// Sorting: stable LSD passes, 8-bit digits for the depth keys and one 11-bit pass for tile ids (up to
-// 2048 tiles; that pass's scatter also writes the tile lists' Gaussian ids and, in block 0, the tile
-// offsets, which are the exclusive scan of its digit totals). A pass is
-// three kernels: per-block digit histograms, a per-digit scan over the blocks, and a scatter whose
-// in-block ranks come from warp match-any votes. Every block owns one contiguous chunk of the items
-// and walks it in rounds of kTile items.
+// In-block ranks of the stable scatters come from warp match-any votes: each warp ranks its items among
+// equal digits and the warps' counts per digit are added in warp order.
 
 #include "tile_cull.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 
 namespace u3dg {
@@ -87,9 +88,7 @@ __device__ __forceinline__ void chunkOf(int n, int G, int b, int &begin, int &en
 }
 
 template <int DB>
-// keys, or with pairs set the (key, value) pairs' keys.
-__global__ void __launch_bounds__(kThreads) radixHistKernel(const uint32_t *keys, const uint2 *pairs, const int *nPtr,
-                                                            int nHost, int shift, int *hist, int G)
+__global__ void __launch_bounds__(kThreads) radixHistKernel(const uint32_t *keys, const int *nPtr, int shift, int *hist, int G)
 {
     pdlEntry();
     constexpr int R = 1 << DB;
@@ -98,9 +97,9 @@ __global__ void __launch_bounds__(kThreads) radixHistKernel(const uint32_t *keys
         counts[d] = 0;
     __syncthreads();
     int begin, end;
-    chunkOf(nPtr ? *nPtr : nHost, G, blockIdx.x, begin, end);
+    chunkOf(*nPtr, G, blockIdx.x, begin, end);
     for (int i = begin + threadIdx.x; i < end; i += kThreads)
-        atomicAdd(&counts[((pairs ? pairs[i].x : keys[i]) >> shift) & uint32_t(R - 1)], 1);
+        atomicAdd(&counts[(keys[i] >> shift) & uint32_t(R - 1)], 1);
     __syncthreads();
     for (int d = threadIdx.x; d < R; d += kThreads)
         hist[size_t(d) * G + blockIdx.x] = counts[d];
@@ -130,25 +129,13 @@ __global__ void __launch_bounds__(kThreads) radixRowScanKernel(int *hist, int G,
 // memory; an item's position is its digit's base + the counts of the warps before it (they hold
 // earlier items) + its rank in its warp. After the round the last item of each (warp, digit) advances
 // the digit's base and clears that count, so only the touched counts are reset.
-// kTiles (the single pass of a tile sort, digit = tile): instead of the sorted keys and values, the
-// scatter writes each entry's Gaussian id (fin.entries[pos]) and its position (fin.listPos), and block 0
-// writes the tile offsets, which are the digit bases it starts from.
-// Where a pass of the depth sort keeps its items: (key, value) pairs in and out, so each item is one
-// load and one scattered 8-byte store; the last pass writes the values only (the keys are done).
-struct PairIO {
-    const uint2 *in;    // when set: the items (keysIn / valsIn unused)
-    uint2 *out;         // when set: write (key, value) pairs
-    uint32_t *valsOnly; // when set: write the values only
-};
-
-template <int DB, bool kTiles = false>
+template <int DB>
 __global__ void __launch_bounds__(kThreads) radixScatterKernel(const uint32_t *keysIn, const uint32_t *valsIn,
                                                                uint32_t *keysOut, uint32_t *valsOut, const int *nPtr,
-                                                               int nHost, int shift, const int *hist, const int *rowTotals,
-                                                               int G, TileFinish fin, PairIO io)
+                                                               int shift, const int *hist, const int *rowTotals, int G)
 {
     pdlEntry();
-    const int n = nPtr ? *nPtr : nHost;
+    const int n = *nPtr;
     constexpr int R = 1 << DB;
     __shared__ uint8_t warpCounts[kWarps][R];
     __shared__ int base[R];
@@ -169,12 +156,6 @@ __global__ void __launch_bounds__(kThreads) radixScatterKernel(const uint32_t *k
         }
     }
     __syncthreads();
-    if (kTiles && blockIdx.x == 0) {
-        for (int d = threadIdx.x; d < fin.tiles; d += kThreads)
-            fin.tileOffsets[d] = base[d]; // block 0's row prefix is zero
-        if (threadIdx.x == 0)
-            fin.tileOffsets[fin.tiles] = n;
-    }
     const uint32_t lanesBelow = (1u << lane) - 1u;
     uint8_t *myCounts = warpCounts[warp];
     for (int r0 = begin; r0 < end; r0 += kTile) {
@@ -185,14 +166,8 @@ __global__ void __launch_bounds__(kThreads) radixScatterKernel(const uint32_t *k
         for (int r = 0; r < kItemsPerThread; ++r) {
             const int i = first + r * 32 + lane;
             const bool valid = i < end;
-            if (io.in) {
-                const uint2 kv = valid ? io.in[i] : make_uint2(0u, 0u);
-                key[r] = kv.x;
-                val[r] = kv.y;
-            } else {
-                key[r] = valid ? keysIn[i] : 0u;
-                val[r] = valid ? (valsIn ? valsIn[i] : uint32_t(i)) : 0u;
-            }
+            key[r] = valid ? keysIn[i] : 0u;
+            val[r] = valid ? (valsIn ? valsIn[i] : uint32_t(i)) : 0u;
             const int d = valid ? int((key[r] >> shift) & uint32_t(R - 1)) : R;
             digit[r] = d;
             local[r] = 0;
@@ -218,17 +193,8 @@ __global__ void __launch_bounds__(kThreads) radixScatterKernel(const uint32_t *k
                 for (int w = 0; w < warp; ++w)
                     cross += warpCounts[w][d];
                 const int pos = base[d] + cross + local[r];
-                if (kTiles) {
-                    fin.entries[pos] = fin.emitGid[val[r]];
-                    fin.listPos[val[r]] = make_int2(pos, d);
-                } else if (io.out) {
-                    io.out[pos] = make_uint2(key[r], val[r]);
-                } else if (io.valsOnly) {
-                    io.valsOnly[pos] = val[r];
-                } else {
-                    keysOut[pos] = key[r];
-                    valsOut[pos] = val[r];
-                }
+                keysOut[pos] = key[r];
+                valsOut[pos] = val[r];
                 last[r] = local[r] == int(myCounts[d]) - 1;
             }
         }
@@ -346,6 +312,473 @@ __global__ void capacityKernel(const int *total, int capacity, BinCounts *c, int
     checkCapacity(*total, capacity, c, iteration, desc);
 }
 
+// ---------------------------------------------------------------- depth sort
+
+// A pass is two kernels over chunks of the items: chunk histograms (hist[chunk][digit], so a chunk's row
+// and the rows of a digit range are contiguous), and a scatter whose blocks add up the rows themselves.
+// Every block reads every row, so the chunks are kept to about one per SM (148 rows of 1 KB: 22 MB from L2
+// per pass) and the rows are dealt out to four groups of the block's threads.
+constexpr int kDigits = 256;
+constexpr int kDepthThreads = 1024, kDepthWarps = kDepthThreads / 32, kDepthGroups = kDepthThreads / kDigits;
+constexpr int kDepthItems = 2;
+constexpr int kDepthTile = kDepthThreads * kDepthItems;
+constexpr int kDepthChunks = 160;
+
+__device__ __forceinline__ uint32_t depthDigit(uint32_t key, int shift) { return (key >> shift) & uint32_t(kDigits - 1); }
+
+__global__ void __launch_bounds__(kDepthThreads) depthHistKernel(const uint32_t *keys, const uint2 *pairs, int n, int shift,
+                                                                 int chunk, int *hist)
+{
+    pdlEntry();
+    __shared__ int counts[kDigits];
+    if (threadIdx.x < kDigits)
+        counts[threadIdx.x] = 0;
+    __syncthreads();
+    const int begin = blockIdx.x * chunk, end = min(n, begin + chunk), lane = threadIdx.x & 31;
+    for (int i0 = begin; i0 < end; i0 += kDepthThreads) {
+        const int i = i0 + threadIdx.x;
+        const int d = i < end ? int(depthDigit(pairs ? pairs[i].x : keys[i], shift)) : kDigits;
+        // One addition per distinct digit of a warp: the upper digits of depths hold few values.
+        const uint32_t peers = __match_any_sync(0xffffffffu, d);
+        if (d < kDigits && lane == __ffs(peers) - 1)
+            atomicAdd(&counts[d], __popc(peers));
+    }
+    __syncthreads();
+    if (threadIdx.x < kDigits)
+        hist[blockIdx.x * kDigits + threadIdx.x] = counts[threadIdx.x];
+}
+
+// Where a pass of the depth sort keeps its items: (key, value) pairs in and out, so each item is one
+// load and one scattered 8-byte store; the last pass writes the values only (the keys are done).
+struct PairIO {
+    const uint2 *in;    // when null: the keys, valued by their index
+    uint2 *out;         // when set: write (key, value) pairs
+    uint32_t *valsOnly; // when set: write the values only
+};
+
+__global__ void __launch_bounds__(kDepthThreads) depthScatterKernel(const uint32_t *keys, int n, int shift, int chunk,
+                                                                    const int *hist, PairIO io)
+{
+    pdlEntry();
+    __shared__ uint16_t counts[kDepthWarps][kDigits];
+    __shared__ int base[kDigits], before[kDepthGroups][kDigits], all[kDepthGroups][kDigits], warpSums[kDigits / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int begin = blockIdx.x * chunk, end = min(n, begin + chunk);
+    {
+        // This chunk's first position of a digit: all items of lower digits, plus the digit's in the chunks
+        // before.
+        const int d = tid % kDigits, group = tid / kDigits;
+        int sumBefore = 0, sumAll = 0;
+#pragma unroll 8
+        for (int c = group; c < int(gridDim.x); c += kDepthGroups) {
+            const int v = hist[c * kDigits + d];
+            sumAll += v;
+            sumBefore += c < int(blockIdx.x) ? v : 0;
+        }
+        before[group][d] = sumBefore;
+        all[group][d] = sumAll;
+        __syncthreads();
+        int total = 0, scan = 0;
+        if (tid < kDigits) {
+#pragma unroll
+            for (int g = 0; g < kDepthGroups; ++g)
+                total += all[g][tid];
+            scan = total;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, scan, o);
+                if (lane >= o)
+                    scan += y;
+            }
+            if (lane == 31)
+                warpSums[warp] = scan;
+        }
+        __syncthreads();
+        if (tid < kDigits) {
+            int at = scan - total;
+            for (int w = 0; w < warp; ++w)
+                at += warpSums[w];
+#pragma unroll
+            for (int g = 0; g < kDepthGroups; ++g)
+                at += before[g][tid];
+            base[tid] = at;
+        }
+    }
+    const uint32_t below = (1u << lane) - 1u;
+    for (int r0 = begin; r0 < end; r0 += kDepthTile) {
+        const int first = r0 + warp * (32 * kDepthItems);
+        uint2 item[kDepthItems];
+        int local[kDepthItems];
+#pragma unroll
+        for (int r = 0; r < kDepthItems; ++r) {
+            const int i = first + r * 32 + lane;
+            item[r] = i >= end ? make_uint2(0u, 0u) : io.in ? io.in[i] : make_uint2(keys[i], uint32_t(i));
+        }
+#pragma unroll
+        for (int k = 0; k < kDigits / 32; ++k)
+            counts[warp][k * 32 + lane] = 0;
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < kDepthItems; ++r) {
+            const bool valid = first + r * 32 + lane < end;
+            const int d = valid ? int(depthDigit(item[r].x, shift)) : kDigits;
+            const uint32_t peers = __match_any_sync(0xffffffffu, d);
+            int seen = 0;
+            if (valid) {
+                seen = counts[warp][d];
+                local[r] = seen + __popc(peers & below);
+            }
+            __syncwarp();
+            if (valid && lane == __ffs(peers) - 1)
+                counts[warp][d] = uint16_t(seen + __popc(peers));
+            __syncwarp();
+        }
+        __syncthreads();
+        int run = 0; // digit `tid`: the warps' counts to what the warps before hold
+        if (tid < kDigits) {
+#pragma unroll 8
+            for (int w = 0; w < kDepthWarps; ++w) {
+                const int c = counts[w][tid];
+                counts[w][tid] = uint16_t(run);
+                run += c;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kDepthItems; ++r) {
+            if (first + r * 32 + lane >= end)
+                continue;
+            const int d = int(depthDigit(item[r].x, shift));
+            const int pos = base[d] + counts[warp][d] + local[r];
+            if (io.out)
+                io.out[pos] = item[r];
+            else
+                io.valsOnly[pos] = item[r].y;
+        }
+        __syncthreads();
+        if (tid < kDigits)
+            base[tid] += run;
+    }
+}
+
+// ---------------------------------------------------------------- tile lists of up to 2048 tiles
+
+// A chunk is kRanks ranks, one per thread, a warp owning 32 consecutive ones.
+constexpr int kMaxTiles = 1 << kWideBits;
+constexpr int kRanks = 512, kRankWarps = kRanks / 32;
+
+inline int rankChunks(int n) { return std::max(1, (n + kRanks - 1) / kRanks); }
+
+// The k-th tile (row-major) in which Gaussian g with rectangle q is listed.
+__device__ __forceinline__ int2 listedTile(const SplatRec *cullRec, const uint32_t *rowTab, int tileSize, int g,
+                                           const int4 &q, int k)
+{
+    if (cullRec == nullptr) {
+        const int wdt = q.z - q.x;
+        return make_int2(q.x + k % wdt, q.y + k / wdt);
+    }
+    // The k-th reachable tile: the Gaussian's row table (one 32-byte row, two vector loads; entries past its
+    // rows are unused), then (rows beyond it, rare) the rows' spans.
+    const uint4 *tab = reinterpret_cast<const uint4 *>(rowTab + size_t(g) * kCullRows);
+    const uint4 t0 = tab[0], t1 = tab[1];
+    const uint32_t tv[kCullRows] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w};
+    const int rows = q.w - q.y;
+    int before = 0;
+#pragma unroll
+    for (int i = 0; i < kCullRows; ++i) {
+        if (i >= rows)
+            break;
+        const int through = int(tv[i] & 0xffffu);
+        if (k < through)
+            return make_int2(int(tv[i] >> 16) + (k - before), q.y + i);
+        before = through;
+    }
+    k -= before;
+    const CullShape cs = cullShape(cullRec, g);
+    for (int row = q.y + kCullRows; row < q.w; ++row) {
+        int c0, c1;
+        cullSpan(cs, q, row, tileSize, c0, c1);
+        if (k < c1 - c0)
+            return make_int2(c0 + k, row);
+        k -= c1 - c0;
+    }
+    return make_int2(q.x, q.y);
+}
+
+// A rank's Gaussian: its rectangle and, culling, the first rows' spans in registers.
+struct Listed {
+    int gid = 0, count = 0;
+    int4 q = make_int4(0, 0, 0, 0);
+    uint32_t tab[kCullRows] = {};
+};
+
+__device__ __forceinline__ Listed loadListed(const uint32_t *sortedIds, const int *tileCount, const int4 *rect,
+                                             const uint32_t *rowTab, bool cull, int r, int n)
+{
+    Listed l;
+    if (r < n) {
+        l.gid = int(sortedIds[r]);
+        l.count = tileCount[l.gid];
+        l.q = rect[l.gid];
+        if (cull) {
+            const uint4 *t = reinterpret_cast<const uint4 *>(rowTab + size_t(l.gid) * kCullRows);
+            const uint4 t0 = t[0], t1 = t[1];
+            const uint32_t v[kCullRows] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w};
+#pragma unroll
+            for (int i = 0; i < kCullRows; ++i)
+                l.tab[i] = v[i];
+        }
+    }
+    return l;
+}
+
+// f(tile) for every tile of the rank, row-major.
+template <class F>
+__device__ __forceinline__ void eachTile(const Listed &l, const SplatRec *cullRec, int tileSize, int tilesX, F &&f)
+{
+    if (l.count == 0)
+        return;
+    if (cullRec == nullptr) {
+        for (int row = l.q.y; row < l.q.w; ++row)
+            for (int c = l.q.x; c < l.q.z; ++c)
+                f(row * tilesX + c);
+        return;
+    }
+    const int rows = l.q.w - l.q.y;
+    int before = 0;
+#pragma unroll
+    for (int i = 0; i < kCullRows; ++i) {
+        if (i >= rows)
+            break;
+        const int through = int(l.tab[i] & 0xffffu), t0 = (l.q.y + i) * tilesX + int(l.tab[i] >> 16);
+        for (int c = 0; c < through - before; ++c)
+            f(t0 + c);
+        before = through;
+    }
+    if (rows > kCullRows) {
+        const CullShape cs = cullShape(cullRec, l.gid);
+        for (int row = l.q.y + kCullRows; row < l.q.w; ++row) {
+            int c0, c1;
+            cullSpan(cs, l.q, row, tileSize, c0, c1);
+            for (int c = c0; c < c1; ++c)
+                f(row * tilesX + c);
+        }
+    }
+}
+
+// hist[chunk][tile]: intersections of the chunk's ranks per tile; chunkTotals[chunk]: all of them.
+__global__ void __launch_bounds__(kRanks) tileCountKernel(TileBins b, int *hist, int *chunkTotals)
+{
+    pdlEntry();
+    extern __shared__ int counts[]; // per tile
+    __shared__ int total;
+    for (int d = threadIdx.x; d < b.tiles; d += kRanks)
+        counts[d] = 0;
+    if (threadIdx.x == 0)
+        total = 0;
+    const Listed l = loadListed(b.sortedIds, b.tileCount, b.rect, b.rowTab, b.cullRec != nullptr,
+                                blockIdx.x * kRanks + threadIdx.x, b.n);
+    __syncthreads();
+    eachTile(l, b.cullRec, b.tileSize, b.tilesX, [&](int tile) { atomicAdd(&counts[tile], 1); });
+    const int sum = __reduce_add_sync(0xffffffffu, l.count); // at most 32 * kMaxTiles
+    if ((threadIdx.x & 31) == 0)
+        atomicAdd(&total, sum);
+    __syncthreads();
+    if (threadIdx.x == 0)
+        chunkTotals[blockIdx.x] = total;
+    for (int d = threadIdx.x; d < b.tiles; d += kRanks)
+        hist[size_t(blockIdx.x) * b.tiles + d] = counts[d];
+}
+
+// Blocks of 32 tiles (a warp's lanes) by 32 groups of chunks: hist to the tile's intersections in the chunks
+// before, in place, and tileTotals. The last block: chunkTotals to the chunks' first emission, in place,
+// and the capacity check on their sum.
+constexpr int kScanThreads = 1024, kScanGroups = kScanThreads / 32;
+
+__global__ void __launch_bounds__(kScanThreads) tileScanKernel(int *hist, int chunks, int tiles, int *tileTotals,
+                                                               int *chunkTotals, ScanCapacity cap)
+{
+    pdlEntry();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (int(blockIdx.x) == int(gridDim.x) - 1) {
+        if (warp > 0)
+            return;
+        long long carry = 0;
+        for (int c0 = 0; c0 < chunks; c0 += 32) {
+            const int c = c0 + lane, v = c < chunks ? chunkTotals[c] : 0; // at most kRanks * kMaxTiles = 2^20
+            int incl = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o)
+                    incl += y;
+            }
+            if (c < chunks)
+                chunkTotals[c] = int(min(carry + incl - v, (long long)INT_MAX));
+            carry += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (lane == 0)
+            checkCapacity(int(min(carry, (long long)INT_MAX)), cap.capacity, cap.counts, cap.iteration, cap.desc);
+        return;
+    }
+    __shared__ int groupSums[kScanGroups][32];
+    const int t = blockIdx.x * 32 + lane, per = (chunks + kScanGroups - 1) / kScanGroups;
+    const int c0 = warp * per, c1 = min(chunks, c0 + per);
+    int sum = 0;
+    if (t < tiles) {
+#pragma unroll 8
+        for (int c = c0; c < c1; ++c)
+            sum += hist[size_t(c) * tiles + t];
+    }
+    groupSums[warp][lane] = sum;
+    __syncthreads();
+    if (t >= tiles)
+        return;
+    int run = 0;
+    for (int w = 0; w < warp; ++w)
+        run += groupSums[w][lane];
+    if (warp == kScanGroups - 1)
+        tileTotals[t] = run + sum;
+#pragma unroll 8
+    for (int c = c0; c < c1; ++c) {
+        const int v = hist[size_t(c) * tiles + t];
+        hist[size_t(c) * tiles + t] = run;
+        run += v;
+    }
+}
+
+// Writes the chunk's Gaussian ids to the tile lists (and, with listPos, where each emission went, and with
+// offsById each Gaussian's first emission). A warp first lists its ranks' intersections (tile and lane, in
+// rank order) and counts them per tile, the counts are added up over the block's warps in order, and each
+// warp then goes through its list, 32 intersections at a time, ranking equal tiles by match-any votes, with
+// no barrier on the way. A chunk with more than kListed intersections finds each one's rank and tile by a
+// search over the warp's lanes instead. Block 0 writes the tile offsets.
+constexpr int kListed = 10240; // 20 KB; a chunk of 512 ranks has about 4,000 on a 300k model at 640x480
+static_assert(kMaxTiles * 32 == 65536, "a tile and a lane fit in 16 bits");
+
+__global__ void __launch_bounds__(kRanks, 3) tileScatterKernel(TileBins b, const int *hist, const int *tileTotals,
+                                                            const int *chunkFirst, const BinCounts *bc)
+{
+    pdlEntry();
+    extern __shared__ int dyn[];
+    const int tiles = b.tiles, stride = (tiles + 1) / 2 * 2;
+    int *base = dyn;                                                      // per tile: the chunk's first position
+    uint16_t *offset = reinterpret_cast<uint16_t *>(dyn + stride);        // per warp and tile: the warp's next, from base
+    __shared__ int warpSums[kRankWarps], scanSums[kRankWarps];
+    __shared__ uint16_t listed[kListed];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (bc->effTotal <= 0) { // nothing listed, or an overflow
+        if (blockIdx.x == 0)
+            for (int d = tid; d <= tiles; d += kRanks)
+                b.tileOffsets[d] = 0;
+        return;
+    }
+    const Listed l = loadListed(b.sortedIds, b.tileCount, b.rect, b.rowTab, b.cullRec != nullptr, blockIdx.x * kRanks + tid, b.n);
+    for (int k = tid; k < kRankWarps * stride / 2; k += kRanks)
+        reinterpret_cast<uint32_t *>(offset)[k] = 0;
+    auto warpScan = [&](int v) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o)
+                v += y;
+        }
+        return v;
+    };
+    const int incl = warpScan(l.count), o = incl - l.count; // the rank's first intersection in its warp
+    if (lane == 31)
+        warpSums[warp] = incl;
+    // The tile lists' starts: every thread scans consecutive tiles.
+    const int per = (tiles + kRanks - 1) / kRanks;
+    int own = 0;
+    for (int k = 0; k < per; ++k)
+        own += tid * per + k < tiles ? tileTotals[tid * per + k] : 0;
+    const int scan = warpScan(own);
+    if (lane == 31)
+        scanSums[warp] = scan;
+    __syncthreads();
+    int start = scan - own, l0 = 0, all = 0; // l0: the warp's first intersection in the chunk
+#pragma unroll
+    for (int w = 0; w < kRankWarps; ++w) {
+        start += w < warp ? scanSums[w] : 0;
+        l0 += w < warp ? warpSums[w] : 0;
+        all += warpSums[w];
+    }
+    const int e0 = chunkFirst[blockIdx.x] + l0;
+    const bool fits = all <= kListed;
+    for (int k = 0; k < per; ++k) {
+        const int d = tid * per + k;
+        if (d >= tiles)
+            break;
+        base[d] = start + hist[size_t(blockIdx.x) * tiles + d];
+        if (blockIdx.x == 0)
+            b.tileOffsets[d] = start;
+        start += tileTotals[d];
+        if (blockIdx.x == 0 && d == tiles - 1)
+            b.tileOffsets[tiles] = start;
+    }
+    if (b.offsById && int(blockIdx.x) * kRanks + tid < b.n)
+        b.offsById[l.gid] = e0 + o;
+    uint16_t *mine = offset + warp * stride;
+    // (Two tiles share a word; a warp's ranks add at most 32 to each.)
+    int at = l0 + o;
+    eachTile(l, b.cullRec, b.tileSize, b.tilesX, [&](int tile) {
+        atomicAdd(reinterpret_cast<uint32_t *>(mine) + (tile >> 1), 1u << (16 * (tile & 1)));
+        if (fits)
+            listed[at++] = uint16_t(tile << 5 | lane);
+    });
+    __syncthreads();
+    for (int d = tid; d < tiles; d += kRanks) {
+        int run = 0; // at most kRanks
+#pragma unroll
+        for (int w = 0; w < kRankWarps; ++w) {
+            const int c = offset[w * stride + d];
+            offset[w * stride + d] = uint16_t(run);
+            run += c;
+        }
+    }
+    __syncthreads();
+    const int items = __shfl_sync(0xffffffffu, incl, 31);
+    const uint32_t below = (1u << lane) - 1u;
+    for (int i0 = 0; i0 < items; i0 += 32) {
+        const int i = i0 + lane;
+        int tile = kMaxTiles, gid;
+        if (fits) {
+            const int v = i < items ? listed[l0 + i] : 0;
+            gid = __shfl_sync(0xffffffffu, l.gid, v & 31);
+            if (i < items)
+                tile = v >> 5;
+        } else {
+            int owner = 0; // the last lane whose first intersection is not above i (empty ranks share the next one's)
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1)
+                if (__shfl_sync(0xffffffffu, o, owner + step) <= i)
+                    owner += step;
+            const int k = i - __shfl_sync(0xffffffffu, o, owner);
+            gid = __shfl_sync(0xffffffffu, l.gid, owner);
+            const int4 q = make_int4(__shfl_sync(0xffffffffu, l.q.x, owner), __shfl_sync(0xffffffffu, l.q.y, owner),
+                                     __shfl_sync(0xffffffffu, l.q.z, owner), __shfl_sync(0xffffffffu, l.q.w, owner));
+            if (i < items) {
+                const int2 t = listedTile(b.cullRec, b.rowTab, b.tileSize, gid, q, k);
+                tile = t.y * b.tilesX + t.x;
+            }
+        }
+        const uint32_t peers = __match_any_sync(0xffffffffu, tile);
+        int seen = 0;
+        if (i < items) {
+            seen = mine[tile];
+            const int pos = base[tile] + seen + __popc(peers & below);
+            b.entries[pos] = gid;
+            if (b.listPos)
+                b.listPos[e0 + i] = make_int2(pos, tile);
+        }
+        __syncwarp();
+        if (i < items && lane == __ffs(peers) - 1)
+            mine[tile] = uint16_t(seen + __popc(peers));
+        __syncwarp();
+    }
+}
+
 // One warp per 32 consecutive depth ranks (grid-stride): the warp writes its ranks' intersections in
 // order, 32 at a time. Each lane finds the rank of its intersection as the last of the warp's 32 start
 // offsets not above it (a binary search over lanes with shuffles; empty ranks share their start with
@@ -386,54 +819,8 @@ __global__ void __launch_bounds__(256) emitKernel(const uint32_t *sortedIds, con
             const int qx = __shfl_sync(0xffffffffu, q.x, l), qy = __shfl_sync(0xffffffffu, q.y, l);
             const int qz = __shfl_sync(0xffffffffu, q.z, l), qw = __shfl_sync(0xffffffffu, q.w, l);
             if (e < last) {
-                int k = e - ol;
-                int ty, tx;
-                if (cullRec == nullptr) {
-                    const int wdt = qz - qx;
-                    ty = qy + k / wdt;
-                    tx = qx + k % wdt;
-                } else {
-                    // The k-th reachable tile in row-major order: the Gaussian's row table, then (rows
-                    // beyond it) the rows' spans.
-                    // One 32-byte row (two vector loads) per Gaussian; entries past its rows are unused.
-                    const uint4 *tab = reinterpret_cast<const uint4 *>(rowTab + size_t(gl) * kCullRows);
-                    const uint4 t0 = tab[0], t1 = tab[1];
-                    const uint32_t tv[kCullRows] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w};
-                    const int rows = qw - qy;
-                    ty = -1;
-                    tx = qx;
-                    int before = 0;
-#pragma unroll
-                    for (int i = 0; i < kCullRows; ++i) {
-                        if (i >= rows)
-                            break;
-                        const uint32_t v = tv[i];
-                        const int through = int(v & 0xffffu);
-                        if (k < through) {
-                            ty = qy + i;
-                            tx = int(v >> 16) + (k - before);
-                            break;
-                        }
-                        before = through;
-                    }
-                    if (ty < 0) { // rare: more rows than the table holds
-                        k -= before;
-                        const CullShape csl = cullShape(cullRec, gl);
-                        const int4 qq = make_int4(qx, qy, qz, qw);
-                        ty = qy;
-                        for (int row = qy + kCullRows; row < qw; ++row) {
-                            int c0, c1;
-                            cullSpan(csl, qq, row, tileSize, c0, c1);
-                            if (k < c1 - c0) {
-                                ty = row;
-                                tx = c0 + k;
-                                break;
-                            }
-                            k -= c1 - c0;
-                        }
-                    }
-                }
-                keys[e] = uint32_t(ty * tilesX + tx);
+                const int2 t = listedTile(cullRec, rowTab, tileSize, gl, make_int4(qx, qy, qz, qw), e - ol);
+                keys[e] = uint32_t(t.y * tilesX + t.x);
                 emitGid[e] = gl;
             }
         }
@@ -448,7 +835,8 @@ __global__ void finalizeKernel(const uint32_t *sortedKeys, const uint32_t *sorte
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < total; s += gridDim.x * blockDim.x) {
         const uint32_t e = sortedEmit[s];
         entries[s] = emitGid[e];
-        listPos[e] = make_int2(s, int(sortedKeys[s]));
+        if (listPos)
+            listPos[e] = make_int2(s, int(sortedKeys[s]));
     }
 }
 
@@ -474,39 +862,42 @@ inline int grid(long long n, int t) { return int((n + t - 1) / t); }
 
 } // namespace
 
+// Lets a kernel that is about to use `need` bytes of shared memory, more than the default 48 KB, use up to
+// `most` on the current device: once per kernel and device, since the attribute belongs to the device's
+// copy of the kernel.
+template <class K>
+static void allowShared(K kernel, size_t need, size_t most, std::atomic<uint64_t> &done)
+{
+    if (need <= 48 * 1024)
+        return;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint64_t bit = uint64_t(1) << (dev & 63);
+    if (dev > 63 || !(done.load(std::memory_order_acquire) & bit)) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most));
+        done.fetch_or(bit, std::memory_order_release);
+    }
+}
+
 int radixBlocks(int nMax) { return std::max(1, std::min(kMaxBlocks, (nMax + kTile - 1) / kTile)); }
 
-size_t radixHistEntries(int nMax) { return size_t(1 << kWideBits) * size_t(radixBlocks(nMax)); }
+size_t radixHistEntries(int nMax) { return size_t(1 << 8) * size_t(radixBlocks(nMax)); }
 
-int radixDigits() { return 1 << kWideBits; }
+int radixDigits() { return kMaxTiles; }
+
+bool binsByTile(int tiles) { return tiles <= kMaxTiles; }
 
 int radixSortPairs(uint32_t *keysA, uint32_t *keysB, uint32_t *valsA, uint32_t *valsB, const int *nDev, int nMax,
-                   int bits, int *hist, int *rowTotals, uint32_t **keysOut, uint32_t **valsOut, cudaStream_t s,
-                   const TileFinish *fin, int nHost)
+                   int bits, int *hist, int *rowTotals, uint32_t **keysOut, uint32_t **valsOut, cudaStream_t s)
 {
     uint32_t *kin = keysA, *kout = keysB, *vout = valsB;
     const uint32_t *vin = nullptr;
     const int G = radixBlocks(nMax);
-    // Keys of up to 11 bits (tile ids) in one pass of 2048 digits; longer keys in 8-bit passes (three
-    // 11-bit passes over 32-bit depth keys measured slower than four 8-bit ones).
-    const bool wide = bits <= kWideBits;
-    if (!wide)
-        fin = nullptr;
-    const int db = wide ? kWideBits : 8;
     int passes = 0;
-    for (int shift = 0; shift < bits; shift += db, ++passes) {
-        if (wide) {
-            { launchPdl(radixHistKernel<kWideBits>, G, kThreads, 0, s, kin, nullptr, nDev, nHost, shift, hist, G); countLaunch(); }
-            { launchPdl(radixRowScanKernel, 1 << kWideBits, kThreads, 0, s, hist, G, rowTotals); countLaunch(); }
-            if (fin != nullptr)
-                { launchPdl(radixScatterKernel<kWideBits, true>, G, kThreads, 0, s, kin, vin, kout, vout, nDev, nHost, shift, hist, rowTotals, G, *fin, PairIO{}); countLaunch(); }
-            else
-                { launchPdl(radixScatterKernel<kWideBits>, G, kThreads, 0, s, kin, vin, kout, vout, nDev, nHost, shift, hist, rowTotals, G, TileFinish{}, PairIO{}); countLaunch(); }
-        } else {
-            { launchPdl(radixHistKernel<8>, G, kThreads, 0, s, kin, nullptr, nDev, nHost, shift, hist, G); countLaunch(); }
-            { launchPdl(radixRowScanKernel, 1 << 8, kThreads, 0, s, hist, G, rowTotals); countLaunch(); }
-            { launchPdl(radixScatterKernel<8>, G, kThreads, 0, s, kin, vin, kout, vout, nDev, nHost, shift, hist, rowTotals, G, TileFinish{}, PairIO{}); countLaunch(); }
-        }
+    for (int shift = 0; shift < bits; shift += 8, ++passes) {
+        { launchPdl(radixHistKernel<8>, G, kThreads, 0, s, kin, nDev, shift, hist, G); countLaunch(); }
+        { launchPdl(radixRowScanKernel, 1 << 8, kThreads, 0, s, hist, G, rowTotals); countLaunch(); }
+        { launchPdl(radixScatterKernel<8>, G, kThreads, 0, s, kin, vin, kout, vout, nDev, shift, hist, rowTotals, G); countLaunch(); }
         uint32_t *nk = kin;
         kin = kout;
         kout = nk;
@@ -518,20 +909,43 @@ int radixSortPairs(uint32_t *keysA, uint32_t *keysB, uint32_t *valsA, uint32_t *
     return passes;
 }
 
+// Items per depth chunk: whole tiles, at most kDepthChunks chunks.
+static int depthChunk(int n) { return kDepthTile * std::max(1, (n + kDepthTile * kDepthChunks - 1) / (kDepthTile * kDepthChunks)); }
+
 void radixSortDepth(const uint32_t *keys, uint2 *pairsA, uint2 *pairsB, uint32_t *sortedIds, int n, int *hist,
-                    int *rowTotals, cudaStream_t s)
+                    cudaStream_t s)
 {
-    const int G = radixBlocks(std::max(n, 1));
+    if (n <= 0)
+        return;
+    const int chunk = depthChunk(n), G = (n + chunk - 1) / chunk;
     const uint2 *pin = nullptr;
     uint2 *bufs[2] = {pairsA, pairsB};
     for (int pass = 0; pass < 4; ++pass) {
         const int shift = 8 * pass;
         const PairIO io{pin, pass < 3 ? bufs[pass & 1] : nullptr, pass < 3 ? nullptr : sortedIds};
-        { launchPdl(radixHistKernel<8>, G, kThreads, 0, s, keys, pin, nullptr, n, shift, hist, G); countLaunch(); }
-        { launchPdl(radixRowScanKernel, 1 << 8, kThreads, 0, s, hist, G, rowTotals); countLaunch(); }
-        { launchPdl(radixScatterKernel<8>, G, kThreads, 0, s, keys, nullptr, nullptr, nullptr, nullptr, n, shift, hist, rowTotals, G, TileFinish{}, io); countLaunch(); }
+        { launchPdl(depthHistKernel, G, kDepthThreads, 0, s, keys, pin, n, shift, chunk, hist); countLaunch(); }
+        { launchPdl(depthScatterKernel, G, kDepthThreads, 0, s, keys, n, shift, chunk, hist, io); countLaunch(); }
         pin = io.out;
     }
+}
+
+size_t binChunkEntries(int n) { return size_t(rankChunks(n)); }
+
+size_t binHistEntries(int n, int tiles)
+{
+    const size_t depth = size_t(kDepthChunks) * kDigits;
+    return binsByTile(tiles) ? std::max(depth, binChunkEntries(n) * size_t(std::max(tiles, 1))) : depth;
+}
+
+void binByTile(const TileBins &b, int *hist, int *tileTotals, int *chunkTotals, const ScanCapacity &cap, cudaStream_t s)
+{
+    const int G = rankChunks(b.n), stride = (b.tiles + 1) / 2 * 2;
+    const size_t scatterShared = size_t(stride) * (sizeof(int) + kRankWarps * sizeof(uint16_t)); // 36 bytes per tile
+    static std::atomic<uint64_t> allowed{0};
+    allowShared(tileScatterKernel, scatterShared + 24 * 1024, size_t(kMaxTiles) * 36, allowed); // with the static arrays
+    { launchPdl(tileCountKernel, G, kRanks, b.tiles * sizeof(int), s, b, hist, chunkTotals); countLaunch(); }
+    { launchPdl(tileScanKernel, (b.tiles + 31) / 32 + 1, kScanThreads, 0, s, hist, G, b.tiles, tileTotals, chunkTotals, cap); countLaunch(); }
+    { launchPdl(tileScatterKernel, G, kRanks, scatterShared, s, b, hist, tileTotals, chunkTotals, cap.counts); countLaunch(); }
 }
 
 size_t scanPartialEntries(int n) { return size_t((n + kScanTile - 1) / kScanTile) + 1; }

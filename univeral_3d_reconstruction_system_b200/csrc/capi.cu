@@ -379,7 +379,7 @@ int u3dg_trainer_set_intersection_capacity(u3dg_trainer *trainer, size_t capacit
         capacity = std::max<size_t>(capacity, 1024);
         if (capacity > size_t(INT_MAX / 16))
             throw StatusError(U3DG_ERR_CAPACITY, "capacity too large");
-        t.ws.iKeys0.release();
+        t.ws.entries.release();
         t.ws.icap = 0;
         t.ws.reserveIntersections(capacity);
     });
@@ -726,7 +726,7 @@ int u3dg_bin_tiles(const float *depth, const int *radius, const int *rect, size_
                 U3DG_CUDA(cudaMemcpyAsync(ws.cnt.p, cnt.data(), n * sizeof(int), cudaMemcpyHostToDevice, st.s));
             }
             ws.clearCounts(st.s);
-            ws.bin(st.s, 0);
+            ws.bin(st.s, 0, false);
             U3DG_CUDA(cudaGetLastError());
             U3DG_CUDA(cudaMemcpyAsync(ws.hostCounts.p, ws.counts.p, sizeof(BinCounts), cudaMemcpyDeviceToHost, st.s));
             st.sync();

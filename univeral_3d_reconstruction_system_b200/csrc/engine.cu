@@ -126,33 +126,43 @@ size_t RasterWorkspace::checkedIntersections(size_t capacity)
     return capacity;
 }
 
+// What only a binning of more than 2048 tiles needs: the emitted intersections and their sort buffers.
 template <class F>
-void RasterWorkspace::eachIntersectionBuffer(size_t capacity, F &&f)
+void RasterWorkspace::eachEmissionBuffer(size_t capacity, F &&f)
 {
     f(iKeys0, capacity);
     f(iKeys1, capacity);
     f(iVals0, capacity);
     f(iVals1, capacity);
     f(emitGid, capacity);
-    f(entries, capacity);
-    f(listPos, capacity);
-    f(partial, capacity * kPartial * size_t(partialSlots));
 }
 
 void RasterWorkspace::reserveIntersections(size_t capacity)
 {
     capacity = checkedIntersections(capacity);
-    if (int(capacity) <= icap && iKeys0.p)
+    if (int(capacity) <= icap && entries.p)
         return;
-    eachIntersectionBuffer(capacity, [](auto &b, size_t c) { b.reserve(c, true); });
+    entries.reserve(capacity, true);
     icap = int(capacity);
+    if (partial.p)
+        reservePartials();
+    if (iKeys0.p)
+        reserveEmission();
+}
+
+void RasterWorkspace::reservePartials()
+{
+    listPos.reserve(size_t(icap), true);
+    partial.reserve(size_t(icap) * kPartial * size_t(partialSlots), true);
 }
 
 void RasterWorkspace::planIntersections(DeviceSlab &slab, size_t capacity)
 {
     capacity = checkedIntersections(capacity);
-    eachIntersectionBuffer(capacity, [&](auto &b, size_t c) { slab.add(b, c); });
+    slab.add(entries, capacity);
     icap = std::max(icap, int(capacity));
+    slab.add(listPos, size_t(icap));
+    slab.add(partial, size_t(icap) * kPartial * size_t(partialSlots));
 }
 
 void RasterWorkspace::project(const Params &P, int count, const u3dg_camera &c, const u3dg_raster_settings &s,
@@ -172,7 +182,8 @@ void RasterWorkspace::project(const Params &P, int count, const u3dg_camera &c, 
     const int per = st.tile_size > 16 ? st.tile_size / 16 : 1;
     if (per * per > partialSlots) { // a tile size spanning more backward CTAs than before
         partialSlots = per * per;
-        partial.reserve(size_t(icap) * kPartial * size_t(partialSlots), true);
+        if (partial.p)
+            reservePartials();
     }
     ProjOut out{rec.p, depthKey.p, depth.p, rect.p, radius.p, flags.p, cov2d.p, cnt.p, rowTab.p, culled() ? 1 : 0};
     launchProject(P, n, cam, st, tilesX, tilesY, shRest, shDegree, out, stream, desc);
@@ -196,7 +207,7 @@ void RasterWorkspace::eachGaussianBuffer(size_t nn, F &&f)
     f(scanPartial, scanPartialEntries(int(nn)) + 1);
     f(flags, nn);
     f(cov2d, nn);
-    f(hist, std::max(radixHistEntries(std::max(int(nn), icap)), size_t(256)));
+    f(chunkTotals, binChunkEntries(int(nn)));
 }
 
 void RasterWorkspace::reserveGaussians(size_t nn)
@@ -209,7 +220,7 @@ void RasterWorkspace::planGaussians(DeviceSlab &slab, size_t nn)
     eachGaussianBuffer(std::max<size_t>(nn, 1), [&](auto &b, size_t c) { slab.add(b, c); });
 }
 
-void RasterWorkspace::planPixels(DeviceSlab &slab, size_t pixels, int tx, int ty, int tileSize)
+void RasterWorkspace::planPixels(DeviceSlab &slab, size_t count, size_t pixels, int tx, int ty, int tileSize)
 {
     // The sizes bin() and composite() reserve for such a view.
     slab.add(rgb, pixels * 3);
@@ -217,6 +228,12 @@ void RasterWorkspace::planPixels(DeviceSlab &slab, size_t pixels, int tx, int ty
     slab.add(nContrib, pixels);
     slab.add(tileOffsets, size_t(tx) * ty + 1);
     slab.add(rowTotals, size_t(radixDigits()));
+    size_t histEntries = binHistEntries(int(count), tx * ty);
+    if (!binsByTile(tx * ty)) {
+        eachEmissionBuffer(size_t(icap), [&](auto &b, size_t c) { slab.add(b, c); });
+        histEntries = std::max(histEntries, radixHistEntries(icap));
+    }
+    slab.add(hist, histEntries);
     const int pb = tileSize <= 8 ? 8 : 16;
     const int per = tileSize > pb ? tileSize / pb : 1;
     slab.add(blockStop, size_t(std::max(1, tx * per * ty * per)));
@@ -227,32 +244,45 @@ void RasterWorkspace::planPixels(DeviceSlab &slab, size_t pixels, int tx, int ty
     slab.add(unitCount, 1);
 }
 
-void RasterWorkspace::bin(cudaStream_t stream, int iteration, const StepDesc *desc)
+void RasterWorkspace::reserveEmission()
 {
+    eachEmissionBuffer(size_t(icap), [](auto &b, size_t c) { b.reserve(c, true); });
+    hist.reserve(radixHistEntries(icap));
+}
+
+void RasterWorkspace::bin(cudaStream_t stream, int iteration, bool keep, const StepDesc *desc)
+{
+    if (keep)
+        reservePartials();
     const int tiles = tilesX * tilesY;
-    hist.reserve(std::max(radixHistEntries(std::max(n, icap)), size_t(256)));
+    const bool direct = binsByTile(tiles);
+    if (!direct)
+        reserveEmission();
+    hist.reserve(binHistEntries(n, tiles));
+    chunkTotals.reserve(binChunkEntries(n));
     rowTotals.reserve(size_t(radixDigits()));
     tileOffsets.reserve(size_t(tiles) + 1);
-    uint32_t *keysOut = nullptr, *valsOut = nullptr;
-    radixSortDepth(depthKey.p, depthPairs[0].p, depthPairs[1].p, depthOrder.p, n, hist.p, rowTotals.p, stream);
-    sortedIds = depthOrder.p;
-    // The projection counted each Gaussian's tiles (and, culling, its row table); the scan takes the
-    // counts in depth-rank order.
+    radixSortDepth(depthKey.p, depthPairs[0].p, depthPairs[1].p, depthOrder.p, n, hist.p, stream);
+    // The projection counted each Gaussian's tiles (and, culling, its row table).
     const SplatRec *cullRec = culled() ? rec.p : nullptr;
-    exclusiveScanChecked(cnt.p, sortedIds, offs.p, offsById.p, n, scanPartial.p, ScanCapacity{icap, counts.p, iteration, desc},
-                         stream);
-    launchEmit(sortedIds, offs.p, rect.p, n, counts.p, icap, tilesX, cullRec, st.tile_size, rowTab.p, iKeys0.p,
+    const ScanCapacity cap{icap, counts.p, iteration, desc};
+    int2 *const positions = keep ? listPos.p : nullptr;
+    if (direct) {
+        binByTile(TileBins{depthOrder.p, cnt.p, rect.p, n, tilesX, tiles, cullRec, st.tile_size, rowTab.p, tileOffsets.p,
+                           entries.p, positions, keep ? offsById.p : nullptr},
+                  hist.p, rowTotals.p, chunkTotals.p, cap, stream);
+        return;
+    }
+    uint32_t *keysOut = nullptr, *valsOut = nullptr;
+    exclusiveScanChecked(cnt.p, depthOrder.p, offs.p, offsById.p, n, scanPartial.p, cap, stream);
+    launchEmit(depthOrder.p, offs.p, rect.p, n, counts.p, icap, tilesX, cullRec, st.tile_size, rowTab.p, iKeys0.p,
                emitGid.p, stream);
     int bits = 0;
     while ((1 << bits) < tiles)
         ++bits;
-    bits = std::max(bits, 1);
-    // Up to 2048 tiles: one pass whose scatter also writes the lists' entries and the tile offsets.
-    const TileFinish fin{emitGid.p, entries.p, listPos.p, tileOffsets.p, tiles};
-    const int tilePasses = radixSortPairs(iKeys0.p, iKeys1.p, iVals0.p, iVals1.p, &counts.p->effTotal, icap, bits,
-                                          hist.p, rowTotals.p, &keysOut, &valsOut, stream, &fin);
-    if (tilePasses != 1)
-        launchFinalizeBins(keysOut, valsOut, emitGid.p, counts.p, icap, tiles, entries.p, listPos.p, tileOffsets.p, stream);
+    radixSortPairs(iKeys0.p, iKeys1.p, iVals0.p, iVals1.p, &counts.p->effTotal, icap, bits, hist.p, rowTotals.p, &keysOut,
+                   &valsOut, stream);
+    launchFinalizeBins(keysOut, valsOut, emitGid.p, counts.p, icap, tiles, entries.p, positions, tileOffsets.p, stream);
 }
 
 void RasterWorkspace::forwardChecked(const Params &P, int count, const u3dg_camera &c, const u3dg_raster_settings &s,
@@ -451,7 +481,7 @@ TrainerImpl::TrainerImpl(const u3dg_model &initial, const u3dg_image *imgs, int 
     ws.partialSlots = std::max(ws.partialSlots, per * per);
     ws.planIntersections(slab, std::max<size_t>(size_t(1) << 20, 16 * cap));
     ws.planGaussians(slab, cap);
-    ws.planPixels(slab, maxP, maxTx, maxTy, ts);
+    ws.planPixels(slab, cap, maxP, maxTx, maxTy, ts);
     for (DevBuf<int> *b : {&keep, &cost, &costScan, &accCost, &accScan, &isSplit, &splitScan, &keepScan})
         slab.add(*b, cap + 1);
     slab.add(firstSecond, 2);
@@ -761,7 +791,7 @@ void TrainerImpl::launchStep(const StepValues &sv, const StepDesc *desc, BinCoun
     ws.project(params(), n, cam, o.raster, nullptr, 0, stream, desc);
     if (tm)
         tm->mark(1, stream);
-    ws.bin(stream, sv.d.iteration, desc);
+    ws.bin(stream, sv.d.iteration, true, desc);
     if (tm)
         tm->mark(2, stream);
     ws.composite(stream, true);

@@ -198,7 +198,7 @@ struct RasterWorkspace {
     DevBuf<uint2> depthPairs[2];           // the depth sort's (key, id) pairs between passes
     DevBuf<float> depth;
     DevBuf<int4> rect;
-    DevBuf<int> radius, cnt, offs, offsById, scanPartial, hist, rowTotals; // cnt: tiles per Gaussian (projection)
+    DevBuf<int> radius, cnt, offs, offsById, scanPartial, hist, rowTotals, chunkTotals; // cnt: tiles per Gaussian (projection)
     DevBuf<uint32_t> rowTab; // tile culling: per Gaussian, the first rows' spans (emission lookup)
     DevBuf<uint8_t> flags;
     DevBuf<float4> cov2d;
@@ -233,7 +233,6 @@ struct RasterWorkspace {
     bool culled() const { return cullTiles && tilesX < 8192; }
     u3dg_camera cam{};
     u3dg_raster_settings st{};
-    uint32_t *sortedIds = nullptr;
 
     RasterWorkspace();
     // Sizes the intersection buffers for `capacity` entries (waits for the device if they grow).
@@ -244,7 +243,7 @@ struct RasterWorkspace {
     // the tile size st.tile_size), planned into a slab instead of allocated one by one.
     void planIntersections(DeviceSlab &slab, size_t capacity);
     void planGaussians(DeviceSlab &slab, size_t count);
-    void planPixels(DeviceSlab &slab, size_t pixels, int tilesX, int tilesY, int tileSize);
+    void planPixels(DeviceSlab &slab, size_t count, size_t pixels, int tilesX, int tilesY, int tileSize);
     // Clears the overflow / abort record (stream-ordered).
     void clearCounts(cudaStream_t stream);
     // desc (may be null): the camera of a graph-captured step (see StepDesc).
@@ -252,7 +251,8 @@ struct RasterWorkspace {
                  int shDegree, cudaStream_t stream, const StepDesc *desc = nullptr);
     // Depth sort + tile binning from depthKey / rect / radius. Never waits for the device: an overflow of
     // the intersection buffers is recorded in `counts` (tagged with `iteration`) and bins nothing.
-    void bin(cudaStream_t stream, int iteration, const StepDesc *desc = nullptr);
+    // keep: also what a backward needs.
+    void bin(cudaStream_t stream, int iteration, bool keep, const StepDesc *desc = nullptr);
     // keep: also what a backward needs (RasterArgs::segment).
     void composite(cudaStream_t stream, bool keep);
     // Entries per segment of a tile list, and the segment slots and units that the intersection capacity
@@ -260,11 +260,13 @@ struct RasterWorkspace {
     static int segmentOf(int tileSize);
     size_t segmentSlots(size_t tiles) const { return size_t(icap) / size_t(segmentOf(st.tile_size)) + tiles + 1; }
     void reserveSegments();
+    // The buffers only a backward needs (listPos, partial), at the current intersection capacity.
+    void reservePartials();
     void forward(const Params &P, int count, const u3dg_camera &c, const u3dg_raster_settings &s, const float *shRest,
                  int shDegree, cudaStream_t stream, int iteration, bool keep)
     {
         project(P, count, c, s, shRest, shDegree, stream);
-        bin(stream, iteration);
+        bin(stream, iteration, keep);
         composite(stream, keep);
     }
     // A forward that is complete when it returns: waits, and on an overflow grows the intersection
@@ -283,7 +285,8 @@ struct RasterWorkspace {
     template <class F>
     void eachGaussianBuffer(size_t nn, F &&f);
     template <class F>
-    void eachIntersectionBuffer(size_t capacity, F &&f);
+    void eachEmissionBuffer(size_t capacity, F &&f);
+    void reserveEmission();
     static size_t checkedIntersections(size_t capacity);
 };
 

@@ -126,46 +126,53 @@ void launchOpacityReset(float *opac, float *mOpac, float *vOpac, int n, float ca
                         cudaStream_t s);
 
 // binning.cu
-// Blocks of a radix pass sized for at most nMax items, and the histogram entries it needs.
-int radixBlocks(int nMax);
-size_t radixHistEntries(int nMax);
-// Outputs of a tile sort done in one pass (keys of at most 11 bits, digit = tile): instead of the
-// sorted keys and values, the scatter writes every sorted entry's Gaussian id (entries[pos] =
-// emitGid[emission index]), where each emission went (listPos[emission index] = (pos, tile), in
-// emission order and so coalesced) and the tile offsets (tiles + 1 entries; the last is the item
-// count). The one scattered store per entry is 4 bytes: the scatter's cost is its scattered stores.
-struct TileFinish {
-    const int *emitGid;
-    int *entries;
-    int2 *listPos;
-    int *tileOffsets;
-    int tiles;
-};
-// Stable LSD radix sort of (key, value) pairs on key bits [0, bits); the item count is read on the
-// device from *nDev (at most nMax), or, with nDev null, is nHost (known on the host; at most nMax);
-// the initial values are the item indices. Result in *keysOut / *valsOut (one of the two buffers).
-// Returns the number of passes; rowTotals needs radixDigits() entries. fin (may be null) applies when
-// bits <= 11 (one pass): the sorted keys and values are then not written (fin->entries instead).
-int radixSortPairs(uint32_t *keysA, uint32_t *keysB, uint32_t *valsA, uint32_t *valsB, const int *nDev, int nMax,
-                   int bits, int *hist, int *rowTotals, uint32_t **keysOut, uint32_t **valsOut, cudaStream_t s,
-                   const TileFinish *fin = nullptr, int nHost = 0);
-int radixDigits();
 // The depth sort: stable sort of the n 32-bit keys (four 8-bit passes; ties keep index order), items
 // kept as (key, index) pairs between passes (pairsA / pairsB: n each); sortedIds receives the
-// indices in key order.
+// indices in key order. hist needs binHistEntries(n, 0) entries.
 void radixSortDepth(const uint32_t *keys, uint2 *pairsA, uint2 *pairsB, uint32_t *sortedIds, int n, int *hist,
-                    int *rowTotals, cudaStream_t s);
-// Exclusive prefix sum of n ints: out[0..n], out[n] = total. partial needs scanPartialEntries(n).
-size_t scanPartialEntries(int n);
-void exclusiveScan(const int *in, int *out, int n, int *partial, cudaStream_t s);
-// The scan of in[perm[i]] (the per-Gaussian tile counts in depth-rank order), fused with the bin pass's
-// capacity check (launchCapacityCheck on the total out[n], done by the scan's last kernel).
+                    cudaStream_t s);
+// The capacity check of a bin pass on its intersection count (see BinCounts).
 struct ScanCapacity {
     int capacity;
     BinCounts *counts;
     int iteration;
     const StepDesc *desc;
 };
+// Tile lists of up to 2048 tiles (binsByTile) from the depth order: the Gaussians' tiles in rank order,
+// stably by tile.
+struct TileBins {
+    const uint32_t *sortedIds; // Gaussian id per depth rank
+    const int *tileCount;      // per Gaussian: tiles it is listed in
+    const int4 *rect;
+    int n, tilesX, tiles;
+    const SplatRec *cullRec; // tile culling: the records and row tables; else null
+    int tileSize;
+    const uint32_t *rowTab;
+    int *tileOffsets; // tiles + 1
+    int *entries;     // per list position: Gaussian id
+    int2 *listPos;    // per emission: list position, tile (may be null)
+    int *offsById;    // per Gaussian: first emission (may be null)
+};
+bool binsByTile(int tiles);
+// hist needs binHistEntries(n, tiles) entries, tileTotals radixDigits(), chunkTotals binChunkEntries(n).
+void binByTile(const TileBins &b, int *hist, int *tileTotals, int *chunkTotals, const ScanCapacity &cap, cudaStream_t s);
+size_t binHistEntries(int n, int tiles);
+size_t binChunkEntries(int n);
+// With more tiles the intersections are written out (launchEmit) and sorted by tile id in 8-bit passes:
+// stable LSD radix sort of (key, value) pairs on key bits [0, bits); the item count is read on the device
+// from *nDev (at most nMax); the initial values are the item indices. Result in *keysOut / *valsOut (one
+// of the two buffers). Returns the number of passes; hist needs radixHistEntries(nMax) entries and
+// rowTotals radixDigits().
+int radixBlocks(int nMax);
+size_t radixHistEntries(int nMax);
+int radixDigits();
+int radixSortPairs(uint32_t *keysA, uint32_t *keysB, uint32_t *valsA, uint32_t *valsB, const int *nDev, int nMax,
+                   int bits, int *hist, int *rowTotals, uint32_t **keysOut, uint32_t **valsOut, cudaStream_t s);
+// Exclusive prefix sum of n ints: out[0..n], out[n] = total. partial needs scanPartialEntries(n).
+size_t scanPartialEntries(int n);
+void exclusiveScan(const int *in, int *out, int n, int *partial, cudaStream_t s);
+// The scan of in[perm[i]] (the per-Gaussian tile counts in depth-rank order), fused with the bin pass's
+// capacity check (launchCapacityCheck on the total out[n], done by the scan's last kernel).
 // outById[perm[i]] gets out[i].
 void exclusiveScanChecked(const int *in, const uint32_t *perm, int *out, int *outById, int n, int *partial,
                           const ScanCapacity &cap, cudaStream_t s);
@@ -180,9 +187,8 @@ void launchCapacityCheck(const int *total, int capacity, BinCounts *c, int itera
 void launchEmit(const uint32_t *sortedIds, const int *offs, const int4 *rect, int n, const BinCounts *c, int capacity,
                 int tilesX, const SplatRec *cullRec, int tileSize, const uint32_t *rowTab, uint32_t *keys, int *emitGid,
                 cudaStream_t s);
-// After a tile sort of several passes (more than 2048 tiles): the Gaussian id of every sorted entry, the
-// list position and tile of every emission and the tile offsets (a binary search in the sorted keys). A one-pass tile sort
-// writes both itself (TileFinish).
+// After that sort: the Gaussian id of every sorted entry, the list position and tile of every emission
+// (listPos may be null) and the tile offsets (a binary search in the sorted keys).
 void launchFinalizeBins(const uint32_t *sortedKeys, const uint32_t *sortedEmit, const int *emitGid, const BinCounts *c,
                         int capacity, int tiles, int *entries, int2 *listPos, int *tileOffsets, cudaStream_t s);
 
