@@ -13,7 +13,7 @@ void countLaunch();
 
 constexpr float kShC0 = 0.28209479177387814f; // degree-0 SH (GaussianModel.h:10)
 constexpr float kMaxAlpha = 0.99f;            // Rasterizer.cpp:13
-constexpr int kG2d = 9;                       // per-Gaussian 2D gradient: dmx dmy dA dB dC dr dg db dalpha
+constexpr int kG2d = 9;                       // per-Gaussian 2D gradient: dmx dmy da db dc dr dg db dalpha (a, b, c: 2D covariance)
 constexpr int kPartial = 12;                  // floats per list entry of the backward's partials (kG2d, padded to 3 x float4)
 
 // Device view of a GaussianModel arena: the five groups one after the other, each strided by the

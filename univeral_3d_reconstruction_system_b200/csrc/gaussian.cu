@@ -221,12 +221,10 @@ __device__ __forceinline__ void addPartial(const ChainArgs &a, const int2 &lp, f
     }
 }
 
-__device__ __forceinline__ void gatherPartials(const ChainArgs &a, int start, int cnt, float (&g)[kG2d])
+__device__ __forceinline__ void gatherPartials(const ChainArgs &a, int start, int cnt, float (&out)[kG2d])
 {
     const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int k = 0; k < kG2d; ++k)
-        g[k] = 0.0f;
+    float g[kG2d] = {};
     const int own = cnt <= kGatherLane ? cnt : 0;
     for (int k = 0; k < own; k += 4) {
         int2 lp[4];
@@ -252,6 +250,9 @@ __device__ __forceinline__ void gatherPartials(const ChainArgs &a, int start, in
                 g[k] = h[k];
         }
     }
+#pragma unroll
+    for (int k = 0; k < kG2d; ++k)
+        out[k] = float(g[k]);
 }
 
 // Rasterizer::backward pass 2 (Rasterizer.cpp:432-544) for one Gaussian per thread, fused either with
@@ -282,7 +283,7 @@ __global__ void __launch_bounds__(256, U3DG_CHAIN_MIN_BLOCKS) chainKernel(ChainA
     float gMeans[3] = {0, 0, 0}, gScales[3] = {0, 0, 0}, gQuats[4] = {0, 0, 0, 0}, gOpac = 0, gColors[3] = {0, 0, 0};
     if (a.radius[i] > 0) {
         const u3dg_camera &cam = a.desc ? a.desc->cam : a.cam;
-        const float dmx = g[0], dmy = g[1], dA = g[2], dB = g[3], dC = g[4];
+        const float dmx = g[0], dmy = g[1];
         if (a.gradAccum != nullptr) {
             const float nx = dmx * 0.5f * float(cam.width), ny = dmy * 0.5f * float(cam.height);
             a.gradAccum[i] += sqrtf(nx * nx + ny * ny);
@@ -303,13 +304,7 @@ __global__ void __launch_bounds__(256, U3DG_CHAIN_MIN_BLOCKS) chainKernel(ChainA
         Ewa p;
         ewaProject(mu, qr, ls, cam, a.st, p);
         const float z = p.pc[2];
-        const float aa = p.a, bb = p.b, cc = p.c;
-        const float det = aa * cc - bb * bb;
-        const float det2 = det * det;
-        const float da = (dA * -cc * cc + dB * bb * cc + dC * -bb * bb) / det2;
-        const float db = (dA * 2 * bb * cc + dC * 2 * aa * bb) / det2 + dB * (-1.0f / det - 2 * bb * bb / det2);
-        const float dc = (dA * -bb * bb + dB * aa * bb + dC * -aa * aa) / det2;
-        const float G00 = da, G01 = 0.5f * db, G11 = dc;
+        const float G00 = g[2], G01 = 0.5f * g[3], G11 = g[4]; // dL/dcovariance
         float dSigma[9];
 #pragma unroll
         for (int k = 0; k < 3; ++k)

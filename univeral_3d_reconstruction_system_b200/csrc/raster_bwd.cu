@@ -8,7 +8,7 @@
 // the SMs were idle 40 % of 0.33 ms; on 96x72 pixels 30 CTAs took 0.13 ms), and the transmittance
 // recovered over a whole list carried the rounding of every division.
 // A batch of entries is staged in shared memory with per-block masks as in the forward
-// (raster_common.cuh). The 9 sums per list entry (dmean2d xy, dconic ABC, drgb, dalpha) go through a
+// (raster_common.cuh). The 9 sums per list entry (dmean2d xy, dcovariance abc, drgb, dalpha) go through a
 // reduce-scatter over a block's lanes, land in a per-block shared-memory slot, and are added over the
 // 8x8 blocks in order after the batch: the result does not depend on scheduling. Each (tile, Gaussian)
 // partial is stored once, at the entry's list position (a tile's partials are contiguous); entries
@@ -51,17 +51,19 @@ struct BackwardShape {
     static constexpr int NT = BLOCKS * LPB;
 };
 
-// Turns an entry's summed moments (the entry loop) into dL/dmean2d and dL/dconic (Rasterizer.cpp:405-412):
-// with m the moments of dPow = alpha t, dmean = -(A m_x + B m_y, C m_y + B m_x), dA = -m_xx / 2,
-// dB = -m_xy, dC = -m_yy / 2.
+// Turns an entry's sums into dL/dmean2d and dL/dcovariance. With dPow = alpha t and w = conic (mean - pixel)
+// per pixel, dmean = -sum dPow w, and the covariance's gradient, which the reference reaches through the
+// conic's (Rasterizer.cpp:405-412, 432-446), is sum dPow w w^T / 2: da = sum dPow w_x^2 / 2, db = sum dPow
+// w_x w_y, dc = sum dPow w_y^2 / 2. Taken through the moments of the pixel offsets instead, an elongated
+// footprint's gradient is a difference of sums larger by its condition number; w has cancelled its square
+// root of it already.
 __device__ __forceinline__ void finishEntry(const float4 &Q, float g[kG2d])
 {
-    const float mx = Q.w * g[0], my = Q.w * g[1];
-    g[0] = -(Q.x * mx + Q.y * my);
-    g[1] = -(Q.z * my + Q.y * mx);
-    g[2] = -0.5f * (Q.w * g[2]);
-    g[3] = -(Q.w * g[3]);
-    g[4] = -0.5f * (Q.w * g[4]);
+    g[0] = -(Q.w * g[0]);
+    g[1] = -(Q.w * g[1]);
+    g[2] = 0.5f * (Q.w * g[2]);
+    g[3] = Q.w * g[3];
+    g[4] = 0.5f * (Q.w * g[4]);
 }
 
 // Sum of c[0..8] over the LPB lanes of a block: values 0..7 by reduce-scatter (three exchanges halve the
@@ -256,7 +258,8 @@ __device__ __forceinline__ void backwardUnit(const RasterArgs &a, int block, int
             if (!__any_sync(0xffffffffu, act))
                 continue;
             const float4 R = sR[jj];
-            float2 s5, s6, s7, st, sy, syy;
+            const float adx = Q.x * dx;
+            float2 s5, s6, s7, st, sx, sy, sxx, sxy, syy;
 #pragma unroll
             for (int p = 0; p < PAIRS; ++p) {
                 // One back-to-front step of Rasterizer.cpp:385-416 for two pixels. Transmittance before
@@ -292,23 +295,25 @@ __device__ __forceinline__ void backwardUnit(const RasterArgs &a, int block, int
                     e2 = only(e2);
                 }
                 acc[p] = next;
-                // Colour sums, and the moments of t in the pixel offsets: the mean and conic gradients are
-                // linear in them (finishEntry combines them with the conic and alpha once per entry); the
-                // lane's pixels share dx, which multiplies their sums once.
-                const float2 ty = mul2rn(t, dy[p]);
+                // Colour sums, and the sums of t, t w and t w w^T (finishEntry).
+                const float2 wx = fma2rn(both(Q.y), dy[p], both(adx)), wy = fma2rn(both(Q.z), dy[p], both(ct.bx));
+                const float2 tx = mul2rn(t, wx), ty = mul2rn(t, wy);
                 s5 = p ? fma2rn(wv, e0, s5) : mul2rn(wv, e0);
                 s6 = p ? fma2rn(wv, e1, s6) : mul2rn(wv, e1);
                 s7 = p ? fma2rn(wv, e2, s7) : mul2rn(wv, e2);
                 st = p ? add2rn(st, t) : t;
+                sx = p ? add2rn(sx, tx) : tx;
                 sy = p ? add2rn(sy, ty) : ty;
-                syy = p ? fma2rn(ty, dy[p], syy) : mul2rn(ty, dy[p]);
+                sxx = p ? fma2rn(tx, wx, sxx) : mul2rn(tx, wx);
+                sxy = p ? fma2rn(tx, wy, sxy) : mul2rn(tx, wy);
+                syy = p ? fma2rn(ty, wy, syy) : mul2rn(ty, wy);
             }
             float c[kG2d];
             c[8] = st.x + st.y;
-            c[0] = dx * c[8];
+            c[0] = sx.x + sx.y;
             c[1] = sy.x + sy.y;
-            c[2] = dx * c[0];
-            c[3] = dx * c[1];
+            c[2] = sxx.x + sxx.y;
+            c[3] = sxy.x + sxy.y;
             c[4] = syy.x + syy.y;
             c[5] = s5.x + s5.y;
             c[6] = s6.x + s6.y;
