@@ -140,40 +140,65 @@ __device__ __forceinline__ void backwardUnit(const RasterArgs &a, int block, int
     // what the forward kept where the next segment begins, and acc the colours it kept of the segments
     // behind (positive terms, added from the back) over T.
     float2 T[PAIRS], acc[PAIRS], d0[PAIRS], d1[PAIRS], d2[PAIRS], nfy[PAIRS], fb[PAIRS];
-    int nC[PPL];
-    int bMax = 0; // no pixel of this 8x8 block has a contributor at or beyond bMax: entries from there are skipped
-    bool odd = false; // a non-finite dL/dpixel or kept colour
+    int nC[PPL], last[PPL];
+    size_t pix[PPL];
+    int lastSegment = 0; // the furthest segment a pixel of the lane blends in
 #pragma unroll
     for (int k = 0; k < PPL; ++k) {
         const int y = py + k * RS;
         const bool in = px < a.width && y < a.height;
-        const size_t pix = in ? size_t(y) * a.width + px : 0;
-        const float g0 = in ? dLdRgb[pix * 3] : 0.0f, g1 = in ? dLdRgb[pix * 3 + 1] : 0.0f,
-                    g2 = in ? dLdRgb[pix * 3 + 2] : 0.0f;
-        const int last = in ? nContribIn[pix] : 0;
-        const float fT = in && (kBg || last <= jEnd) ? finalTIn[pix] : 0.0f;
-        float behind = 0.0f, t = fT;
-        if (last > jEnd) {
-            const float4 *ck = a.ck + slotPixel(a.tileSize, px, y);
-            const int slot = start / a.segment + tile, area = a.tileSize * a.tileSize;
-            for (int s = (last - 1) / a.segment; s > segment; --s) {
-                const float4 c = ck[size_t(slot + s) * area];
-                behind += c.x * g0 + c.y * g1 + c.z * g2;
-                t = c.w;
+        pix[k] = in ? size_t(y) * a.width + px : 0;
+        last[k] = in ? nContribIn[pix[k]] : 0;
+        lastSegment = max(lastSegment, (last[k] - 1) / a.segment);
+    }
+    float behind[PPL], t[PPL], fT[PPL], g0[PPL], g1[PPL], g2[PPL];
+#pragma unroll
+    for (int k = 0; k < PPL; ++k) {
+        const bool in = last[k] > 0;
+        g0[k] = in ? dLdRgb[pix[k] * 3] : 0.0f;
+        g1[k] = in ? dLdRgb[pix[k] * 3 + 1] : 0.0f;
+        g2[k] = in ? dLdRgb[pix[k] * 3 + 2] : 0.0f;
+        fT[k] = in && (kBg || last[k] <= jEnd) ? finalTIn[pix[k]] : 0.0f;
+        t[k] = fT[k];
+        behind[k] = 0.0f;
+    }
+    {
+        // The segments behind, for all of the lane's pixels at a time so that their loads overlap.
+        const int area = a.tileSize * a.tileSize;
+        const float4 *ck = a.ck + size_t(start / a.segment + tile) * area;
+#pragma unroll 2
+        for (int s = lastSegment; s > segment; --s) {
+            float4 c[PPL];
+#pragma unroll
+            for (int k = 0; k < PPL; ++k)
+                c[k] = last[k] > s * a.segment ? ck[size_t(s) * area + slotPixel(a.tileSize, px, py + k * RS)]
+                                               : make_float4(0.0f, 0.0f, 0.0f, t[k]);
+#pragma unroll
+            for (int k = 0; k < PPL; ++k) {
+                if (last[k] > s * a.segment) {
+                    behind[k] += c[k].x * g0[k] + c[k].y * g1[k] + c[k].z * g2[k];
+                    t[k] = c[k].w;
+                }
             }
-            behind = t > 0.0f ? behind / t : 0.0f; // (an underflown T: nothing behind is seen)
         }
-        nC[k] = min(last, jEnd);
+    }
+    int bMax = 0; // no pixel of this 8x8 block has a contributor at or beyond bMax: entries from there are skipped
+    bool odd = false; // a non-finite dL/dpixel or kept colour
+#pragma unroll
+    for (int k = 0; k < PPL; ++k) {
+        if (last[k] > jEnd)
+            behind[k] = t[k] > 0.0f ? behind[k] / t[k] : 0.0f; // (an underflown T: nothing behind is seen)
+        nC[k] = min(last[k], jEnd);
         bMax = max(bMax, nC[k]);
-        const float b = kBg ? -fT * (a.bg[0] * g0 + a.bg[1] * g1 + a.bg[2] * g2) : 0.0f;
-        odd = odd || !finite(g0) || !finite(g1) || !finite(g2) || !finite(t) || !finite(b) || !finite(behind);
+        const float b = kBg ? -fT[k] * (a.bg[0] * g0[k] + a.bg[1] * g1[k] + a.bg[2] * g2[k]) : 0.0f;
+        odd = odd || !finite(g0[k]) || !finite(g1[k]) || !finite(g2[k]) || !finite(t[k]) || !finite(b) || !finite(behind[k]);
         auto set = [&](float2 *v, float x) { (k & 1 ? v[k / 2].y : v[k / 2].x) = x; };
-        set(T, t);
-        set(acc, behind);
-        set(d0, g0);
-        set(d1, g1);
-        set(d2, g2);
-        set(nfy, -float(y));
+        set(T, t[k]);
+        set(acc, behind[k]);
+        set(d0, g0[k]);
+        set(d1, g1[k]);
+        set(d2, g2[k]);
+        set(nfy, -float(py + k * RS));
         set(fb, b);
     }
 #pragma unroll
