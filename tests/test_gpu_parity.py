@@ -728,3 +728,17 @@ def test_training_recovers_a_synthetic_scene(u3dg, oracle):
     assert after > before + 8.0, (before, after)
     assert after > 26.0, after
     assert t.model().size() != init.size()
+
+
+def test_stats_are_those_of_the_last_step(u3dg, tiny_scene, oracle):
+    """stats() straight after a single step, against a second trainer whose stream was waited for first."""
+    sc = tiny_scene
+    init = oracle.init_from_points(sc.init_xyz, sc.init_rgb)
+    a, b = (u3dg.Trainer(init, sc.images, sc.extent, TrainOptions.for_iterations(400)) for _ in range(2))
+    for k in range(100):
+        a.step(1)
+        sa = a.stats()
+        b.step(1)
+        b.model()
+        sb = b.stats()
+        assert (sa.iteration, sa.loss, sa.psnr) == (sb.iteration, sb.loss, sb.psnr), k

@@ -834,6 +834,8 @@ void TrainerImpl::enqueueStep()
     f.slot = nextSlot;
     nextSlot = (nextSlot + 1) % kSlots;
     launchStep(sv, nullptr, statusSlots.p + f.slot);
+    // Before the event that finish() waits for: stats() reads the copy.
+    U3DG_CUDA(cudaMemcpyAsync(hStats.p, dStats.p, sizeof(DevStats), cudaMemcpyDeviceToHost, stream));
     ++normalSteps;
     ++iteration;
     if (freeEvents.empty()) {
@@ -856,7 +858,6 @@ void TrainerImpl::enqueueStep()
     }
     if (o.opacity_reset_interval > 0 && iteration < o.refine_stop && iteration % o.opacity_reset_interval == 0)
         resetOpacity();
-    U3DG_CUDA(cudaMemcpyAsync(hStats.p, dStats.p, sizeof(DevStats), cudaMemcpyDeviceToHost, stream));
     PhaseTimer *tm = profiling ? timer : nullptr;
     if (tm) {
         tm->mark(7, stream);
