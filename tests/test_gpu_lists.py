@@ -63,6 +63,17 @@ def test_backward_at_segment_edges(u3dg, oracle, n, tile):
     _close(u3dg, oracle, mixed, cam, RasterSettings(tile_size=tile), w, 1e-4)
 
 
+@pytest.mark.parametrize("width, height, n", [(368, 400, 40), (480, 352, 40), (480, 352, 90)])
+@pytest.mark.parametrize("background", [(0.0, 0.0, 0.0), (0.2, 0.4, 0.1)])
+def test_backward_with_few_and_many_units(u3dg, oracle, width, height, n, background):
+    # 575 blocks of 16x16 with one segment each (a unit per CTA at 592 CTAs and more), 660, and 660 with two.
+    # Sums of up to 170,000 pixels in another order: 2^-24 sqrt(170,000) times a cancellation of 10 is 2.5e-4.
+    rng = np.random.default_rng(n)
+    w = rng.uniform(-1, 1, (height, width, 3)).astype(np.float32)
+    _close(u3dg, oracle, _stack(n, rng, 0.05), make_camera(width, height, 1.5 * width), RasterSettings(background=background), w,
+           3e-4)
+
+
 def test_a_non_finite_pixel_gradient_reaches_only_what_blends_there(u3dg):
     rng = np.random.default_rng(3)
     m = random_model(200, rng, 1.0, 3.0, 0.02, 0.1)

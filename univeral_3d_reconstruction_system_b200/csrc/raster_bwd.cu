@@ -38,17 +38,18 @@ namespace u3dg {
 
 namespace {
 
-// Pixels and threads of the backward: LPB lanes own one 8x8 pixel block, PPL = 64 / LPB pixels each, in
-// one column (rows r, r + LPB / 8, ...). LPB = 16 (16x16 CTAs): a warp holds two blocks, left and right,
-// that walk their own entry masks in step, so the reduction (12 shuffles over 16 lanes), the entry's
-// loads and the loop are paid once for two (block, entry) pairs and a lane adds four pixels before it.
-// LPB = 32 (8x8 CTAs, tile size 8): one block per warp.
-template <int PB>
+// Pixels and threads of a unit: L lanes own one 8x8 pixel block, PPL = 64 / L pixels each, in one column
+// (rows r, r + L / 8, ...). L = 16: a warp holds two blocks, left and right, that walk their own entry masks
+// in step, so the reduction (12 shuffles over 16 lanes), the entry's loads and the loop are paid once for two
+// (block, entry) pairs and a lane adds four pixels before it. L = 32: one block per warp, which takes 1.3
+// times the instructions for the same entries but 0.6 of the time for one of them.
+template <int PB, int L>
 struct BackwardShape {
-    static constexpr int LPB = PB == 8 ? 32 : 16;
+    static constexpr int LPB = L;
     static constexpr int PPL = 64 / LPB, PAIRS = PPL / 2;
     static constexpr int WX = PB / 8, BLOCKS = WX * WX;
     static constexpr int NT = BLOCKS * LPB;
+    static constexpr int BATCH = PB == 8 ? 32 : 64; // entries staged at a time (times the depth)
 };
 
 // Turns an entry's sums into dL/dmean2d and dL/dcovariance. With dPow = alpha t and w = conic (mean - pixel)
@@ -112,18 +113,25 @@ __device__ __forceinline__ float rcpApprox(float x)
     return y;
 }
 
-template <int PB, int BD, bool kBg>
+// Barrier of the NT threads that work on one unit.
+template <int NT>
+__device__ __forceinline__ void teamSync(int barrier)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(barrier), "r"(NT) : "memory");
+}
+
+template <int PB, int L, int BD, bool kBg>
 __device__ __forceinline__ void backwardUnit(const RasterArgs &a, int block, int segment, const float *dLdRgb,
                                              const float *finalTIn, const int *nContribIn, float *partial,
                                              const int *stop, float4 *sP, float4 *sQ, float4 *sR,
-                                             uint32_t (*mask)[BackwardShape<PB>::NT * BD / 32], int &sOdd,
-                                             float *sBlock)
+                                             uint32_t (*mask)[BackwardShape<PB, L>::BATCH * BD / 32], int &sOdd,
+                                             float *sBlock, int tid, int barrier)
 {
-    using S = BackwardShape<PB>;
+    using S = BackwardShape<PB, L>;
     constexpr int NT = S::NT, LPB = S::LPB, PPL = S::PPL, PAIRS = S::PAIRS, BLOCKS = S::BLOCKS;
-    constexpr int NB = NT * BD, NG = NB / 32, RS = LPB / 8; // batch entries, mask words, row step of a lane's pixels
+    constexpr int NB = S::BATCH * BD, NG = NB / 32, RS = LPB / 8; // batch entries, mask words, row step of a lane's pixels
     const int bx = block % a.blocksX, by = block / a.blocksX;
-    const int tid = threadIdx.x, lane = tid & 31, blk = tid / LPB, bl = tid % LPB;
+    const int lane = tid & 31, blk = tid / LPB, bl = tid % LPB;
     const int tile = tileOf<PB>(a, bx, by);
     const int start = a.tileOffsets[tile];
     // The unit's entries [jBegin, jEnd) of the tile's list.
@@ -213,7 +221,7 @@ __device__ __forceinline__ void backwardUnit(const RasterArgs &a, int block, int
     const float4 *rec = reinterpret_cast<const float4 *>(a.rec);
     for (int bEnd = jEnd; bEnd > jBegin; bEnd -= NB) {
         const int bStart = max(jBegin, bEnd - NB), cnt = bEnd - bStart;
-        __syncthreads();
+        teamSync<NT>(barrier);
         if (tid == 0)
             sOdd = 0;
         {
@@ -221,17 +229,19 @@ __device__ __forceinline__ void backwardUnit(const RasterArgs &a, int block, int
             for (int k = tid; k < BLOCKS * NB * kG2d / 4; k += NT)
                 z[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
-        __syncthreads();
+        teamSync<NT>(barrier);
 #pragma unroll
-        for (int r = 0; r < BD; ++r) {
+        for (int r = 0; r < (NB + NT - 1) / NT; ++r) {
             const int slot = r * NT + tid;
+            if (slot >= NB) // whole warps
+                break;
             const bool valid = slot < cnt;
             stage<S::WX, NG>(loadRecord(rec, valid ? a.entries[start + bStart + slot] : -1), valid, slot, sP, sQ, sR, mask, bx,
                           by);
             if (valid && !(finite(sR[slot].x) && finite(sR[slot].y) && finite(sR[slot].z)))
                 sOdd = 1;
         }
-        __syncthreads();
+        teamSync<NT>(barrier);
         // A non-finite colour or dL/dpixel must reach only the pixels and entries that blend: then the
         // factors of pixels that do not are replaced by zeros (0 * inf is not 0).
         const bool strict = odd || sOdd != 0;
@@ -348,9 +358,9 @@ __device__ __forceinline__ void backwardUnit(const RasterArgs &a, int block, int
             if (has && (storeV || store8))
                 mine[jj * kG2d + storeAt] = storeV ? v : v8;
         }
-        __syncthreads();
+        teamSync<NT>(barrier);
 #pragma unroll
-        for (int r = 0; r < BD; ++r) {
+        for (int r = 0; r < (NB + NT - 1) / NT; ++r) {
             const int e = r * NT + tid;
             if (e >= cnt)
                 break;
@@ -371,31 +381,69 @@ __device__ __forceinline__ void backwardUnit(const RasterArgs &a, int block, int
     }
 }
 
-// Resident CTAs per SM the compiler must allow for at 64 threads (16x16 blocks): caps registers per
-// thread at 65536 / (64 * n).
+// Teams of 64 threads per SM the compiler must allow for (16x16 blocks): caps registers per thread at
+// 65536 / (64 * n).
 #ifndef U3DG_BWD_MIN_BLOCKS
 #define U3DG_BWD_MIN_BLOCKS 8
 #endif
 
+// A CTA of 16x16 blocks has 128 threads: two teams of 64 (16 lanes per 8x8 block), each with a unit of its
+// own, or, where the launch has no more units than CTAs, one team of 128 (32 lanes). Then the launch lasts as
+// long as one unit, 64 entries at about 800 cycles each by 16 lanes (a warp alone on its scheduler): 52 us
+// against 38 us on 4k Gaussians at 96x72. With more units than CTAs the instructions count: at two units
+// per CTA the two shapes are even (+-2 us of 60), on 300k Gaussians at 640x480 32 lanes take 169 us against
+// 143.
+template <int PB>
+constexpr int kTeams = PB == 8 ? 1 : 2;
+template <int PB>
+constexpr int kThreads = PB == 8 ? 32 : 128;
+
+template <int PB, int L, int BD, bool kBg>
+__device__ __forceinline__ void backwardUnits(const RasterArgs &a, const float *dLdRgb, const float *finalTIn,
+                                              const int *nContribIn, float *partial, const int *stop, const int2 *units,
+                                              int count, float4 *sP, float4 *sQ, float4 *sR,
+                                              uint32_t (*mask)[BackwardShape<PB, L>::BATCH * BD / 32], int &sOdd,
+                                              int &sNext, float *sBlock)
+{
+    constexpr int NT = BackwardShape<PB, L>::NT;
+    const int tid = threadIdx.x % NT, barrier = threadIdx.x / NT;
+    for (;;) {
+        teamSync<NT>(barrier); // every thread is done with the previous unit's shared memory
+        if (tid == 0)
+            sNext = takeUnit(count, a.counters, gridDim.x * (kThreads<PB> / NT));
+        teamSync<NT>(barrier);
+        const int u = sNext;
+        if (u >= count)
+            break;
+        const int2 unit = units[u];
+        backwardUnit<PB, L, BD, kBg>(a, unit.x, unit.y, dLdRgb, finalTIn, nContribIn, partial, stop, sP, sQ, sR, mask,
+                                     sOdd, sBlock, tid, barrier);
+    }
+}
+
 template <int PB, int BD, bool kBg>
-__global__ void __launch_bounds__(BackwardShape<PB>::NT, U3DG_BWD_MIN_BLOCKS * 64 / BackwardShape<PB>::NT)
+__global__ void __launch_bounds__(kThreads<PB>, U3DG_BWD_MIN_BLOCKS * 64 / kThreads<PB>)
     compositeBackwardKernel(RasterArgs a, const float *dLdRgb, const float *finalTIn, const int *nContribIn,
                             float *partial, const int *stop, const int2 *units, const int *unitCount)
 {
     pdlEntry();
-    using S = BackwardShape<PB>;
-    constexpr int NB = S::NT * BD, NG = NB / 32;
-    __shared__ float4 sP[NB];
-    __shared__ float4 sQ[NB];
-    __shared__ float4 sR[NB];
-    __shared__ uint32_t mask[S::BLOCKS][NG];
-    __shared__ int sOdd, sNext;
-    extern __shared__ __align__(16) float sBlock[]; // per 8x8 block: NB entries x 9 sums
+    using S = BackwardShape<PB, PB == 8 ? 32 : 16>;
+    constexpr int NB = S::BATCH * BD, NG = NB / 32, TEAMS = kTeams<PB>;
+    __shared__ float4 sP[TEAMS][NB];
+    __shared__ float4 sQ[TEAMS][NB];
+    __shared__ float4 sR[TEAMS][NB];
+    __shared__ uint32_t mask[TEAMS][S::BLOCKS][NG];
+    __shared__ int sOdd[TEAMS], sNext[TEAMS];
+    extern __shared__ __align__(16) float sBlock[]; // per team and 8x8 block: NB entries x 9 sums
     const int count = *unitCount;
-    for (int u = nextUnit(count, a.counters, &sNext); u < count; u = nextUnit(count, a.counters, &sNext)) {
-        const int2 unit = units[u];
-        backwardUnit<PB, BD, kBg>(a, unit.x, unit.y, dLdRgb, finalTIn, nContribIn, partial, stop, sP, sQ, sR, mask,
-                                  sOdd, sBlock);
+    if (PB == 8 || count <= int(gridDim.x)) {
+        backwardUnits<PB, 32, BD, kBg>(a, dLdRgb, finalTIn, nContribIn, partial, stop, units, count, sP[0], sQ[0], sR[0],
+                                       mask[0], sOdd[0], sNext[0], sBlock);
+    } else {
+        const int team = threadIdx.x / S::NT;
+        backwardUnits<PB, PB == 8 ? 32 : 16, BD, kBg>(a, dLdRgb, finalTIn, nContribIn, partial, stop, units, count, sP[team], sQ[team],
+                                       sR[team], mask[team], sOdd[team], sNext[team],
+                                       sBlock + size_t(team) * S::BLOCKS * NB * kG2d);
     }
 }
 
@@ -469,13 +517,13 @@ template <int PB, int BD, bool kBg>
 static void launchBackward(const RasterArgs &a, const float *dLdRgb, const float *finalT, const int *nContrib,
                            float *partial, const int *stop, const int2 *units, const int *unitCount, cudaStream_t s)
 {
-    using S = BackwardShape<PB>;
-    const size_t smem = size_t(S::BLOCKS) * S::NT * BD * kG2d * sizeof(float); // 9 KB or 18 KB at PB 16
+    using S = BackwardShape<PB, 32>;
+    const size_t smem = size_t(kTeams<PB>) * S::BLOCKS * S::BATCH * BD * kG2d * sizeof(float); // 18 KB or 36 KB at PB 16
     static const int ctas = [&] {
         cudaFuncSetAttribute(compositeBackwardKernel<PB, BD, kBg>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        return residentCtas(compositeBackwardKernel<PB, BD, kBg>, S::NT, smem);
+        return residentCtas(compositeBackwardKernel<PB, BD, kBg>, kThreads<PB>, smem);
     }();
-    { launchPdl(compositeBackwardKernel<PB, BD, kBg>, ctas, S::NT, smem, s, a, dLdRgb, finalT, nContrib, partial, stop, units, unitCount); countLaunch(); }
+    { launchPdl(compositeBackwardKernel<PB, BD, kBg>, ctas, kThreads<PB>, smem, s, a, dLdRgb, finalT, nContrib, partial, stop, units, unitCount); countLaunch(); }
 }
 
 void launchBackwardUnits(const RasterArgs &a, int *stop, int2 *units, int *unitCount, cudaStream_t s)

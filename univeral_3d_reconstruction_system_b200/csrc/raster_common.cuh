@@ -50,25 +50,20 @@ __device__ __forceinline__ int tileOf(const RasterArgs &a, int bx, int by)
     return (by * PB / a.tileSize) * a.tilesX + bx * PB / a.tileSize;
 }
 
-// Persistent scheduling: every CTA takes work units from a device counter until none are left. Returns
-// the next unit's index for the whole CTA (>= units: done); the last CTA to run out resets the counter
-// for the next launch. counter[0] hands out units, counter[1] counts finished CTAs.
-__device__ __forceinline__ int nextUnit(int units, int *counter, int *sNext)
+// Persistent scheduling: every team of threads takes work units from a device counter until none are left.
+// Called by one thread of a team; returns the next unit's index (>= units: done). The last team to run out
+// resets the counter for the next launch. counter[0] hands out units, counter[1] counts finished teams.
+__device__ __forceinline__ int takeUnit(int units, int *counter, int teams)
 {
-    __syncthreads(); // every thread is done with the previous unit's shared memory
-    if (threadIdx.x == 0) {
-        int u = atomicAdd(counter, 1);
-        if (u >= units) {
-            __threadfence();
-            if (atomicAdd(counter + 1, 1) == int(gridDim.x) - 1) {
-                atomicExch(counter, 0);
-                atomicExch(counter + 1, 0);
-            }
+    const int u = atomicAdd(counter, 1);
+    if (u >= units) {
+        __threadfence();
+        if (atomicAdd(counter + 1, 1) == teams - 1) {
+            atomicExch(counter, 0);
+            atomicExch(counter + 1, 0);
         }
-        *sNext = u;
     }
-    __syncthreads();
-    return *sNext;
+    return u;
 }
 
 // Index of a pixel in its tile's segment slot (RasterArgs::ck).
