@@ -742,3 +742,30 @@ def test_stats_are_those_of_the_last_step(u3dg, tiny_scene, oracle):
         b.model()
         sb = b.stats()
         assert (sa.iteration, sa.loss, sa.psnr) == (sb.iteration, sb.loss, sb.psnr), k
+
+
+@pytest.mark.parametrize("lr", [1e-32, 1e-2, 1e22])
+def test_first_adam_step_at_any_step_size(u3dg, oracle, tiny_scene, lr):
+    """The first step moves an element with gradient g by lr |g| / (|g| + 1e-15) (Adam.cpp's bias-corrected
+    moments): by lr where |g| is above 1e-9, whatever the size of lr (the fused quotient has a range of its
+    own and the operators outside it). 32-bit rounding of m, v, the root and the quotient: 1e-6, and of
+    p + lr at lr = 0.01: |p| 2^-24 / 0.01 < 6e-5 for |p| < 10. At 1e-32 nothing moves."""
+    from univeral_3d_reconstruction_system_b200.types import LearningRates
+
+    sc = tiny_scene
+    init = oracle.init_from_points(sc.init_xyz, sc.init_rgb)
+    opt = TrainOptions.for_iterations(400).replace(lr=LearningRates(means=lr, scales=lr, quats=lr, opacities=lr, colors=lr),
+                                                   means_lr_final=lr)
+    t = u3dg.Trainer(init, sc.images, sc.extent, opt)
+    t.step(1)
+    m = t.model()
+    for k in ("scales", "opacities", "colors"):  # (quats of spheres have no gradient)
+        a, b = getattr(init, k).astype(np.float64).ravel(), getattr(m, k).astype(np.float64).ravel()
+        moved = np.abs(b - a)
+        if lr < 1e-20:
+            assert np.array_equal(a, b), k
+            continue
+        assert moved.max() <= lr * (1 + 1e-4), k
+        some = moved[moved > 0.5 * lr]
+        assert some.size > 0.3 * a.size, (k, some.size, a.size)
+        assert np.median(np.abs(some / lr - 1)) <= 1e-4, k

@@ -94,10 +94,40 @@ struct Ewa {
     float a, b, c;
 };
 
+// Several divisions by one divisor, each correctly rounded by Markstein's sequence (IBM Journal of Research
+// and Development 34, 1990): the quotient by the correctly rounded reciprocal, corrected by its exact
+// remainder. For |a| and quotients between 2^-100 and 2^100 the result has the bits of a / b (3.7e10 quotients
+// compared); an infinite quotient, whose remainder is NaN, is kept.
+struct Divisor {
+    float b, y;
+    __device__ __forceinline__ explicit Divisor(float d) : b(d), y(1.0f / d) {}
+    __device__ __forceinline__ float under(float a) const
+    {
+        const float q = __fmul_rn(a, y);
+        const float c = __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+        return c == c ? c : q;
+    }
+};
+
+// Bounds of x / z and y / z outside which the projection's Jacobian is clamped, the same for all Gaussians of
+// a view. All lanes of a warp call it; four of them divide.
+struct ViewLimits {
+    float xPos, xNeg, yPos, yNeg;
+};
+
+__device__ __forceinline__ ViewLimits viewLimits(const u3dg_camera &cam)
+{
+    const int which = threadIdx.x & 3;
+    const float size = float(which < 2 ? cam.width : cam.height), f = which < 2 ? cam.fx : cam.fy, c = which < 2 ? cam.cx : cam.cy;
+    const float lim = (which & 1 ? c : size - c) / f + 0.3f * 0.5f * size / f;
+    return {__shfl_sync(0xffffffffu, lim, 0), __shfl_sync(0xffffffffu, lim, 1), __shfl_sync(0xffffffffu, lim, 2),
+            __shfl_sync(0xffffffffu, lim, 3)};
+}
+
 // EWA projection of Gaussian i (computeProjection, Rasterizer.cpp:48-110), same operation order;
 // files including this are compiled with -fmad=false so no multiply-add is contracted.
 __device__ __forceinline__ bool ewaProject(const float mu[3], const float qr[4], const float ls[3],
-                                           const u3dg_camera &cam, const u3dg_raster_settings &st, Ewa &p)
+                                           const u3dg_camera &cam, const ViewLimits &lim, const u3dg_raster_settings &st, Ewa &p)
 {
     const float *R = cam.R;
     p.pc[0] = R[0] * mu[0] + R[1] * mu[1] + R[2] * mu[2] + cam.t[0];
@@ -112,9 +142,10 @@ __device__ __forceinline__ bool ewaProject(const float mu[3], const float qr[4],
         p.q[0] = 1;
         p.q[1] = p.q[2] = p.q[3] = 0;
     } else {
+        const Divisor byNorm(p.qNorm);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            p.q[k] = qr[k] / p.qNorm;
+            p.q[k] = byNorm.under(qr[k]);
     }
     quatToRot(p.q[0], p.q[1], p.q[2], p.q[3], p.Rq);
 #pragma unroll
@@ -130,25 +161,21 @@ __device__ __forceinline__ bool ewaProject(const float mu[3], const float qr[4],
 #pragma unroll
         for (int c = 0; c < 3; ++c)
             p.Sigma[r * 3 + c] = p.M[r * 3] * p.M[c * 3] + p.M[r * 3 + 1] * p.M[c * 3 + 1] + p.M[r * 3 + 2] * p.M[c * 3 + 2];
-    const float W = float(cam.width), H = float(cam.height);
-    const float limXPos = (W - cam.cx) / cam.fx + 0.3f * 0.5f * W / cam.fx;
-    const float limXNeg = cam.cx / cam.fx + 0.3f * 0.5f * W / cam.fx;
-    const float limYPos = (H - cam.cy) / cam.fy + 0.3f * 0.5f * H / cam.fy;
-    const float limYNeg = cam.cy / cam.fy + 0.3f * 0.5f * H / cam.fy;
-    const float xz = p.pc[0] / z, yz = p.pc[1] / z;
+    const Divisor byZ(z), byZ2(z * z);
+    const float xz = byZ.under(p.pc[0]), yz = byZ.under(p.pc[1]);
     // std::min(a, b) = (b < a) ? b : a and std::max(a, b) = (a < b) ? b : a, kept literally.
-    const float mxz = (-limXNeg < xz) ? xz : -limXNeg;
-    const float cxz = (mxz < limXPos) ? mxz : limXPos;
-    const float myz = (-limYNeg < yz) ? yz : -limYNeg;
-    const float cyz = (myz < limYPos) ? myz : limYPos;
+    const float mxz = (-lim.xNeg < xz) ? xz : -lim.xNeg;
+    const float cxz = (mxz < lim.xPos) ? mxz : lim.xPos;
+    const float myz = (-lim.yNeg < yz) ? yz : -lim.yNeg;
+    const float cyz = (myz < lim.yPos) ? myz : lim.yPos;
     p.clampX = cxz != xz;
     p.clampY = cyz != yz;
     p.limTx = cxz;
     p.limTy = cyz;
     p.tx = z * cxz;
     p.ty = z * cyz;
-    const float J00 = cam.fx / z, J02 = -cam.fx * p.tx / (z * z);
-    const float J11 = cam.fy / z, J12 = -cam.fy * p.ty / (z * z);
+    const float J00 = byZ.under(cam.fx), J02 = byZ2.under(-cam.fx * p.tx);
+    const float J11 = byZ.under(cam.fy), J12 = byZ2.under(-cam.fy * p.ty);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         p.T0[k] = J00 * R[k] + J02 * R[6 + k];

@@ -57,9 +57,10 @@ __global__ void __launch_bounds__(256) projectKernel(Params P, int n, u3dg_camer
 {
     pdlEntry();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const u3dg_camera cam = desc ? desc->cam : camArg;
+    const ViewLimits lim = viewLimits(cam);
     if (i >= n)
         return;
-    const u3dg_camera cam = desc ? desc->cam : camArg;
     const float mu[3] = {P.means[3 * i], P.means[3 * i + 1], P.means[3 * i + 2]};
     const float qr[4] = {P.quats[4 * i], P.quats[4 * i + 1], P.quats[4 * i + 2], P.quats[4 * i + 3]};
     const float ls[3] = {P.scales[3 * i], P.scales[3 * i + 1], P.scales[3 * i + 2]};
@@ -67,7 +68,7 @@ __global__ void __launch_bounds__(256) projectKernel(Params P, int n, u3dg_camer
     Ewa p;
     int radius = 0;
     int4 rect = make_int4(0, 0, 0, 0);
-    bool visible = ewaProject(mu, qr, ls, cam, st, p);
+    bool visible = ewaProject(mu, qr, ls, cam, lim, st, p);
     float det = 0.0f, u = 0.0f, v = 0.0f;
     if (visible) {
         det = p.a * p.c - p.b * p.b;
@@ -75,8 +76,9 @@ __global__ void __launch_bounds__(256) projectKernel(Params P, int n, u3dg_camer
     }
     if (visible) {
         const float z = p.pc[2];
-        u = cam.fx * p.pc[0] / z + cam.cx;
-        v = cam.fy * p.pc[1] / z + cam.cy;
+        const Divisor byZ(z);
+        u = byZ.under(cam.fx * p.pc[0]) + cam.cx;
+        v = byZ.under(cam.fy * p.pc[1]) + cam.cy;
         const float mid = 0.5f * (p.a + p.c);
         const float lambda = mid + sqrtf(stdMax(0.1f, mid * mid - det));
         const float rf = ceilf(3.0f * sqrtf(lambda));
@@ -87,10 +89,11 @@ __global__ void __launch_bounds__(256) projectKernel(Params P, int n, u3dg_camer
         if (u + fr < 0 || v + fr < 0 || u - fr >= float(cam.width) || v - fr >= float(cam.height)) {
             visible = false;
         } else {
-            const int tx0 = max(0, int(floorf((u - fr) / float(ts))));
-            const int ty0 = max(0, int(floorf((v - fr) / float(ts))));
-            const int tx1 = min(tilesX, int(floorf((u + fr) / float(ts))) + 1);
-            const int ty1 = min(tilesY, int(floorf((v + fr) / float(ts))) + 1);
+            const Divisor byTile{float(ts)};
+            const int tx0 = max(0, int(floorf(byTile.under(u - fr))));
+            const int ty0 = max(0, int(floorf(byTile.under(v - fr))));
+            const int tx1 = min(tilesX, int(floorf(byTile.under(u + fr))) + 1);
+            const int ty1 = min(tilesY, int(floorf(byTile.under(v + fr))) + 1);
             if (tx0 >= tx1 || ty0 >= ty1)
                 visible = false;
             else
@@ -180,67 +183,208 @@ __global__ void __launch_bounds__(256) projectKernel(Params P, int n, u3dg_camer
 }
 
 // One Adam element update (adamArray, Adam.cpp:13-28), same order as the reference.
-__device__ __forceinline__ void adamOne(float &p, float &m, float &v, float g, float stepSize, float invSqrtBc2)
+__device__ __forceinline__ void adamMoments(float &m, float &v, float g)
 {
     m = 0.9f * m + (1.0f - 0.9f) * g;
     v = 0.999f * v + (1.0f - 0.999f) * g * g;
-    p -= stepSize * m / (sqrtf(v) * invSqrtBc2 + 1e-15f);
 }
 
-// The 9 summed 2D gradients of Gaussian i: its partials of the compositing backward, in emission order.
-// Every intersection names its list position and tile (listPos); those behind the last contributor of
-// their block's pixels (stop) have no partial and are passed over, so a Gaussian deep behind others
-// costs its 8-byte positions only. A lane adds up its own Gaussian, four intersections' loads in flight
-// at a time; Gaussians in more tiles than kGatherLane are added by the whole warp (lanes strided, then a
-// butterfly), so that a few image-sized ones do not hold up a kernel. Both orders are fixed, so the sums
-// are deterministic. All lanes of a warp call it (cnt = 0 without a Gaussian).
-constexpr int kGatherLane = 32;
-
-__device__ __forceinline__ void addPartial(const ChainArgs &a, const int2 &lp, float (&g)[kG2d])
+__device__ __forceinline__ float adamQuotient(float m, float v, float stepSize, float invSqrtBc2)
 {
-    for (int sl = 0; sl < a.subSlots; ++sl) {
-        int block = lp.y;
-        if (a.subSlots > 1) { // tiles covered by several blocks: slot sl is its block's position, row-major
-            const int per = a.blocksX / a.tilesX;
-            block = (lp.y / a.tilesX * per + sl / per) * a.blocksX + lp.y % a.tilesX * per + sl % per;
-        }
-        if (lp.x >= a.stop[block])
-            continue;
-        const float4 *p = reinterpret_cast<const float4 *>(a.partial + sl * a.subStride) + size_t(lp.x) * (kPartial / 4);
-        const float4 u = p[0], v = p[1];
-        const float w = p[2].x;
-        g[0] += u.x;
-        g[1] += u.y;
-        g[2] += u.z;
-        g[3] += u.w;
-        g[4] += v.x;
-        g[5] += v.y;
-        g[6] += v.z;
-        g[7] += v.w;
-        g[8] += w;
+    return stepSize * m / (sqrtf(v) * invSqrtBc2 + 1e-15f);
+}
+
+__device__ __forceinline__ void adamOne(float &p, float &m, float &v, float g, float stepSize, float invSqrtBc2)
+{
+    adamMoments(m, v, g);
+    p -= adamQuotient(m, v, stepSize, invSqrtBc2);
+}
+
+__device__ __forceinline__ float rcpApprox(float x)
+{
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+__device__ __forceinline__ float rsqrtApprox(float x)
+{
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// Adam of a Gaussian's elements in two groups of K and L values per Gaussian: adamOne's arithmetic with
+// Markstein's correctly rounded square root and quotient (Divisor) in their range: v 0 or from 2^-100 to 2^100
+// (all such v compared with the correctly rounded root) and |step m| 0 or from 2^-90 to 2^60; a lane with any
+// other value takes the operators.
+template <int K, int L>
+__device__ __forceinline__ void adamGroups(float *p, float *m, float *v, const float *g, float step, float *p2, float *m2, float *v2,
+                                           const float *g2, float step2, int i, float inv)
+{
+    float x[K + L], y[K + L], z[K + L], q[K + L];
+#pragma unroll
+    for (int k = 0; k < K + L; ++k) {
+        x[k] = k < K ? p[K * i + k] : p2[L * i + k - K];
+        y[k] = k < K ? m[K * i + k] : m2[L * i + k - K];
+        z[k] = k < K ? v[K * i + k] : v2[L * i + k - K];
+    }
+    auto within = [](float t, int lo, int hi) { // 2^lo <= t < 2^hi
+        return __float_as_uint(t) - (uint32_t(lo + 127) << 23) < (uint32_t(hi - lo) << 23);
+    };
+    bool usual = true;
+#pragma unroll
+    for (int k = 0; k < K + L; ++k) {
+        adamMoments(y[k], z[k], k < K ? g[k] : g2[k - K]);
+        const float a = (k < K ? step : step2) * y[k];
+        usual = usual && (z[k] == 0.0f || within(z[k], -100, 100)) && (a == 0.0f || within(fabsf(a), -90, 60));
+        const float r = rsqrtApprox(z[k]), s0 = __fmul_rn(z[k], r);
+        const float s = z[k] == 0.0f ? 0.0f : __fmaf_rn(__fmaf_rn(-s0, s0, z[k]), __fmul_rn(0.5f, r), s0);
+        const float den = s * inv + 1e-15f;
+        float w = rcpApprox(den);
+        w = __fmaf_rn(w, __fmaf_rn(-den, w, 1.0f), w);
+        const float q0 = __fmul_rn(a, w);
+        q[k] = __fmaf_rn(__fmaf_rn(-den, q0, a), w, q0);
+    }
+    if (!usual)
+#pragma unroll
+        for (int k = 0; k < K + L; ++k)
+            q[k] = adamQuotient(y[k], z[k], k < K ? step : step2, inv);
+#pragma unroll
+    for (int k = 0; k < K + L; ++k) {
+        (k < K ? p[K * i + k] : p2[L * i + k - K]) = x[k] - q[k];
+        (k < K ? m[K * i + k] : m2[L * i + k - K]) = y[k];
+        (k < K ? v[K * i + k] : v2[L * i + k - K]) = z[k];
     }
 }
 
-__device__ __forceinline__ void gatherPartials(const ChainArgs &a, int start, int cnt, float (&out)[kG2d])
+// The 9 summed 2D gradients of a lane's Gaussian: its partials of the compositing backward, in emission
+// order. Every intersection names its list position and tile (listPos); those behind the last contributor of
+// their block's pixels (stop) have no partial and are passed over, so a Gaussian deep behind others costs its
+// 8-byte positions only. A warp goes through the intersections of its 32 Gaussians as one sequence, two a lane
+// at a time, and copies the partials that exist, three lanes to one, into rows of shared memory; when those
+// are full each lane adds its own Gaussian's. A lane that looked up and loaded its own, four at a time, waited
+// three memory latencies for each four of the warp's longest (update of 300k Gaussians at 640x480, 2.3M
+// intersections: 79 us, 68 by rows; two rounds and 96 rows against 1..3 and 64..128: 68 to 71).
+// Gaussians in more tiles than kGatherLane are added by the whole warp (lanes strided, then a butterfly), so
+// that a few image-sized ones do not hold up a kernel. Both orders are fixed, so the sums are deterministic.
+// All lanes of a warp call it (cnt = 0 without a Gaussian).
+constexpr int kGatherLane = 32;
+constexpr int kPartialF4 = kPartial / 4;
+constexpr int kGatherRounds = 2, kGatherRows = 96; // 32 intersections looked up at a time; rows of a batch
+
+struct GatherBuffer { // a warp's
+    float4 rows[kGatherRows * kPartialF4];
+    size_t at[32 * kGatherRounds]; // partials to load, float4 index
+};
+
+// The partial of intersection lp in slot array sl: its list position, or -1.
+__device__ __forceinline__ int partialAt(const ChainArgs &a, const int2 &lp, int sl)
 {
-    const int lane = threadIdx.x & 31;
-    float g[kG2d] = {};
-    const int own = cnt <= kGatherLane ? cnt : 0;
-    for (int k = 0; k < own; k += 4) {
-        int2 lp[4];
+    int block = lp.y;
+    if (a.subSlots > 1) { // tiles covered by several blocks: slot sl is its block's position, row-major
+        const int per = a.blocksX / a.tilesX;
+        block = (lp.y / a.tilesX * per + sl / per) * a.blocksX + lp.y % a.tilesX * per + sl % per;
+    }
+    return lp.x < a.stop[block] ? lp.x : -1;
+}
+
+__device__ __forceinline__ void addPartial(const float4 *p, float (&g)[kG2d])
+{
+    const float4 u = p[0], v = p[1];
+    const float w = p[2].x;
+    g[0] += u.x;
+    g[1] += u.y;
+    g[2] += u.z;
+    g[3] += u.w;
+    g[4] += v.x;
+    g[5] += v.y;
+    g[6] += v.z;
+    g[7] += v.w;
+    g[8] += w;
+}
+
+__device__ __forceinline__ void copyAsync(float4 *shared, const float4 *global)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(uint32_t(__cvta_generic_to_shared(shared))), "l"(global)
+                 : "memory");
+}
+
+__device__ __forceinline__ void gatherPartials(const ChainArgs &a, int start, int cnt, GatherBuffer &buf, float (&g)[kG2d])
+{
+    const int lane = threadIdx.x & 31, sub = a.subSlots;
+    const float4 *partial = reinterpret_cast<const float4 *>(a.partial);
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-            lp[r] = k + r < own ? a.listPos[start + k + r] : make_int2(INT_MAX, 0);
+    for (int k = 0; k < kG2d; ++k)
+        g[k] = 0.0f;
+    // The warp's sequence of (intersection, slot) pairs: this lane's are [before, before + own).
+    const int own = cnt <= kGatherLane ? cnt * sub : 0;
+    int before = own;
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-            addPartial(a, lp[r], g);
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o)
+            before += y;
+    }
+    const int total = __shfl_sync(0xffffffffu, before, 31);
+    before -= own;
+    for (int b = 0; b < total;) {
+        int rows = 0, first = 0, last = 0; // rows of the batch; this lane's are [first, last)
+        for (; b < total && rows <= kGatherRows - 32 * kGatherRounds; b += 32 * kGatherRounds) {
+            int2 lp[kGatherRounds];
+            int sl[kGatherRounds];
+#pragma unroll
+            for (int r = 0; r < kGatherRounds; ++r) {
+                // Owner of the sequence's element e: the last lane that begins at or before it.
+                const int e = b + r * 32 + lane;
+                int owner = 0;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+                    if (__shfl_sync(0xffffffffu, before, owner + o) <= e)
+                        owner += o;
+                const int k = e - __shfl_sync(0xffffffffu, before, owner), s0 = __shfl_sync(0xffffffffu, start, owner);
+                sl[r] = sub > 1 ? k % sub : 0;
+                lp[r] = e < total ? a.listPos[s0 + (sub > 1 ? k / sub : k)] : make_int2(INT_MAX, 0);
+            }
+            int at[kGatherRounds], got = 0;
+#pragma unroll
+            for (int r = 0; r < kGatherRounds; ++r)
+                at[r] = partialAt(a, lp[r], sl[r]);
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < kGatherRounds; ++r) {
+                const uint32_t valid = __ballot_sync(0xffffffffu, at[r] >= 0);
+                if (at[r] >= 0)
+                    buf.at[got + __popc(valid & ((1u << lane) - 1u))] =
+                        size_t(sl[r]) * (a.subStride / 4) + size_t(at[r]) * kPartialF4;
+                const int lo = before - b - r * 32, hi = lo + own;
+                first += __popc(valid & (lo <= 0 ? 0u : lo < 32 ? (1u << lo) - 1u : ~0u));
+                last += __popc(valid & (hi <= 0 ? 0u : hi < 32 ? (1u << hi) - 1u : ~0u));
+                got += __popc(valid);
+            }
+            __syncwarp();
+            for (int f = lane; f < got * kPartialF4; f += 32)
+                copyAsync(buf.rows + rows * kPartialF4 + f, partial + buf.at[f / kPartialF4] + f % kPartialF4);
+            rows += got;
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+        for (int k = first; k < last; ++k)
+            addPartial(buf.rows + k * kPartialF4, g);
+        __syncwarp();
     }
     for (uint32_t many = __ballot_sync(0xffffffffu, cnt > kGatherLane); many; many &= many - 1) {
         const int owner = __ffs(many) - 1;
         const int s0 = __shfl_sync(0xffffffffu, start, owner), c0 = __shfl_sync(0xffffffffu, cnt, owner);
         float h[kG2d] = {};
-        for (int k = lane; k < c0; k += 32)
-            addPartial(a, a.listPos[s0 + k], h);
+        for (int k = lane; k < c0; k += 32) {
+            const int2 lp = a.listPos[s0 + k];
+            for (int sl = 0; sl < sub; ++sl) {
+                const int pos = partialAt(a, lp, sl);
+                if (pos >= 0)
+                    addPartial(partial + size_t(sl) * (a.subStride / 4) + size_t(pos) * kPartialF4, h);
+            }
+        }
 #pragma unroll
         for (int k = 0; k < kG2d; ++k) {
 #pragma unroll
@@ -250,39 +394,39 @@ __device__ __forceinline__ void gatherPartials(const ChainArgs &a, int start, in
                 g[k] = h[k];
         }
     }
-#pragma unroll
-    for (int k = 0; k < kG2d; ++k)
-        out[k] = float(g[k]);
 }
 
 // Rasterizer::backward pass 2 (Rasterizer.cpp:432-544) for one Gaussian per thread, fused either with
 // Adam::step (kAdam: the trainer; gradients never leave registers) or with adding the gradients into
 // caller arrays (the unit entry point). It starts from the Gaussian's summed partials (gatherPartials),
 // which never go through memory.
-// Resident CTAs per SM the compiler must allow for: caps registers per thread at 65536 / (256 * n)
-// (64 at 4; the kernel is latency-bound, and 4 CTAs per SM beat fewer with more registers).
-#ifndef U3DG_CHAIN_MIN_BLOCKS
-#define U3DG_CHAIN_MIN_BLOCKS 4
-#endif
+// Bound by the latency of its loads and by instructions (57 us on 300k Gaussians at 640x480, where its 190 MB
+// take 29 us): loads of a group of parameters stand ahead of the group's stores, quotients share their
+// divisors' reciprocals (68 us with the division operator, whose slow path every zero takes). Small CTAs
+// spread few Gaussians over the chip (4k: 22 us at 256 threads, 21.5 at 64, the rest even). Registers are capped
+// at 64 for 32 warps per SM (28 warps: 63 us, 40: 80 us).
+constexpr int kChainThreads = 64, kChainWarps = 32;
 
 template <bool kAdam>
-__global__ void __launch_bounds__(256, U3DG_CHAIN_MIN_BLOCKS) chainKernel(ChainArgs a)
+__global__ void __launch_bounds__(kChainThreads, kChainWarps * 32 / kChainThreads) chainKernel(ChainArgs a)
 {
     pdlEntry();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (a.counts != nullptr && a.counts->abortIter >= 0)
         return;
+    const u3dg_camera &cam = a.desc ? a.desc->cam : a.cam;
+    const ViewLimits lim = viewLimits(cam);
+    __shared__ GatherBuffer sGather[kChainThreads / 32];
     float g[kG2d];
     {
         const bool seen = i < a.n && a.radius[i] > 0;
-        gatherPartials(a, seen ? a.offs[i] : 0, seen ? a.tileCount[i] : 0, g);
+        gatherPartials(a, seen ? a.offs[i] : 0, seen ? a.tileCount[i] : 0, sGather[threadIdx.x >> 5], g);
     }
     if (i >= a.n)
         return;
     const Params &P = a.params;
     float gMeans[3] = {0, 0, 0}, gScales[3] = {0, 0, 0}, gQuats[4] = {0, 0, 0, 0}, gOpac = 0, gColors[3] = {0, 0, 0};
     if (a.radius[i] > 0) {
-        const u3dg_camera &cam = a.desc ? a.desc->cam : a.cam;
         const float dmx = g[0], dmy = g[1];
         if (a.gradAccum != nullptr) {
             const float nx = dmx * 0.5f * float(cam.width), ny = dmy * 0.5f * float(cam.height);
@@ -302,7 +446,7 @@ __global__ void __launch_bounds__(256, U3DG_CHAIN_MIN_BLOCKS) chainKernel(ChainA
         const float qr[4] = {P.quats[4 * i], P.quats[4 * i + 1], P.quats[4 * i + 2], P.quats[4 * i + 3]};
         const float ls[3] = {P.scales[3 * i], P.scales[3 * i + 1], P.scales[3 * i + 2]};
         Ewa p;
-        ewaProject(mu, qr, ls, cam, a.st, p);
+        ewaProject(mu, qr, ls, cam, lim, a.st, p);
         const float z = p.pc[2];
         const float G00 = g[2], G01 = 0.5f * g[3], G11 = g[4]; // dL/dcovariance
         float dSigma[9];
@@ -346,20 +490,23 @@ __global__ void __launch_bounds__(256, U3DG_CHAIN_MIN_BLOCKS) chainKernel(ChainA
         const float dy = 2 * (-2 * y * dRq[0] + x * dRq[1] + w * dRq[2] + x * dRq[3] + zq * dRq[5] - w * dRq[6] + zq * dRq[7] - 2 * y * dRq[8]);
         const float dz = 2 * (-2 * zq * dRq[0] - w * dRq[1] + x * dRq[2] + w * dRq[3] - 2 * zq * dRq[4] + y * dRq[5] + x * dRq[6] + y * dRq[7]);
         const float dq[4] = {dw, dx, dy, dz};
+        const Divisor byNorm(p.qNorm);
         const float qdot = dq[0] * p.q[0] + dq[1] * p.q[1] + dq[2] * p.q[2] + dq[3] * p.q[3];
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            gQuats[k] = (dq[k] - qdot * p.q[k]) / p.qNorm;
+            gQuats[k] = byNorm.under(dq[k] - qdot * p.q[k]);
         const float *R = cam.R;
         const float dJ00 = dT0[0] * R[0] + dT0[1] * R[1] + dT0[2] * R[2];
         const float dJ02 = dT0[0] * R[6] + dT0[1] * R[7] + dT0[2] * R[8];
         const float dJ11 = dT1[0] * R[3] + dT1[1] * R[4] + dT1[2] * R[5];
         const float dJ12 = dT1[0] * R[6] + dT1[1] * R[7] + dT1[2] * R[8];
         const float z2 = z * z, z3 = z2 * z;
+        const Divisor byZ(z), byZ2(z2), byZ3(z3);
         float dpc[3] = {0, 0, 0};
-        dpc[2] += dJ00 * -cam.fx / z2 + dJ02 * 2 * cam.fx * p.tx / z3 + dJ11 * -cam.fy / z2 + dJ12 * 2 * cam.fy * p.ty / z3;
-        const float dtx = dJ02 * -cam.fx / z2;
-        const float dty = dJ12 * -cam.fy / z2;
+        dpc[2] += byZ2.under(dJ00 * -cam.fx) + byZ3.under(dJ02 * 2 * cam.fx * p.tx) + byZ2.under(dJ11 * -cam.fy) +
+                  byZ3.under(dJ12 * 2 * cam.fy * p.ty);
+        const float dtx = byZ2.under(dJ02 * -cam.fx);
+        const float dty = byZ2.under(dJ12 * -cam.fy);
         if (p.clampX)
             dpc[2] += dtx * p.limTx;
         else
@@ -368,9 +515,9 @@ __global__ void __launch_bounds__(256, U3DG_CHAIN_MIN_BLOCKS) chainKernel(ChainA
             dpc[2] += dty * p.limTy;
         else
             dpc[1] += dty;
-        dpc[0] += dmx * cam.fx / z;
-        dpc[1] += dmy * cam.fy / z;
-        dpc[2] += -dmx * cam.fx * p.pc[0] / z2 - dmy * cam.fy * p.pc[1] / z2;
+        dpc[0] += byZ.under(dmx * cam.fx);
+        dpc[1] += byZ.under(dmy * cam.fy);
+        dpc[2] += byZ2.under(-dmx * cam.fx * p.pc[0]) - byZ2.under(dmy * cam.fy * p.pc[1]);
 #pragma unroll
         for (int k = 0; k < 3; ++k)
             gMeans[k] = R[k] * dpc[0] + R[3 + k] * dpc[1] + R[6 + k] * dpc[2];
@@ -380,19 +527,10 @@ __global__ void __launch_bounds__(256, U3DG_CHAIN_MIN_BLOCKS) chainKernel(ChainA
         const Params &M = a.m, &V = a.v;
         const float inv = a.desc ? a.desc->invSqrtBc2 : a.invSqrtBc2;
         const float *lr = a.desc ? a.desc->stepSize : a.stepSize;
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            adamOne(P.means[3 * i + k], M.means[3 * i + k], V.means[3 * i + k], gMeans[k], lr[0], inv);
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            adamOne(P.scales[3 * i + k], M.scales[3 * i + k], V.scales[3 * i + k], gScales[k], lr[1], inv);
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            adamOne(P.quats[4 * i + k], M.quats[4 * i + k], V.quats[4 * i + k], gQuats[k], lr[2], inv);
-        adamOne(P.opac[i], M.opac[i], V.opac[i], gOpac, lr[3], inv);
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            adamOne(P.colors[3 * i + k], M.colors[3 * i + k], V.colors[3 * i + k], gColors[k], lr[4], inv);
+        // Loads ahead of the stores, which the compiler may not exchange.
+        adamGroups<3, 3>(P.means, M.means, V.means, gMeans, lr[0], P.scales, M.scales, V.scales, gScales, lr[1], i, inv);
+        adamGroups<4, 1>(P.quats, M.quats, V.quats, gQuats, lr[2], P.opac, M.opac, V.opac, &gOpac, lr[3], i, inv);
+        adamGroups<3, 0>(P.colors, M.colors, V.colors, gColors, lr[4], P.colors, M.colors, V.colors, gColors, lr[4], i, inv);
     } else {
         const Params &G = a.grads;
         if (a.radius[i] > 0) {
@@ -602,9 +740,9 @@ void launchChain(const ChainArgs &a, bool adam, cudaStream_t s)
     if (a.n <= 0)
         return;
     if (adam)
-        { launchPdl(chainKernel<true>, blocks(a.n, 256), 256, 0, s, a); countLaunch(); }
+        { launchPdl(chainKernel<true>, blocks(a.n, kChainThreads), kChainThreads, 0, s, a); countLaunch(); }
     else
-        { launchPdl(chainKernel<false>, blocks(a.n, 256), 256, 0, s, a); countLaunch(); }
+        { launchPdl(chainKernel<false>, blocks(a.n, kChainThreads), kChainThreads, 0, s, a); countLaunch(); }
 }
 
 void launchAdamSegment(float *p, const float *g, float *m, float *v, int len, float stepSize, float invSqrtBc2,
