@@ -769,3 +769,19 @@ def test_first_adam_step_at_any_step_size(u3dg, oracle, tiny_scene, lr):
         some = moved[moved > 0.5 * lr]
         assert some.size > 0.3 * a.size, (k, some.size, a.size)
         assert np.median(np.abs(some / lr - 1)) <= 1e-4, k
+
+
+@pytest.mark.parametrize("lam", [0.0, 0.2, 1.0])
+@pytest.mark.parametrize("width, height", [(1, 1), (31, 15), (32, 16), (33, 17), (97, 50)])
+def test_loss_at_tile_edges(u3dg, oracle, width, height, lam):
+    """The loss kernels' tiles are 32x16 with a halo of 5: bounds of test_loss_matches_oracle."""
+    rng = np.random.default_rng(width)
+    render = rng.uniform(0, 1, (height, width, 3)).astype(np.float32)
+    target = np.clip(render + rng.normal(0, 0.1, render.shape), 0, 1).astype(np.float32)
+    render[0, 0] = target[0, 0]
+    gv, gg = u3dg.photometricLoss(render, target, width, height, lam)
+    ov, og = oracle.photometric_loss(render, target, width, height, lam)
+    assert abs(gv.l1 - ov.l1) <= 1e-7 * max(1.0, abs(ov.l1))
+    assert abs(gv.ssim - ov.ssim) <= 1e-6
+    assert abs(gv.total - ov.total) <= 1e-6
+    np.testing.assert_allclose(gg.reshape(-1), og.reshape(-1), rtol=1e-5, atol=1e-9)

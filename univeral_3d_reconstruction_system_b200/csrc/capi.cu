@@ -771,8 +771,7 @@ int u3dg_photometric_loss(const float *render, const float *target, int width, i
         U3DG_CUDA(cudaMemcpyAsync(dr.p, render, P * 12, cudaMemcpyHostToDevice, st.s));
         U3DG_CUDA(cudaMemcpyAsync(dt.p, target, P * 12, cudaMemcpyHostToDevice, st.s));
         LossScratch ls{dabc.p, sums.p, blocks};
-        launchLoss(dr.p, dt.p, nullptr, width, height, lambda, dg.p, ls, st.s);
-        launchLossFinalize(ls, width, height, lambda, nullptr, 0, nullptr, vals.p, vals.p + 3, st.s);
+        launchLoss(dr.p, dt.p, nullptr, width, height, lambda, dg.p, ls, nullptr, 0, nullptr, vals.p, vals.p + 3, st.s);
         U3DG_CUDA(cudaGetLastError());
         float v[4];
         U3DG_CUDA(cudaMemcpyAsync(v, vals.p, sizeof(v), cudaMemcpyDeviceToHost, st.s));

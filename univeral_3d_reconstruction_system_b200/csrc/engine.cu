@@ -801,9 +801,8 @@ void TrainerImpl::launchStep(const StepValues &sv, const StepDesc *desc, BinCoun
     const int lb = lossBlocks(W, H);
     lossBlockSums.reserve(size_t(lb) * 3);
     LossScratch ls{abc.p, lossBlockSums.p, lb};
-    launchLoss(ws.rgb.p, nullptr, sv.d.target, W, H, o.ssim_lambda, dLoss.p, ls, stream, desc);
-    launchLossFinalize(ls, W, H, o.ssim_lambda, dStats.p, sv.d.iteration + 1, ws.counts.p, nullptr, nullptr, stream,
-                       desc);
+    launchLoss(ws.rgb.p, nullptr, sv.d.target, W, H, o.ssim_lambda, dLoss.p, ls, dStats.p, sv.d.iteration + 1, ws.counts.p,
+               nullptr, nullptr, stream, desc);
     if (tm)
         tm->mark(4, stream);
     ws.backwardComposite(dLoss.p, stream);

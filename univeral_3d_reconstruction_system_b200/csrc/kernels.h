@@ -239,15 +239,12 @@ struct LossScratch {
 int lossBlocks(int width, int height);
 // target is either float (targetF) or uint8 (targetU8, converted as float(u8) * (1/255f)).
 // desc (may be null): the uint8 target comes from desc->target.
+// Also reduces the block sums into the step's LossValue / PSNR and updates the EMA stats (may be null;
+// Trainer.cpp:88-92) unless counts (may be null) records an aborted step. out3 (may be null) gets
+// total, l1, ssim; psnrOut (may be null) the PSNR. With desc, iteration is desc->iteration + 1.
 void launchLoss(const float *render, const float *targetF, const uint8_t *targetU8, int width, int height, float lambda,
-                float *grad, const LossScratch &ls, cudaStream_t s, const StepDesc *desc = nullptr);
-// Reduces the block sums into the step's LossValue / PSNR and updates the EMA stats
-// (Trainer.cpp:88-92) unless counts (may be null) records an aborted step. out3 (may be null) gets
-// total, l1, ssim; psnrOut (may be null) the PSNR.
-// desc (may be null): iteration is desc->iteration + 1.
-void launchLossFinalize(const LossScratch &ls, int width, int height, float lambda, DevStats *stats, int iteration,
-                        const BinCounts *counts, float *out3, float *psnrOut, cudaStream_t s,
-                        const StepDesc *desc = nullptr);
+                float *grad, const LossScratch &ls, DevStats *stats, int iteration, const BinCounts *counts, float *out3,
+                float *psnrOut, cudaStream_t s, const StepDesc *desc = nullptr);
 // PSNR of the render against a uint8 target, accumulated in double (evaluatePsnr).
 void launchPsnrU8(const float *render, const uint8_t *target, size_t count, double *sumOut, cudaStream_t s);
 void launchPsnrF(const float *a, const float *b, size_t count, double *sumOut, cudaStream_t s);

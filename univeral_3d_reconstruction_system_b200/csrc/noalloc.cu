@@ -115,8 +115,7 @@ extern "C" int u3dg_photometric_loss_noalloc(const float *render, const float *t
         const cudaStream_t s = static_cast<cudaStream_t>(stream);
         const LossScratch ls{reinterpret_cast<float *>(base + kMapsOffset), base, blocks};
         float *vals = reinterpret_cast<float *>(base + kValsOffset);
-        launchLoss(render, target, nullptr, width, height, lambda, grad, ls, s);
-        launchLossFinalize(ls, width, height, lambda, nullptr, 0, nullptr, vals, vals + 3, s);
+        launchLoss(render, target, nullptr, width, height, lambda, grad, ls, nullptr, 0, nullptr, vals, vals + 3, s);
         U3DG_CUDA(cudaGetLastError());
         float v[4] = {0, 0, 0, 0};
         if (out)
