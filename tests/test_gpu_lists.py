@@ -180,3 +180,17 @@ def test_tile_lists_at_chunk_and_path_edges(u3dg, oracle, n, tiles_x, tiles_y, w
                     lists[ty * tiles_x + tx].append(i)
     np.testing.assert_array_equal(offsets, np.concatenate([[0], np.cumsum([len(x) for x in lists])]))
     np.testing.assert_array_equal(ids, np.concatenate([np.array(x, np.int32) for x in lists]) if len(ids) else ids)
+
+
+@pytest.mark.parametrize("n", [1, 32, 33, 127, 128, 1025, 4095, 4096, 4097, 6145])
+def test_depth_order_by_one_and_several_blocks(u3dg, n):
+    # One kernel sorts up to 4096 Gaussians. Depths over many octaves, a third of them equal, a tenth of the
+    # Gaussians invisible. Exact.
+    rng = np.random.default_rng(n)
+    depth = rng.choice(np.exp(rng.uniform(-8, 8, max(1, 2 * n // 3))).astype(np.float32), n)
+    radius = (rng.random(n) < 0.9).astype(np.int32) * 3
+    rect = np.tile(np.array([0, 0, 2, 1], np.int32), (n, 1))
+    offsets, ids = u3dg.binTiles(depth, radius, rect, 2, 1)
+    want = [i for i in np.argsort(depth, kind="stable") if radius[i] > 0]
+    np.testing.assert_array_equal(offsets, [0, len(want), 2 * len(want)])
+    np.testing.assert_array_equal(ids, np.array(want + want, np.int32))

@@ -4,8 +4,8 @@
 // radix sort (ties keep index order), then buckets them per tile in that order, so every tile list
 // is depth-sorted. Here the same order comes from two stable sorts:
 //   1. (depth bits, Gaussian id) over all Gaussians -> depth rank; invisible ones get key
-//      0xFFFFFFFF and sort last: four passes of 8 bits, a histogram and a scatter kernel each
-//      (radixSortDepth);
+//      0xFFFFFFFF and sort last: four passes of 8 bits, a histogram and a scatter kernel each, or
+//      one kernel for up to 4096 Gaussians (radixSortDepth);
 //   2. the ranks' intersections, in rank order, by tile. Up to 2048 tiles (binByTile) they are never
 //      written out: a chunk of ranks counts its intersections per tile, the counts are scanned over the
 //      chunks, and the chunk then goes through its intersections again and writes each one's Gaussian id
@@ -20,7 +20,7 @@
 // the buffers and replays the step). Grids of the first path follow the host-known Gaussian count; those
 // of the second are sized for the capacity.
 //
-// In-block ranks of the stable scatters come from warp match-any votes: each warp ranks its items among
+// In-block ranks of the stable scatters come from warp votes: each warp ranks its items among
 // equal digits and the warps' counts per digit are added in warp order.
 
 #include "tile_cull.cuh"
@@ -324,7 +324,45 @@ constexpr int kDepthItems = 2;
 constexpr int kDepthTile = kDepthThreads * kDepthItems;
 constexpr int kDepthChunks = 160;
 
+// The lanes of the warp with the same digit d (0 .. 255, or kDigits for none). Nine votes: match-any takes
+// about 64 cycles of the SM per warp on 32 different digits (tile lists of 4k Gaussians 47 us, 44.6 with votes,
+// of 300k 116 and 113.5).
+__device__ __forceinline__ uint32_t digitPeers(int d)
+{
+    uint32_t peers = 0xffffffffu;
+#pragma unroll
+    for (int b = 0; b < 9; ++b) {
+        const uint32_t set = __ballot_sync(0xffffffffu, d >> b & 1);
+        peers &= d >> b & 1 ? set : ~set;
+    }
+    return peers;
+}
+
 __device__ __forceinline__ uint32_t depthDigit(uint32_t key, int shift) { return (key >> shift) & uint32_t(kDigits - 1); }
+
+// Stable ranks of a warp's items (32 consecutive ones per round) among those with the same digit, and the
+// digits' counts, which start at zero. left: items from this lane's first one on.
+template <int kItems>
+__device__ __forceinline__ void rankInWarp(const uint2 (&item)[kItems], int shift, int left, uint16_t *counts,
+                                           int (&local)[kItems])
+{
+    const int lane = threadIdx.x & 31;
+    uint32_t peers[kItems];
+#pragma unroll
+    for (int r = 0; r < kItems; ++r)
+        peers[r] = digitPeers(r * 32 < left ? int(depthDigit(item[r].x, shift)) : kDigits);
+#pragma unroll
+    for (int r = 0; r < kItems; ++r) {
+        const bool valid = r * 32 < left;
+        const int d = int(depthDigit(item[r].x, shift));
+        const int seen = counts[d];
+        local[r] = seen + __popc(peers[r] & ((1u << lane) - 1u));
+        __syncwarp();
+        if (valid && lane == __ffs(peers[r]) - 1)
+            counts[d] = uint16_t(seen + __popc(peers[r]));
+        __syncwarp();
+    }
+}
 
 __global__ void __launch_bounds__(kDepthThreads) depthHistKernel(const uint32_t *keys, const uint2 *pairs, int n, int shift,
                                                                  int chunk, int *hist)
@@ -339,7 +377,7 @@ __global__ void __launch_bounds__(kDepthThreads) depthHistKernel(const uint32_t 
         const int i = i0 + threadIdx.x;
         const int d = i < end ? int(depthDigit(pairs ? pairs[i].x : keys[i], shift)) : kDigits;
         // One addition per distinct digit of a warp: the upper digits of depths hold few values.
-        const uint32_t peers = __match_any_sync(0xffffffffu, d);
+        const uint32_t peers = digitPeers(d);
         if (d < kDigits && lane == __ffs(peers) - 1)
             atomicAdd(&counts[d], __popc(peers));
     }
@@ -404,7 +442,6 @@ __global__ void __launch_bounds__(kDepthThreads) depthScatterKernel(const uint32
             base[tid] = at;
         }
     }
-    const uint32_t below = (1u << lane) - 1u;
     for (int r0 = begin; r0 < end; r0 += kDepthTile) {
         const int first = r0 + warp * (32 * kDepthItems);
         uint2 item[kDepthItems];
@@ -418,21 +455,7 @@ __global__ void __launch_bounds__(kDepthThreads) depthScatterKernel(const uint32
         for (int k = 0; k < kDigits / 32; ++k)
             counts[warp][k * 32 + lane] = 0;
         __syncwarp();
-#pragma unroll
-        for (int r = 0; r < kDepthItems; ++r) {
-            const bool valid = first + r * 32 + lane < end;
-            const int d = valid ? int(depthDigit(item[r].x, shift)) : kDigits;
-            const uint32_t peers = __match_any_sync(0xffffffffu, d);
-            int seen = 0;
-            if (valid) {
-                seen = counts[warp][d];
-                local[r] = seen + __popc(peers & below);
-            }
-            __syncwarp();
-            if (valid && lane == __ffs(peers) - 1)
-                counts[warp][d] = uint16_t(seen + __popc(peers));
-            __syncwarp();
-        }
+        rankInWarp<kDepthItems>(item, shift, end - first - lane, counts[warp], local);
         __syncthreads();
         int run = 0; // digit `tid`: the warps' counts to what the warps before hold
         if (tid < kDigits) {
@@ -458,6 +481,98 @@ __global__ void __launch_bounds__(kDepthThreads) depthScatterKernel(const uint32
         __syncthreads();
         if (tid < kDigits)
             base[tid] += run;
+    }
+}
+
+// Few items: all four passes in one CTA, the items in its registers (a warp's ones consecutive) and exchanged
+// through shared memory; bound by the latency of its steps (3.5 us per pass). 4k items: sort and tile lists
+// 44.6 us with eight launches, 35.5 with this one; 6k (8 items a thread): even, 12k: 48.0 and 61.0. So it takes
+// what 4 items a thread hold.
+constexpr int kSmallItems = 4, kSmallSort = kSmallItems * kDepthThreads;
+
+__global__ void __launch_bounds__(kDepthThreads) depthSortSmallKernel(const uint32_t *keys, int n, uint32_t *sortedIds)
+{
+    pdlEntry();
+    extern __shared__ __align__(16) uint8_t shared[];
+    uint2 *exchange = reinterpret_cast<uint2 *>(shared);
+    uint16_t(*counts)[kDigits] = reinterpret_cast<uint16_t(*)[kDigits]>(exchange + kSmallItems * kDepthThreads);
+    __shared__ int groups[kDepthGroups][kDigits], warpSums[kDigits / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, first = warp * (32 * kSmallItems) + lane;
+    uint2 item[kSmallItems];
+#pragma unroll
+    for (int r = 0; r < kSmallItems; ++r) {
+        const int i = first + r * 32;
+        item[r] = make_uint2(i < n ? keys[i] : 0u, uint32_t(i));
+    }
+    for (int shift = 0; shift < 32; shift += 8) {
+        int local[kSmallItems];
+#pragma unroll
+        for (int k = 0; k < kDigits / 32; ++k)
+            counts[warp][k * 32 + lane] = 0;
+        __syncwarp();
+        rankInWarp<kSmallItems>(item, shift, n - first, counts[warp], local);
+        __syncthreads();
+        {
+            // A digit's counts of a group of warps to what the group's warps before hold.
+            const int d = tid % kDigits, group = tid / kDigits;
+            constexpr int per = kDepthWarps / kDepthGroups;
+            int c[per], sum = 0;
+#pragma unroll
+            for (int w = 0; w < per; ++w)
+                c[w] = counts[group * per + w][d];
+#pragma unroll
+            for (int w = 0; w < per; ++w) {
+                counts[group * per + w][d] = uint16_t(sum);
+                sum += c[w];
+            }
+            groups[group][d] = sum;
+        }
+        __syncthreads();
+        int total = 0, scan = 0;
+        if (tid < kDigits) {
+#pragma unroll
+            for (int g = 0; g < kDepthGroups; ++g)
+                total += groups[g][tid];
+            scan = total;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, scan, o);
+                if (lane >= o)
+                    scan += y;
+            }
+            if (lane == 31)
+                warpSums[warp] = scan;
+        }
+        __syncthreads();
+        if (tid < kDigits) {
+            int at = scan - total;
+            for (int w = 0; w < warp; ++w)
+                at += warpSums[w];
+#pragma unroll
+            for (int g = 0; g < kDepthGroups; ++g) {
+                const int c = groups[g][tid];
+                groups[g][tid] = at; // the group's first position of the digit
+                at += c;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kSmallItems; ++r)
+            if (first + r * 32 < n) {
+                const int d = int(depthDigit(item[r].x, shift));
+                const int pos = groups[warp / (kDepthWarps / kDepthGroups)][d] + counts[warp][d] + local[r];
+                if (shift < 24)
+                    exchange[pos] = item[r];
+                else
+                    sortedIds[pos] = item[r].y;
+            }
+        if (shift < 24) {
+            __syncthreads();
+#pragma unroll
+            for (int r = 0; r < kSmallItems; ++r)
+                if (first + r * 32 < n)
+                    item[r] = exchange[first + r * 32];
+        }
     }
 }
 
@@ -917,6 +1032,13 @@ void radixSortDepth(const uint32_t *keys, uint2 *pairsA, uint2 *pairsB, uint32_t
 {
     if (n <= 0)
         return;
+    if (n <= kSmallSort) {
+        constexpr size_t shared = kSmallSort * sizeof(uint2) + size_t(kDepthWarps) * kDigits * sizeof(uint16_t);
+        static std::atomic<uint64_t> allowed{0};
+        allowShared(depthSortSmallKernel, shared + 8192, shared, allowed); // with the static arrays
+        { launchPdl(depthSortSmallKernel, 1, kDepthThreads, shared, s, keys, n, sortedIds); countLaunch(); }
+        return;
+    }
     const int chunk = depthChunk(n), G = (n + chunk - 1) / chunk;
     const uint2 *pin = nullptr;
     uint2 *bufs[2] = {pairsA, pairsB};
