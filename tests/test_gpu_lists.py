@@ -194,3 +194,17 @@ def test_depth_order_by_one_and_several_blocks(u3dg, n):
     want = [i for i in np.argsort(depth, kind="stable") if radius[i] > 0]
     np.testing.assert_array_equal(offsets, [0, len(want), 2 * len(want)])
     np.testing.assert_array_equal(ids, np.array(want + want, np.int32))
+
+
+@pytest.mark.parametrize("width, height, tile", [(240, 236, 16), (240, 240, 16), (235, 243, 16), (243, 235, 32), (235, 243, 64),
+                                                 (350, 391, 8), (397, 405, 16)])
+def test_tiles_in_order_of_their_lists(u3dg, oracle, width, height, tile):
+    # On both sides of 888 blocks of 8x8, from which tiles are taken by descending list length, and with tiles
+    # that reach over the image's edges; lists of 0 to 600 entries. Image within 1e-5, gradients as above.
+    rng = np.random.default_rng(width)
+    m = random_model(600, rng, 1.0, 3.0, 0.02, 0.3)
+    m.means[:, 0] = np.abs(m.means[:, 0]) ** 2
+    cam, st = make_camera(width, height, 0.8 * width), RasterSettings(tile_size=tile, background=(0.1, 0.2, 0.3))
+    w = rng.uniform(-1, 1, (height, width, 3)).astype(np.float32)
+    r = _close(u3dg, oracle, m, cam, st, w, 3e-4)
+    np.testing.assert_allclose(r.forward(m, cam, st), oracle.raster(1).forward(m, cam, st), rtol=0, atol=1e-5)

@@ -771,6 +771,44 @@ __global__ void __launch_bounds__(kScanThreads) tileScanKernel(int *hist, int ch
 constexpr int kListed = 10240; // 20 KB; a chunk of 512 ranks has about 4,000 on a 300k model at 640x480
 static_assert(kMaxTiles * 32 == 65536, "a tile and a lane fit in 16 bits");
 
+// Tiles by descending list length, in kLengths steps of the longest (one block of kRanks threads): the forward
+// starts the longest lists first. Within a step the order is open; it changes no result.
+constexpr int kLengths = 64;
+
+__device__ __forceinline__ void orderTiles(const int *lengths, int tiles, int *order)
+{
+    __shared__ int longest, count[kLengths];
+    const int tid = threadIdx.x;
+    if (tid == 0)
+        longest = 0;
+    if (tid < kLengths)
+        count[tid] = 0;
+    __syncthreads();
+    int most = 0;
+    for (int d = tid; d < tiles; d += kRanks)
+        most = max(most, lengths[d]);
+    most = __reduce_max_sync(0xffffffffu, most);
+    if ((tid & 31) == 0)
+        atomicMax(&longest, most);
+    __syncthreads();
+    const float scale = float(kLengths) / (float(longest) + 1.0f);
+    auto step = [&](int d) { return kLengths - 1 - min(kLengths - 1, int(float(lengths[d]) * scale)); };
+    for (int d = tid; d < tiles; d += kRanks)
+        atomicAdd(&count[step(d)], 1);
+    __syncthreads();
+    if (tid == 0) {
+        int run = 0;
+        for (int k = 0; k < kLengths; ++k) {
+            const int c = count[k];
+            count[k] = run;
+            run += c;
+        }
+    }
+    __syncthreads();
+    for (int d = tid; d < tiles; d += kRanks)
+        order[atomicAdd(&count[step(d)], 1)] = d;
+}
+
 __global__ void __launch_bounds__(kRanks, 3) tileScatterKernel(TileBins b, const int *hist, const int *tileTotals,
                                                             const int *chunkFirst, const BinCounts *bc)
 {
@@ -782,13 +820,18 @@ __global__ void __launch_bounds__(kRanks, 3) tileScatterKernel(TileBins b, const
     __shared__ int warpSums[kRankWarps], scanSums[kRankWarps];
     __shared__ uint16_t listed[kListed];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int chunk = int(blockIdx.x) - (b.tileOrder ? 1 : 0); // the first block orders the tiles
+    if (chunk < 0) {
+        orderTiles(tileTotals, tiles, b.tileOrder);
+        return;
+    }
     if (bc->effTotal <= 0) { // nothing listed, or an overflow
-        if (blockIdx.x == 0)
+        if (chunk == 0)
             for (int d = tid; d <= tiles; d += kRanks)
                 b.tileOffsets[d] = 0;
         return;
     }
-    const Listed l = loadListed(b.sortedIds, b.tileCount, b.rect, b.rowTab, b.cullRec != nullptr, blockIdx.x * kRanks + tid, b.n);
+    const Listed l = loadListed(b.sortedIds, b.tileCount, b.rect, b.rowTab, b.cullRec != nullptr, chunk * kRanks + tid, b.n);
     for (int k = tid; k < kRankWarps * stride / 2; k += kRanks)
         reinterpret_cast<uint32_t *>(offset)[k] = 0;
     auto warpScan = [&](int v) {
@@ -819,20 +862,20 @@ __global__ void __launch_bounds__(kRanks, 3) tileScatterKernel(TileBins b, const
         l0 += w < warp ? warpSums[w] : 0;
         all += warpSums[w];
     }
-    const int e0 = chunkFirst[blockIdx.x] + l0;
+    const int e0 = chunkFirst[chunk] + l0;
     const bool fits = all <= kListed;
     for (int k = 0; k < per; ++k) {
         const int d = tid * per + k;
         if (d >= tiles)
             break;
-        base[d] = start + hist[size_t(blockIdx.x) * tiles + d];
-        if (blockIdx.x == 0)
+        base[d] = start + hist[size_t(chunk) * tiles + d];
+        if (chunk == 0)
             b.tileOffsets[d] = start;
         start += tileTotals[d];
-        if (blockIdx.x == 0 && d == tiles - 1)
+        if (chunk == 0 && d == tiles - 1)
             b.tileOffsets[tiles] = start;
     }
-    if (b.offsById && int(blockIdx.x) * kRanks + tid < b.n)
+    if (b.offsById && chunk * kRanks + tid < b.n)
         b.offsById[l.gid] = e0 + o;
     uint16_t *mine = offset + warp * stride;
     // (Two tiles share a word; a warp's ranks add at most 32 to each.)
@@ -1067,7 +1110,7 @@ void binByTile(const TileBins &b, int *hist, int *tileTotals, int *chunkTotals, 
     allowShared(tileScatterKernel, scatterShared + 24 * 1024, size_t(kMaxTiles) * 36, allowed); // with the static arrays
     { launchPdl(tileCountKernel, G, kRanks, b.tiles * sizeof(int), s, b, hist, chunkTotals); countLaunch(); }
     { launchPdl(tileScanKernel, (b.tiles + 31) / 32 + 1, kScanThreads, 0, s, hist, G, b.tiles, tileTotals, chunkTotals, cap); countLaunch(); }
-    { launchPdl(tileScatterKernel, G, kRanks, scatterShared, s, b, hist, tileTotals, chunkTotals, cap.counts); countLaunch(); }
+    { launchPdl(tileScatterKernel, G + (b.tileOrder ? 1 : 0), kRanks, scatterShared, s, b, hist, tileTotals, chunkTotals, cap.counts); countLaunch(); }
 }
 
 size_t scanPartialEntries(int n) { return size_t((n + kScanTile - 1) / kScanTile) + 1; }

@@ -227,6 +227,7 @@ void RasterWorkspace::planPixels(DeviceSlab &slab, size_t count, size_t pixels, 
     slab.add(finalT, pixels);
     slab.add(nContrib, pixels);
     slab.add(tileOffsets, size_t(tx) * ty + 1);
+    slab.add(tileOrder, size_t(tx) * ty);
     slab.add(rowTotals, size_t(radixDigits()));
     size_t histEntries = binHistEntries(int(count), tx * ty);
     if (!binsByTile(tx * ty)) {
@@ -262,6 +263,7 @@ void RasterWorkspace::bin(cudaStream_t stream, int iteration, bool keep, const S
     chunkTotals.reserve(binChunkEntries(n));
     rowTotals.reserve(size_t(radixDigits()));
     tileOffsets.reserve(size_t(tiles) + 1);
+    tileOrder.reserve(size_t(tiles));
     radixSortDepth(depthKey.p, depthPairs[0].p, depthPairs[1].p, depthOrder.p, n, hist.p, stream);
     // The projection counted each Gaussian's tiles (and, culling, its row table).
     const SplatRec *cullRec = culled() ? rec.p : nullptr;
@@ -269,7 +271,7 @@ void RasterWorkspace::bin(cudaStream_t stream, int iteration, bool keep, const S
     int2 *const positions = keep ? listPos.p : nullptr;
     if (direct) {
         binByTile(TileBins{depthOrder.p, cnt.p, rect.p, n, tilesX, tiles, cullRec, st.tile_size, rowTab.p, tileOffsets.p,
-                           entries.p, positions, keep ? offsById.p : nullptr},
+                           ordersTiles() ? tileOrder.p : nullptr, entries.p, positions, keep ? offsById.p : nullptr},
                   hist.p, rowTotals.p, chunkTotals.p, cap, stream);
         return;
     }
@@ -300,11 +302,18 @@ void RasterWorkspace::forwardChecked(const Params &P, int count, const u3dg_came
     throw StatusError(U3DG_ERR_CAPACITY, "intersection buffers could not be sized");
 }
 
+bool RasterWorkspace::ordersTiles() const
+{
+    const int tiles = tilesX * tilesY;
+    return binsByTile(tiles) && forwardOrdersTiles(tiles, st.tile_size);
+}
+
 RasterArgs RasterWorkspace::rasterArgs() const
 {
     RasterArgs a;
     a.tileOffsets = tileOffsets.p;
     a.entries = entries.p;
+    a.tileOrder = ordersTiles() ? tileOrder.p : nullptr;
     a.rec = rec.p;
     a.width = cam.width;
     a.height = cam.height;

@@ -211,7 +211,7 @@ struct RasterWorkspace {
     int icap = 0;
     int partialSlots = 1;              // slot arrays the backward needs: (tile size / 16)^2 above 16
     // per tile / pixel
-    DevBuf<int> tileOffsets, nContrib;
+    DevBuf<int> tileOffsets, tileOrder, nContrib;
     DevBuf<int> blockStop; // per backward block: list position behind its last contributor
     DevBuf<float4> segments;                      // RasterArgs::ck
     DevBuf<int> blockMax, unitCount;
@@ -231,6 +231,7 @@ struct RasterWorkspace {
     bool cullTiles = false;
     // Culling applies while tile rows fit the row table's 16-bit cumulative counts (< 8192 tiles).
     bool culled() const { return cullTiles && tilesX < 8192; }
+    bool ordersTiles() const;
     u3dg_camera cam{};
     u3dg_raster_settings st{};
 

@@ -149,6 +149,7 @@ struct TileBins {
     int tileSize;
     const uint32_t *rowTab;
     int *tileOffsets; // tiles + 1
+    int *tileOrder;   // tiles, the longest lists first (in 64 steps of length; may be null)
     int *entries;     // per list position: Gaussian id
     int2 *listPos;    // per emission: list position, tile (may be null)
     int *offsById;    // per Gaussian: first emission (may be null)
@@ -196,6 +197,7 @@ void launchFinalizeBins(const uint32_t *sortedKeys, const uint32_t *sortedEmit, 
 struct RasterArgs {
     const int *tileOffsets;
     const int *entries; // per tile-sorted entry: Gaussian id
+    const int *tileOrder; // the order in which the forward takes the tiles (null: row-major pixel blocks)
     const SplatRec *rec;
     int width, height, tileSize, tilesX;
     float bg[3];
@@ -223,6 +225,8 @@ struct RasterArgs {
 // their number into unitCount, and per pixel block the list position behind its last contributor into
 // stop.
 void launchBackwardUnits(const RasterArgs &a, int *stop, int2 *units, int *unitCount, cudaStream_t s);
+// Whether the forward of so many tiles takes them in the order of their list lengths (RasterArgs::tileOrder).
+bool forwardOrdersTiles(int tiles, int tileSize);
 void launchCompositeForward(const RasterArgs &a, float *rgb, float *finalT, int *nContrib, cudaStream_t s);
 // partial: kPartial floats per list position, in a.subSlots slot arrays. Partials from a block's stop on
 // are not written: they are zero, and ChainArgs' reader skips them.

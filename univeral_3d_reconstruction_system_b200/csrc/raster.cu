@@ -199,12 +199,30 @@ __device__ __forceinline__ void soloBatch(const SoloShared &sh, Blend<kKeep> &px
     }
 }
 
+// The 8x8 block of this CTA: the tiles' blocks in tile order, or row-major blocks of the image. False outside
+// the image.
+__device__ __forceinline__ bool forwardBlock(const RasterArgs &a, int &bx, int &by)
+{
+    const int i = int(blockIdx.x);
+    if (a.tileOrder) {
+        const int side = a.tileSize >> 3, tile = a.tileOrder[i / (side * side)], at = i % (side * side);
+        bx = tile % a.tilesX * side + at % side;
+        by = tile / a.tilesX * side + at / side;
+    } else {
+        bx = i % a.blocksX;
+        by = i / a.blocksX;
+    }
+    return bx < a.blocksX && by < a.blocksY;
+}
+
 template <bool kKeep>
 __global__ void __launch_bounds__(32, 20) compositeForwardKernel(RasterArgs a, float *rgb, float *finalT, int *nContrib)
 {
     pdlEntry();
     __shared__ SoloShared sh;
-    const int bx = int(blockIdx.x) % a.blocksX, by = int(blockIdx.x) / a.blocksX; // 8x8 blocks
+    int bx, by; // 8x8 blocks
+    if (!forwardBlock(a, bx, by))
+        return;
     const int lane = threadIdx.x;
     const WarpBlock wb(lane, bx, by);
     const int tile = tileOf<8>(a, bx, by);
@@ -327,7 +345,9 @@ __global__ void __launch_bounds__(kTeamThreads, 6) compositeForwardTeamKernel(Ra
 {
     pdlEntry();
     __shared__ TeamShared sh;
-    const int bx = int(blockIdx.x) % a.blocksX, by = int(blockIdx.x) / a.blocksX; // 8x8 blocks
+    int bx, by; // 8x8 blocks
+    if (!forwardBlock(a, bx, by))
+        return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const WarpBlock wb(lane, bx, by);
     const int tile = tileOf<8>(a, bx, by);
@@ -398,17 +418,24 @@ __global__ void __launch_bounds__(kTeamThreads, 6) compositeForwardTeamKernel(Ra
 
 // Blocks up to which the team is faster (between 1,200 and 2,700, see above): about 14 per SM.
 constexpr int kTeamLimit = 2048;
+// Blocks up to which all teams run at once (6 on each of 148 SMs), so that their order does not matter. Beyond,
+// the longest lists go first: forward of 1,200 blocks 55.8 -> 51.4 us, of 2,700 75.8 -> 73.0, of 4,800 104.1 ->
+// 100.0; of 108 blocks 26.8 -> 27.2, and the lists 34.6 -> 35.1.
+constexpr int kTeamsResident = 888;
 
 } // namespace
+
+bool forwardOrdersTiles(int tiles, int tileSize) { return tiles * (tileSize / 8) * (tileSize / 8) > kTeamsResident; }
 
 template <bool kKeep>
 static void launchForward(const RasterArgs &a, float *rgb, float *finalT, int *nContrib, cudaStream_t s)
 {
-    const int blocks = a.blocksX * a.blocksY;
+    const int blocks = a.blocksX * a.blocksY, side = a.tileSize / 8;
+    const int grid = a.tileOrder ? a.tilesX * ((a.height + a.tileSize - 1) / a.tileSize) * side * side : blocks;
     if (blocks <= kTeamLimit)
-        { launchPdl(compositeForwardTeamKernel<kKeep>, blocks, kTeamThreads, 0, s, a, rgb, finalT, nContrib); countLaunch(); }
+        { launchPdl(compositeForwardTeamKernel<kKeep>, grid, kTeamThreads, 0, s, a, rgb, finalT, nContrib); countLaunch(); }
     else
-        { launchPdl(compositeForwardKernel<kKeep>, blocks, 32, 0, s, a, rgb, finalT, nContrib); countLaunch(); }
+        { launchPdl(compositeForwardKernel<kKeep>, grid, 32, 0, s, a, rgb, finalT, nContrib); countLaunch(); }
 }
 
 void launchCompositeForward(const RasterArgs &a, float *rgb, float *finalT, int *nContrib, cudaStream_t s)
