@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from helpers import make_camera, random_model, rel_l2
-from univeral_3d_reconstruction_system_b200.types import RasterSettings
+from univeral_3d_reconstruction_system_b200.types import RasterSettings, TrainImage, TrainOptions
 
 pytestmark = pytest.mark.gpu
 
@@ -208,3 +208,26 @@ def test_tiles_in_order_of_their_lists(u3dg, oracle, width, height, tile):
     w = rng.uniform(-1, 1, (height, width, 3)).astype(np.float32)
     r = _close(u3dg, oracle, m, cam, st, w, 3e-4)
     np.testing.assert_allclose(r.forward(m, cam, st), oracle.raster(1).forward(m, cam, st), rtol=0, atol=1e-5)
+
+
+def test_views_whose_lists_do_not_fit_at_first(u3dg):
+    # 400 Gaussians over all of 4,800 tiles of 8x8: 1.9M intersections, above the first capacity of 2^20, between
+    # views that fit. The bytes and the PSNR are those of views rendered one by one.
+    rng = np.random.default_rng(8)
+    m = _stack(400, rng, 0.1)
+    m.scales += 2.0
+    cams = [make_camera(w, h, 300.0) for w, h in ((64, 48), (640, 480), (640, 480), (97, 33), (640, 479))]
+    st = RasterSettings(tile_size=8, background=(0.1, 0.2, 0.3))
+    views = u3dg.renderViewsSh(m, None, 0, cams, st)
+    r = u3dg.Rasterizer()
+    images = [r.forward(m, c, st).reshape(c.height, c.width, 3) for c in cams]
+    for view, image in zip(views, images):
+        np.testing.assert_array_equal(view, TrainImage.quantize(image))
+    photos = [TrainImage(c, rng.integers(0, 256, (c.height, c.width, 3)).astype(np.uint8)) for c in cams]
+    t = u3dg.Trainer(m, photos, 1.0, TrainOptions(max_gaussians=400, raster=st))
+    psnr = t.evaluatePsnr()
+    want = []
+    for p, image in zip(photos, images):
+        d = image.astype(np.float64) - (p.rgb.astype(np.float32) * np.float32(1 / 255)).astype(np.float64)
+        want.append(-10 * np.log10(np.mean(d * d)))
+    assert abs(psnr - np.mean(want)) < 1e-5 * np.mean(want)

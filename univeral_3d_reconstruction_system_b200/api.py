@@ -551,7 +551,7 @@ def renderViewsSh(model: GaussianModel, sh_rest: np.ndarray | None, degree: int,
         cams[k] = _cam(c)
         sizes.append((cams[k].height, cams[k].width))
     total = sum(h * w * 3 for h, w in sizes)
-    out = np.zeros(max(total, 1), np.uint8)
+    out = np.empty(max(total, 1), np.uint8)
     mv = model.view()
     ss = _settings(settings)
     shp = _abi.fptr(np.ascontiguousarray(sh_rest, np.float32).reshape(-1)) if (sh_rest is not None and degree > 0) \
@@ -560,7 +560,7 @@ def renderViewsSh(model: GaussianModel, sh_rest: np.ndarray | None, degree: int,
                                       out.ctypes.data_as(_abi.u8p)))
     res, o = [], 0
     for h, w in sizes:
-        res.append(out[o:o + h * w * 3].reshape(h, w, 3).copy())
+        res.append(out[o:o + h * w * 3].reshape(h, w, 3))
         o += h * w * 3
     return res
 

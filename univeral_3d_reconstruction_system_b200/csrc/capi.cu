@@ -83,6 +83,16 @@ struct Stream {
     void sync() { U3DG_CUDA(cudaStreamSynchronize(s)); }
 };
 
+struct Event {
+    cudaEvent_t e = nullptr;
+    Event() { U3DG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming)); }
+    ~Event()
+    {
+        if (e)
+            cudaEventDestroy(e);
+    }
+};
+
 } // namespace
 
 struct u3dg_rasterizer {
@@ -1224,30 +1234,83 @@ int u3dg_render_views_sh(const u3dg_model *model, const float *sh_rest, int degr
         if (degree < 0 || degree > 3)
             throw StatusError(U3DG_ERR_INVALID_ARG, "SH degree must be 0..3");
         checkSettings(*settings);
+        size_t pixels = 0;
+        int tx = 0, ty = 0;
+        for (int v = 0; v < count; ++v) {
+            checkCamera(cameras[v]);
+            const int ts = settings->tile_size;
+            pixels = std::max(pixels, size_t(cameras[v].width) * cameras[v].height);
+            tx = std::max(tx, (cameras[v].width + ts - 1) / ts);
+            ty = std::max(ty, (cameras[v].height + ts - 1) / ts);
+        }
+        const size_t K = size_t((degree + 1) * (degree + 1) - 1), shCount = sh_rest ? model->count * K * 3 : 0;
+        // One allocation for all buffers (each of its own took 0.3 ms, and as much to free), sized for the
+        // largest view; lists that do not fit grow as elsewhere.
+        DeviceSlab slab;
         u3dg_rasterizer r;
         U3DG_CUDA(cudaGetDevice(&r.device));
         cudaStream_t s = r.stream.s;
-        r.model.upload(*model, s);
         DevBuf<float> sh;
+        DevBuf<uint8_t> q[2];
+        slab.add(r.model.buf, 14 * std::max<size_t>(model->count, 1));
+        if (shCount)
+            slab.add(sh, shCount);
+        if (count > 0) {
+            r.ws.cullTiles = true; // shorter lists, the same images
+            r.ws.planEntries(slab, RasterWorkspace::firstCapacity(std::max<size_t>(model->count, 1)));
+            r.ws.planGaussians(slab, model->count);
+            r.ws.planForward(slab, model->count, pixels, tx, ty);
+            for (auto &buf : q)
+                slab.add(buf, pixels * 3);
+        }
+        slab.commit();
+        r.model.upload(*model, s);
         const float *shDev = nullptr;
-        if (sh_rest && degree > 0 && model->count > 0) {
-            const size_t K = size_t((degree + 1) * (degree + 1) - 1);
-            sh.reserve(model->count * K * 3, true);
-            U3DG_CUDA(cudaMemcpyAsync(sh.p, sh_rest, model->count * K * 3 * sizeof(float), cudaMemcpyHostToDevice, s));
+        if (shCount) {
+            sh.reserve(shCount, true);
+            U3DG_CUDA(cudaMemcpyAsync(sh.p, sh_rest, shCount * sizeof(float), cudaMemcpyHostToDevice, s));
             shDev = sh.p;
         }
-        DevBuf<uint8_t> q;
-        size_t offset = 0;
-        for (int v = 0; v < count; ++v) {
-            checkCamera(cameras[v]);
-            const size_t P3 = size_t(cameras[v].width) * cameras[v].height * 3;
-            r.ws.forwardChecked(r.model.params(), int(model->count), cameras[v], *settings, shDev, degree, s);
-            q.reserve(P3);
-            launchQuantize(r.ws.rgb.p, P3, q.p, s);
-            U3DG_CUDA(cudaGetLastError());
-            U3DG_CUDA(cudaMemcpyAsync(rgb8 + offset, q.p, P3, cudaMemcpyDeviceToHost, s));
+        if (count == 0) {
             r.stream.sync();
-            offset += P3;
+            return;
+        }
+        // The next view is rendered while this one's bytes go to the host (16 views of 250k Gaussians with
+        // degree 3 at 640x480: 9.4 ms, of which 5 are the upload; 21 with a wait and a copy after each view and
+        // the buffers allocated one by one).
+        Stream copies;
+        Event rendered[2];
+        HostPinned<BinCounts> counts;
+        counts.reserve(2);
+        auto bytes = [&](int v) { return size_t(cameras[v].width) * cameras[v].height * 3; };
+        auto quantize = [&](int v) {
+            launchQuantize(r.ws.rgb.p, bytes(v), q[v & 1].p, s);
+            U3DG_CUDA(cudaGetLastError());
+        };
+        auto render = [&](int v) {
+            r.ws.clearCounts(s);
+            r.ws.forward(r.model.params(), int(model->count), cameras[v], *settings, shDev, degree, s, 0, false);
+            quantize(v);
+            U3DG_CUDA(cudaMemcpyAsync(counts.p + (v & 1), r.ws.counts.p, sizeof(BinCounts), cudaMemcpyDeviceToHost, s));
+            U3DG_CUDA(cudaEventRecord(rendered[v & 1].e, s));
+        };
+        size_t offset = 0;
+        render(0);
+        for (int v = 0; v < count; ++v) {
+            if (v + 1 < count)
+                render(v + 1);
+            U3DG_CUDA(cudaEventSynchronize(rendered[v & 1].e));
+            if (counts.p[v & 1].abortIter >= 0) { // its lists did not fit
+                r.stream.sync();
+                r.ws.forwardChecked(r.model.params(), int(model->count), cameras[v], *settings, shDev, degree, s);
+                quantize(v);
+                r.stream.sync();
+                if (v + 1 < count)
+                    render(v + 1);
+            }
+            U3DG_CUDA(cudaMemcpyAsync(rgb8 + offset, q[v & 1].p, bytes(v), cudaMemcpyDeviceToHost, copies.s));
+            copies.sync();
+            offset += bytes(v);
         }
     });
 }

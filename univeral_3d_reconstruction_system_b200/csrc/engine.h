@@ -242,6 +242,10 @@ struct RasterWorkspace {
     void reserveGaussians(size_t count);
     // The same sizes (and the per-pixel buffers for views of up to `pixels` pixels and `tiles` tiles at
     // the tile size st.tile_size), planned into a slab instead of allocated one by one.
+    // planEntries, planForward: what a forward without backward needs of them.
+    static size_t firstCapacity(size_t count) { return std::max<size_t>(size_t(1) << 20, 16 * count); }
+    void planEntries(DeviceSlab &slab, size_t capacity);
+    void planForward(DeviceSlab &slab, size_t count, size_t pixels, int tilesX, int tilesY);
     void planIntersections(DeviceSlab &slab, size_t capacity);
     void planGaussians(DeviceSlab &slab, size_t count);
     void planPixels(DeviceSlab &slab, size_t count, size_t pixels, int tilesX, int tilesY, int tileSize);
@@ -399,6 +403,7 @@ struct TrainerImpl {
     DevBuf<double> lossBlockSums, psnrSums;
     DevBuf<DevStats> dStats;
     HostPinned<DevStats> hStats;
+    HostPinned<BinCounts> viewCounts; // evaluatePsnr: per view
     // densification scratch
     DevBuf<int> keep, cost, costScan, accCost, accScan, isSplit, splitScan, keepScan, firstSecond, dScanPartial;
     DevBuf<float> normals;
