@@ -11,16 +11,19 @@ pytestmark = pytest.mark.gpu
 
 
 def _close(u3dg, oracle, model, cam, st, w, rel):
-    r = u3dg.Rasterizer()
-    r.forward(model, cam, st)
-    ndc = np.zeros(model.size(), np.float32)
-    g = r.backward(model, w, None, ndc)
+    """Both backwards: over whole lists (the rasterizer's) and over segments (culled lists, the trainers')."""
     o = oracle.raster(1)
     o.forward(model, cam, st)
     og, ondc = o.backward(w)
-    for k in ("means", "scales", "quats", "opacities", "colors"):
-        assert rel_l2(getattr(g, k), getattr(og, k)) <= rel, k
-    assert rel_l2(ndc, ondc) <= rel
+    for culled in (True, False):
+        r = u3dg.Rasterizer()
+        r.set_tile_culling(culled)
+        r.forward(model, cam, st)
+        ndc = np.zeros(model.size(), np.float32)
+        g = r.backward(model, w, None, ndc)
+        for k in ("means", "scales", "quats", "opacities", "colors"):
+            assert rel_l2(getattr(g, k), getattr(og, k)) <= rel, (k, culled)
+        assert rel_l2(ndc, ondc) <= rel
     return r
 
 
@@ -74,12 +77,14 @@ def test_backward_with_few_and_many_units(u3dg, oracle, width, height, n, backgr
            3e-4)
 
 
-def test_a_non_finite_pixel_gradient_reaches_only_what_blends_there(u3dg):
+@pytest.mark.parametrize("culled", [False, True])
+def test_a_non_finite_pixel_gradient_reaches_only_what_blends_there(u3dg, culled):
     rng = np.random.default_rng(3)
     m = random_model(200, rng, 1.0, 3.0, 0.02, 0.1)
     cam, st = make_camera(64, 48, 50.0), RasterSettings()
     w = rng.uniform(-1, 1, (48, 64, 3)).astype(np.float32)
     r = u3dg.Rasterizer()
+    r.set_tile_culling(culled)
     r.forward(m, cam, st)
     clean = r.backward(m, w)
     w[20, 30, 1] = np.inf
@@ -100,14 +105,16 @@ def test_a_non_finite_pixel_gradient_reaches_only_what_blends_there(u3dg):
         np.testing.assert_array_equal(a, b)
 
 
+@pytest.mark.parametrize("culled", [False, True])
 @pytest.mark.parametrize("background", [(0.0, 0.0, 0.0), (0.2, 0.4, 0.1)])
-def test_a_non_finite_colour_reaches_only_the_pixels_it_covers(u3dg, background):
+def test_a_non_finite_colour_reaches_only_the_pixels_it_covers(u3dg, background, culled):
     rng = np.random.default_rng(4)
     m = random_model(120, rng, 1.0, 3.0, 0.02, 0.08)
     m.means[7] = [0.0, 0.0, 2.5]
     cam, st = make_camera(64, 48, 50.0), RasterSettings(background=background)
     w = rng.uniform(-1, 1, (48, 64, 3)).astype(np.float32)
     r = u3dg.Rasterizer()
+    r.set_tile_culling(culled)
     clean_image = r.forward(m, cam, st)
     clean = r.backward(m, w)
     m.colors[7, 0] = np.inf

@@ -99,8 +99,8 @@ struct u3dg_rasterizer {
     int device = 0;
     Stream stream;
     RasterWorkspace ws;
-    DevModel model;
-    DevBuf<float> dl;
+    DevModel model, grads;
+    DevBuf<float> dl, ndc; // with grads: kept, as a buffer allocated per call can cost 0.3 ms to map and as much to free
     bool haveForward = false;
 };
 
@@ -498,6 +498,7 @@ int u3dg_rasterizer_create(u3dg_rasterizer **out)
         requireDevice();
         auto r = std::make_unique<u3dg_rasterizer>();
         U3DG_CUDA(cudaGetDevice(&r->device));
+        r->ws.wholeLists = true;
         *out = r.release();
     });
 }
@@ -563,22 +564,20 @@ int u3dg_rasterizer_backward(u3dg_rasterizer *r, const u3dg_model *model, const 
         R.model.upload(*model, s);
         R.dl.reserve(P * 3);
         U3DG_CUDA(cudaMemcpyAsync(R.dl.p, dl_drgb, P * 3 * sizeof(float), cudaMemcpyHostToDevice, s));
-        DevModel g;
-        g.upload(*grads, s);
-        DevBuf<float> ndc;
-        ndc.reserve(std::max<size_t>(n, 1), true);
+        R.grads.upload(*grads, s);
+        R.ndc.reserve(std::max<size_t>(n, 1), true);
         if (mean2d_grad_ndc && n > 0)
-            U3DG_CUDA(cudaMemcpyAsync(ndc.p, mean2d_grad_ndc, n * sizeof(float), cudaMemcpyHostToDevice, s));
+            U3DG_CUDA(cudaMemcpyAsync(R.ndc.p, mean2d_grad_ndc, n * sizeof(float), cudaMemcpyHostToDevice, s));
         R.ws.backwardComposite(R.dl.p, s);
         ChainArgs a = R.ws.chainArgs(R.model.params());
-        a.grads = g.params();
-        a.gradAccum = mean2d_grad_ndc ? ndc.p : nullptr;
+        a.grads = R.grads.params();
+        a.gradAccum = mean2d_grad_ndc ? R.ndc.p : nullptr;
         a.gradCount = nullptr;
         launchChain(a, false, s);
         U3DG_CUDA(cudaGetLastError());
-        g.download(*grads, n, s);
+        R.grads.download(*grads, n, s);
         if (mean2d_grad_ndc && n > 0)
-            U3DG_CUDA(cudaMemcpyAsync(mean2d_grad_ndc, ndc.p, n * sizeof(float), cudaMemcpyDeviceToHost, s));
+            U3DG_CUDA(cudaMemcpyAsync(mean2d_grad_ndc, R.ndc.p, n * sizeof(float), cudaMemcpyDeviceToHost, s));
         R.stream.sync();
     });
 }
@@ -674,6 +673,7 @@ int u3dg_rasterizer_set_tile_culling(u3dg_rasterizer *r, int enable)
     return guarded([&] {
         u3dg_rasterizer &R = rz(r);
         R.ws.cullTiles = enable != 0;
+        R.ws.wholeLists = !enable; // culled lists are the trainers', and so is their backward
         R.haveForward = false; // the next backward needs a forward with the new lists
     });
 }

@@ -378,10 +378,11 @@ void RasterWorkspace::composite(cudaStream_t stream, bool keep)
     const int pb = st.tile_size <= 8 ? 8 : 16;
     const int per = st.tile_size > pb ? st.tile_size / pb : 1;
     blockStop.reserve(size_t(std::max(1, tilesX * per * tilesY * per)));
-    if (keep)
+    segmented = keep && !wholeLists;
+    if (segmented)
         reserveSegments();
     RasterArgs a = rasterArgs();
-    if (!keep)
+    if (!segmented)
         a.segment = 0;
     launchCompositeForward(a, rgb.p, finalT.p, nContrib.p, stream);
 }
@@ -389,6 +390,11 @@ void RasterWorkspace::composite(cudaStream_t stream, bool keep)
 void RasterWorkspace::backwardComposite(const float *dLdRgb, cudaStream_t stream)
 {
     const RasterArgs a = rasterArgs();
+    if (!segmented) {
+        sums.reserve(size_t(std::max(n, 1)) * kG2d);
+        launchCompositeBackwardList(a, dLdRgb, finalT.p, nContrib.p, partial.p, blockStop.p, stream);
+        return;
+    }
     launchBackwardUnits(a, blockStop.p, units.p, unitCount.p, stream);
     launchCompositeBackward(a, dLdRgb, finalT.p, nContrib.p, partial.p, blockStop.p, units.p, unitCount.p, stream);
 }
@@ -414,6 +420,8 @@ ChainArgs RasterWorkspace::chainArgs(const Params &P) const
     a.tilesX = tilesX;
     a.blocksX = tilesX * per;
     a.counts = counts.p;
+    a.order = depthOrder.p;
+    a.sums = segmented ? nullptr : sums.p;
     return a;
 }
 

@@ -218,6 +218,7 @@ struct RasterWorkspace {
     DevBuf<int2> units;                           // the backward's (block, segment) units
     DevBuf<int> unitCounters; // RasterArgs::counters
     DevBuf<float> rgb, finalT;
+    DevBuf<float> sums; // backward over whole lists: 9 sums per Gaussian
     // device-side sizes of the last pass and their pinned host copy
     DevBuf<BinCounts> counts;
     HostPinned<BinCounts> hostCounts;
@@ -232,6 +233,9 @@ struct RasterWorkspace {
     // Culling applies while tile rows fit the row table's 16-bit cumulative counts (< 8192 tiles).
     bool culled() const { return cullTiles && tilesX < 8192; }
     bool ordersTiles() const;
+    // Backward over whole lists (the rasterizer's, launchCompositeBackwardList) instead of segments; and what
+    // the last forward was for.
+    bool wholeLists = false, segmented = false;
     u3dg_camera cam{};
     u3dg_raster_settings st{};
 

@@ -396,6 +396,69 @@ __device__ __forceinline__ void gatherPartials(const ChainArgs &a, int start, in
     }
 }
 
+// The sums of partials of launchCompositeBackwardList, in a fixed tree over the emission order: one warp per 32
+// depth ranks, a segmented scan over the lanes.
+__global__ void __launch_bounds__(256) partialSumKernel(ChainArgs a)
+{
+    pdlEntry();
+    if (a.counts != nullptr && a.counts->abortIter >= 0)
+        return;
+    const int lane = threadIdx.x & 31, w = int((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (w * 32 >= a.n)
+        return;
+    const int r = w * 32 + lane, total = a.counts->effTotal;
+    const bool valid = r < a.n;
+    auto firstOf = [&](int rank) { return rank < a.n ? a.offs[a.order[rank]] : total; };
+    const int o = valid ? firstOf(r) : INT_MAX, oEnd = valid ? firstOf(r + 1) : INT_MAX;
+    const int first = __shfl_sync(0xffffffffu, o, 0), last = firstOf(min(w * 32 + 32, a.n));
+    const float4 *partial = reinterpret_cast<const float4 *>(a.partial);
+    float acc[kG2d] = {};
+    for (int c0 = first; c0 < last; c0 += 32) {
+        const int e = c0 + lane;
+        const int2 lp = e < last ? a.listPos[e] : make_int2(INT_MAX, 0);
+        // Owner of entry e: the last lane whose start offset is not above e.
+        int owner = 0;
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1)
+            if (__shfl_sync(0xffffffffu, o, owner + step) <= e)
+                owner += step;
+        float v[kG2d] = {};
+        // Tiles covered by several CTAs: their slots, added in slot order.
+        for (int sl = 0; sl < a.subSlots; ++sl) {
+            const int pos = partialAt(a, lp, sl);
+            if (pos >= 0)
+                addPartial(partial + size_t(sl) * (a.subStride / 4) + size_t(pos) * kPartialF4, v);
+        }
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int ownerUp = __shfl_up_sync(0xffffffffu, owner, d);
+            const bool same = lane >= d && ownerUp == owner;
+#pragma unroll
+            for (int k = 0; k < kG2d; ++k) {
+                const float up = __shfl_up_sync(0xffffffffu, v[k], d);
+                if (same)
+                    v[k] += up;
+            }
+        }
+        // This lane's rank: its last entry inside the chunk, if any.
+        const int lastE = min(min(oEnd, last), c0 + 32) - 1;
+        const bool has = valid && o < c0 + 32 && oEnd > c0 && lastE >= max(o, c0);
+        const int src = has ? lastE - c0 : lane;
+#pragma unroll
+        for (int k = 0; k < kG2d; ++k) {
+            const float got = __shfl_sync(0xffffffffu, v[k], src);
+            if (has)
+                acc[k] += got;
+        }
+    }
+    if (valid) {
+        float *dst = a.sums + size_t(a.order[r]) * kG2d;
+#pragma unroll
+        for (int k = 0; k < kG2d; ++k)
+            dst[k] = acc[k];
+    }
+}
+
 // Rasterizer::backward pass 2 (Rasterizer.cpp:432-544) for one Gaussian per thread, fused either with
 // Adam::step (kAdam: the trainer; gradients never leave registers) or with adding the gradients into
 // caller arrays (the unit entry point). It starts from the Gaussian's summed partials (gatherPartials),
@@ -420,7 +483,13 @@ __global__ void __launch_bounds__(kChainThreads, kChainWarps * 32 / kChainThread
     float g[kG2d];
     {
         const bool seen = i < a.n && a.radius[i] > 0;
-        gatherPartials(a, seen ? a.offs[i] : 0, seen ? a.tileCount[i] : 0, sGather[threadIdx.x >> 5], g);
+        if (kAdam || a.sums == nullptr) {
+            gatherPartials(a, seen ? a.offs[i] : 0, seen ? a.tileCount[i] : 0, sGather[threadIdx.x >> 5], g);
+        } else {
+#pragma unroll
+            for (int k = 0; k < kG2d; ++k)
+                g[k] = seen ? a.sums[size_t(i) * kG2d + k] : 0.0f;
+        }
     }
     if (i >= a.n)
         return;
@@ -448,6 +517,14 @@ __global__ void __launch_bounds__(kChainThreads, kChainWarps * 32 / kChainThread
         Ewa p;
         ewaProject(mu, qr, ls, cam, lim, a.st, p);
         const float z = p.pc[2];
+        if (!kAdam && a.sums != nullptr) { // dL/dconic to dL/dcovariance (Rasterizer.cpp:432-446)
+            const float dA = g[2], dB = g[3], dC = g[4], aa = p.a, bb = p.b, cc = p.c;
+            const float det = aa * cc - bb * bb;
+            const float det2 = det * det;
+            g[2] = (dA * -cc * cc + dB * bb * cc + dC * -bb * bb) / det2;
+            g[3] = (dA * 2 * bb * cc + dC * 2 * aa * bb) / det2 + dB * (-1.0f / det - 2 * bb * bb / det2);
+            g[4] = (dA * -bb * bb + dB * aa * bb + dC * -aa * aa) / det2;
+        }
         const float G00 = g[2], G01 = 0.5f * g[3], G11 = g[4]; // dL/dcovariance
         float dSigma[9];
 #pragma unroll
@@ -741,7 +818,9 @@ void launchChain(const ChainArgs &a, bool adam, cudaStream_t s)
         return;
     if (adam)
         { launchPdl(chainKernel<true>, blocks(a.n, kChainThreads), kChainThreads, 0, s, a); countLaunch(); }
-    else
+    if (!adam && a.sums)
+        { launchPdl(partialSumKernel, blocks((long long)(a.n + 31) / 32 * 32, 256), 256, 0, s, a); countLaunch(); }
+    if (!adam)
         { launchPdl(chainKernel<false>, blocks(a.n, kChainThreads), kChainThreads, 0, s, a); countLaunch(); }
 }
 

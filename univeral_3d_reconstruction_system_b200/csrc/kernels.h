@@ -97,6 +97,10 @@ struct ChainArgs {
     const BinCounts *counts; // the kernel does nothing when counts->abortIter >= 0
     float *gradAccum;     // |dL/dmean2d| NDC statistic (may be null)
     int *gradCount;       // visibility count (may be null)
+    // Non-Adam mode, partials of launchCompositeBackwardList: the Gaussians by depth rank, and space for 9 sums
+    // per Gaussian (null: the partials are gathered by the chain rule).
+    const uint32_t *order;
+    float *sums;
     Params grads;         // non-Adam mode: gradients are added here
     Params m, v;          // Adam mode: moments
     float stepSize[5];    // Adam mode: lr / bc1 per group
@@ -233,6 +237,10 @@ void launchCompositeForward(const RasterArgs &a, float *rgb, float *finalT, int 
 void launchCompositeBackward(const RasterArgs &a, const float *dLdRgb, const float *finalT, const int *nContrib,
                              float *partial, const int *stop, const int2 *units, const int *unitCount,
                              cudaStream_t s);
+// The same over whole lists: partials hold dL/dmean2d and dL/dconic, stop is written, and a forward with
+// segment 0 is enough.
+void launchCompositeBackwardList(const RasterArgs &a, const float *dLdRgb, const float *finalT, const int *nContrib,
+                                 float *partial, int *stop, cudaStream_t s);
 
 // loss.cu
 struct LossScratch {

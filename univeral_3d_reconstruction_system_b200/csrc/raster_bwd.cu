@@ -447,6 +447,221 @@ __global__ void __launch_bounds__(kThreads<PB>, U3DG_BWD_MIN_BLOCKS * 64 / kThre
     }
 }
 
+// ---------------------------------------------------------------- whole lists
+
+// The rasterizer's own backward, for lists that are not culled: a 16x16 (or 8x8) block replays its whole list,
+// two pixels of a column per thread, and sums the moments of the pixel offsets. A program that takes gradients
+// from the rasterizer gets them in this order of summation: a few ill-conditioned Gaussians' (of 250k at
+// 640x480) come out of sums that cancel to 1e-3 of their terms' rounding, and any other order moves those by
+// up to 1e-2 of the gradients' root mean square. The trainers take units of segments (40 % of the time).
+struct PixelPair {
+    float2 T, nacc, lcd, nla; // transmittance, -(colour dot behind), last contributor's colour dot, -its alpha
+    float2 d0, d1, d2, fy;    // dL/dpixel per channel, pixel row
+    float2 fT, bgDot;         // final transmittance, background . dL/dpixel (background term only)
+    int nC0, nC1;             // contributor counts
+};
+
+// dL/dmean2d and dL/dconic of an entry's summed moments (Rasterizer.cpp:405-412): dmean = -(A m_x + B m_y,
+// C m_y + B m_x), dA = -m_xx / 2, dB = -m_xy, dC = -m_yy / 2.
+__device__ __forceinline__ void finishMoments(const float4 &Q, float g[kG2d])
+{
+    const float mx = g[0], my = g[1];
+    g[0] = -(Q.x * mx + Q.y * my);
+    g[1] = -(Q.z * my + Q.y * mx);
+    g[2] = -0.5f * g[2];
+    g[3] = -g[3];
+    g[4] = -0.5f * g[4];
+}
+
+__device__ __forceinline__ PixelPair initPair(bool in0, bool in1, size_t pix0, size_t pix1, float fy0, float fy1,
+                                              const float *dLdRgb, const float *finalT, const int *nContrib,
+                                              const float *bg)
+{
+    PixelPair p;
+    p.nC0 = in0 ? nContrib[pix0] : 0;
+    p.nC1 = in1 ? nContrib[pix1] : 0;
+    p.fT = make_float2(in0 ? finalT[pix0] : 0.0f, in1 ? finalT[pix1] : 0.0f);
+    p.d0 = make_float2(in0 ? dLdRgb[pix0 * 3] : 0.0f, in1 ? dLdRgb[pix1 * 3] : 0.0f);
+    p.d1 = make_float2(in0 ? dLdRgb[pix0 * 3 + 1] : 0.0f, in1 ? dLdRgb[pix1 * 3 + 1] : 0.0f);
+    p.d2 = make_float2(in0 ? dLdRgb[pix0 * 3 + 2] : 0.0f, in1 ? dLdRgb[pix1 * 3 + 2] : 0.0f);
+    p.bgDot = make_float2(bg[0] * p.d0.x + bg[1] * p.d1.x + bg[2] * p.d2.x, bg[0] * p.d0.y + bg[1] * p.d1.y + bg[2] * p.d2.y);
+    p.T = p.fT;
+    p.nacc = p.lcd = p.nla = both(0.0f);
+    p.fy = make_float2(fy0, fy1);
+    return p;
+}
+
+template <int PB>
+constexpr int kListWarps = PB * PB / 64;
+
+template <int PB, bool kBg>
+__global__ void __launch_bounds__(32 * kListWarps<PB>, 6) compositeBackwardListKernel(RasterArgs a, const float *dLdRgb,
+                                                                                      const float *finalTIn,
+                                                                                      const int *nContribIn, float *partial,
+                                                                                      int *stop)
+{
+    pdlEntry();
+    constexpr int NW = kListWarps<PB>, NT = 32 * NW, NB = NT, NG = NB / 32, WX = PB / 8;
+    __shared__ float4 sP[NB], sQ[NB], sR[NB];
+    __shared__ uint32_t mask[NW][NG];
+    __shared__ int sMax;
+    __shared__ __align__(16) float sWarp[NW * NB * kG2d]; // per warp: NB entries x 9 sums
+    int bx = int(blockIdx.x) % a.blocksX, by = int(blockIdx.x) / a.blocksX;
+    if (a.tileOrder) {
+        const int per = a.tileSize / PB, t = a.tileOrder[int(blockIdx.x) / (per * per)], at = int(blockIdx.x) % (per * per);
+        bx = t % a.tilesX * per + at % per;
+        by = t / a.tilesX * per + at / per;
+    }
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const WarpBlock wb(lane, bx * WX + warp % WX, by * WX + warp / WX);
+    const int tile = tileOf<PB>(a, bx, by);
+    const int start = a.tileOffsets[tile];
+    const bool in0 = wb.px < a.width && wb.py0 < a.height, in1 = wb.px < a.width && wb.py1 < a.height;
+    if (a.subSlots > 1) { // this block's slot array: its position in the tile, row-major
+        const int per = a.tileSize / PB;
+        partial += size_t((by % per) * per + bx % per) * a.subStride;
+    }
+    PixelPair pp = initPair(in0, in1, in0 ? size_t(wb.py0) * a.width + wb.px : 0,
+                            in1 ? size_t(wb.py1) * a.width + wb.px : 0, float(wb.py0), float(wb.py1), dLdRgb,
+                            finalTIn, nContribIn, a.bg);
+    const float2 one2 = both(1.0f);
+    const float fx = float(wb.px), minA = a.minAlpha;
+    const float4 *rec = reinterpret_cast<const float4 *>(a.rec);
+    if (tid == 0)
+        sMax = 0;
+    __syncthreads();
+    const int nMax = max(pp.nC0, pp.nC1);
+    if (nMax > 0)
+        atomicMax(&sMax, nMax);
+    // This warp's pixels have no contributor at or beyond wMax: the warp skips those entries.
+    const int wMax = __reduce_max_sync(0xffffffffu, nMax);
+    __syncthreads();
+    const int jmax = sMax;
+    if (tid == 0)
+        stop[by * a.blocksX + bx] = start + jmax;
+    float *myWarp = sWarp + size_t(warp) * NB * kG2d;
+    for (int bEnd = jmax; bEnd > 0; bEnd -= NB) {
+        const int bStart = max(0, bEnd - NB), cnt = bEnd - bStart;
+        __syncthreads();
+        stage<WX, NG>(loadRecord(rec, tid < cnt ? a.entries[start + bStart + tid] : -1), tid < cnt, tid, sP, sQ, sR, mask, bx, by);
+        {
+            float4 *z = reinterpret_cast<float4 *>(sWarp);
+            for (int k = tid; k < NW * NB * kG2d / 4; k += NT)
+                z[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+        __syncthreads();
+        for (int k = NG - 1; k >= 0; --k) {
+            uint32_t bits = mask[warp][k];
+            const int lim = wMax - bStart - 32 * k; // entries of this group below wMax
+            if (lim <= 0)
+                continue;
+            if (lim < 32)
+                bits &= (1u << lim) - 1u;
+            while (bits) {
+                const int hb = 31 - __clz(bits);
+                bits &= ~(1u << hb);
+                const int jj = 32 * k + hb;
+                const int j = bStart + jj;
+                float c[kG2d];
+#pragma unroll
+                for (int q = 0; q < kG2d; ++q)
+                    c[q] = 0.0f;
+                bool act = false;
+                if (j < pp.nC0 || j < pp.nC1) {
+                    const float4 P = sP[jj], Q = sQ[jj];
+                    const float dx = __fsub_rn(P.x, fx);
+                    const ColumnTerms ct = columnTerms(Q, dx);
+                    // Falloff exponents exactly as the forward decides (powerAt's order; products
+                    // paired, sums scalar).
+                    const float2 dy = make_float2(__fsub_rn(P.y, pp.fy.x), __fsub_rn(P.y, pp.fy.y));
+                    const float2 cdd = mul2rn(mul2rn(both(Q.z), dy), dy);
+                    const float2 bdy = mul2rn(both(ct.bx), dy);
+                    const float2 hq = mul2rn(both(-0.5f), make_float2(__fadd_rn(ct.axx, cdd.x), __fadd_rn(ct.axx, cdd.y)));
+                    const float2 pw = make_float2(__fsub_rn(hq.x, bdy.x), __fsub_rn(hq.y, bdy.y));
+                    bool v0 = j < pp.nC0 && !(pw.x > 0.0f || pw.x < P.z);
+                    bool v1 = j < pp.nC1 && !(pw.y > 0.0f || pw.y < P.z);
+                    if (v0 || v1) {
+                        // One back-to-front step of Rasterizer.cpp:385-416 for both pixels (a pixel that
+                        // is out gets exp(0) and zero weights, and keeps its state).
+                        const float2 G = make_float2(rasterExp(v0 ? pw.x : 0.0f), rasterExp(v1 ? pw.y : 0.0f));
+                        const float2 raw = mul2rn(both(Q.w), G);
+                        const float al0 = (raw.x < kMaxAlpha) ? raw.x : kMaxAlpha;
+                        const float al1 = (raw.y < kMaxAlpha) ? raw.y : kMaxAlpha;
+                        v0 = v0 && !(al0 < minA);
+                        v1 = v1 && !(al1 < minA);
+                        if (v0 || v1) {
+                            act = true;
+                            const float4 R = sR[jj];
+                            // Transmittance before this entry: T / (1 - alpha), correctly rounded.
+                            const float2 om = add2rn(one2, make_float2(-al0, -al1));
+                            const float Tn0 = __fdiv_rn(pp.T.x, om.x), Tn1 = __fdiv_rn(pp.T.y, om.y);
+                            pp.T = make_float2(v0 ? Tn0 : pp.T.x, v1 ? Tn1 : pp.T.y);
+                            const float2 w = mul2rn(make_float2(v0 ? al0 : 0.0f, v1 ? al1 : 0.0f), pp.T);
+                            // dAlpha = (colour . dpix - accum . dpix) T (Rasterizer.cpp:393-399), on the
+                            // dot products; accum takes the previous contributor's colour first.
+                            const float2 rd = fma2rn(both(R.z), pp.d2, fma2rn(both(R.y), pp.d1, mul2rn(both(R.x), pp.d0)));
+                            const float2 nacc = fma2rn(pp.nla, add2rn(pp.lcd, pp.nacc), pp.nacc);
+                            float2 dAl = mul2rn(add2rn(rd, nacc), pp.T);
+                            pp.nacc = make_float2(v0 ? nacc.x : pp.nacc.x, v1 ? nacc.y : pp.nacc.y);
+                            pp.lcd = make_float2(v0 ? rd.x : pp.lcd.x, v1 ? rd.y : pp.lcd.y);
+                            pp.nla = make_float2(v0 ? -al0 : pp.nla.x, v1 ? -al1 : pp.nla.y);
+                            // (An infinite dL/dpixel of a pixel that is out stays out: 0 * inf is not 0.)
+                            auto only = [&](const float2 &d) { return make_float2(v0 ? d.x : 0.0f, v1 ? d.y : 0.0f); };
+                            const float2 wd0 = mul2rn(w, only(pp.d0)), wd1 = mul2rn(w, only(pp.d1)), wd2 = mul2rn(w, only(pp.d2));
+                            c[5] = wd0.x + wd0.y;
+                            c[6] = wd1.x + wd1.y;
+                            c[7] = wd2.x + wd2.y;
+                            if (kBg) {
+                                dAl.x += -pp.fT.x / om.x * pp.bgDot.x;
+                                dAl.y += -pp.fT.y / om.y * pp.bgDot.y;
+                            }
+                            // A clamped alpha has a colour gradient only.
+                            const bool m0 = v0 && !(raw.x > kMaxAlpha), m1 = v1 && !(raw.y > kMaxAlpha);
+                            float2 t = mul2rn(G, dAl);
+                            t = make_float2(m0 ? t.x : 0.0f, m1 ? t.y : 0.0f);
+                            c[8] = t.x + t.y;
+                            // Per-pixel moments of dPow; both pixels share dx, so dx multiplies the thread's
+                            // sums once.
+                            const float2 dPow = mul2rn(both(Q.w), t);
+                            const float2 pdy = mul2rn(dPow, dy);
+                            const float2 pdyy = mul2rn(pdy, dy);
+                            c[1] = pdy.x + pdy.y;
+                            c[4] = pdyy.x + pdyy.y;
+                            c[0] = dx * (dPow.x + dPow.y);
+                            c[2] = dx * c[0];
+                            c[3] = dx * c[1];
+                        }
+                    }
+                }
+                if (__any_sync(0xffffffffu, act)) {
+                    float v8;
+                    const float v = blockReduce9<32>(c, lane, &v8);
+                    if ((lane & 3) == 0)
+                        myWarp[jj * kG2d + (lane >> 2)] = v;
+                    if (lane == 1)
+                        myWarp[jj * kG2d + 8] = v8;
+                }
+            }
+        }
+        __syncthreads();
+        if (tid < cnt) {
+            float sum[kG2d];
+#pragma unroll
+            for (int q = 0; q < kG2d; ++q)
+                sum[q] = sWarp[tid * kG2d + q];
+            for (int w = 1; w < NW; ++w)
+#pragma unroll
+                for (int q = 0; q < kG2d; ++q)
+                    sum[q] += sWarp[(size_t(w) * NB + tid) * kG2d + q];
+            finishMoments(sQ[tid], sum);
+            float4 *dst = reinterpret_cast<float4 *>(partial) + size_t(start + bStart + tid) * (kPartial / 4);
+            dst[0] = make_float4(sum[0], sum[1], sum[2], sum[3]);
+            dst[1] = make_float4(sum[4], sum[5], sum[6], sum[7]);
+            dst[2] = make_float4(sum[8], 0.0f, 0.0f, 0.0f);
+        }
+    }
+}
+
 // One CTA: the backward's units (block, segment) in block order, by an exclusive scan of the blocks'
 // segment counts.
 __global__ void __launch_bounds__(1024) backwardUnitsKernel(RasterArgs a, int pb, int *stop, int2 *units, int *unitCount)
@@ -529,6 +744,29 @@ static void launchBackward(const RasterArgs &a, const float *dLdRgb, const float
 void launchBackwardUnits(const RasterArgs &a, int *stop, int2 *units, int *unitCount, cudaStream_t s)
 {
     { launchPdl(backwardUnitsKernel, 1, 1024, 0, s, a, a.tileSize <= 8 ? 8 : 16, stop, units, unitCount); countLaunch(); }
+}
+
+void launchCompositeBackwardList(const RasterArgs &a, const float *dLdRgb, const float *finalT, const int *nContrib,
+                                 float *partial, int *stop, cudaStream_t s)
+{
+    const int blocks = a.blocksX * a.blocksY;
+    if (blocks <= 0)
+        return;
+    const bool bg = a.bg[0] != 0.0f || a.bg[1] != 0.0f || a.bg[2] != 0.0f;
+    auto run = [&](auto pb, auto kBg) {
+        constexpr int PB = decltype(pb)::value;
+        { launchPdl(compositeBackwardListKernel<PB, decltype(kBg)::value>, blocks, 32 * kListWarps<PB>, 0, s, a, dLdRgb, finalT, nContrib, partial, stop); countLaunch(); }
+    };
+    auto sized = [&](auto kBg) {
+        if (a.tileSize <= 8)
+            run(std::integral_constant<int, 8>{}, kBg);
+        else
+            run(std::integral_constant<int, 16>{}, kBg);
+    };
+    if (bg)
+        sized(std::true_type{});
+    else
+        sized(std::false_type{});
 }
 
 void launchCompositeBackward(const RasterArgs &a, const float *dLdRgb, const float *finalT, const int *nContrib,
