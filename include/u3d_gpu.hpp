@@ -554,8 +554,8 @@ public:
         check(u3dg_batch_tile_size(m_b, scene, &t, nullptr));
         return t;
     }
-    // Compositing schedule chosen with the tile size: the forward kernel's pixel block edge and the
-    // list entries each forward / backward thread stages per batch (u3dg_trainer_set_raster_schedule).
+    // Compositing schedule chosen with the tile size: the list entries the backward stages per batch; the
+    // forward's values choose nothing (u3dg_trainer_set_raster_schedule).
     struct RasterSchedule {
         int forwardBlock, forwardDepth, backwardDepth;
     };

@@ -270,8 +270,9 @@ int u3dg_rasterizer_pixel_state(u3dg_rasterizer *r, float *final_t, int *n_contr
 /* No reference counterpart (the trainers' tile culling at the unit boundary): with enable = 1 the
  * following forwards list each Gaussian only in the tiles of its rectangle that its contributing
  * ellipse (alpha >= min_alpha) can reach, as the trainers do by default; every tile list is then an
- * order-preserving subsequence of Rasterizer::binTiles' list (Rasterizer.cpp:206-261) and images,
- * pixel state and gradients are unchanged. 0 (the default) keeps the reference's lists. */
+ * order-preserving subsequence of Rasterizer::binTiles' list (Rasterizer.cpp:206-261), images and
+ * final transmittances are unchanged, and gradients agree to rounding (a backward then adds its sums in
+ * the trainers' order, else over whole lists). 0 (the default) keeps the reference's lists. */
 int u3dg_rasterizer_set_tile_culling(u3dg_rasterizer *r, int enable);
 void u3dg_rasterizer_destroy(u3dg_rasterizer *r);
 
