@@ -238,3 +238,32 @@ def test_views_whose_lists_do_not_fit_at_first(u3dg):
         d = image.astype(np.float64) - (p.rgb.astype(np.float32) * np.float32(1 / 255)).astype(np.float64)
         want.append(-10 * np.log10(np.mean(d * d)))
     assert abs(psnr - np.mean(want)) < 1e-5 * np.mean(want)
+
+
+@pytest.mark.parametrize("width, height", [(161, 121), (1040, 800)])
+@pytest.mark.parametrize("culled", [False, True])
+@pytest.mark.parametrize("n", [0, 1, 32, 33, 513, 5000])
+def test_backward_with_nothing_in_view(u3dg, n, culled, width, height):
+    # Every Gaussian behind the camera, in a new rasterizer, in one that has seen them, and in one that has seen
+    # fewer: no list has an entry (up to 2048 tiles and above), and every gradient is exactly zero.
+    rng = np.random.default_rng(n)
+    seen = random_model(n, rng, 1.0, 3.0, 0.02, 0.1)
+    behind = seen.copy()
+    behind.means[:, 2] = -behind.means[:, 2] - 10.0
+    cam, st = make_camera(width, height, 0.8 * width), RasterSettings(background=(0.1, 0.2, 0.3))
+    w = rng.uniform(-1, 1, (height, width, 3)).astype(np.float32)
+    for before in (None, seen, random_model(max(1, n // 3), rng, 1.0, 3.0, 0.02, 0.1)):
+        r = u3dg.Rasterizer()
+        r.set_tile_culling(culled)
+        if before is not None:
+            r.forward(before, cam, st)
+            r.backward(before, w)
+        image = r.forward(behind, cam, st)
+        np.testing.assert_array_equal(image, np.broadcast_to(np.float32(st.background), image.shape))
+        ndc = np.zeros(n, np.float32)
+        g = r.backward(behind, w, None, ndc)
+        for k in ("means", "scales", "quats", "opacities", "colors"):
+            assert not np.any(getattr(g, k)), k
+        assert not np.any(ndc)
+        offsets, ids = r.tiles()
+        assert not np.any(offsets) and len(ids) == 0

@@ -829,6 +829,9 @@ __global__ void __launch_bounds__(kRanks, 3) tileScatterKernel(TileBins b, const
         if (chunk == 0)
             for (int d = tid; d <= tiles; d += kRanks)
                 b.tileOffsets[d] = 0;
+        // A backward takes its loop bounds from the first emissions, of unseen Gaussians too.
+        if (b.offsById && chunk * kRanks + tid < b.n)
+            b.offsById[b.sortedIds[chunk * kRanks + tid]] = 0;
         return;
     }
     const Listed l = loadListed(b.sortedIds, b.tileCount, b.rect, b.rowTab, b.cullRec != nullptr, chunk * kRanks + tid, b.n);
