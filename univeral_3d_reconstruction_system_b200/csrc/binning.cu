@@ -26,7 +26,6 @@
 #include "tile_cull.cuh"
 
 #include <algorithm>
-#include <atomic>
 #include <climits>
 
 namespace u3dg {
@@ -1023,23 +1022,6 @@ inline int grid(long long n, int t) { return int((n + t - 1) / t); }
 
 } // namespace
 
-// Lets a kernel that is about to use `need` bytes of shared memory, more than the default 48 KB, use up to
-// `most` on the current device: once per kernel and device, since the attribute belongs to the device's
-// copy of the kernel.
-template <class K>
-static void allowShared(K kernel, size_t need, size_t most, std::atomic<uint64_t> &done)
-{
-    if (need <= 48 * 1024)
-        return;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const uint64_t bit = uint64_t(1) << (dev & 63);
-    if (dev > 63 || !(done.load(std::memory_order_acquire) & bit)) {
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most));
-        done.fetch_or(bit, std::memory_order_release);
-    }
-}
-
 int radixBlocks(int nMax) { return std::max(1, std::min(kMaxBlocks, (nMax + kTile - 1) / kTile)); }
 
 size_t radixHistEntries(int nMax) { return size_t(1 << 8) * size_t(radixBlocks(nMax)); }
@@ -1080,7 +1062,7 @@ void radixSortDepth(const uint32_t *keys, uint2 *pairsA, uint2 *pairsB, uint32_t
         return;
     if (n <= kSmallSort) {
         constexpr size_t shared = kSmallSort * sizeof(uint2) + size_t(kDepthWarps) * kDigits * sizeof(uint16_t);
-        static std::atomic<uint64_t> allowed{0};
+        static PerDevice allowed;
         allowShared(depthSortSmallKernel, shared + 8192, shared, allowed); // with the static arrays
         { launchPdl(depthSortSmallKernel, 1, kDepthThreads, shared, s, keys, n, sortedIds); countLaunch(); }
         return;
@@ -1109,7 +1091,7 @@ void binByTile(const TileBins &b, int *hist, int *tileTotals, int *chunkTotals, 
 {
     const int G = rankChunks(b.n), stride = (b.tiles + 1) / 2 * 2;
     const size_t scatterShared = size_t(stride) * (sizeof(int) + kRankWarps * sizeof(uint16_t)); // 36 bytes per tile
-    static std::atomic<uint64_t> allowed{0};
+    static PerDevice allowed;
     allowShared(tileScatterKernel, scatterShared + 24 * 1024, size_t(kMaxTiles) * 36, allowed); // with the static arrays
     { launchPdl(tileCountKernel, G, kRanks, b.tiles * sizeof(int), s, b, hist, chunkTotals); countLaunch(); }
     { launchPdl(tileScanKernel, (b.tiles + 31) / 32 + 1, kScanThreads, 0, s, hist, G, b.tiles, tileTotals, chunkTotals, cap); countLaunch(); }

@@ -2,6 +2,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "per_device.h"
 
 #include <utility>
 
@@ -38,6 +39,21 @@ inline void launchPdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sm
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+// Lets a kernel that is about to use `need` bytes of shared memory, static arrays among them, have up to `most`
+// of dynamic shared memory on the current device, where `need` is above the default 48 KB.
+template <class K>
+inline void allowShared(K kernel, size_t need, size_t most, PerDevice &done)
+{
+    if (need <= 48 * 1024)
+        return;
+    int device = 0;
+    cudaGetDevice(&device);
+    done.get(device, [&] {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most));
+        return 1;
+    });
 }
 
 // Device-side sizes of one bin pass. The host never waits for them inside a step: it reads the

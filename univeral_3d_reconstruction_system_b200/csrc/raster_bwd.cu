@@ -717,11 +717,10 @@ __global__ void __launch_bounds__(1024) backwardUnitsKernel(RasterArgs a, int pb
 }
 
 template <class K>
-int residentCtas(K kernel, int threads, size_t smem)
+int residentCtas(int device, K kernel, int threads, size_t smem)
 {
-    int dev = 0, sms = 0, perSm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int sms = 0, perSm = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, threads, smem);
     return std::max(1, sms * std::max(1, perSm));
 }
@@ -734,10 +733,12 @@ static void launchBackward(const RasterArgs &a, const float *dLdRgb, const float
 {
     using S = BackwardShape<PB, 32>;
     const size_t smem = size_t(kTeams<PB>) * S::BLOCKS * S::BATCH * BD * kG2d * sizeof(float); // 18 KB or 36 KB at PB 16
-    static const int ctas = [&] {
-        cudaFuncSetAttribute(compositeBackwardKernel<PB, BD, kBg>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        return residentCtas(compositeBackwardKernel<PB, BD, kBg>, kThreads<PB>, smem);
-    }();
+    static PerDevice allowed, resident;
+    allowShared(compositeBackwardKernel<PB, BD, kBg>, smem + 16 * 1024, smem, allowed); // with the static arrays
+    int device = 0;
+    cudaGetDevice(&device);
+    const int ctas = resident.get(
+        device, [&] { return residentCtas(device, compositeBackwardKernel<PB, BD, kBg>, kThreads<PB>, smem); });
     { launchPdl(compositeBackwardKernel<PB, BD, kBg>, ctas, kThreads<PB>, smem, s, a, dLdRgb, finalT, nContrib, partial, stop, units, unitCount); countLaunch(); }
 }
 
