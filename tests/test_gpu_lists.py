@@ -77,6 +77,25 @@ def test_backward_with_few_and_many_units(u3dg, oracle, width, height, n, backgr
            3e-4)
 
 
+@pytest.mark.parametrize("tile", [32, 64])
+@pytest.mark.parametrize("width, height, n", [(368, 400, 40), (480, 352, 40), (480, 352, 700)])
+def test_batch_depths_give_the_same_model(u3dg, tile, width, height, n):
+    # On both sides of 592 units of the backward (4 per SM), where the order in which an entry's pixels are added
+    # changes: 575, 660, and lists of more segments than one. The same bits.
+    rng = np.random.default_rng(n)
+    m = _stack(n, rng, 0.02)
+    cam = make_camera(width, height, 1.5 * width)
+    photo = TrainImage(cam, rng.integers(0, 256, (height, width, 3)).astype(np.uint8))
+    flat = []
+    for depth in (1, 2):
+        t = u3dg.Trainer(m, [photo], 1.0, TrainOptions(max_gaussians=n, refine_stop=0, raster=RasterSettings(tile_size=tile)))
+        t.set_raster_schedule(8, 1, depth)
+        t.step(3)
+        flat.append(t.model().flat())
+    assert not np.array_equal(flat[0], m.flat())
+    np.testing.assert_array_equal(flat[0], flat[1])
+
+
 @pytest.mark.parametrize("culled", [False, True])
 def test_a_non_finite_pixel_gradient_reaches_only_what_blends_there(u3dg, culled):
     rng = np.random.default_rng(3)

@@ -388,11 +388,15 @@ __device__ __forceinline__ void backwardUnit(const RasterArgs &a, int block, int
 #endif
 
 // A CTA of 16x16 blocks has 128 threads: two teams of 64 (16 lanes per 8x8 block), each with a unit of its
-// own, or, where the launch has no more units than CTAs, one team of 128 (32 lanes). Then the launch lasts as
+// own, or, where the launch has no more than `few` units (kFewUnits per SM, about one per CTA), one team of
+// 128 (32 lanes). Then the launch lasts as
 // long as one unit, 64 entries at about 800 cycles each by 16 lanes (a warp alone on its scheduler): 52 us
 // against 38 us on 4k Gaussians at 96x72. With more units than CTAs the instructions count: at two units
 // per CTA the two shapes are even (+-2 us of 60), on 300k Gaussians at 640x480 32 lanes take 169 us against
-// 143.
+// 143. The two shapes add an entry's pixels in another order, so the line is a number of units of its own and
+// not the grid: it must not move with the registers or the shared memory of one instance (the batch depths
+// give the same bits).
+constexpr int kFewUnits = 4;
 template <int PB>
 constexpr int kTeams = PB == 8 ? 1 : 2;
 template <int PB>
@@ -424,7 +428,7 @@ __device__ __forceinline__ void backwardUnits(const RasterArgs &a, const float *
 template <int PB, int BD, bool kBg>
 __global__ void __launch_bounds__(kThreads<PB>, U3DG_BWD_MIN_BLOCKS * 64 / kThreads<PB>)
     compositeBackwardKernel(RasterArgs a, const float *dLdRgb, const float *finalTIn, const int *nContribIn,
-                            float *partial, const int *stop, const int2 *units, const int *unitCount)
+                            float *partial, const int *stop, const int2 *units, const int *unitCount, int few)
 {
     pdlEntry();
     using S = BackwardShape<PB, PB == 8 ? 32 : 16>;
@@ -436,7 +440,7 @@ __global__ void __launch_bounds__(kThreads<PB>, U3DG_BWD_MIN_BLOCKS * 64 / kThre
     __shared__ int sOdd[TEAMS], sNext[TEAMS];
     extern __shared__ __align__(16) float sBlock[]; // per team and 8x8 block: NB entries x 9 sums
     const int count = *unitCount;
-    if (PB == 8 || count <= int(gridDim.x)) {
+    if (PB == 8 || count <= few) {
         backwardUnits<PB, 32, BD, kBg>(a, dLdRgb, finalTIn, nContribIn, partial, stop, units, count, sP[0], sQ[0], sR[0],
                                        mask[0], sOdd[0], sNext[0], sBlock);
     } else {
@@ -716,13 +720,14 @@ __global__ void __launch_bounds__(1024) backwardUnitsKernel(RasterArgs a, int pb
         *unitCount = carry;
 }
 
-template <class K>
-int residentCtas(int device, K kernel, int threads, size_t smem)
+int multiprocessors(int device)
 {
-    int sms = 0, perSm = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, threads, smem);
-    return std::max(1, sms * std::max(1, perSm));
+    static PerDevice count;
+    return count.get(device, [&] {
+        int sms = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        return std::max(1, sms);
+    });
 }
 
 } // namespace
@@ -737,9 +742,12 @@ static void launchBackward(const RasterArgs &a, const float *dLdRgb, const float
     allowShared(compositeBackwardKernel<PB, BD, kBg>, smem + 16 * 1024, smem, allowed); // with the static arrays
     int device = 0;
     cudaGetDevice(&device);
-    const int ctas = resident.get(
-        device, [&] { return residentCtas(device, compositeBackwardKernel<PB, BD, kBg>, kThreads<PB>, smem); });
-    { launchPdl(compositeBackwardKernel<PB, BD, kBg>, ctas, kThreads<PB>, smem, s, a, dLdRgb, finalT, nContrib, partial, stop, units, unitCount); countLaunch(); }
+    const int sms = multiprocessors(device), perSm = resident.get(device, [&] {
+        int n = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, compositeBackwardKernel<PB, BD, kBg>, kThreads<PB>, smem);
+        return std::max(1, n);
+    });
+    { launchPdl(compositeBackwardKernel<PB, BD, kBg>, sms * perSm, kThreads<PB>, smem, s, a, dLdRgb, finalT, nContrib, partial, stop, units, unitCount, kFewUnits * sms); countLaunch(); }
 }
 
 void launchBackwardUnits(const RasterArgs &a, int *stop, int2 *units, int *unitCount, cudaStream_t s)
