@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/u3dg.h"
+#include "rounded.cuh"
 
 namespace u3dg {
 
@@ -94,21 +95,6 @@ struct Ewa {
     float a, b, c;
 };
 
-// Several divisions by one divisor, each correctly rounded by Markstein's sequence (IBM Journal of Research
-// and Development 34, 1990): the quotient by the correctly rounded reciprocal, corrected by its exact
-// remainder. For |a| and quotients between 2^-100 and 2^100 the result has the bits of a / b (3.7e10 quotients
-// compared); an infinite quotient, whose remainder is NaN, is kept.
-struct Divisor {
-    float b, y;
-    __device__ __forceinline__ explicit Divisor(float d) : b(d), y(1.0f / d) {}
-    __device__ __forceinline__ float under(float a) const
-    {
-        const float q = __fmul_rn(a, y);
-        const float c = __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
-        return c == c ? c : q;
-    }
-};
-
 // Bounds of x / z and y / z outside which the projection's Jacobian is clamped, the same for all Gaussians of
 // a view. All lanes of a warp call it; four of them divide.
 struct ViewLimits {
@@ -125,9 +111,11 @@ __device__ __forceinline__ ViewLimits viewLimits(const u3dg_camera &cam)
 }
 
 // EWA projection of Gaussian i (computeProjection, Rasterizer.cpp:48-110), same operation order;
-// files including this are compiled with -fmad=false so no multiply-add is contracted.
-__device__ __forceinline__ bool ewaProject(const float mu[3], const float qr[4], const float ls[3],
-                                           const u3dg_camera &cam, const ViewLimits &lim, const u3dg_raster_settings &st, Ewa &p)
+// files including this are compiled with -fmad=false so no multiply-add is contracted. D: Division, or Divisor
+// where the caller looks at ops.
+template <class D>
+__device__ __forceinline__ bool ewaProjectBy(const float mu[3], const float qr[4], const float ls[3], const u3dg_camera &cam,
+                                             const ViewLimits &lim, const u3dg_raster_settings &st, Ewa &p, Operands &ops)
 {
     const float *R = cam.R;
     p.pc[0] = R[0] * mu[0] + R[1] * mu[1] + R[2] * mu[2] + cam.t[0];
@@ -142,10 +130,10 @@ __device__ __forceinline__ bool ewaProject(const float mu[3], const float qr[4],
         p.q[0] = 1;
         p.q[1] = p.q[2] = p.q[3] = 0;
     } else {
-        const Divisor byNorm(p.qNorm);
+        const D byNorm(p.qNorm, ops);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            p.q[k] = byNorm.under(qr[k]);
+            p.q[k] = byNorm.under(qr[k], ops);
     }
     quatToRot(p.q[0], p.q[1], p.q[2], p.q[3], p.Rq);
 #pragma unroll
@@ -161,8 +149,8 @@ __device__ __forceinline__ bool ewaProject(const float mu[3], const float qr[4],
 #pragma unroll
         for (int c = 0; c < 3; ++c)
             p.Sigma[r * 3 + c] = p.M[r * 3] * p.M[c * 3] + p.M[r * 3 + 1] * p.M[c * 3 + 1] + p.M[r * 3 + 2] * p.M[c * 3 + 2];
-    const Divisor byZ(z), byZ2(z * z);
-    const float xz = byZ.under(p.pc[0]), yz = byZ.under(p.pc[1]);
+    const D byZ(z, ops), byZ2(z * z, ops);
+    const float xz = byZ.under(p.pc[0], ops), yz = byZ.under(p.pc[1], ops);
     // std::min(a, b) = (b < a) ? b : a and std::max(a, b) = (a < b) ? b : a, kept literally.
     const float mxz = (-lim.xNeg < xz) ? xz : -lim.xNeg;
     const float cxz = (mxz < lim.xPos) ? mxz : lim.xPos;
@@ -174,8 +162,8 @@ __device__ __forceinline__ bool ewaProject(const float mu[3], const float qr[4],
     p.limTy = cyz;
     p.tx = z * cxz;
     p.ty = z * cyz;
-    const float J00 = byZ.under(cam.fx), J02 = byZ2.under(-cam.fx * p.tx);
-    const float J11 = byZ.under(cam.fy), J12 = byZ2.under(-cam.fy * p.ty);
+    const float J00 = byZ.under(cam.fx, ops), J02 = byZ2.under(-cam.fx * p.tx, ops);
+    const float J11 = byZ.under(cam.fy, ops), J12 = byZ2.under(-cam.fy * p.ty, ops);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         p.T0[k] = J00 * R[k] + J02 * R[6 + k];

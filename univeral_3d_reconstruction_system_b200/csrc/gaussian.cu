@@ -68,7 +68,8 @@ __global__ void __launch_bounds__(256) projectKernel(Params P, int n, u3dg_camer
     Ewa p;
     int radius = 0;
     int4 rect = make_int4(0, 0, 0, 0);
-    bool visible = ewaProject(mu, qr, ls, cam, lim, st, p);
+    Operands any;
+    bool visible = ewaProjectBy<Division>(mu, qr, ls, cam, lim, st, p, any);
     float det = 0.0f, u = 0.0f, v = 0.0f;
     if (visible) {
         det = p.a * p.c - p.b * p.b;
@@ -76,9 +77,8 @@ __global__ void __launch_bounds__(256) projectKernel(Params P, int n, u3dg_camer
     }
     if (visible) {
         const float z = p.pc[2];
-        const Divisor byZ(z);
-        u = byZ.under(cam.fx * p.pc[0]) + cam.cx;
-        v = byZ.under(cam.fy * p.pc[1]) + cam.cy;
+        u = cam.fx * p.pc[0] / z + cam.cx;
+        v = cam.fy * p.pc[1] / z + cam.cy;
         const float mid = 0.5f * (p.a + p.c);
         const float lambda = mid + sqrtf(stdMax(0.1f, mid * mid - det));
         const float rf = ceilf(3.0f * sqrtf(lambda));
@@ -89,11 +89,10 @@ __global__ void __launch_bounds__(256) projectKernel(Params P, int n, u3dg_camer
         if (u + fr < 0 || v + fr < 0 || u - fr >= float(cam.width) || v - fr >= float(cam.height)) {
             visible = false;
         } else {
-            const Divisor byTile{float(ts)};
-            const int tx0 = max(0, int(floorf(byTile.under(u - fr))));
-            const int ty0 = max(0, int(floorf(byTile.under(v - fr))));
-            const int tx1 = min(tilesX, int(floorf(byTile.under(u + fr))) + 1);
-            const int ty1 = min(tilesY, int(floorf(byTile.under(v + fr))) + 1);
+            const int tx0 = max(0, int(floorf((u - fr) / float(ts))));
+            const int ty0 = max(0, int(floorf((v - fr) / float(ts))));
+            const int tx1 = min(tilesX, int(floorf((u + fr) / float(ts))) + 1);
+            const int ty1 = min(tilesY, int(floorf((v + fr) / float(ts))) + 1);
             if (tx0 >= tx1 || ty0 >= ty1)
                 visible = false;
             else
@@ -200,24 +199,8 @@ __device__ __forceinline__ void adamOne(float &p, float &m, float &v, float g, f
     p -= adamQuotient(m, v, stepSize, invSqrtBc2);
 }
 
-__device__ __forceinline__ float rcpApprox(float x)
-{
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-__device__ __forceinline__ float rsqrtApprox(float x)
-{
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // Adam of a Gaussian's elements in two groups of K and L values per Gaussian: adamOne's arithmetic with
-// Markstein's correctly rounded square root and quotient (Divisor) in their range: v 0 or from 2^-100 to 2^100
-// (all such v compared with the correctly rounded root) and |step m| 0 or from 2^-90 to 2^60; a lane with any
-// other value takes the operators.
+// roundedRoot and roundedQuotient where these are right for all of a lane's values (adamUsual), else the operators.
 template <int K, int L>
 __device__ __forceinline__ void adamGroups(float *p, float *m, float *v, const float *g, float step, float *p2, float *m2, float *v2,
                                            const float *g2, float step2, int i, float inv)
@@ -229,22 +212,13 @@ __device__ __forceinline__ void adamGroups(float *p, float *m, float *v, const f
         y[k] = k < K ? m[K * i + k] : m2[L * i + k - K];
         z[k] = k < K ? v[K * i + k] : v2[L * i + k - K];
     }
-    auto within = [](float t, int lo, int hi) { // 2^lo <= t < 2^hi
-        return __float_as_uint(t) - (uint32_t(lo + 127) << 23) < (uint32_t(hi - lo) << 23);
-    };
     bool usual = true;
 #pragma unroll
     for (int k = 0; k < K + L; ++k) {
         adamMoments(y[k], z[k], k < K ? g[k] : g2[k - K]);
         const float a = (k < K ? step : step2) * y[k];
-        usual = usual && (z[k] == 0.0f || within(z[k], -100, 100)) && (a == 0.0f || within(fabsf(a), -90, 60));
-        const float r = rsqrtApprox(z[k]), s0 = __fmul_rn(z[k], r);
-        const float s = z[k] == 0.0f ? 0.0f : __fmaf_rn(__fmaf_rn(-s0, s0, z[k]), __fmul_rn(0.5f, r), s0);
-        const float den = s * inv + 1e-15f;
-        float w = rcpApprox(den);
-        w = __fmaf_rn(w, __fmaf_rn(-den, w, 1.0f), w);
-        const float q0 = __fmul_rn(a, w);
-        q[k] = __fmaf_rn(__fmaf_rn(-den, q0, a), w, q0);
+        usual = usual && adamUsual(a, z[k]);
+        q[k] = roundedQuotient(a, roundedRoot(z[k]) * inv + 1e-15f);
     }
     if (!usual)
 #pragma unroll
@@ -459,13 +433,109 @@ __global__ void __launch_bounds__(256) partialSumKernel(ChainArgs a)
     }
 }
 
+// The chain rule of one seen Gaussian from its 2D gradients g (listed: with dL/dconic, else dL/dcovariance) to its
+// means, scales and quaternion (Rasterizer.cpp:432-544). D: Divisor, right for usual operands, or Division.
+template <class D>
+__device__ __forceinline__ void chainRule(const ChainArgs &a, const u3dg_camera &cam, const ViewLimits &lim, const float mu[3],
+                                          const float qr[4], const float ls[3], const float (&g)[kG2d], bool listed, float gMeans[3],
+                                          float gScales[3], float gQuats[4], Operands &ops)
+{
+    Ewa p;
+    ewaProjectBy<D>(mu, qr, ls, cam, lim, a.st, p, ops);
+    const float z = p.pc[2];
+    const float dmx = g[0], dmy = g[1];
+    float G00 = g[2], db = g[3], G11 = g[4];
+    if (listed) { // dL/dconic to dL/dcovariance (Rasterizer.cpp:432-446)
+        const float dA = g[2], dB = g[3], dC = g[4], aa = p.a, bb = p.b, cc = p.c;
+        const float det = aa * cc - bb * bb;
+        const float det2 = det * det;
+        G00 = (dA * -cc * cc + dB * bb * cc + dC * -bb * bb) / det2;
+        db = (dA * 2 * bb * cc + dC * 2 * aa * bb) / det2 + dB * (-1.0f / det - 2 * bb * bb / det2);
+        G11 = (dA * -bb * bb + dB * aa * bb + dC * -aa * aa) / det2;
+    }
+    const float G01 = 0.5f * db;
+    float dSigma[9];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int l = 0; l < 3; ++l)
+            dSigma[k * 3 + l] = p.T0[k] * (G00 * p.T0[l] + G01 * p.T1[l]) + p.T1[k] * (G01 * p.T0[l] + G11 * p.T1[l]);
+    float TS0[3], TS1[3];
+#pragma unroll
+    for (int col = 0; col < 3; ++col) {
+        TS0[col] = p.T0[0] * p.Sigma[col] + p.T0[1] * p.Sigma[3 + col] + p.T0[2] * p.Sigma[6 + col];
+        TS1[col] = p.T1[0] * p.Sigma[col] + p.T1[1] * p.Sigma[3 + col] + p.T1[2] * p.Sigma[6 + col];
+    }
+    float dT0[3], dT1[3];
+#pragma unroll
+    for (int col = 0; col < 3; ++col) {
+        dT0[col] = 2.0f * (G00 * TS0[col] + G01 * TS1[col]);
+        dT1[col] = 2.0f * (G01 * TS0[col] + G11 * TS1[col]);
+    }
+    float dM[9];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int col = 0; col < 3; ++col)
+            dM[r * 3 + col] = 2.0f * (dSigma[r * 3] * p.M[col] + dSigma[r * 3 + 1] * p.M[3 + col] + dSigma[r * 3 + 2] * p.M[6 + col]);
+    float dRq[9];
+#pragma unroll
+    for (int col = 0; col < 3; ++col) {
+        float ds = 0;
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            ds += dM[r * 3 + col] * p.Rq[r * 3 + col];
+            dRq[r * 3 + col] = dM[r * 3 + col] * p.s[col];
+        }
+        gScales[col] = ds * p.s[col];
+    }
+    const float w = p.q[0], x = p.q[1], y = p.q[2], zq = p.q[3];
+    const float dw = 2 * (-zq * dRq[1] + y * dRq[2] + zq * dRq[3] - x * dRq[5] - y * dRq[6] + x * dRq[7]);
+    const float dx = 2 * (y * dRq[1] + zq * dRq[2] + y * dRq[3] - 2 * x * dRq[4] - w * dRq[5] + zq * dRq[6] + w * dRq[7] - 2 * x * dRq[8]);
+    const float dy = 2 * (-2 * y * dRq[0] + x * dRq[1] + w * dRq[2] + x * dRq[3] + zq * dRq[5] - w * dRq[6] + zq * dRq[7] - 2 * y * dRq[8]);
+    const float dz = 2 * (-2 * zq * dRq[0] - w * dRq[1] + x * dRq[2] + w * dRq[3] - 2 * zq * dRq[4] + y * dRq[5] + x * dRq[6] + y * dRq[7]);
+    const float dq[4] = {dw, dx, dy, dz};
+    const D byNorm(p.qNorm, ops);
+    const float qdot = dq[0] * p.q[0] + dq[1] * p.q[1] + dq[2] * p.q[2] + dq[3] * p.q[3];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        gQuats[k] = byNorm.under(dq[k] - qdot * p.q[k], ops);
+    const float *R = cam.R;
+    const float dJ00 = dT0[0] * R[0] + dT0[1] * R[1] + dT0[2] * R[2];
+    const float dJ02 = dT0[0] * R[6] + dT0[1] * R[7] + dT0[2] * R[8];
+    const float dJ11 = dT1[0] * R[3] + dT1[1] * R[4] + dT1[2] * R[5];
+    const float dJ12 = dT1[0] * R[6] + dT1[1] * R[7] + dT1[2] * R[8];
+    const float z2 = z * z, z3 = z2 * z;
+    const D byZ(z, ops), byZ2(z2, ops), byZ3(z3, ops);
+    float dpc[3] = {0, 0, 0};
+    dpc[2] += byZ2.under(dJ00 * -cam.fx, ops) + byZ3.under(dJ02 * 2 * cam.fx * p.tx, ops) + byZ2.under(dJ11 * -cam.fy, ops) +
+              byZ3.under(dJ12 * 2 * cam.fy * p.ty, ops);
+    const float dtx = byZ2.under(dJ02 * -cam.fx, ops);
+    const float dty = byZ2.under(dJ12 * -cam.fy, ops);
+    if (p.clampX)
+        dpc[2] += dtx * p.limTx;
+    else
+        dpc[0] += dtx;
+    if (p.clampY)
+        dpc[2] += dty * p.limTy;
+    else
+        dpc[1] += dty;
+    dpc[0] += byZ.under(dmx * cam.fx, ops);
+    dpc[1] += byZ.under(dmy * cam.fy, ops);
+    dpc[2] += byZ2.under(-dmx * cam.fx * p.pc[0], ops) - byZ2.under(dmy * cam.fy * p.pc[1], ops);
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        gMeans[k] = R[k] * dpc[0] + R[3 + k] * dpc[1] + R[6 + k] * dpc[2];
+}
+
 // Rasterizer::backward pass 2 (Rasterizer.cpp:432-544) for one Gaussian per thread, fused either with
 // Adam::step (kAdam: the trainer; gradients never leave registers) or with adding the gradients into
 // caller arrays (the unit entry point). It starts from the Gaussian's summed partials (gatherPartials),
 // which never go through memory.
-// Bound by the latency of its loads and by instructions (57 us on 300k Gaussians at 640x480, where its 190 MB
+// Bound by the latency of its loads and by instructions (60 us on 300k Gaussians at 640x480, where its 190 MB
 // take 29 us): loads of a group of parameters stand ahead of the group's stores, quotients share their
-// divisors' reciprocals (68 us with the division operator, whose slow path every zero takes). Small CTAs
+// divisors' reciprocals (68 us with the division operator, whose slow path every zero takes; 56 without a look
+// at the operands, which made quotients by a subnormal z^3 NaN). Small CTAs
 // spread few Gaussians over the chip (4k: 22 us at 256 threads, 21.5 at 64, the rest even). Registers are capped
 // at 64 for 32 warps per SM (28 warps: 63 us, 40: 80 us).
 constexpr int kChainThreads = 64, kChainWarps = 32;
@@ -514,90 +584,10 @@ __global__ void __launch_bounds__(kChainThreads, kChainWarps * 32 / kChainThread
         const float mu[3] = {P.means[3 * i], P.means[3 * i + 1], P.means[3 * i + 2]};
         const float qr[4] = {P.quats[4 * i], P.quats[4 * i + 1], P.quats[4 * i + 2], P.quats[4 * i + 3]};
         const float ls[3] = {P.scales[3 * i], P.scales[3 * i + 1], P.scales[3 * i + 2]};
-        Ewa p;
-        ewaProject(mu, qr, ls, cam, lim, a.st, p);
-        const float z = p.pc[2];
-        if (!kAdam && a.sums != nullptr) { // dL/dconic to dL/dcovariance (Rasterizer.cpp:432-446)
-            const float dA = g[2], dB = g[3], dC = g[4], aa = p.a, bb = p.b, cc = p.c;
-            const float det = aa * cc - bb * bb;
-            const float det2 = det * det;
-            g[2] = (dA * -cc * cc + dB * bb * cc + dC * -bb * bb) / det2;
-            g[3] = (dA * 2 * bb * cc + dC * 2 * aa * bb) / det2 + dB * (-1.0f / det - 2 * bb * bb / det2);
-            g[4] = (dA * -bb * bb + dB * aa * bb + dC * -aa * aa) / det2;
-        }
-        const float G00 = g[2], G01 = 0.5f * g[3], G11 = g[4]; // dL/dcovariance
-        float dSigma[9];
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-#pragma unroll
-            for (int l = 0; l < 3; ++l)
-                dSigma[k * 3 + l] = p.T0[k] * (G00 * p.T0[l] + G01 * p.T1[l]) + p.T1[k] * (G01 * p.T0[l] + G11 * p.T1[l]);
-        float TS0[3], TS1[3];
-#pragma unroll
-        for (int col = 0; col < 3; ++col) {
-            TS0[col] = p.T0[0] * p.Sigma[col] + p.T0[1] * p.Sigma[3 + col] + p.T0[2] * p.Sigma[6 + col];
-            TS1[col] = p.T1[0] * p.Sigma[col] + p.T1[1] * p.Sigma[3 + col] + p.T1[2] * p.Sigma[6 + col];
-        }
-        float dT0[3], dT1[3];
-#pragma unroll
-        for (int col = 0; col < 3; ++col) {
-            dT0[col] = 2.0f * (G00 * TS0[col] + G01 * TS1[col]);
-            dT1[col] = 2.0f * (G01 * TS0[col] + G11 * TS1[col]);
-        }
-        float dM[9];
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-#pragma unroll
-            for (int col = 0; col < 3; ++col)
-                dM[r * 3 + col] = 2.0f * (dSigma[r * 3] * p.M[col] + dSigma[r * 3 + 1] * p.M[3 + col] + dSigma[r * 3 + 2] * p.M[6 + col]);
-        float dRq[9];
-#pragma unroll
-        for (int col = 0; col < 3; ++col) {
-            float ds = 0;
-#pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                ds += dM[r * 3 + col] * p.Rq[r * 3 + col];
-                dRq[r * 3 + col] = dM[r * 3 + col] * p.s[col];
-            }
-            gScales[col] = ds * p.s[col];
-        }
-        const float w = p.q[0], x = p.q[1], y = p.q[2], zq = p.q[3];
-        const float dw = 2 * (-zq * dRq[1] + y * dRq[2] + zq * dRq[3] - x * dRq[5] - y * dRq[6] + x * dRq[7]);
-        const float dx = 2 * (y * dRq[1] + zq * dRq[2] + y * dRq[3] - 2 * x * dRq[4] - w * dRq[5] + zq * dRq[6] + w * dRq[7] - 2 * x * dRq[8]);
-        const float dy = 2 * (-2 * y * dRq[0] + x * dRq[1] + w * dRq[2] + x * dRq[3] + zq * dRq[5] - w * dRq[6] + zq * dRq[7] - 2 * y * dRq[8]);
-        const float dz = 2 * (-2 * zq * dRq[0] - w * dRq[1] + x * dRq[2] + w * dRq[3] - 2 * zq * dRq[4] + y * dRq[5] + x * dRq[6] + y * dRq[7]);
-        const float dq[4] = {dw, dx, dy, dz};
-        const Divisor byNorm(p.qNorm);
-        const float qdot = dq[0] * p.q[0] + dq[1] * p.q[1] + dq[2] * p.q[2] + dq[3] * p.q[3];
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            gQuats[k] = byNorm.under(dq[k] - qdot * p.q[k]);
-        const float *R = cam.R;
-        const float dJ00 = dT0[0] * R[0] + dT0[1] * R[1] + dT0[2] * R[2];
-        const float dJ02 = dT0[0] * R[6] + dT0[1] * R[7] + dT0[2] * R[8];
-        const float dJ11 = dT1[0] * R[3] + dT1[1] * R[4] + dT1[2] * R[5];
-        const float dJ12 = dT1[0] * R[6] + dT1[1] * R[7] + dT1[2] * R[8];
-        const float z2 = z * z, z3 = z2 * z;
-        const Divisor byZ(z), byZ2(z2), byZ3(z3);
-        float dpc[3] = {0, 0, 0};
-        dpc[2] += byZ2.under(dJ00 * -cam.fx) + byZ3.under(dJ02 * 2 * cam.fx * p.tx) + byZ2.under(dJ11 * -cam.fy) +
-                  byZ3.under(dJ12 * 2 * cam.fy * p.ty);
-        const float dtx = byZ2.under(dJ02 * -cam.fx);
-        const float dty = byZ2.under(dJ12 * -cam.fy);
-        if (p.clampX)
-            dpc[2] += dtx * p.limTx;
-        else
-            dpc[0] += dtx;
-        if (p.clampY)
-            dpc[2] += dty * p.limTy;
-        else
-            dpc[1] += dty;
-        dpc[0] += byZ.under(dmx * cam.fx);
-        dpc[1] += byZ.under(dmy * cam.fy);
-        dpc[2] += byZ2.under(-dmx * cam.fx * p.pc[0]) - byZ2.under(dmy * cam.fy * p.pc[1]);
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            gMeans[k] = R[k] * dpc[0] + R[3 + k] * dpc[1] + R[6 + k] * dpc[2];
+        Operands ops;
+        chainRule<Divisor>(a, cam, lim, mu, qr, ls, g, !kAdam && a.sums != nullptr, gMeans, gScales, gQuats, ops);
+        if (!ops.usual())
+            chainRule<Division>(a, cam, lim, mu, qr, ls, g, !kAdam && a.sums != nullptr, gMeans, gScales, gQuats, ops);
     }
 
     if constexpr (kAdam) {

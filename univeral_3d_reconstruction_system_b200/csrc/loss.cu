@@ -217,14 +217,23 @@ __global__ void __launch_bounds__(kThreads) lossForwardKernel(const float *rende
             const float vx = square[r].x - mx * mx, vy = square[r].y - my * my, vxy = cross[r] - mx * my;
             const float a1 = 2 * mx * my + kC1, a2 = 2 * vxy + kC2;
             const float b1 = mx * mx + my * my + kC1, b2 = vx + vy + kC2;
-            const Divisor by1(b1), by2(b2), by12(b1 * b2);
-            const float v = by12.under(a1 * a2);
+            // SSIM and its partials, dLds apart.
+            float v, dmu, dsq, dxy;
+            auto partials = [&](auto by1, auto by2, auto by12, Operands &ops) {
+                v = by12.under(a1 * a2, ops);
+                dmu = by12.under(2 * my * a2 - 2 * my * a1, ops) - v * (by1.under(2 * mx, ops) - by2.under(2 * mx, ops));
+                dsq = by2.under(-v, ops);
+                dxy = by12.under(2 * a1, ops);
+            };
+            Operands ops;
+            partials(Divisor(b1, ops), Divisor(b2, ops), Divisor(b1 * b2, ops), ops);
+            if (!ops.usual())
+                partials(Division(b1, ops), Division(b2, ops), Division(b1 * b2, ops), ops);
             ssim += double(v);
-            const float dmu = by12.under(2 * my * a2 - 2 * my * a1) - v * (by1.under(2 * mx) - by2.under(2 * mx));
             const size_t o = size_t(c) * P + size_t(gy) * W + gx;
             abc[o] = dLds * dmu;
-            abc[3 * P + o] = dLds * by2.under(-v);
-            abc[6 * P + o] = dLds * by12.under(2 * a1);
+            abc[3 * P + o] = dLds * dsq;
+            abc[6 * P + o] = dLds * dxy;
         }
     }
     __shared__ double warpSums[3][kThreads / 32];

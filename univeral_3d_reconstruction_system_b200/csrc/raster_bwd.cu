@@ -106,13 +106,6 @@ __device__ __forceinline__ float blockReduce9(const float c[kG2d], int lane, flo
     return v;
 }
 
-__device__ __forceinline__ float rcpApprox(float x)
-{
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // Barrier of the NT threads that work on one unit.
 template <int NT>
 __device__ __forceinline__ void teamSync(int barrier)
@@ -298,15 +291,10 @@ __device__ __forceinline__ void backwardUnit(const RasterArgs &a, int block, int
 #pragma unroll
             for (int p = 0; p < PAIRS; ++p) {
                 // One back-to-front step of Rasterizer.cpp:385-416 for two pixels. Transmittance before
-                // this entry: T / (1 - alpha), correctly rounded by Markstein's sequence (IBM Journal of
-                // Research and Development 34, 1990): reciprocal refined by one Newton step, quotient
-                // corrected by its exact remainder. 1 - alpha is a multiple of 2^-24 in [0.01, 1]; for all
-                // of those the refined reciprocal was compared with the correctly rounded one.
+                // this entry: T / (1 - alpha), rounded like the division (roundedQuotient2).
                 const float2 nom = add2rn(al[p], both(-1.0f)); // -(1 - alpha)
-                float2 y = make_float2(rcpApprox(-nom.x), rcpApprox(-nom.y));
-                y = fma2rn(y, fma2rn(nom, y, both(1.0f)), y);
-                float2 Tq = mul2rn(T[p], y);
-                Tq = fma2rn(fma2rn(nom, Tq, T[p]), y, Tq);
+                float2 y;
+                const float2 Tq = roundedQuotient2(T[p], nom, y);
                 T[p] = Tq;
                 const float2 w = mul2rn(al[p], Tq);
                 // dAlpha = (colour . dpix - acc) T (Rasterizer.cpp:393-399) on the dot products; this entry's
