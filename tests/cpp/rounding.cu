@@ -8,7 +8,7 @@ namespace {
 
 using namespace u3dg;
 
-enum Kind { kDivisor, kQuotient, kQuotient2, kRoot };
+enum Kind { kDivisor, kQuotient, kQuotient2, kRoot, kAdam1, kAdam32 };
 
 __global__ void compareKernel(int kind, const float *a, const float *b, size_t n, float *fused, float *exact, unsigned char *usual)
 {
@@ -27,11 +27,15 @@ __global__ void compareKernel(int kind, const float *a, const float *b, size_t n
             const float2 q = roundedQuotient2(make_float2(a[j], a[i]), make_float2(-b[j], -b[i]), y);
             fused[i] = i & 1 ? q.y : roundedQuotient2(make_float2(a[i], a[j]), make_float2(-b[i], -b[j]), y).x;
             exact[i] = __fdiv_rn(a[i], b[i]);
-        } else {
+        } else if (kind == kRoot) {
             fused[i] = roundedRoot(a[i]);
             exact[i] = __fsqrt_rn(a[i]);
+        } else {
+            const float inv = kind == kAdam1 ? 1.0f : 31.9f;
+            fused[i] = roundedQuotient(a[i], __fadd_rn(__fmul_rn(roundedRoot(b[i]), inv), 1e-15f));
+            exact[i] = __fdiv_rn(a[i], __fadd_rn(__fmul_rn(__fsqrt_rn(b[i]), inv), 1e-15f));
         }
-        usual[i] = ops.usual();
+        usual[i] = kind >= kAdam1 ? adamUsual(a[i], b[i]) : ops.usual();
     }
 }
 

@@ -15,7 +15,7 @@ import numpy as np
 import pytest
 
 CPP = Path(__file__).resolve().parent / "cpp"
-DIVISOR, QUOTIENT, QUOTIENT2, ROOT = range(4)
+DIVISOR, QUOTIENT, QUOTIENT2, ROOT, ADAM1, ADAM32 = range(6)
 N = 1 << 22
 
 
@@ -111,15 +111,34 @@ def test_any_other_operands_are_known_as_such(lib):
 @pytest.mark.gpu
 def test_adam_s_quotients(lib):
     rng = np.random.default_rng(3)
-    for a, b in ((powers(rng, -90, 60), np.abs(powers(rng, -50, 34))), hard(rng, -90, 60, -50, 34),
-                 (np.zeros(N, np.float32), np.abs(powers(rng, -50, 34)))):
+    for a, b in ((powers(rng, -90, 60), np.abs(powers(rng, -50, 55))), hard(rng, -90, 60, -50, 55),
+                 (np.zeros(N, np.float32), np.abs(powers(rng, -50, 55)))):
         same, _ = compare(lib, QUOTIENT, a, b)
-        same |= (a == 0)  # (a zero's sign does not matter there; its value does, below)
+        same |= (a == 0)  # (a zero's sign does not matter there)
         assert same.all(), (a[~same][:3], b[~same][:3])
     # Every significand of a divisor.
     every = np.arange(1 << 23, 1 << 24).astype(np.float32) * np.float32(2.0 ** -23)
     for a in (np.ones(1 << 23, np.float32), powers(rng, 0, 1, 1 << 23)):
         assert compare(lib, QUOTIENT, a, every)[0].all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", [ADAM1, ADAM32])  # the smallest and the largest bias correction
+def test_adam_s_range(lib, kind):
+    # Step sizes times first moments over second moments of every size, their extremes together among them: where
+    # the fused quotient is taken it is the operators', subnormal ones included.
+    rng = np.random.default_rng(6)
+    any_a, any_v = (rng.integers(0, 1 << 32, N, dtype=np.uint64).astype(np.uint32).view(np.float32) for _ in range(2))
+    small, large = powers(rng, -92, -80), np.abs(powers(rng, 40, 102))
+    some = 0
+    for a, v in ((any_a, np.abs(any_v)), (any_a, any_v), (small, large), (powers(rng, -92, 62), np.abs(powers(rng, -102, 102))),
+                 (powers(rng, 50, 62), np.abs(powers(rng, -102, -90))), (small, np.zeros(N, np.float32)),
+                 (np.zeros(N, np.float32), large), (powers(rng, -60, 0), np.abs(powers(rng, -80, 10)))):
+        same, usual = compare(lib, kind, a, v)
+        same |= (a == 0)  # (a zero's sign does not matter there)
+        assert (same | ~usual).all(), (a[~same & usual][:3], v[~same & usual][:3])
+        some += usual.sum()
+    assert some > 2 * N
 
 
 @pytest.mark.gpu

@@ -79,7 +79,8 @@ __device__ __forceinline__ float roundedRoot(float v)
     return v == 0.0f ? 0.0f : __fmaf_rn(__fmaf_rn(-s, s, v), __fmul_rn(0.5f, r), s);
 }
 
-// a / b for a = 0 or |a| from 2^-90 to 2^60, b from 2^-50 to 2^34 (the quotient stays normal).
+// a / b for a = 0 or |a| from 2^-90 to 2^60, b from 2^-50 to 2^55 (a subnormal quotient is right too: the remainder
+// is exact and the last step rounds once).
 __device__ __forceinline__ float roundedQuotient(float a, float b)
 {
     float y = rcpApprox(b);
