@@ -67,3 +67,32 @@ def test_batch_matches_scenes_trained_alone(u3dg, autotune, tile):
         s2 = t.stats()
         assert (s2.iteration, s2.loss, s2.psnr, s2.gaussians) == (st.iteration, st.loss, st.psnr, st.gaussians)
     b.close()
+
+
+def test_autotuner_times_what_makes_a_difference(u3dg):
+    # At tile 16 the backward's batch depth does nothing: one run is timed there, two at tiles 8 and 32, and a
+    # scene that takes tile 16 is given depth 1. Counted in kernel launches: 33 steps of the one run (13 of
+    # warm-up, 20 timed) and 43 of each of the others (10 profiled), within what recordings of graphs and odd
+    # launches add.
+    from univeral_3d_reconstruction_system_b200 import _lib
+
+    def launches():
+        return int(_lib.load().u3dg_launch_count())
+
+    for init, images, extent, options in _scenes(u3dg):
+        expected = 0
+        for tile, runs in ((16, 1), (8, 2), (32, 2)):
+            o = dataclasses.replace(options, raster=dataclasses.replace(options.raster, tile_size=tile), iterations=64)
+            t = u3dg.Trainer(init, images, extent, o)
+            n0 = launches()
+            t.step(43 if runs == 2 else 33)
+            t.synchronize()
+            expected += runs * (launches() - n0)
+            t.close()
+        n0 = launches()
+        b = u3dg.Batch([(init, images, extent, options)], autotune=True)
+        counted = launches() - n0
+        assert counted <= 1.08 * expected, (counted, expected)
+        tile, schedule, _ = b.schedule(0)
+        assert tile != 16 or schedule[2] == 1
+        b.close()

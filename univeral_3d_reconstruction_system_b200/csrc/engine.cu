@@ -1278,11 +1278,12 @@ RasterSchedule autotuneSchedule(const u3dg_model &initial, const u3dg_image *img
     static const int kTiles[3] = {16, 8, 32};
     RasterSchedule best{opt.raster.tile_size, 8, 1, 1, 0.0f};
     for (int tile : kTiles) {
-        // Two runs per tile, the backward at depth 1 and 2. Each times graph runs of whole steps, then
-        // profiled steps for the backward's own time; the tile's step time is the first run's corrected by
-        // the gain.
+        // A run times graph runs of whole steps. Where the backward's batch depth makes a difference there are
+        // two, at depth 1 and 2, each followed by profiled steps for the backward's own time; the tile's step
+        // time is the first run's corrected by the gain.
         float stepMs[2] = {}, bwdMs[2] = {};
-        for (int d = 0; d < 2; ++d) {
+        const int runs = backwardTakesDepth(tile) ? 2 : 1;
+        for (int d = 0; d < runs; ++d) {
             u3dg_train_options o = opt;
             o.raster.tile_size = tile;
             o.iterations = std::max(o.iterations, 64);
@@ -1302,6 +1303,8 @@ RasterSchedule autotuneSchedule(const u3dg_model &initial, const u3dg_image *img
             cudaEventDestroy(e0);
             cudaEventDestroy(e1);
             stepMs[d] /= float(2 * TrainerImpl::kGraphSteps);
+            if (runs == 1)
+                break;
             t.timer = new PhaseTimer();
             t.profiling = true;
             t.stepTo(t.iteration + TrainerImpl::kGraphSteps);
@@ -1309,7 +1312,7 @@ RasterSchedule autotuneSchedule(const u3dg_model &initial, const u3dg_image *img
             const u3dg_phase_times &acc = t.timer->acc;
             bwdMs[d] = acc.steps ? acc.backward_ms / float(acc.steps) : 0.0f;
         }
-        const int b = bwdMs[1] < bwdMs[0] ? 1 : 0;
+        const int b = runs == 2 && bwdMs[1] < bwdMs[0] ? 1 : 0;
         const float ms = stepMs[0] - (bwdMs[0] - bwdMs[b]);
         if (best.msPerStep == 0.0f || ms < best.msPerStep)
             best = RasterSchedule{tile, 8, 1, b + 1, ms};

@@ -771,7 +771,7 @@ void launchCompositeBackward(const RasterArgs &a, const float *dLdRgb, const flo
 {
     if (a.blocksX * a.blocksY <= 0)
         return;
-    const bool deep = a.backwardDepth >= 2 && a.tileSize != 16; // segments of 64 entries are one batch at tile 16
+    const bool deep = a.backwardDepth >= 2 && backwardTakesDepth(a.tileSize);
     const bool bg = a.bg[0] != 0.0f || a.bg[1] != 0.0f || a.bg[2] != 0.0f;
     auto run = [&](auto kBg) {
         constexpr bool B = decltype(kBg)::value;
