@@ -286,3 +286,26 @@ def test_backward_with_nothing_in_view(u3dg, n, culled, width, height):
         assert not np.any(ndc)
         offsets, ids = r.tiles()
         assert not np.any(offsets) and len(ids) == 0
+
+
+@pytest.mark.parametrize("culled", [False, True])
+@pytest.mark.parametrize("width, height", [(33, 37), (403, 340)])
+@pytest.mark.parametrize("minimum", [float("nan"), -0.5, -2.0, float("-inf")])
+def test_a_minimum_transmittance_that_nothing_is_below(u3dg, minimum, width, height, culled):
+    # No pixel terminates, as with a minimum of 0: the same image and gradients, by a team per block and by one
+    # warp (2,193 blocks of 8x8).
+    rng = np.random.default_rng(width)
+    m = _stack(90, rng, 0.3)
+    m.scales -= 1.0
+    cam = make_camera(width, height, 0.9 * width)
+    w = rng.uniform(-1, 1, (height, width, 3)).astype(np.float32)
+    out = []
+    for least in (0.0, minimum):
+        st = RasterSettings(background=(0.1, 0.2, 0.3), min_transmittance=least)
+        r = u3dg.Rasterizer()
+        r.set_tile_culling(culled)
+        image = r.forward(m, cam, st)
+        out.append([image, *r.pixel_state(), r.backward(m, w).flat()])
+    assert out[0][2].max() == 90 and out[0][1].min() < 1e-4
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)

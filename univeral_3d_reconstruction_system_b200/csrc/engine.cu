@@ -24,6 +24,7 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <limits>
 
 namespace u3dg {
 
@@ -332,7 +333,9 @@ RasterArgs RasterWorkspace::rasterArgs() const
     for (int k = 0; k < 3; ++k)
         a.bg[k] = st.background[k];
     a.minAlpha = st.min_alpha;
-    a.minTransmittance = st.min_transmittance;
+    // A pixel stops where its transmittance is below the minimum, which is nowhere if that is NaN; the forward
+    // asks where it is not (Blend::entry).
+    a.minTransmittance = std::isnan(st.min_transmittance) ? -std::numeric_limits<float>::infinity() : st.min_transmittance;
     const int pb = st.tile_size <= 8 ? 8 : 16;
     // Whole tiles of pixel blocks: a block past the image edge composites nothing, but (for tiles of
     // several blocks) still writes its slot of every entry of its tile.
