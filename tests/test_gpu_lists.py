@@ -309,3 +309,32 @@ def test_a_minimum_transmittance_that_nothing_is_below(u3dg, minimum, width, hei
     assert out[0][2].max() == 90 and out[0][1].min() < 1e-4
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("culled", [False, True])
+@pytest.mark.parametrize("background", [(0.0, 0.0, 0.0), (0.2, 0.4, 0.1)])
+@pytest.mark.parametrize("colour, weight", [(2.0 ** 102, 2.0 ** 40), (2.0 ** 70, 2.0 ** 70), (2.0 ** 125, 16.0)])
+def test_an_overflowing_product_reaches_only_what_blends_there(u3dg, colour, weight, background, culled):
+    # A finite colour and a finite dL/dpixel whose product is infinite: Gaussians that blend at no pixel of the
+    # bright one keep their gradients to the bit.
+    rng = np.random.default_rng(6)
+    m = random_model(150, rng, 1.0, 3.0, 0.02, 0.08)
+    m.means[7] = [0.0, 0.0, 2.5]
+    cam, st = make_camera(64, 48, 50.0), RasterSettings(background=background)
+    w = (rng.uniform(0.5, 1, (48, 64, 3)) * weight).astype(np.float32)
+    r = u3dg.Rasterizer()
+    r.set_tile_culling(culled)
+    image = r.forward(m, cam, st)
+    clean = r.backward(m, w)
+    bright = m.copy()
+    bright.colors[7] = colour / 0.2820948
+    covered = np.any(r.forward(bright, cam, st) != image, axis=-1)
+    got = r.backward(bright, w)
+    assert not np.isfinite(got.opacities[7])
+    # Who blends at the covered pixels: whose opacity has a gradient from them.
+    r.forward(m, cam, st)
+    there = r.backward(m, np.repeat(covered[..., None], 3, axis=2).astype(np.float32))
+    apart = there.opacities.reshape(-1) == 0
+    assert apart.sum() > 50 and 0 < covered.sum() < covered.size // 4
+    for k in ("means", "scales", "quats", "opacities", "colors"):
+        np.testing.assert_array_equal(getattr(got, k)[apart], getattr(clean, k)[apart])

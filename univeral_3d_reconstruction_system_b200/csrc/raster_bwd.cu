@@ -106,6 +106,9 @@ __device__ __forceinline__ float blockReduce9(const float c[kG2d], int lane, flo
     return v;
 }
 
+// Below 2^60, so that a product of two such values, and the sums of a few, are finite.
+__device__ __forceinline__ bool moderate(float v) { return fabsf(v) < 1.152921504606846976e18f; }
+
 // Barrier of the NT threads that work on one unit.
 template <int NT>
 __device__ __forceinline__ void teamSync(int barrier)
@@ -184,7 +187,7 @@ __device__ __forceinline__ void backwardUnit(const RasterArgs &a, int block, int
         }
     }
     int bMax = 0; // no pixel of this 8x8 block has a contributor at or beyond bMax: entries from there are skipped
-    bool odd = false; // a non-finite dL/dpixel or kept colour
+    bool odd = false; // a huge or non-finite dL/dpixel or kept colour
 #pragma unroll
     for (int k = 0; k < PPL; ++k) {
         if (last[k] > jEnd)
@@ -192,7 +195,7 @@ __device__ __forceinline__ void backwardUnit(const RasterArgs &a, int block, int
         nC[k] = min(last[k], jEnd);
         bMax = max(bMax, nC[k]);
         const float b = kBg ? -fT[k] * (a.bg[0] * g0[k] + a.bg[1] * g1[k] + a.bg[2] * g2[k]) : 0.0f;
-        odd = odd || !finite(g0[k]) || !finite(g1[k]) || !finite(g2[k]) || !finite(t[k]) || !finite(b) || !finite(behind[k]);
+        odd = odd || !moderate(g0[k]) || !moderate(g1[k]) || !moderate(g2[k]) || !moderate(t[k]) || !moderate(b) || !moderate(behind[k]);
         auto set = [&](float2 *v, float x) { (k & 1 ? v[k / 2].y : v[k / 2].x) = x; };
         set(T, t[k]);
         set(acc, behind[k]);
@@ -231,12 +234,12 @@ __device__ __forceinline__ void backwardUnit(const RasterArgs &a, int block, int
             const bool valid = slot < cnt;
             stage<S::WX, NG>(loadRecord(rec, valid ? a.entries[start + bStart + slot] : -1), valid, slot, sP, sQ, sR, mask, bx,
                           by);
-            if (valid && !(finite(sR[slot].x) && finite(sR[slot].y) && finite(sR[slot].z)))
+            if (valid && !(moderate(sR[slot].x) && moderate(sR[slot].y) && moderate(sR[slot].z)))
                 sOdd = 1;
         }
         teamSync<NT>(barrier);
-        // A non-finite colour or dL/dpixel must reach only the pixels and entries that blend: then the
-        // factors of pixels that do not are replaced by zeros (0 * inf is not 0).
+        // A non-finite colour or dL/dpixel, or a product of two that is, must reach only the pixels and entries
+        // that blend: then the factors of pixels that do not are replaced by zeros (0 * inf is not 0).
         const bool strict = odd || sOdd != 0;
         int k = NG;
         uint32_t bits = 0;

@@ -150,7 +150,6 @@ __device__ __forceinline__ float powerAt(const float4 &Q, const ColumnTerms &c, 
 
 __device__ __forceinline__ float rasterExp(float x) { return expf(x); }
 
-
 __device__ __forceinline__ bool finite(float v) { return fabsf(v) < __int_as_float(0x7f800000); }
 
 } // namespace u3dg
