@@ -61,21 +61,38 @@ int u3dg_batch_create(const u3dg_model *initial, const u3dg_image *const *images
         }
         auto b = std::make_unique<u3dg_batch>();
         U3DG_CUDA(cudaGetDevice(&b->device));
+        bool compact = false; // once the device had no room for all scenes' trainers otherwise
+        auto create = [&](int s) {
+            const RasterSchedule &rs = b->schedules[size_t(s)];
+            u3dg_train_options o = options[s];
+            o.raster.tile_size = rs.tileSize;
+            auto t = std::make_unique<u3dg_trainer>();
+            t->impl = std::make_unique<TrainerImpl>(initial[s], images[s], image_counts[s], extents[s], o, false, compact);
+            t->impl->ws.backwardDepth = rs.backwardDepth;
+            t->ownedByBatch = true;
+            b->scenes.push_back(std::move(t));
+        };
+        auto add = [&](int s) {
+            if (int(b->schedules.size()) == s)
+                b->schedules.push_back(autotune ? autotuneSchedule(initial[s], images[s], image_counts[s], extents[s], options[s])
+                                                : RasterSchedule{options[s].raster.tile_size, 8, 1, 1, 0.0f});
+            create(s);
+        };
         for (int s = 0; s < scenes; ++s) {
             if (initial[s].count > 0 && (!initial[s].means || !initial[s].scales || !initial[s].quats ||
                                          !initial[s].opacities || !initial[s].colors))
                 throw StatusError(U3DG_ERR_INVALID_ARG, "scene " + std::to_string(s) + ": model has NULL arrays");
-            u3dg_train_options o = options[s];
-            RasterSchedule rs{o.raster.tile_size, 8, 1, 1, 0.0f};
-            if (autotune)
-                rs = autotuneSchedule(initial[s], images[s], image_counts[s], extents[s], options[s]);
-            o.raster.tile_size = rs.tileSize;
-            auto t = std::make_unique<u3dg_trainer>();
-            t->impl = std::make_unique<TrainerImpl>(initial[s], images[s], image_counts[s], extents[s], o);
-            t->impl->ws.backwardDepth = rs.backwardDepth;
-            t->ownedByBatch = true;
-            b->schedules.push_back(rs);
-            b->scenes.push_back(std::move(t));
+            try {
+                add(s);
+            } catch (const StatusError &e) {
+                if (e.status != U3DG_ERR_OOM || compact)
+                    throw;
+                compact = true;
+                b->scenes.clear();
+                for (int k = 0; k < s; ++k)
+                    create(k);
+                add(s);
+            }
         }
         *out = b.release();
     });

@@ -153,8 +153,18 @@ void RasterWorkspace::reserveIntersections(size_t capacity)
 
 void RasterWorkspace::reservePartials()
 {
-    listPos.reserve(size_t(icap), true);
-    partial.reserve(size_t(icap) * kPartial * size_t(partialSlots), true);
+    auto grow = [&] {
+        listPos.reserve(size_t(icap), true);
+        partial.reserve(size_t(icap) * kPartial * size_t(partialSlots), true);
+    };
+    try {
+        grow();
+    } catch (const StatusError &e) {
+        if (e.status != U3DG_ERR_OOM || wholeLists)
+            throw;
+        releaseSegments();
+        grow();
+    }
 }
 
 void RasterWorkspace::planEntries(DeviceSlab &slab, size_t capacity)
@@ -249,6 +259,10 @@ void RasterWorkspace::planPixels(DeviceSlab &slab, size_t count, size_t pixels, 
     const int pb = tileSize <= 8 ? 8 : 16;
     const int per = tileSize > pb ? tileSize / pb : 1;
     slab.add(blockStop, size_t(std::max(1, tx * per * ty * per)));
+    if (wholeLists) {
+        slab.add(sums, std::max<size_t>(count, 1) * kG2d);
+        return;
+    }
     const size_t slots = icap / segmentOf(tileSize) + size_t(tx) * ty + 1;
     slab.add(segments, slots * tileSize * tileSize);
     slab.add(units, slots * per * per);
@@ -362,14 +376,30 @@ int RasterWorkspace::segmentOf(int tileSize)
     return tileSize <= 16 ? 64 : tileSize * tileSize / 4;
 }
 
-void RasterWorkspace::reserveSegments()
+bool RasterWorkspace::reserveSegments()
 {
     const int ts = st.tile_size, pb = ts <= 8 ? 8 : 16, per = ts > pb ? ts / pb : 1;
     const size_t tiles = size_t(tilesX) * tilesY, slots = segmentSlots(tiles);
-    segments.reserve(slots * ts * ts);
-    units.reserve(slots * per * per);
-    blockMax.reserve(tiles * (ts / 8) * (ts / 8));
-    unitCount.reserve(1);
+    try {
+        segments.reserve(slots * ts * ts);
+        units.reserve(slots * per * per);
+        blockMax.reserve(tiles * (ts / 8) * (ts / 8));
+        unitCount.reserve(1);
+    } catch (const StatusError &e) {
+        if (e.status != U3DG_ERR_OOM)
+            throw;
+        releaseSegments();
+    }
+    return !wholeLists;
+}
+
+void RasterWorkspace::releaseSegments()
+{
+    segments.release();
+    units.release();
+    blockMax.release();
+    unitCount.release();
+    wholeLists = true;
 }
 
 void RasterWorkspace::composite(cudaStream_t stream, bool keep)
@@ -381,9 +411,7 @@ void RasterWorkspace::composite(cudaStream_t stream, bool keep)
     const int pb = st.tile_size <= 8 ? 8 : 16;
     const int per = st.tile_size > pb ? st.tile_size / pb : 1;
     blockStop.reserve(size_t(std::max(1, tilesX * per * tilesY * per)));
-    segmented = keep && !wholeLists;
-    if (segmented)
-        reserveSegments();
+    segmented = keep && !wholeLists && reserveSegments();
     RasterArgs a = rasterArgs();
     if (!segmented)
         a.segment = 0;
@@ -456,7 +484,7 @@ static void copyArenaToModel(const float *base, size_t cap, size_t n, u3dg_model
 }
 
 TrainerImpl::TrainerImpl(const u3dg_model &initial, const u3dg_image *imgs, int count, float sceneExtent,
-                         const u3dg_train_options &opt, bool backgroundUpload)
+                         const u3dg_train_options &opt, bool backgroundUpload, bool compact)
     : o(opt), rng(opt.seed)
 {
     checkSettings(o.raster);
@@ -496,28 +524,44 @@ TrainerImpl::TrainerImpl(const u3dg_model &initial, const u3dg_image *imgs, int 
     // largest view, in one device allocation: nothing is allocated during a schedule (allocations wait
     // for the device), and creation pays for one cudaMalloc instead of one per buffer. Intersection
     // buffers start at 16 tiles per Gaussian at the capacity and grow on demand.
-    for (auto &a : arena)
-        slab.add(a, 42 * cap);
-    slab.add(gradAccum, cap);
-    slab.add(gradCount, cap);
-    slab.add(images, std::max<size_t>(total, 1));
-    slab.add(dLoss, maxP * 3);
-    slab.add(abc, maxP * 9);
-    slab.add(lossBlockSums, size_t(maxLossBlocks) * 3);
-    slab.add(dStats, 1);
-    slab.add(descDev, kGraphSteps);
-    slab.add(statusDev, kGraphSteps);
-    const int per = ts > 16 ? ts / 16 : 1;
-    ws.partialSlots = std::max(ws.partialSlots, per * per);
-    ws.planIntersections(slab, std::max<size_t>(size_t(1) << 20, 16 * cap));
-    ws.planGaussians(slab, cap);
-    ws.planPixels(slab, cap, maxP, maxTx, maxTy, ts);
-    for (DevBuf<int> *b : {&keep, &cost, &costScan, &accCost, &accScan, &isSplit, &splitScan, &keepScan})
-        slab.add(*b, cap + 1);
-    slab.add(firstSecond, 2);
-    slab.add(dScanPartial, scanPartialEntries(int(cap)) + 1);
-    slab.add(normals, 6 * cap);
-    slab.commit();
+    auto plan = [&] {
+        for (auto &a : arena)
+            slab.add(a, 42 * cap);
+        slab.add(gradAccum, cap);
+        slab.add(gradCount, cap);
+        slab.add(images, std::max<size_t>(total, 1));
+        slab.add(dLoss, maxP * 3);
+        slab.add(abc, maxP * 9);
+        slab.add(lossBlockSums, size_t(maxLossBlocks) * 3);
+        slab.add(dStats, 1);
+        slab.add(descDev, kGraphSteps);
+        slab.add(statusDev, kGraphSteps);
+        const int per = ts > 16 ? ts / 16 : 1;
+        ws.partialSlots = std::max(ws.partialSlots, per * per);
+        ws.planIntersections(slab, RasterWorkspace::firstCapacity(cap, ws.wholeLists && per > 1 ? 12 : 16));
+        ws.planGaussians(slab, cap);
+        ws.planPixels(slab, cap, maxP, maxTx, maxTy, ts);
+        for (DevBuf<int> *b : {&keep, &cost, &costScan, &accCost, &accScan, &isSplit, &splitScan, &keepScan})
+            slab.add(*b, cap + 1);
+        slab.add(firstSecond, 2);
+        slab.add(dScanPartial, scanPartialEntries(int(cap)) + 1);
+        slab.add(normals, 6 * cap);
+    };
+    // Where there is no room for that, without the backward's segments (and, at tiles of more than 16 pixels,
+    // whose lists are short, for 12 tiles per Gaussian).
+    ws.wholeLists = compact;
+    plan();
+    try {
+        slab.commit();
+    } catch (const StatusError &e) {
+        if (e.status != U3DG_ERR_OOM || ws.wholeLists)
+            throw;
+        slab.drop();
+        ws.icap = 0;
+        ws.wholeLists = true;
+        plan();
+        slab.commit();
+    }
     U3DG_CUDA(cudaMemsetAsync(arena[cur].p, 0, 42 * cap * sizeof(float), stream));
     copyModelToArena(arena[cur].p, cap, initial, stream);
     U3DG_CUDA(cudaMemsetAsync(gradAccum.p, 0, cap * sizeof(float), stream));

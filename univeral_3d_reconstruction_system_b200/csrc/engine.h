@@ -143,8 +143,9 @@ class DeviceSlab {
             return;
         items.push_back({&b, n * sizeof(T), n, [](void *buf, void *mem, size_t k) { static_cast<DevBuf<T> *>(buf)->adopt(mem, k); }});
     }
-    // Allocates everything planned since the last commit and hands out the slices.
+    // Allocates everything planned since the last commit and hands out the slices. drop: forgets it instead.
     void commit();
+    void drop() { items.clear(); }
     size_t bytes() const { return total; }
 
   private:
@@ -233,8 +234,9 @@ struct RasterWorkspace {
     // Culling applies while tile rows fit the row table's 16-bit cumulative counts (< 8192 tiles).
     bool culled() const { return cullTiles && tilesX < 8192; }
     bool ordersTiles() const;
-    // Backward over whole lists (the rasterizer's, launchCompositeBackwardList) instead of segments; and what
-    // the last forward was for.
+    // Backward over whole lists (launchCompositeBackwardList) instead of segments: the rasterizer's, and the
+    // trainers' where the device has no room for segments, which are half of what an intersection takes (60
+    // bytes without them at tiles of up to 16 pixels, 124 with). And what the last forward was for.
     bool wholeLists = false, segmented = false;
     u3dg_camera cam{};
     u3dg_raster_settings st{};
@@ -247,7 +249,10 @@ struct RasterWorkspace {
     // The same sizes (and the per-pixel buffers for views of up to `pixels` pixels and `tiles` tiles at
     // the tile size st.tile_size), planned into a slab instead of allocated one by one.
     // planEntries, planForward: what a forward without backward needs of them.
-    static size_t firstCapacity(size_t count) { return std::max<size_t>(size_t(1) << 20, 16 * count); }
+    static size_t firstCapacity(size_t count, size_t tilesPerGaussian = 16)
+    {
+        return std::max<size_t>(size_t(1) << 20, tilesPerGaussian * count);
+    }
     void planEntries(DeviceSlab &slab, size_t capacity);
     void planForward(DeviceSlab &slab, size_t count, size_t pixels, int tilesX, int tilesY);
     void planIntersections(DeviceSlab &slab, size_t capacity);
@@ -268,7 +273,8 @@ struct RasterWorkspace {
     // and tile count need.
     static int segmentOf(int tileSize);
     size_t segmentSlots(size_t tiles) const { return size_t(icap) / size_t(segmentOf(st.tile_size)) + tiles + 1; }
-    void reserveSegments();
+    bool reserveSegments(); // false: no room, and whole lists from now on
+    void releaseSegments();
     // The buffers only a backward needs (listPos, partial), at the current intersection capacity.
     void reservePartials();
     void forward(const Params &P, int count, const u3dg_camera &c, const u3dg_raster_settings &s, const float *shRest,
@@ -456,8 +462,10 @@ struct TrainerImpl {
 
     // backgroundUpload: the images are copied by a host thread while the first steps run (the
     // caller's pixel buffers must stay valid until waitUploads() returns or the trainer is gone).
+    // compact: without the backward's segments (RasterWorkspace::wholeLists), as when the device has no room
+    // for them.
     TrainerImpl(const u3dg_model &initial, const u3dg_image *imgs, int count, float sceneExtent,
-                const u3dg_train_options &opt, bool backgroundUpload = false);
+                const u3dg_train_options &opt, bool backgroundUpload = false, bool compact = false);
     ~TrainerImpl();
     // Blocks until every image is on the device (no-op without background upload); afterwards the
     // caller's pixel buffers may be released.

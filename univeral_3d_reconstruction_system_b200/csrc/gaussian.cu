@@ -540,7 +540,8 @@ __device__ __forceinline__ void chainRule(const ChainArgs &a, const u3dg_camera 
 // at 64 for 32 warps per SM (28 warps: 63 us, 40: 80 us).
 constexpr int kChainThreads = 64, kChainWarps = 32;
 
-template <bool kAdam>
+// kList: the partials are launchCompositeBackwardList's, summed by partialSumKernel.
+template <bool kAdam, bool kList>
 __global__ void __launch_bounds__(kChainThreads, kChainWarps * 32 / kChainThreads) chainKernel(ChainArgs a)
 {
     pdlEntry();
@@ -549,11 +550,11 @@ __global__ void __launch_bounds__(kChainThreads, kChainWarps * 32 / kChainThread
         return;
     const u3dg_camera &cam = a.desc ? a.desc->cam : a.cam;
     const ViewLimits lim = viewLimits(cam);
-    __shared__ GatherBuffer sGather[kChainThreads / 32];
     float g[kG2d];
     {
         const bool seen = i < a.n && a.radius[i] > 0;
-        if (kAdam || a.sums == nullptr) {
+        if constexpr (!kList) {
+            __shared__ GatherBuffer sGather[kChainThreads / 32];
             gatherPartials(a, seen ? a.offs[i] : 0, seen ? a.tileCount[i] : 0, sGather[threadIdx.x >> 5], g);
         } else {
 #pragma unroll
@@ -585,9 +586,9 @@ __global__ void __launch_bounds__(kChainThreads, kChainWarps * 32 / kChainThread
         const float qr[4] = {P.quats[4 * i], P.quats[4 * i + 1], P.quats[4 * i + 2], P.quats[4 * i + 3]};
         const float ls[3] = {P.scales[3 * i], P.scales[3 * i + 1], P.scales[3 * i + 2]};
         Operands ops;
-        chainRule<Divisor>(a, cam, lim, mu, qr, ls, g, !kAdam && a.sums != nullptr, gMeans, gScales, gQuats, ops);
+        chainRule<Divisor>(a, cam, lim, mu, qr, ls, g, kList, gMeans, gScales, gQuats, ops);
         if (!ops.usual())
-            chainRule<Division>(a, cam, lim, mu, qr, ls, g, !kAdam && a.sums != nullptr, gMeans, gScales, gQuats, ops);
+            chainRule<Division>(a, cam, lim, mu, qr, ls, g, kList, gMeans, gScales, gQuats, ops);
     }
 
     if constexpr (kAdam) {
@@ -806,12 +807,11 @@ void launchChain(const ChainArgs &a, bool adam, cudaStream_t s)
 {
     if (a.n <= 0)
         return;
-    if (adam)
-        { launchPdl(chainKernel<true>, blocks(a.n, kChainThreads), kChainThreads, 0, s, a); countLaunch(); }
-    if (!adam && a.sums)
+    if (a.sums)
         { launchPdl(partialSumKernel, blocks((long long)(a.n + 31) / 32 * 32, 256), 256, 0, s, a); countLaunch(); }
-    if (!adam)
-        { launchPdl(chainKernel<false>, blocks(a.n, kChainThreads), kChainThreads, 0, s, a); countLaunch(); }
+    const auto kernel = adam ? (a.sums ? chainKernel<true, true> : chainKernel<true, false>)
+                             : (a.sums ? chainKernel<false, true> : chainKernel<false, false>);
+    { launchPdl(kernel, blocks(a.n, kChainThreads), kChainThreads, 0, s, a); countLaunch(); }
 }
 
 void launchAdamSegment(float *p, const float *g, float *m, float *v, int len, float stepSize, float invSqrtBc2,

@@ -113,8 +113,8 @@ struct ChainArgs {
     const BinCounts *counts; // the kernel does nothing when counts->abortIter >= 0
     float *gradAccum;     // |dL/dmean2d| NDC statistic (may be null)
     int *gradCount;       // visibility count (may be null)
-    // Non-Adam mode, partials of launchCompositeBackwardList: the Gaussians by depth rank, and space for 9 sums
-    // per Gaussian (null: the partials are gathered by the chain rule).
+    // Partials of launchCompositeBackwardList: the Gaussians by depth rank, and space for 9 sums per Gaussian
+    // (null: the partials are gathered by the chain rule).
     const uint32_t *order;
     float *sums;
     Params grads;         // non-Adam mode: gradients are added here
