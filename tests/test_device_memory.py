@@ -99,3 +99,24 @@ def test_a_batch_that_would_not_fit_with_segments(u3dg, fill):
     b.step(23)
     _same_training(one, b.trainer(0))
     b.close()
+
+
+def test_no_backward_after_a_forward_that_ran_out_of_memory(u3dg, fill):
+    rng = np.random.default_rng(2)
+    m = random_model(500, rng, 1.0, 3.0, 0.02, 0.1)
+    cam, st = make_camera(96, 72, 80.0), RasterSettings()
+    w = rng.uniform(-1, 1, (72, 96, 3)).astype(np.float32)
+    r = u3dg.Rasterizer()
+    r.forward(m, cam, st)
+    want = r.backward(m, w)
+    large = m.copy()
+    for k in ("means", "scales", "quats", "opacities", "colors"):
+        setattr(large, k, np.tile(getattr(m, k), (4000,) + (1,) * (getattr(m, k).ndim - 1)))
+    fill(200 * MB)  # 2M Gaussians take 1.5 GB of lists
+    with pytest.raises(u3dg.U3dgError, match="memory"):
+        r.forward(large, cam, st)
+    for model in (large, m):
+        with pytest.raises(u3dg.U3dgError):
+            r.backward(model, w)
+    r.forward(m, cam, st)
+    np.testing.assert_array_equal(r.backward(m, w).flat(), want.flat())

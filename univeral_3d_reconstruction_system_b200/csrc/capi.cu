@@ -522,6 +522,7 @@ static void rasterForward(u3dg_rasterizer &r, const u3dg_model *model, const flo
     checkSettings(*settings);
     checkCamera(*camera);
     cudaStream_t s = r.stream.s;
+    r.haveForward = false; // until this one is complete: its buffers may move or run out of memory
     r.model.upload(*model, s);
     DevBuf<float> sh;
     const float *shDev = nullptr;
