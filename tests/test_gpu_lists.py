@@ -362,3 +362,22 @@ def test_views_are_arrays_of_their_own(u3dg):
     for bad in (-3, 0, 16385):
         with pytest.raises(u3dg.U3dgError):
             u3dg.renderViewsSh(m, None, 0, [cams[0], make_camera(bad, 5, 60.0)])
+
+
+@pytest.mark.parametrize("width, height", [(312, 304), (312, 312)])
+@pytest.mark.parametrize("background", [(0.0, 0.0, 0.0), (0.2, 0.4, 0.1)])
+def test_training_with_either_backward_at_tile_8(u3dg, oracle, width, height, background):
+    # 1,482 and 1,521 tiles of 8, on both sides of the 1,500 beyond which the trainers replay whole lists: five steps
+    # agree with the oracle's trainer, as trainings in another order of summation do.
+    rng = np.random.default_rng(width + height)
+    m = random_model(600, rng, 1.0, 3.0, 0.05, 0.3)
+    cam = make_camera(width, height, 0.9 * width)
+    photos = [TrainImage(cam, rng.integers(0, 256, (height, width, 3)).astype(np.uint8))]
+    opt = TrainOptions(max_gaussians=600, refine_stop=0, raster=RasterSettings(tile_size=8, background=background))
+    t, o = u3dg.Trainer(m, photos, 1.0, opt), oracle.trainer(m, photos, 1.0, opt, threads=4)
+    t.step(5)
+    o.step(5)
+    a, b = t.stats(), o.stats()
+    assert abs(a.loss - b.loss) <= 1e-4 * abs(b.loss) and abs(a.psnr - b.psnr) <= 1e-3
+    for k in ("means", "scales", "quats", "opacities", "colors"):
+        assert rel_l2(getattr(t.model(), k), getattr(o.model(), k)) < 1e-3, k

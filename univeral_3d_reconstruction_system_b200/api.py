@@ -333,8 +333,10 @@ class Rasterizer:
         return ft, nc
 
     def set_tile_culling(self, enable: bool) -> None:
-        """List each Gaussian only in the tiles its contributing ellipse reaches (the trainers'
-        default); the lists become subsequences of the reference's, results are unchanged."""
+        """List each Gaussian only in the tiles its contributing ellipse reaches (the trainers' default); the
+        lists become subsequences of the reference's. Images and final transmittances are unchanged,
+        contributor counts index the shorter lists, and gradients are summed in the trainers' order: they
+        agree to rounding (which a few Gaussians with ill-conditioned covariances amplify)."""
         check(load().u3dg_rasterizer_set_tile_culling(self._h, 1 if enable else 0))
 
 

@@ -569,6 +569,7 @@ int u3dg_rasterizer_backward(u3dg_rasterizer *r, const u3dg_model *model, const 
         R.ndc.reserve(std::max<size_t>(n, 1), true);
         if (mean2d_grad_ndc && n > 0)
             U3DG_CUDA(cudaMemcpyAsync(R.ndc.p, mean2d_grad_ndc, n * sizeof(float), cudaMemcpyHostToDevice, s));
+        R.ws.sums.reserve(std::max<size_t>(n, 1) * kG2d);
         R.ws.backwardComposite(R.dl.p, s);
         ChainArgs a = R.ws.chainArgs(R.model.params());
         a.grads = R.grads.params();

@@ -259,10 +259,8 @@ void RasterWorkspace::planPixels(DeviceSlab &slab, size_t count, size_t pixels, 
     const int pb = tileSize <= 8 ? 8 : 16;
     const int per = tileSize > pb ? tileSize / pb : 1;
     slab.add(blockStop, size_t(std::max(1, tx * per * ty * per)));
-    if (wholeLists) {
-        slab.add(sums, std::max<size_t>(count, 1) * kG2d);
+    if (wholeLists || !takesSegments(tileSize, size_t(tx) * ty))
         return;
-    }
     const size_t slots = icap / segmentOf(tileSize) + size_t(tx) * ty + 1;
     slab.add(segments, slots * tileSize * tileSize);
     slab.add(units, slots * per * per);
@@ -376,6 +374,16 @@ int RasterWorkspace::segmentOf(int tileSize)
     return tileSize <= 16 ? 64 : tileSize * tileSize / 4;
 }
 
+// Whether the trainers' backward replays segments. At tiles of 8 a list's segments cost a warp of 32 lanes twice
+// what the same entries cost in one piece, which many tiles at a time hide: us of the backward and the chain rule,
+// segments / whole lists, of part-trained and of transparent models at 108 tiles 55 / 125 and 61 / 138, at 1,200
+// (20k to 80k Gaussians) 137 / 142 and 214 / 233, 143 / 171 and 291 / 314, at 1,900 177 / 159 and 350 / 303, at 4,800 355 /
+// 246 and 898 / 538, at 19,200 1165 / 640 and 2810 / 1432.
+bool RasterWorkspace::takesSegments(int tileSize, size_t tiles)
+{
+    return tileSize > 8 || tiles <= 1500;
+}
+
 bool RasterWorkspace::reserveSegments()
 {
     const int ts = st.tile_size, pb = ts <= 8 ? 8 : 16, per = ts > pb ? ts / pb : 1;
@@ -411,7 +419,7 @@ void RasterWorkspace::composite(cudaStream_t stream, bool keep)
     const int pb = st.tile_size <= 8 ? 8 : 16;
     const int per = st.tile_size > pb ? st.tile_size / pb : 1;
     blockStop.reserve(size_t(std::max(1, tilesX * per * tilesY * per)));
-    segmented = keep && !wholeLists && reserveSegments();
+    segmented = keep && !wholeLists && takesSegments(st.tile_size, size_t(tilesX) * tilesY) && reserveSegments();
     RasterArgs a = rasterArgs();
     if (!segmented)
         a.segment = 0;
@@ -422,7 +430,6 @@ void RasterWorkspace::backwardComposite(const float *dLdRgb, cudaStream_t stream
 {
     const RasterArgs a = rasterArgs();
     if (!segmented) {
-        sums.reserve(size_t(std::max(n, 1)) * kG2d);
         launchCompositeBackwardList(a, dLdRgb, finalT.p, nContrib.p, partial.p, blockStop.p, stream);
         return;
     }
@@ -451,8 +458,9 @@ ChainArgs RasterWorkspace::chainArgs(const Params &P) const
     a.tilesX = tilesX;
     a.blocksX = tilesX * per;
     a.counts = counts.p;
+    a.conics = !segmented;
     a.order = depthOrder.p;
-    a.sums = segmented ? nullptr : sums.p;
+    a.sums = sums.p;
     return a;
 }
 

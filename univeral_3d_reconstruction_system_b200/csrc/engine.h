@@ -273,6 +273,7 @@ struct RasterWorkspace {
     // and tile count need.
     static int segmentOf(int tileSize);
     size_t segmentSlots(size_t tiles) const { return size_t(icap) / size_t(segmentOf(st.tile_size)) + tiles + 1; }
+    static bool takesSegments(int tileSize, size_t tiles);
     bool reserveSegments(); // false: no room, and whole lists from now on
     void releaseSegments();
     // The buffers only a backward needs (listPos, partial), at the current intersection capacity.

@@ -433,11 +433,11 @@ __global__ void __launch_bounds__(256) partialSumKernel(ChainArgs a)
     }
 }
 
-// The chain rule of one seen Gaussian from its 2D gradients g (listed: with dL/dconic, else dL/dcovariance) to its
+// The chain rule of one seen Gaussian from its 2D gradients g (conics: with dL/dconic, else dL/dcovariance) to its
 // means, scales and quaternion (Rasterizer.cpp:432-544). D: Divisor, right for usual operands, or Division.
 template <class D>
 __device__ __forceinline__ void chainRule(const ChainArgs &a, const u3dg_camera &cam, const ViewLimits &lim, const float mu[3],
-                                          const float qr[4], const float ls[3], const float (&g)[kG2d], bool listed, float gMeans[3],
+                                          const float qr[4], const float ls[3], const float (&g)[kG2d], bool conics, float gMeans[3],
                                           float gScales[3], float gQuats[4], Operands &ops)
 {
     Ewa p;
@@ -445,7 +445,7 @@ __device__ __forceinline__ void chainRule(const ChainArgs &a, const u3dg_camera 
     const float z = p.pc[2];
     const float dmx = g[0], dmy = g[1];
     float G00 = g[2], db = g[3], G11 = g[4];
-    if (listed) { // dL/dconic to dL/dcovariance (Rasterizer.cpp:432-446)
+    if (conics) { // dL/dconic to dL/dcovariance (Rasterizer.cpp:432-446)
         const float dA = g[2], dB = g[3], dC = g[4], aa = p.a, bb = p.b, cc = p.c;
         const float det = aa * cc - bb * bb;
         const float det2 = det * det;
@@ -540,8 +540,9 @@ __device__ __forceinline__ void chainRule(const ChainArgs &a, const u3dg_camera 
 // at 64 for 32 warps per SM (28 warps: 63 us, 40: 80 us).
 constexpr int kChainThreads = 64, kChainWarps = 32;
 
-// kList: the partials are launchCompositeBackwardList's, summed by partialSumKernel.
-template <bool kAdam, bool kList>
+// kConics: the partials are launchCompositeBackwardList's; without Adam (the rasterizer's) partialSumKernel has
+// added them in the order that its callers know.
+template <bool kAdam, bool kConics>
 __global__ void __launch_bounds__(kChainThreads, kChainWarps * 32 / kChainThreads) chainKernel(ChainArgs a)
 {
     pdlEntry();
@@ -553,7 +554,7 @@ __global__ void __launch_bounds__(kChainThreads, kChainWarps * 32 / kChainThread
     float g[kG2d];
     {
         const bool seen = i < a.n && a.radius[i] > 0;
-        if constexpr (!kList) {
+        if constexpr (kAdam || !kConics) {
             __shared__ GatherBuffer sGather[kChainThreads / 32];
             gatherPartials(a, seen ? a.offs[i] : 0, seen ? a.tileCount[i] : 0, sGather[threadIdx.x >> 5], g);
         } else {
@@ -586,9 +587,9 @@ __global__ void __launch_bounds__(kChainThreads, kChainWarps * 32 / kChainThread
         const float qr[4] = {P.quats[4 * i], P.quats[4 * i + 1], P.quats[4 * i + 2], P.quats[4 * i + 3]};
         const float ls[3] = {P.scales[3 * i], P.scales[3 * i + 1], P.scales[3 * i + 2]};
         Operands ops;
-        chainRule<Divisor>(a, cam, lim, mu, qr, ls, g, kList, gMeans, gScales, gQuats, ops);
+        chainRule<Divisor>(a, cam, lim, mu, qr, ls, g, kConics, gMeans, gScales, gQuats, ops);
         if (!ops.usual())
-            chainRule<Division>(a, cam, lim, mu, qr, ls, g, kList, gMeans, gScales, gQuats, ops);
+            chainRule<Division>(a, cam, lim, mu, qr, ls, g, kConics, gMeans, gScales, gQuats, ops);
     }
 
     if constexpr (kAdam) {
@@ -807,10 +808,10 @@ void launchChain(const ChainArgs &a, bool adam, cudaStream_t s)
 {
     if (a.n <= 0)
         return;
-    if (a.sums)
+    if (!adam && a.conics)
         { launchPdl(partialSumKernel, blocks((long long)(a.n + 31) / 32 * 32, 256), 256, 0, s, a); countLaunch(); }
-    const auto kernel = adam ? (a.sums ? chainKernel<true, true> : chainKernel<true, false>)
-                             : (a.sums ? chainKernel<false, true> : chainKernel<false, false>);
+    const auto kernel = adam ? (a.conics ? chainKernel<true, true> : chainKernel<true, false>)
+                             : (a.conics ? chainKernel<false, true> : chainKernel<false, false>);
     { launchPdl(kernel, blocks(a.n, kChainThreads), kChainThreads, 0, s, a); countLaunch(); }
 }
 

@@ -113,8 +113,9 @@ struct ChainArgs {
     const BinCounts *counts; // the kernel does nothing when counts->abortIter >= 0
     float *gradAccum;     // |dL/dmean2d| NDC statistic (may be null)
     int *gradCount;       // visibility count (may be null)
-    // Partials of launchCompositeBackwardList: the Gaussians by depth rank, and space for 9 sums per Gaussian
-    // (null: the partials are gathered by the chain rule).
+    bool conics;          // partials of launchCompositeBackwardList
+    // Non-Adam mode, conics: the Gaussians by depth rank, and space for 9 sums per Gaussian (partialSumKernel;
+    // else the chain rule gathers the partials itself).
     const uint32_t *order;
     float *sums;
     Params grads;         // non-Adam mode: gradients are added here
@@ -204,7 +205,7 @@ size_t cullRowEntries(size_t n);
 void launchCapacityCheck(const int *total, int capacity, BinCounts *c, int iteration, cudaStream_t s,
                          const StepDesc *desc = nullptr);
 // Emission of the intersections in depth-rank order: tile key and Gaussian id per intersection (the
-// same tiles as launchRankCounts counted).
+// tiles that the projection counted, ProjOut::tileCount).
 void launchEmit(const uint32_t *sortedIds, const int *offs, const int4 *rect, int n, const BinCounts *c, int capacity,
                 int tilesX, const SplatRec *cullRec, int tileSize, const uint32_t *rowTab, uint32_t *keys, int *emitGid,
                 cudaStream_t s);

@@ -18,14 +18,14 @@
 //   compositeForwardTeamKernel  four warps per block evaluate for one that blends: 70 cycles per entry, but
 //                               up to a batch of entries evaluated in vain at the end of every block
 // The second where blocks are too few to fill the GPU: us per launch one warp / team / before at 96x72
-// pixels 46 / 27 / 71, 320x240 (1,200 blocks) 65 / 57 / 96, 480x360 (2,700) 76 / 84 / 102, 640x480 106 / 130 /
+// pixels 46 / 27 / 71, 320x240 (1,200 blocks) 64 / 52 / 96, 480x360 (2,700) 73 / 80 / 102, 640x480 106 / 130 /
 // 134.
 //
 // Compiled with -fmad=false: the contribution decisions (power, alpha, the transmittance cut-off) and
 // the transmittance round exactly like the reference's, so the same entries contribute. The colour
 // sums alone use explicit fused multiply-adds (within 1e-7 of the unfused sums; images are compared
 // within 1e-5). A lane's two pixels are blended together in sm_100's paired FP32 instructions
-// (add2rn / mul2rn / fma2rn, raster_common.cuh), which round each lane like the scalar operation.
+// (add2rn / mul2rn / fma2rn, paired.cuh), which round each lane like the scalar operation.
 
 #include "raster_common.cuh"
 
@@ -416,9 +416,12 @@ __global__ void __launch_bounds__(kTeamThreads, 6) compositeForwardTeamKernel(Ra
     px.store(a, slot0, wb.px, wb.py0, in0, in1, rgb, finalT, nContrib);
 }
 
-// Blocks up to which the team is faster (between 1,200 and 2,700, see above): about 14 per SM.
+// Blocks up to which the team is faster: us by a team / one warp with lists of trained models (80k to 150k
+// Gaussians) at 1,200 blocks 51.5 / 63.7, 1,530 58.1 / 63.7, 1,900 65.1 / 69.0, 2,080 68.1 / 69.5, 2,352 73.0 / 71.8,
+// 2,700 79.6 / 73.1. (With the short lists of 20k Gaussians one warp is faster from below 1,900 on: 48.6 / 39.9;
+// the host does not know the lists' lengths.)
 constexpr int kTeamLimit = 2048;
-// Blocks up to which all teams run at once (6 on each of 148 SMs), so that their order does not matter. Beyond,
+// Blocks up to which all teams run at once (6 on each of a B200's 148 SMs), so that their order does not matter. Beyond,
 // the longest lists go first: forward of 1,200 blocks 55.8 -> 51.4 us, of 2,700 75.8 -> 73.0, of 4,800 104.1 ->
 // 100.0; of 108 blocks 26.8 -> 27.2, and the lists 34.6 -> 35.1.
 constexpr int kTeamsResident = 888;

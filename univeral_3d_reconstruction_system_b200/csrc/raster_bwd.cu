@@ -24,7 +24,7 @@
 // reciprocal-multiply made the backward 3 % faster but moved some colour gradients just past 1e-4
 // relative to the reference's.
 //
-// A lane's pixels are replayed in pairs by paired FP32 instructions (raster_common.cuh), one float2 lane
+// A lane's pixels are replayed in pairs by paired FP32 instructions (paired.cuh), one float2 lane
 // per pixel; the falloff exponents' sums stay scalar. A pixel that does not contribute at an entry takes
 // part with alpha 0, which leaves its state as it is.
 
