@@ -364,6 +364,40 @@ def test_views_are_arrays_of_their_own(u3dg):
             u3dg.renderViewsSh(m, None, 0, [cams[0], make_camera(bad, 5, 60.0)])
 
 
+@pytest.mark.parametrize("n, tiles_x, tiles_y, wide", [(31, 4, 4, 2), (32, 7, 5, 3), (33, 64, 32, 64), (257, 64, 32, 64), (16_384, 13, 9, 3),
+                                                       (16_385, 13, 9, 3), (17_001, 32, 24, 9)])
+def test_tile_lists_of_few_and_many_gaussians(u3dg, n, tiles_x, tiles_y, wide):
+    # Blocks of 32 ranks up to 16,384 Gaussians and of 512 beyond, with fewer and more intersections than a block
+    # lists at a time. As above: exact.
+    test_tile_lists_at_chunk_and_path_edges(u3dg, None, n, tiles_x, tiles_y, wide)
+
+
+@pytest.mark.parametrize("n, size", [(40, 2.0), (700, 0.6), (17_000, 0.05)])
+def test_culled_lists_of_large_gaussians(u3dg, n, size):
+    # Rotated Gaussians over tens to hundreds of tiles of 8: a block of ranks lists its culled tiles in several
+    # rounds. Every culled list is a subsequence of the whole one, nothing that blends is missing (same image and
+    # transmittance, to the bit), and a Gaussian is in no tile twice.
+    rng = np.random.default_rng(n)
+    m = random_model(n, rng, 1.0, 3.0, 0.2 * size, size)
+    m.scales[:, 1] -= 1.5
+    cam, st = make_camera(320, 240, 300.0), RasterSettings(tile_size=8, background=(0.1, 0.2, 0.3))
+    out = []
+    for culled in (False, True):
+        r = u3dg.Rasterizer()
+        r.set_tile_culling(culled)
+        out.append((r.forward(m, cam, st), r.pixel_state()[0], *r.tiles()))
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_array_equal(out[0][1], out[1][1])
+    (_, _, whole, ids), (_, _, culled, some) = out
+    assert len(some) < len(ids) and len(some) > 10_240
+    for k in range(len(whole) - 1):
+        full, part = ids[whole[k]:whole[k + 1]], some[culled[k]:culled[k + 1]]
+        assert len(np.unique(part)) == len(part)
+        place = {g: i for i, g in enumerate(full)}
+        at = [place[g] for g in part]
+        assert at == sorted(at)
+
+
 @pytest.mark.parametrize("width, height", [(312, 304), (312, 312)])
 @pytest.mark.parametrize("background", [(0.0, 0.0, 0.0), (0.2, 0.4, 0.1)])
 def test_training_with_either_backward_at_tile_8(u3dg, oracle, width, height, background):

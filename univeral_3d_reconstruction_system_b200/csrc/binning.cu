@@ -577,11 +577,34 @@ __global__ void __launch_bounds__(kDepthThreads) depthSortSmallKernel(const uint
 
 // ---------------------------------------------------------------- tile lists of up to 2048 tiles
 
-// A chunk is kRanks ranks, one per thread, a warp owning 32 consecutive ones.
+// A block of T threads takes a chunk of ranks, each of its warps R consecutive ones (at most one per lane). Few
+// Gaussians are cut finer, as a warp goes through its ranks' tiles one after the other and 512 ranks to a block
+// would leave most of the chip idle. Sort and lists, us, by 512 / 64 / 32 ranks to a block (32 / 32 / 8 to a warp):
+// 5,000 Gaussians at 640x480 389 / 142 / 96, 5,000 at 400x304 in tiles of 8 652 / 208 / 126, without culling 380 /
+// 340 / 175, 1,000 at 200x150 81 / 50 / 40, 15,000 at 640x480 221 / 104 / 82, 4,000 at 96x72 36 / 34 / 32. Beyond,
+// blocks of 512 keep the counts that are scanned few (300k at 640x480: 586 rows of 1,200).
 constexpr int kMaxTiles = 1 << kWideBits;
-constexpr int kRanks = 512, kRankWarps = kRanks / 32;
+template <int T, int R>
+struct RankShape {
+    static constexpr int THREADS = T, WARPS = T / 32, PER_WARP = R, CHUNK = WARPS * R;
+};
+using ManyRanks = RankShape<512, 32>;
+using FewRanks = RankShape<128, 8>;
+constexpr int kFewGaussians = 16384;
 
-inline int rankChunks(int n) { return std::max(1, (n + kRanks - 1) / kRanks); }
+inline int rankChunks(int n)
+{
+    const int chunk = n <= kFewGaussians ? FewRanks::CHUNK : ManyRanks::CHUNK;
+    return std::max(1, (n + chunk - 1) / chunk);
+}
+
+// The rank of a thread, n where it has none.
+template <class S>
+__device__ __forceinline__ int rankOf(int chunk, int n)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    return lane < S::PER_WARP ? min(n, chunk * S::CHUNK + warp * S::PER_WARP + lane) : n;
+}
 
 // The k-th tile (row-major) in which Gaussian g with rectangle q is listed.
 __device__ __forceinline__ int2 listedTile(const SplatRec *cullRec, const uint32_t *rowTab, int tileSize, int g,
@@ -681,17 +704,18 @@ __device__ __forceinline__ void eachTile(const Listed &l, const SplatRec *cullRe
 }
 
 // hist[chunk][tile]: intersections of the chunk's ranks per tile; chunkTotals[chunk]: all of them.
-__global__ void __launch_bounds__(kRanks) tileCountKernel(TileBins b, int *hist, int *chunkTotals)
+template <class S>
+__global__ void __launch_bounds__(S::THREADS) tileCountKernel(TileBins b, int *hist, int *chunkTotals)
 {
     pdlEntry();
     extern __shared__ int counts[]; // per tile
     __shared__ int total;
-    for (int d = threadIdx.x; d < b.tiles; d += kRanks)
+    for (int d = threadIdx.x; d < b.tiles; d += S::THREADS)
         counts[d] = 0;
     if (threadIdx.x == 0)
         total = 0;
     const Listed l = loadListed(b.sortedIds, b.tileCount, b.rect, b.rowTab, b.cullRec != nullptr,
-                                blockIdx.x * kRanks + threadIdx.x, b.n);
+                                rankOf<S>(blockIdx.x, b.n), b.n);
     __syncthreads();
     eachTile(l, b.cullRec, b.tileSize, b.tilesX, [&](int tile) { atomicAdd(&counts[tile], 1); });
     const int sum = __reduce_add_sync(0xffffffffu, l.count); // at most 32 * kMaxTiles
@@ -700,7 +724,7 @@ __global__ void __launch_bounds__(kRanks) tileCountKernel(TileBins b, int *hist,
     __syncthreads();
     if (threadIdx.x == 0)
         chunkTotals[blockIdx.x] = total;
-    for (int d = threadIdx.x; d < b.tiles; d += kRanks)
+    for (int d = threadIdx.x; d < b.tiles; d += S::THREADS)
         hist[size_t(blockIdx.x) * b.tiles + d] = counts[d];
 }
 
@@ -719,7 +743,7 @@ __global__ void __launch_bounds__(kScanThreads) tileScanKernel(int *hist, int ch
             return;
         long long carry = 0;
         for (int c0 = 0; c0 < chunks; c0 += 32) {
-            const int c = c0 + lane, v = c < chunks ? chunkTotals[c] : 0; // at most kRanks * kMaxTiles = 2^20
+            const int c = c0 + lane, v = c < chunks ? chunkTotals[c] : 0; // at most 512 * kMaxTiles = 2^20
             int incl = v;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -762,18 +786,20 @@ __global__ void __launch_bounds__(kScanThreads) tileScanKernel(int *hist, int ch
 }
 
 // Writes the chunk's Gaussian ids to the tile lists (and, with listPos, where each emission went, and with
-// offsById each Gaussian's first emission). A warp first lists its ranks' intersections (tile and lane, in
-// rank order) and counts them per tile, the counts are added up over the block's warps in order, and each
+// offsById each Gaussian's first emission). The chunk first lists its ranks' intersections (tile and lane, in
+// rank order) and counts them per warp and tile, the counts are added up over the block's warps in order, and each
 // warp then goes through its list, 32 intersections at a time, ranking equal tiles by match-any votes, with
-// no barrier on the way. A chunk with more than kListed intersections finds each one's rank and tile by a
-// search over the warp's lanes instead. Block 0 writes the tile offsets.
-constexpr int kListed = 10240; // 20 KB; a chunk of 512 ranks has about 4,000 on a 300k model at 640x480
+// no barrier on the way. A chunk with more than kListed intersections lists so many at a time, and enumerates its
+// ranks' tiles again for each; without culling, where a rank's k-th tile is a division away, it finds each one's
+// rank by a search over the warp's lanes instead. Block 0 writes the tile offsets.
+constexpr int kListed = 10240; // 20 KB; 512 ranks have about 4,000 on a 300k model at 640x480
 static_assert(kMaxTiles * 32 == 65536, "a tile and a lane fit in 16 bits");
 
-// Tiles by descending list length, in kLengths steps of the longest (one block of kRanks threads): the forward
+// Tiles by descending list length, in kLengths steps of the longest (one block): the forward
 // starts the longest lists first. Within a step the order is open; it changes no result.
 constexpr int kLengths = 64;
 
+template <class S>
 __device__ __forceinline__ void orderTiles(const int *lengths, int tiles, int *order)
 {
     __shared__ int longest, count[kLengths];
@@ -784,7 +810,7 @@ __device__ __forceinline__ void orderTiles(const int *lengths, int tiles, int *o
         count[tid] = 0;
     __syncthreads();
     int most = 0;
-    for (int d = tid; d < tiles; d += kRanks)
+    for (int d = tid; d < tiles; d += S::THREADS)
         most = max(most, lengths[d]);
     most = __reduce_max_sync(0xffffffffu, most);
     if ((tid & 31) == 0)
@@ -792,7 +818,7 @@ __device__ __forceinline__ void orderTiles(const int *lengths, int tiles, int *o
     __syncthreads();
     const float scale = float(kLengths) / (float(longest) + 1.0f);
     auto step = [&](int d) { return kLengths - 1 - min(kLengths - 1, int(float(lengths[d]) * scale)); };
-    for (int d = tid; d < tiles; d += kRanks)
+    for (int d = tid; d < tiles; d += S::THREADS)
         atomicAdd(&count[step(d)], 1);
     __syncthreads();
     if (tid == 0) {
@@ -804,14 +830,16 @@ __device__ __forceinline__ void orderTiles(const int *lengths, int tiles, int *o
         }
     }
     __syncthreads();
-    for (int d = tid; d < tiles; d += kRanks)
+    for (int d = tid; d < tiles; d += S::THREADS)
         order[atomicAdd(&count[step(d)], 1)] = d;
 }
 
-__global__ void __launch_bounds__(kRanks, 3) tileScatterKernel(TileBins b, const int *hist, const int *tileTotals,
-                                                            const int *chunkFirst, const BinCounts *bc)
+template <class S, bool kCull>
+__global__ void __launch_bounds__(S::THREADS, S::THREADS == 128 ? 5 : kCull ? 2 : 3)
+    tileScatterKernel(TileBins b, const int *hist, const int *tileTotals, const int *chunkFirst, const BinCounts *bc)
 {
     pdlEntry();
+    constexpr int kRankWarps = S::WARPS;
     extern __shared__ int dyn[];
     const int tiles = b.tiles, stride = (tiles + 1) / 2 * 2;
     int *base = dyn;                                                      // per tile: the chunk's first position
@@ -821,20 +849,20 @@ __global__ void __launch_bounds__(kRanks, 3) tileScatterKernel(TileBins b, const
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int chunk = int(blockIdx.x) - (b.tileOrder ? 1 : 0); // the first block orders the tiles
     if (chunk < 0) {
-        orderTiles(tileTotals, tiles, b.tileOrder);
+        orderTiles<S>(tileTotals, tiles, b.tileOrder);
         return;
     }
     if (bc->effTotal <= 0) { // nothing listed, or an overflow
         if (chunk == 0)
-            for (int d = tid; d <= tiles; d += kRanks)
+            for (int d = tid; d <= tiles; d += S::THREADS)
                 b.tileOffsets[d] = 0;
         // A backward takes its loop bounds from the first emissions, of unseen Gaussians too.
-        if (b.offsById && chunk * kRanks + tid < b.n)
-            b.offsById[b.sortedIds[chunk * kRanks + tid]] = 0;
+        if (b.offsById && rankOf<S>(chunk, b.n) < b.n)
+            b.offsById[b.sortedIds[rankOf<S>(chunk, b.n)]] = 0;
         return;
     }
-    const Listed l = loadListed(b.sortedIds, b.tileCount, b.rect, b.rowTab, b.cullRec != nullptr, chunk * kRanks + tid, b.n);
-    for (int k = tid; k < kRankWarps * stride / 2; k += kRanks)
+    const Listed l = loadListed(b.sortedIds, b.tileCount, b.rect, b.rowTab, kCull, rankOf<S>(chunk, b.n), b.n);
+    for (int k = tid; k < kRankWarps * stride / 2; k += S::THREADS)
         reinterpret_cast<uint32_t *>(offset)[k] = 0;
     auto warpScan = [&](int v) {
 #pragma unroll
@@ -849,7 +877,7 @@ __global__ void __launch_bounds__(kRanks, 3) tileScatterKernel(TileBins b, const
     if (lane == 31)
         warpSums[warp] = incl;
     // The tile lists' starts: every thread scans consecutive tiles.
-    const int per = (tiles + kRanks - 1) / kRanks;
+    const int per = (tiles + S::THREADS - 1) / S::THREADS;
     int own = 0;
     for (int k = 0; k < per; ++k)
         own += tid * per + k < tiles ? tileTotals[tid * per + k] : 0;
@@ -864,8 +892,7 @@ __global__ void __launch_bounds__(kRanks, 3) tileScatterKernel(TileBins b, const
         l0 += w < warp ? warpSums[w] : 0;
         all += warpSums[w];
     }
-    const int e0 = chunkFirst[chunk] + l0;
-    const bool fits = all <= kListed;
+    const int e0 = chunkFirst[chunk];
     for (int k = 0; k < per; ++k) {
         const int d = tid * per + k;
         if (d >= tiles)
@@ -877,65 +904,78 @@ __global__ void __launch_bounds__(kRanks, 3) tileScatterKernel(TileBins b, const
         if (chunk == 0 && d == tiles - 1)
             b.tileOffsets[tiles] = start;
     }
-    if (b.offsById && chunk * kRanks + tid < b.n)
-        b.offsById[l.gid] = e0 + o;
+    if (b.offsById && rankOf<S>(chunk, b.n) < b.n)
+        b.offsById[l.gid] = e0 + l0 + o;
     uint16_t *mine = offset + warp * stride;
-    // (Two tiles share a word; a warp's ranks add at most 32 to each.)
-    int at = l0 + o;
-    eachTile(l, b.cullRec, b.tileSize, b.tilesX, [&](int tile) {
-        atomicAdd(reinterpret_cast<uint32_t *>(mine) + (tile >> 1), 1u << (16 * (tile & 1)));
-        if (fits)
-            listed[at++] = uint16_t(tile << 5 | lane);
-    });
-    __syncthreads();
-    for (int d = tid; d < tiles; d += kRanks) {
-        int run = 0; // at most kRanks
-#pragma unroll
-        for (int w = 0; w < kRankWarps; ++w) {
-            const int c = offset[w * stride + d];
-            offset[w * stride + d] = uint16_t(run);
-            run += c;
-        }
-    }
-    __syncthreads();
     const int items = __shfl_sync(0xffffffffu, incl, 31);
     const uint32_t below = (1u << lane) - 1u;
-    for (int i0 = 0; i0 < items; i0 += 32) {
-        const int i = i0 + lane;
-        int tile = kMaxTiles, gid;
-        if (fits) {
-            const int v = i < items ? listed[l0 + i] : 0;
-            gid = __shfl_sync(0xffffffffu, l.gid, v & 31);
-            if (i < items)
-                tile = v >> 5;
-        } else {
-            int owner = 0; // the last lane whose first intersection is not above i (empty ranks share the next one's)
+    const int first = l0 + o; // the rank's first intersection in the chunk
+    const bool search = !kCull && all > kListed;
+    const int window = search ? all : kListed;
+    for (int from = 0; from < all; from += window) {
+        const int to = from + window;
+        if (from > 0)
+            __syncthreads(); // the warps are done with the last ones listed
+        if (from == 0 || (first < to && first + l.count > from)) {
+            int at = first - from;
+            eachTile(l, kCull ? b.cullRec : nullptr, b.tileSize, b.tilesX, [&](int tile) {
+                // (Two tiles share a word; a warp's ranks add at most 32 to each.)
+                if (from == 0)
+                    atomicAdd(reinterpret_cast<uint32_t *>(mine) + (tile >> 1), 1u << (16 * (tile & 1)));
+                if (at >= 0 && at < kListed)
+                    listed[at] = uint16_t(tile << 5 | lane);
+                ++at;
+            });
+        }
+        __syncthreads();
+        if (from == 0) {
+            for (int d = tid; d < tiles; d += S::THREADS) {
+                int run = 0; // at most S::CHUNK
 #pragma unroll
-            for (int step = 16; step > 0; step >>= 1)
-                if (__shfl_sync(0xffffffffu, o, owner + step) <= i)
-                    owner += step;
-            const int k = i - __shfl_sync(0xffffffffu, o, owner);
-            gid = __shfl_sync(0xffffffffu, l.gid, owner);
-            const int4 q = make_int4(__shfl_sync(0xffffffffu, l.q.x, owner), __shfl_sync(0xffffffffu, l.q.y, owner),
-                                     __shfl_sync(0xffffffffu, l.q.z, owner), __shfl_sync(0xffffffffu, l.q.w, owner));
-            if (i < items) {
-                const int2 t = listedTile(b.cullRec, b.rowTab, b.tileSize, gid, q, k);
-                tile = t.y * b.tilesX + t.x;
+                for (int w = 0; w < kRankWarps; ++w) {
+                    const int c = offset[w * stride + d];
+                    offset[w * stride + d] = uint16_t(run);
+                    run += c;
+                }
             }
+            __syncthreads();
         }
-        const uint32_t peers = __match_any_sync(0xffffffffu, tile);
-        int seen = 0;
-        if (i < items) {
-            seen = mine[tile];
-            const int pos = base[tile] + seen + __popc(peers & below);
-            b.entries[pos] = gid;
-            if (b.listPos)
-                b.listPos[e0 + i] = make_int2(pos, tile);
+        const int end = min(l0 + items, to);
+        for (int i0 = max(l0, from); i0 < end; i0 += 32) {
+            const int i = i0 + lane;
+            int gid, tile = kMaxTiles;
+            if (!search) {
+                const int v = i < end ? listed[i - from] : 0;
+                gid = __shfl_sync(0xffffffffu, l.gid, v & 31);
+                if (i < end)
+                    tile = v >> 5;
+            } else {
+                int owner = 0; // the last lane whose first intersection is not above i (empty ranks share the next one's)
+#pragma unroll
+                for (int step = 16; step > 0; step >>= 1)
+                    if (__shfl_sync(0xffffffffu, first, owner + step) <= i)
+                        owner += step;
+                const int k = i - __shfl_sync(0xffffffffu, first, owner);
+                gid = __shfl_sync(0xffffffffu, l.gid, owner);
+                const int x = __shfl_sync(0xffffffffu, l.q.x, owner), y = __shfl_sync(0xffffffffu, l.q.y, owner);
+                const int wide = __shfl_sync(0xffffffffu, l.q.z, owner) - x;
+                if (i < end)
+                    tile = (y + k / wide) * b.tilesX + x + k % wide;
+            }
+            const uint32_t peers = __match_any_sync(0xffffffffu, tile);
+            int seen = 0;
+            if (i < end) {
+                seen = mine[tile];
+                const int pos = base[tile] + seen + __popc(peers & below);
+                b.entries[pos] = gid;
+                if (b.listPos)
+                    b.listPos[e0 + i] = make_int2(pos, tile);
+            }
+            __syncwarp();
+            if (i < end && lane == __ffs(peers) - 1)
+                mine[tile] = uint16_t(seen + __popc(peers));
+            __syncwarp();
         }
-        __syncwarp();
-        if (i < items && lane == __ffs(peers) - 1)
-            mine[tile] = uint16_t(seen + __popc(peers));
-        __syncwarp();
     }
 }
 
@@ -1079,7 +1119,8 @@ void radixSortDepth(const uint32_t *keys, uint2 *pairsA, uint2 *pairsB, uint32_t
     }
 }
 
-size_t binChunkEntries(int n) { return size_t(rankChunks(n)); }
+// For up to n Gaussians (few of them can be cut into more chunks than many).
+size_t binChunkEntries(int n) { return size_t(std::max(rankChunks(n), rankChunks(std::min(n, kFewGaussians)))); }
 
 size_t binHistEntries(int n, int tiles)
 {
@@ -1087,15 +1128,24 @@ size_t binHistEntries(int n, int tiles)
     return binsByTile(tiles) ? std::max(depth, binChunkEntries(n) * size_t(std::max(tiles, 1))) : depth;
 }
 
-void binByTile(const TileBins &b, int *hist, int *tileTotals, int *chunkTotals, const ScanCapacity &cap, cudaStream_t s)
+template <class S, bool kCull>
+static void launchBins(const TileBins &b, int *hist, int *tileTotals, int *chunkTotals, const ScanCapacity &cap, cudaStream_t s)
 {
     const int G = rankChunks(b.n), stride = (b.tiles + 1) / 2 * 2;
-    const size_t scatterShared = size_t(stride) * (sizeof(int) + kRankWarps * sizeof(uint16_t)); // 36 bytes per tile
+    constexpr size_t perTile = sizeof(int) + S::WARPS * sizeof(uint16_t); // 36 or 12 bytes
     static PerDevice allowed;
-    allowShared(tileScatterKernel, scatterShared + 24 * 1024, size_t(kMaxTiles) * 36, allowed); // with the static arrays
-    { launchPdl(tileCountKernel, G, kRanks, b.tiles * sizeof(int), s, b, hist, chunkTotals); countLaunch(); }
+    allowShared(tileScatterKernel<S, kCull>, stride * perTile + 24 * 1024, size_t(kMaxTiles) * perTile, allowed); // with the static arrays
+    { launchPdl(tileCountKernel<S>, G, S::THREADS, b.tiles * sizeof(int), s, b, hist, chunkTotals); countLaunch(); }
     { launchPdl(tileScanKernel, (b.tiles + 31) / 32 + 1, kScanThreads, 0, s, hist, G, b.tiles, tileTotals, chunkTotals, cap); countLaunch(); }
-    { launchPdl(tileScatterKernel, G + (b.tileOrder ? 1 : 0), kRanks, scatterShared, s, b, hist, tileTotals, chunkTotals, cap.counts); countLaunch(); }
+    { launchPdl(tileScatterKernel<S, kCull>, G + (b.tileOrder ? 1 : 0), S::THREADS, stride * perTile, s, b, hist, tileTotals, chunkTotals, cap.counts); countLaunch(); }
+}
+
+void binByTile(const TileBins &b, int *hist, int *tileTotals, int *chunkTotals, const ScanCapacity &cap, cudaStream_t s)
+{
+    const bool few = b.n <= kFewGaussians, cull = b.cullRec != nullptr;
+    const auto launch = few ? (cull ? launchBins<FewRanks, true> : launchBins<FewRanks, false>)
+                            : (cull ? launchBins<ManyRanks, true> : launchBins<ManyRanks, false>);
+    launch(b, hist, tileTotals, chunkTotals, cap, s);
 }
 
 size_t scanPartialEntries(int n) { return size_t((n + kScanTile - 1) / kScanTile) + 1; }
