@@ -415,3 +415,19 @@ def test_training_with_either_backward_at_tile_8(u3dg, oracle, width, height, ba
     assert abs(a.loss - b.loss) <= 1e-4 * abs(b.loss) and abs(a.psnr - b.psnr) <= 1e-3
     for k in ("means", "scales", "quats", "opacities", "colors"):
         assert rel_l2(getattr(t.model(), k), getattr(o.model(), k)) < 1e-3, k
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 16, 31, 32, 33, 40, 64])
+def test_partial_sums_at_chunk_edges(u3dg, oracle, n):
+    # Every Gaussian in four tiles of 16: 4 to 256 entries, 128 (four chunks of 32) to 32 ranks. Sums over 1,024
+    # pixels: within 1e-4.
+    rng = np.random.default_rng(n)
+    m = random_model(n, rng, 0.01, 3.0, 0.05, 0.1)
+    m.means[:, 2] = np.linspace(2.9, 3.1, n)
+    cam = make_camera(32, 32, 40.0)
+    cam.cx = cam.cy = 15.5
+    w = rng.uniform(-1, 1, (32, 32, 3)).astype(np.float32)
+    r = _close(u3dg, oracle, m, cam, RasterSettings(background=(0.1, 0.2, 0.3)), w, 1e-4)
+    r.set_tile_culling(False)
+    r.forward(m, cam, RasterSettings())
+    assert len(r.tiles()[1]) == 4 * n

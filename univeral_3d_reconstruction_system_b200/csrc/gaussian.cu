@@ -387,42 +387,62 @@ __global__ void __launch_bounds__(256) partialSumKernel(ChainArgs a)
     const int first = __shfl_sync(0xffffffffu, o, 0), last = firstOf(min(w * 32 + 32, a.n));
     const float4 *partial = reinterpret_cast<const float4 *>(a.partial);
     float acc[kG2d] = {};
-    for (int c0 = first; c0 < last; c0 += 32) {
-        const int e = c0 + lane;
-        const int2 lp = e < last ? a.listPos[e] : make_int2(INT_MAX, 0);
-        // Owner of entry e: the last lane whose start offset is not above e.
-        int owner = 0;
+    // Four chunks of 32 entries at a time, so that the loads of a chunk (position, stop, partial: one after the
+    // other) overlap the others' (300 Gaussians over most of 1,900 tiles: a rasterizer's forward and backward
+    // 1.82 -> 1.50 ms).
+    constexpr int kChunks = 4;
+    for (int c4 = first; c4 < last; c4 += 32 * kChunks) {
+        int2 lp[kChunks];
+        float part[kChunks][kG2d] = {};
 #pragma unroll
-        for (int step = 16; step > 0; step >>= 1)
-            if (__shfl_sync(0xffffffffu, o, owner + step) <= e)
-                owner += step;
-        float v[kG2d] = {};
+        for (int u = 0; u < kChunks; ++u) {
+            const int e = c4 + 32 * u + lane;
+            lp[u] = e < last ? a.listPos[e] : make_int2(INT_MAX, 0);
+        }
         // Tiles covered by several CTAs: their slots, added in slot order.
         for (int sl = 0; sl < a.subSlots; ++sl) {
-            const int pos = partialAt(a, lp, sl);
-            if (pos >= 0)
-                addPartial(partial + size_t(sl) * (a.subStride / 4) + size_t(pos) * kPartialF4, v);
+            int pos[kChunks];
+#pragma unroll
+            for (int u = 0; u < kChunks; ++u)
+                pos[u] = partialAt(a, lp[u], sl);
+#pragma unroll
+            for (int u = 0; u < kChunks; ++u)
+                if (pos[u] >= 0)
+                    addPartial(partial + size_t(sl) * (a.subStride / 4) + size_t(pos[u]) * kPartialF4, part[u]);
         }
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int ownerUp = __shfl_up_sync(0xffffffffu, owner, d);
-            const bool same = lane >= d && ownerUp == owner;
+        for (int u = 0; u < kChunks; ++u) {
+            const int c0 = c4 + 32 * u, e = c0 + lane;
+            if (c0 >= last)
+                break;
+            // Owner of entry e: the last lane whose start offset is not above e.
+            int owner = 0;
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1)
+                if (__shfl_sync(0xffffffffu, o, owner + step) <= e)
+                    owner += step;
+            float (&v)[kG2d] = part[u];
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int ownerUp = __shfl_up_sync(0xffffffffu, owner, d);
+                const bool same = lane >= d && ownerUp == owner;
+#pragma unroll
+                for (int k = 0; k < kG2d; ++k) {
+                    const float up = __shfl_up_sync(0xffffffffu, v[k], d);
+                    if (same)
+                        v[k] += up;
+                }
+            }
+            // This lane's rank: its last entry inside the chunk, if any.
+            const int lastE = min(min(oEnd, last), c0 + 32) - 1;
+            const bool has = valid && o < c0 + 32 && oEnd > c0 && lastE >= max(o, c0);
+            const int src = has ? lastE - c0 : lane;
 #pragma unroll
             for (int k = 0; k < kG2d; ++k) {
-                const float up = __shfl_up_sync(0xffffffffu, v[k], d);
-                if (same)
-                    v[k] += up;
+                const float got = __shfl_sync(0xffffffffu, v[k], src);
+                if (has)
+                    acc[k] += got;
             }
-        }
-        // This lane's rank: its last entry inside the chunk, if any.
-        const int lastE = min(min(oEnd, last), c0 + 32) - 1;
-        const bool has = valid && o < c0 + 32 && oEnd > c0 && lastE >= max(o, c0);
-        const int src = has ? lastE - c0 : lane;
-#pragma unroll
-        for (int k = 0; k < kG2d; ++k) {
-            const float got = __shfl_sync(0xffffffffu, v[k], src);
-            if (has)
-                acc[k] += got;
         }
     }
     if (valid) {
