@@ -431,3 +431,27 @@ def test_partial_sums_at_chunk_edges(u3dg, oracle, n):
     r.set_tile_culling(False)
     r.forward(m, cam, RasterSettings())
     assert len(r.tiles()[1]) == 4 * n
+
+
+@pytest.mark.parametrize("tile", [8, 16, 64])
+@pytest.mark.parametrize("n, hidden", [(1, 32_768), (7, 32_768), (8, 32_768), (9, 32_768), (33, 32_768), (32_700, 69)])
+def test_few_and_many_gaussians_are_updated_alike(u3dg, n, hidden, tile):
+    # The chain rule takes 8 Gaussians to a warp up to 32,768 and 32 beyond: n Gaussians, and the same ones with so
+    # many more that no view sees. The same model, to the bit.
+    rng = np.random.default_rng(n)
+    m = random_model(n, rng, 1.0, 3.0, 0.03, 0.4 if n < 100 else 0.05)
+    far = random_model(1, rng, 1.0, 3.0, 0.05, 0.1)
+    far.means[:] = (0.0, 0.0, -9.0)
+    cam = make_camera(128, 96, 110.0)
+    photo = TrainImage(cam, rng.integers(0, 256, (96, 128, 3)).astype(np.uint8))
+    both = m.copy()
+    for k in ("means", "scales", "quats", "opacities", "colors"):
+        setattr(both, k, np.concatenate([getattr(m, k), np.repeat(getattr(far, k), hidden, axis=0)]))
+    out = []
+    for model in (m, both):
+        t = u3dg.Trainer(model, [photo], 1.0, TrainOptions(max_gaussians=model.size(), refine_stop=0, raster=RasterSettings(tile_size=tile)))
+        t.step(4)
+        out.append(t.model())
+    assert not np.array_equal(out[0].colors, m.colors)
+    for k in ("means", "scales", "quats", "opacities", "colors"):
+        np.testing.assert_array_equal(getattr(out[0], k), getattr(out[1], k)[:n], err_msg=k)

@@ -10,6 +10,7 @@
 
 #include <cfloat>
 #include <climits>
+#include <type_traits>
 
 namespace u3dg {
 
@@ -555,18 +556,22 @@ __device__ __forceinline__ void chainRule(const ChainArgs &a, const u3dg_camera 
 // Bound by the latency of its loads and by instructions (60 us on 300k Gaussians at 640x480, where its 190 MB
 // take 29 us): loads of a group of parameters stand ahead of the group's stores, quotients share their
 // divisors' reciprocals (68 us with the division operator, whose slow path every zero takes; 56 without a look
-// at the operands, which made quotients by a subnormal z^3 NaN). Small CTAs
-// spread few Gaussians over the chip (4k: 22 us at 256 threads, 21.5 at 64, the rest even). Registers are capped
-// at 64 for 32 warps per SM (28 warps: 63 us, 40: 80 us).
+// at the operands, which made quotients by a subnormal z^3 NaN). Registers are capped at 64 for 32 warps per SM (28
+// warps: 63 us, 40: 80 us). A warp takes kPerWarp Gaussians: 32, or 8 of few, whose partials then are gathered by
+// four times as many warps (the sums are the same): us by 32 / 8 of 4,000 Gaussians at 96x72 16.3 / 14.2, 5,000 at
+// 640x480 75.6 / 39.4, 12,000 at 320x240 24.1 / 19.6, 33,333 at 357x203 22.4 / 22.5, 60,000 at 640x480 34.7 / 38.2; in tiles
+// of 64, with 16 slots to an intersection, 100 over all of 400x304 301 / 95.
 constexpr int kChainThreads = 64, kChainWarps = 32;
+constexpr int kFewChains = 32768;
 
 // kConics: the partials are launchCompositeBackwardList's; without Adam (the rasterizer's) partialSumKernel has
 // added them in the order that its callers know.
-template <bool kAdam, bool kConics>
+template <bool kAdam, bool kConics, int kPerWarp>
 __global__ void __launch_bounds__(kChainThreads, kChainWarps * 32 / kChainThreads) chainKernel(ChainArgs a)
 {
     pdlEntry();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = int(blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int i = kPerWarp == 32 || lane < kPerWarp ? warp * kPerWarp + lane : INT_MAX;
     if (a.counts != nullptr && a.counts->abortIter >= 0)
         return;
     const u3dg_camera &cam = a.desc ? a.desc->cam : a.cam;
@@ -830,9 +835,16 @@ void launchChain(const ChainArgs &a, bool adam, cudaStream_t s)
         return;
     if (!adam && a.conics)
         { launchPdl(partialSumKernel, blocks((long long)(a.n + 31) / 32 * 32, 256), 256, 0, s, a); countLaunch(); }
-    const auto kernel = adam ? (a.conics ? chainKernel<true, true> : chainKernel<true, false>)
-                             : (a.conics ? chainKernel<false, true> : chainKernel<false, false>);
-    { launchPdl(kernel, blocks(a.n, kChainThreads), kChainThreads, 0, s, a); countLaunch(); }
+    auto launch = [&](auto perWarp) {
+        constexpr int P = decltype(perWarp)::value;
+        const auto kernel = adam ? (a.conics ? chainKernel<true, true, P> : chainKernel<true, false, P>)
+                                 : (a.conics ? chainKernel<false, true, P> : chainKernel<false, false, P>);
+        { launchPdl(kernel, blocks(blocks(a.n, P) * 32ll, kChainThreads), kChainThreads, 0, s, a); countLaunch(); }
+    };
+    if (a.n <= kFewChains)
+        launch(std::integral_constant<int, 8>{});
+    else
+        launch(std::integral_constant<int, 32>{});
 }
 
 void launchAdamSegment(float *p, const float *g, float *m, float *v, int len, float stepSize, float invSqrtBc2,
