@@ -69,12 +69,13 @@ int u3dg_batch_create(const u3dg_model *initial, const u3dg_image *const *images
             auto t = std::make_unique<u3dg_trainer>();
             t->impl = std::make_unique<TrainerImpl>(initial[s], images[s], image_counts[s], extents[s], o, false, compact);
             t->impl->ws.backwardDepth = rs.backwardDepth;
+            t->impl->ws.alone = scenes == 1;
             t->ownedByBatch = true;
             b->scenes.push_back(std::move(t));
         };
         auto add = [&](int s) {
             if (int(b->schedules.size()) == s)
-                b->schedules.push_back(autotune ? autotuneSchedule(initial[s], images[s], image_counts[s], extents[s], options[s])
+                b->schedules.push_back(autotune ? autotuneSchedule(initial[s], images[s], image_counts[s], extents[s], options[s], scenes == 1)
                                                 : RasterSchedule{options[s].raster.tile_size, 8, 1, 1, 0.0f});
             create(s);
         };

@@ -582,7 +582,8 @@ __global__ void __launch_bounds__(kDepthThreads) depthSortSmallKernel(const uint
 // would leave most of the chip idle. Sort and lists, us, by 512 / 64 / 32 ranks to a block (32 / 32 / 8 to a warp):
 // 5,000 Gaussians at 640x480 389 / 142 / 96, 5,000 at 400x304 in tiles of 8 652 / 208 / 126, without culling 380 /
 // 340 / 175, 1,000 at 200x150 81 / 50 / 40, 15,000 at 640x480 221 / 104 / 82, 4,000 at 96x72 36 / 34 / 32. Beyond,
-// blocks of 512 keep the counts that are scanned few (300k at 640x480: 586 rows of 1,200).
+// blocks of 512 keep the counts that are scanned few (300k at 640x480: 586 rows of 1,200); and where other work
+// fills the chip, their warps have no idle lanes (16 scenes at once 4,260 steps per second, 4,200 by 32).
 constexpr int kMaxTiles = 1 << kWideBits;
 template <int T, int R>
 struct RankShape {
@@ -592,10 +593,10 @@ using ManyRanks = RankShape<512, 32>;
 using FewRanks = RankShape<128, 8>;
 constexpr int kFewGaussians = 16384;
 
-inline int rankChunks(int n)
+template <class S>
+int rankChunks(int n)
 {
-    const int chunk = n <= kFewGaussians ? FewRanks::CHUNK : ManyRanks::CHUNK;
-    return std::max(1, (n + chunk - 1) / chunk);
+    return std::max(1, (n + S::CHUNK - 1) / S::CHUNK);
 }
 
 // The rank of a thread, n where it has none.
@@ -1120,7 +1121,7 @@ void radixSortDepth(const uint32_t *keys, uint2 *pairsA, uint2 *pairsB, uint32_t
 }
 
 // For up to n Gaussians (few of them can be cut into more chunks than many).
-size_t binChunkEntries(int n) { return size_t(std::max(rankChunks(n), rankChunks(std::min(n, kFewGaussians)))); }
+size_t binChunkEntries(int n) { return size_t(std::max(rankChunks<ManyRanks>(n), rankChunks<FewRanks>(std::min(n, kFewGaussians)))); }
 
 size_t binHistEntries(int n, int tiles)
 {
@@ -1131,7 +1132,7 @@ size_t binHistEntries(int n, int tiles)
 template <class S, bool kCull>
 static void launchBins(const TileBins &b, int *hist, int *tileTotals, int *chunkTotals, const ScanCapacity &cap, cudaStream_t s)
 {
-    const int G = rankChunks(b.n), stride = (b.tiles + 1) / 2 * 2;
+    const int G = rankChunks<S>(b.n), stride = (b.tiles + 1) / 2 * 2;
     constexpr size_t perTile = sizeof(int) + S::WARPS * sizeof(uint16_t); // 36 or 12 bytes
     static PerDevice allowed;
     allowShared(tileScatterKernel<S, kCull>, stride * perTile + 24 * 1024, size_t(kMaxTiles) * perTile, allowed); // with the static arrays
@@ -1142,7 +1143,7 @@ static void launchBins(const TileBins &b, int *hist, int *tileTotals, int *chunk
 
 void binByTile(const TileBins &b, int *hist, int *tileTotals, int *chunkTotals, const ScanCapacity &cap, cudaStream_t s)
 {
-    const bool few = b.n <= kFewGaussians, cull = b.cullRec != nullptr;
+    const bool few = b.alone && b.n <= kFewGaussians, cull = b.cullRec != nullptr;
     const auto launch = few ? (cull ? launchBins<FewRanks, true> : launchBins<FewRanks, false>)
                             : (cull ? launchBins<ManyRanks, true> : launchBins<ManyRanks, false>);
     launch(b, hist, tileTotals, chunkTotals, cap, s);

@@ -294,7 +294,7 @@ void RasterWorkspace::bin(cudaStream_t stream, int iteration, bool keep, const S
     int2 *const positions = keep ? listPos.p : nullptr;
     if (direct) {
         binByTile(TileBins{depthOrder.p, cnt.p, rect.p, n, tilesX, tiles, cullRec, st.tile_size, rowTab.p, tileOffsets.p,
-                           ordersTiles() ? tileOrder.p : nullptr, entries.p, positions, keep ? offsById.p : nullptr},
+                           ordersTiles() ? tileOrder.p : nullptr, entries.p, positions, keep ? offsById.p : nullptr, alone},
                   hist.p, rowTotals.p, chunkTotals.p, cap, stream);
         return;
     }
@@ -459,6 +459,7 @@ ChainArgs RasterWorkspace::chainArgs(const Params &P) const
     a.blocksX = tilesX * per;
     a.counts = counts.p;
     a.conics = !segmented;
+    a.alone = alone;
     a.order = depthOrder.p;
     a.sums = sums.p;
     return a;
@@ -1326,7 +1327,7 @@ void stepBatch(const std::vector<TrainerImpl *> &trainers, int count, BatchGraph
 }
 
 RasterSchedule autotuneSchedule(const u3dg_model &initial, const u3dg_image *imgs, int count, float extent,
-                                const u3dg_train_options &opt)
+                                const u3dg_train_options &opt, bool alone)
 {
     // Every candidate is deterministic: tile 32 spans four backward CTAs per tile, each with its own
     // partial slots, added in a fixed order by the chain rule.
@@ -1343,6 +1344,7 @@ RasterSchedule autotuneSchedule(const u3dg_model &initial, const u3dg_image *img
             o.raster.tile_size = tile;
             o.iterations = std::max(o.iterations, 64);
             TrainerImpl t(initial, imgs, count, extent, o);
+            t.ws.alone = alone;
             t.ws.backwardDepth = d + 1;
             t.stepTo(3 + TrainerImpl::kGraphSteps); // warm-up, including the first graph capture
             t.finish();

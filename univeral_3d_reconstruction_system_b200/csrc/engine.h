@@ -228,6 +228,9 @@ struct RasterWorkspace {
     // List entries each thread of the compositing backward stages per shared-memory batch (1 or 2; no
     // effect on a result).
     int backwardDepth = 1;
+    // Whether nothing else is on the GPU (TileBins::alone; false in batches of several scenes; no effect on a
+    // result).
+    bool alone = true;
     // Tile culling: list a Gaussian only in the tiles of its rectangle that its contributing ellipse
     // can reach (trainers; the rasterizer unit boundary keeps the reference's lists).
     bool cullTiles = false;
@@ -594,7 +597,7 @@ struct RasterSchedule {
     float msPerStep;
 };
 RasterSchedule autotuneSchedule(const u3dg_model &initial, const u3dg_image *imgs, int count, float extent,
-                                const u3dg_train_options &opt);
+                                const u3dg_train_options &opt, bool alone);
 
 } // namespace u3dg
 

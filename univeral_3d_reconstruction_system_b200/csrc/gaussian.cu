@@ -560,7 +560,8 @@ __device__ __forceinline__ void chainRule(const ChainArgs &a, const u3dg_camera 
 // warps: 63 us, 40: 80 us). A warp takes kPerWarp Gaussians: 32, or 8 of few, whose partials then are gathered by
 // four times as many warps (the sums are the same): us by 32 / 8 of 4,000 Gaussians at 96x72 16.3 / 14.2, 5,000 at
 // 640x480 75.6 / 39.4, 12,000 at 320x240 24.1 / 19.6, 33,333 at 357x203 22.4 / 22.5, 60,000 at 640x480 34.7 / 38.2; in tiles
-// of 64, with 16 slots to an intersection, 100 over all of 400x304 301 / 95.
+// of 64, with 16 slots to an intersection, 100 over all of 400x304 301 / 95. Not where other work fills the chip (16
+// scenes at once: 4,310 steps per second with 32, 4,250 with 8).
 constexpr int kChainThreads = 64, kChainWarps = 32;
 constexpr int kFewChains = 32768;
 
@@ -841,7 +842,7 @@ void launchChain(const ChainArgs &a, bool adam, cudaStream_t s)
                                  : (a.conics ? chainKernel<false, true, P> : chainKernel<false, false, P>);
         { launchPdl(kernel, blocks(blocks(a.n, P) * 32ll, kChainThreads), kChainThreads, 0, s, a); countLaunch(); }
     };
-    if (a.n <= kFewChains)
+    if (a.alone && a.n <= kFewChains)
         launch(std::integral_constant<int, 8>{});
     else
         launch(std::integral_constant<int, 32>{});

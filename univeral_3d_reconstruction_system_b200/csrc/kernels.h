@@ -114,6 +114,7 @@ struct ChainArgs {
     float *gradAccum;     // |dL/dmean2d| NDC statistic (may be null)
     int *gradCount;       // visibility count (may be null)
     bool conics;          // partials of launchCompositeBackwardList
+    bool alone;           // TileBins::alone
     // Non-Adam mode, conics: the Gaussians by depth rank, and space for 9 sums per Gaussian (partialSumKernel;
     // else the chain rule gathers the partials itself).
     const uint32_t *order;
@@ -174,6 +175,7 @@ struct TileBins {
     int *entries;     // per list position: Gaussian id
     int2 *listPos;    // per emission: list position, tile (may be null)
     int *offsById;    // per Gaussian: first emission (may be null)
+    bool alone;       // nothing else is on the GPU: few Gaussians may be spread over more threads than they fill
 };
 bool binsByTile(int tiles);
 // hist needs binHistEntries(n, tiles) entries, tileTotals radixDigits(), chunkTotals binChunkEntries(n).
