@@ -729,14 +729,13 @@ int u3dg_bin_tiles(const float *depth, const int *radius, const int *rect, size_
             cnt[i] = radius[i] > 0 ? (rc[i].z - rc[i].x) * (rc[i].w - rc[i].y) : 0;
         }
         ws.reserveIntersections(std::max<size_t>(size_t(1) << 16, 4 * nn));
+        if (n) {
+            U3DG_CUDA(cudaMemcpyAsync(ws.depthKey.p, keys.data(), n * 4, cudaMemcpyHostToDevice, st.s));
+            U3DG_CUDA(cudaMemcpyAsync(ws.rect.p, rc.data(), n * sizeof(int4), cudaMemcpyHostToDevice, st.s));
+            U3DG_CUDA(cudaMemcpyAsync(ws.radius.p, radius, n * sizeof(int), cudaMemcpyHostToDevice, st.s));
+            U3DG_CUDA(cudaMemcpyAsync(ws.cnt.p, cnt.data(), n * sizeof(int), cudaMemcpyHostToDevice, st.s));
+        }
         for (int attempt = 0;; ++attempt) {
-            // The depth sort overwrites its keys, so every attempt uploads them again.
-            if (n) {
-                U3DG_CUDA(cudaMemcpyAsync(ws.depthKey.p, keys.data(), n * 4, cudaMemcpyHostToDevice, st.s));
-                U3DG_CUDA(cudaMemcpyAsync(ws.rect.p, rc.data(), n * sizeof(int4), cudaMemcpyHostToDevice, st.s));
-                U3DG_CUDA(cudaMemcpyAsync(ws.radius.p, radius, n * sizeof(int), cudaMemcpyHostToDevice, st.s));
-                U3DG_CUDA(cudaMemcpyAsync(ws.cnt.p, cnt.data(), n * sizeof(int), cudaMemcpyHostToDevice, st.s));
-            }
             ws.clearCounts(st.s);
             ws.bin(st.s, 0, false);
             U3DG_CUDA(cudaGetLastError());
