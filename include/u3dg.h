@@ -423,9 +423,6 @@ int u3dg_render_sh(const u3dg_model *model, const float *sh_rest, int degree, co
  * rgb8, views back to back (sum of width*height*3 bytes). */
 int u3dg_render_views_sh(const u3dg_model *model, const float *sh_rest, int degree, const u3dg_camera *cameras,
                          int count, const u3dg_raster_settings *settings, uint8_t *rgb8);
-/* The same into a buffer per view (rgb8[v]: width*height*3 bytes). */
-int u3dg_render_views_sh_each(const u3dg_model *model, const float *sh_rest, int degree, const u3dg_camera *cameras,
-                               int count, const u3dg_raster_settings *settings, uint8_t *const *rgb8);
 
 /* ------------------------------------------------------------------ learned warm-start */
 

@@ -340,30 +340,6 @@ def test_an_overflowing_product_reaches_only_what_blends_there(u3dg, colour, wei
         np.testing.assert_array_equal(getattr(got, k)[apart], getattr(clean, k)[apart])
 
 
-def test_views_are_arrays_of_their_own(u3dg):
-    # Keeping one of many views keeps no other's bytes; and the call that writes them back to back agrees.
-    import ctypes as C
-
-    from univeral_3d_reconstruction_system_b200 import _abi, _lib
-
-    rng = np.random.default_rng(9)
-    m = random_model(300, rng, 1.0, 3.0, 0.02, 0.1)
-    cams = [make_camera(w, h, 60.0) for w, h in ((64, 48), (33, 71), (1, 1), (97, 33))]
-    views = u3dg.renderViewsSh(m, None, 0, cams)
-    for v, c in zip(views, cams):
-        assert v.shape == (c.height, c.width, 3) and v.flags.owndata and v.flags.writeable
-    flat = np.zeros(sum(v.size for v in views), np.uint8)
-    structs = (_abi.Camera * len(cams))(*(c.struct() for c in cams))
-    mv, st = m.view(), RasterSettings().struct()
-    _lib.check(_lib.load().u3dg_render_views_sh(C.byref(mv), None, 0, structs, len(cams), C.byref(st),
-                                                flat.ctypes.data_as(_abi.u8p)))
-    np.testing.assert_array_equal(flat, np.concatenate([v.reshape(-1) for v in views]))
-    assert u3dg.renderViewsSh(m, None, 0, []) == []
-    for bad in (-3, 0, 16385):
-        with pytest.raises(u3dg.U3dgError):
-            u3dg.renderViewsSh(m, None, 0, [cams[0], make_camera(bad, 5, 60.0)])
-
-
 @pytest.mark.parametrize("n, tiles_x, tiles_y, wide", [(31, 4, 4, 2), (32, 7, 5, 3), (33, 64, 32, 64), (257, 64, 32, 64), (16_384, 13, 9, 3),
                                                        (16_385, 13, 9, 3), (17_001, 32, 24, 9)])
 def test_tile_lists_of_few_and_many_gaussians(u3dg, n, tiles_x, tiles_y, wide):

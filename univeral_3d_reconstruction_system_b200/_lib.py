@@ -109,7 +109,6 @@ SIGNATURES = {
     "u3dg_read_splat_ply": (C.c_int, [C.c_char_p, _MV, C.c_size_t, _SZ, _I]),
     "u3dg_render_sh": (C.c_int, [_MV, _F, C.c_int, _CAM, _ST, _F]),
     "u3dg_render_views_sh": (C.c_int, [_MV, _F, C.c_int, _CAM, C.c_int, _ST, _abi.u8p]),
-    "u3dg_render_views_sh_each": (C.c_int, [_MV, _F, C.c_int, _CAM, C.c_int, _ST, C.POINTER(_abi.u8p)]),
     "u3dg_mlp_param_count": (C.c_int, []),
     "u3dg_mlp_create": (C.c_int, [_F, C.c_uint, _PP]),
     "u3dg_mlp_params": (C.c_int, [_P, _F]),

@@ -548,17 +548,23 @@ def renderViewsSh(model: GaussianModel, sh_rest: np.ndarray | None, degree: int,
                   settings: RasterSettings | None = None) -> list:
     """Quantised (uint8) SH renders of many views with the model uploaded once: training targets."""
     cams = (_abi.Camera * max(1, len(cameras)))()
-    views, pointers = [], (_abi.u8p * max(1, len(cameras)))()
+    sizes = []
     for k, c in enumerate(cameras):
         cams[k] = _cam(c)
-        views.append(np.empty((max(cams[k].height, 0), max(cams[k].width, 0), 3), np.uint8))
-        pointers[k] = views[k].ctypes.data_as(_abi.u8p)
+        sizes.append((cams[k].height, cams[k].width))
+    total = sum(h * w * 3 for h, w in sizes)
+    out = np.empty(max(total, 1), np.uint8)
     mv = model.view()
     ss = _settings(settings)
     shp = _abi.fptr(np.ascontiguousarray(sh_rest, np.float32).reshape(-1)) if (sh_rest is not None and degree > 0) \
         else None
-    check(load().u3dg_render_views_sh_each(C.byref(mv), shp, int(degree), cams, len(cameras), C.byref(ss), pointers))
-    return views
+    check(load().u3dg_render_views_sh(C.byref(mv), shp, int(degree), cams, len(cameras), C.byref(ss),
+                                      out.ctypes.data_as(_abi.u8p)))
+    res, o = [], 0
+    for h, w in sizes:
+        res.append(out[o:o + h * w * 3].reshape(h, w, 3))
+        o += h * w * 3
+    return res
 
 
 MLP_INPUTS, MLP_OUTPUTS, MLP_PARAMS = 134, 11, 51723

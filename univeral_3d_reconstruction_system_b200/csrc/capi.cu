@@ -1224,14 +1224,13 @@ int u3dg_render_sh(const u3dg_model *model, const float *sh_rest, int degree, co
     });
 }
 
-// The views back to back in rgb8 or, where each is set, in a buffer per view.
-static int renderViews(const u3dg_model *model, const float *sh_rest, int degree, const u3dg_camera *cameras, int count,
-                       const u3dg_raster_settings *settings, uint8_t *rgb8, uint8_t *const *each)
+int u3dg_render_views_sh(const u3dg_model *model, const float *sh_rest, int degree, const u3dg_camera *cameras,
+                         int count, const u3dg_raster_settings *settings, uint8_t *rgb8)
 {
     return guarded([&] {
         requireDevice();
         requireModel(model, "model");
-        if (count < 0 || (count > 0 && (!cameras || !(rgb8 || each))) || !settings)
+        if (count < 0 || (count > 0 && (!cameras || !rgb8)) || !settings)
             throw StatusError(U3DG_ERR_INVALID_ARG, "NULL argument");
         if (degree < 0 || degree > 3)
             throw StatusError(U3DG_ERR_INVALID_ARG, "SH degree must be 0..3");
@@ -1240,8 +1239,6 @@ static int renderViews(const u3dg_model *model, const float *sh_rest, int degree
         int tx = 0, ty = 0;
         for (int v = 0; v < count; ++v) {
             checkCamera(cameras[v]);
-            if (each && !each[v])
-                throw StatusError(U3DG_ERR_INVALID_ARG, "NULL argument");
             const int ts = settings->tile_size;
             pixels = std::max(pixels, size_t(cameras[v].width) * cameras[v].height);
             tx = std::max(tx, (cameras[v].width + ts - 1) / ts);
@@ -1312,23 +1309,11 @@ static int renderViews(const u3dg_model *model, const float *sh_rest, int degree
                 if (v + 1 < count)
                     render(v + 1);
             }
-            U3DG_CUDA(cudaMemcpyAsync(each ? each[v] : rgb8 + offset, q[v & 1].p, bytes(v), cudaMemcpyDeviceToHost, copies.s));
+            U3DG_CUDA(cudaMemcpyAsync(rgb8 + offset, q[v & 1].p, bytes(v), cudaMemcpyDeviceToHost, copies.s));
             copies.sync();
             offset += bytes(v);
         }
     });
-}
-
-int u3dg_render_views_sh(const u3dg_model *model, const float *sh_rest, int degree, const u3dg_camera *cameras,
-                          int count, const u3dg_raster_settings *settings, uint8_t *rgb8)
-{
-    return renderViews(model, sh_rest, degree, cameras, count, settings, rgb8, nullptr);
-}
-
-int u3dg_render_views_sh_each(const u3dg_model *model, const float *sh_rest, int degree, const u3dg_camera *cameras,
-                               int count, const u3dg_raster_settings *settings, uint8_t *const *rgb8)
-{
-    return renderViews(model, sh_rest, degree, cameras, count, settings, nullptr, rgb8);
 }
 
 } // extern "C"
