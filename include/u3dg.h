@@ -229,7 +229,8 @@ int u3dg_trainer_set_graphs(u3dg_trainer *trainer, int enable);
 int u3dg_trainer_graph_launches(u3dg_trainer *trainer, long long *launches);
 /* No reference counterpart. Compositing schedule: backward_depth is the list entries each thread of the
  * backward kernel stages per shared-memory batch, 1 (default) or 2 (deeper batches halve the block
- * barriers per Gaussian at the cost of shared memory; no effect at tile size 16). forward_block (8 or
+ * barriers per Gaussian at the cost of shared memory; no effect at tile size 16, nor at 8 in views of more than
+ * 1,500 tiles). forward_block (8 or
  * 16) and forward_depth (1 or 2) have no effect: the forward kernel picks its own from the image size.
  * The rendered images, gradients and trained models are bit-identical for every setting. */
 int u3dg_trainer_set_raster_schedule(u3dg_trainer *trainer, int forward_block, int forward_depth,

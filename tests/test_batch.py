@@ -71,7 +71,8 @@ def test_batch_matches_scenes_trained_alone(u3dg, autotune, tile):
 
 def test_autotuner_times_what_makes_a_difference(u3dg):
     # At tile 16 the backward's batch depth does nothing: one run is timed there, two at tiles 8 and 32, and a
-    # scene that takes tile 16 is given depth 1. Counted in kernel launches: 33 steps of the one run (13 of
+    # scene that takes tile 16 is given depth 1; nor does it at tile 8 in views of more than 1,500 tiles, whose lists
+    # are replayed whole (the last scene's 312x320). Counted in kernel launches: 33 steps of the one run (13 of
     # warm-up, 20 timed) and 43 of each of the others (10 profiled), within what recordings of graphs and odd
     # launches add.
     from univeral_3d_reconstruction_system_b200 import _lib
@@ -79,9 +80,13 @@ def test_autotuner_times_what_makes_a_difference(u3dg):
     def launches():
         return int(_lib.load().u3dg_launch_count())
 
-    for init, images, extent, options in _scenes(u3dg):
+    scenes = _scenes(u3dg)
+    init, images, extent, options = scenes[0]
+    large = [TrainImage(dataclasses.replace(im.camera, width=312, height=320), np.zeros((320, 312, 3), np.uint8)) for im in images[:3]]
+    scenes.append((init, large, extent, options))
+    for init, images, extent, options in scenes:
         expected = 0
-        for tile, runs in ((16, 1), (8, 2), (32, 2)):
+        for tile, runs in ((16, 1), (8, 1 if images[0].camera.width == 312 else 2), (32, 2)):
             o = dataclasses.replace(options, raster=dataclasses.replace(options.raster, tile_size=tile), iterations=64)
             t = u3dg.Trainer(init, images, extent, o)
             n0 = launches()
@@ -94,5 +99,5 @@ def test_autotuner_times_what_makes_a_difference(u3dg):
         counted = launches() - n0
         assert counted <= 1.08 * expected, (counted, expected)
         tile, schedule, _ = b.schedule(0)
-        assert tile != 16 or schedule[2] == 1
+        assert schedule[2] == 1 or tile == 32 or (tile == 8 and images[0].camera.width != 312)
         b.close()

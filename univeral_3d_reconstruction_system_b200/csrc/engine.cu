@@ -1338,7 +1338,7 @@ RasterSchedule autotuneSchedule(const u3dg_model &initial, const u3dg_image *img
         // two, at depth 1 and 2, each followed by profiled steps for the backward's own time; the tile's step
         // time is the first run's corrected by the gain.
         float stepMs[2] = {}, bwdMs[2] = {};
-        const int runs = backwardTakesDepth(tile) ? 2 : 1;
+        int runs = 2;
         for (int d = 0; d < runs; ++d) {
             u3dg_train_options o = opt;
             o.raster.tile_size = tile;
@@ -1360,6 +1360,8 @@ RasterSchedule autotuneSchedule(const u3dg_model &initial, const u3dg_image *img
             cudaEventDestroy(e0);
             cudaEventDestroy(e1);
             stepMs[d] /= float(2 * TrainerImpl::kGraphSteps);
+            if (!backwardTakesDepth(tile) || !t.ws.segmented)
+                runs = 1;
             if (runs == 1)
                 break;
             t.timer = new PhaseTimer();

@@ -256,7 +256,8 @@ void launchCompositeForward(const RasterArgs &a, float *rgb, float *finalT, int 
 void launchCompositeBackward(const RasterArgs &a, const float *dLdRgb, const float *finalT, const int *nContrib,
                              float *partial, const int *stop, const int2 *units, const int *unitCount,
                              cudaStream_t s);
-// Whether RasterArgs::backwardDepth makes a difference: at tiles of 16 a segment of 64 entries is one batch.
+// Whether RasterArgs::backwardDepth makes a difference to launchCompositeBackward: at tiles of 16 a segment of 64
+// entries is one batch.
 inline bool backwardTakesDepth(int tileSize) { return tileSize != 16; }
 // The same over whole lists: partials hold dL/dmean2d and dL/dconic, stop is written, and a forward with
 // segment 0 is enough.
